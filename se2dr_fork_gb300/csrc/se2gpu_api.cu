@@ -1,8 +1,7 @@
 // se2gpu_api.cu -- C-ABI of libse2gpu.so (see include/se2gpu.h).
 //
 // FP64 mode keeps the reference's state (u, v, a) in the reference's packed
-// [node][component] layout and runs the tiled reference-order kernel
-// (se2gpu_kernels.cuh).  FP32 modes keep the leapfrog state (u, w = half-step
+// [node][component] layout and runs the reference-order kernels (se2gpu_f64.cuh).  FP32 modes keep the leapfrog state (u, w = half-step
 // velocity, Kahan terms) in a padded layout (row pitch a multiple of 16 nodes,
 // as the TMA copies require) and run the persistent TMA-pipelined kernel
 // (se2gpu_persist.cuh); set/get_fields convert to and from the reference's
@@ -27,6 +26,7 @@
 #include <vector>
 
 #include "se2gpu.h"
+#include "se2gpu_f64_launch.h"
 #include "se2gpu_internal.h"
 #include "se2gpu_launch.h"
 #include "se2gpu_persist_launch.h"
@@ -56,6 +56,11 @@ static int fail(se2gpu_solver *h, int code, const char *fmt, ...)
   } while (0)
 
 static bool is_f64(const se2gpu_solver *h) { return h->precision == SE2GPU_FP64; }
+// FP64 u, v, a (f = 0, 1, 2) between blocks of steps
+static double *f64_field(const se2gpu_solver *h, int f)
+{
+  return reinterpret_cast<double *>(f < 2 ? h->f64[h->cur][f] : h->a64);
+}
 // FP32 modes that keep compensation terms of u and w (Kahan and two-float)
 static bool is_kahan(const se2gpu_solver *h) { return h->precision == SE2GPU_FP32_KAHAN || h->precision == SE2GPU_FP32_DF; }
 static bool is_df(const se2gpu_solver *h) { return h->precision == SE2GPU_FP32_DF; }
@@ -358,10 +363,11 @@ extern "C" void se2gpu_destroy(se2gpu_solver *h)
     if (ev) { cudaEventSynchronize(ev); cudaEventDestroy(ev); ev = nullptr; }
   if (h->stream) cudaStreamSynchronize(h->stream);
   for (int b = 0; b < 2; b++) {
-    for (int f = 0; f < 3; f++) dfree(h, h->f64[b][f]);
+    for (int f = 0; f < 2; f++) dfree(h, h->f64[b][f]);
+    dfree(h, h->ef[b]);
     dfree(h, h->pu[b]); dfree(h, h->pw[b]); dfree(h, h->pcu[b]); dfree(h, h->pcw[b]); dfree(h, h->rbuf[b]);
   }
-  void *ptrs[] = {h->pa, h->pminv, h->mass_bad, h->err_dev, h->mass, h->lam, h->mu, h->J00, h->J11, h->iJ00, h->iJ11, h->D, h->wq,
+  void *ptrs[] = {h->a64, h->rmass, h->Dx, h->Dy, h->f64_consts, h->src_xy, h->pa, h->pminv, h->mass_bad, h->err_dev, h->mass, h->lam, h->mu, h->J00, h->J11, h->iJ00, h->iJ11, h->D, h->wq,
                   h->src_vals, h->Dd, h->iJ00d, h->iJ11d, h->stf_dev, h->traces, h->norm_part, h->src_elem,
                   h->rec_node, h->rec_elem, h->rec_gll, h->scratch_u, h->scratch_f, h->tile_src_off,
                   h->tile_src_idx, h->tile_rec_off, h->tile_rec_idx, h->cellc, h->tile_bounds};
@@ -560,10 +566,6 @@ extern "C" int se2gpu_create(const se2gpu_problem *P, int precision, int trace_c
   h->precision = precision; h->nsrc = P->nsrc; h->nrec = P->nrec; h->trace_cap = trace_capacity;
   h->dt = P->dt;
   h->tsize = (precision == SE2GPU_FP64) ? 8 : 4;
-  const int te = se2::tile_edge(P->p);
-  h->ntx = (P->mx + te - 1) / te;
-  h->nty = (P->my + te - 1) / te;
-  h->nblocks = h->ntx * h->nty + 1;
   int rc;
 #define TRY(x) do { if ((rc = (x)) != 0) { snprintf(g_create_err, sizeof(g_create_err), "%s", h->err); se2gpu_destroy(h); return rc; } } while (0)
   if (cudaGetDevice(&h->device) != cudaSuccess) { cudaGetLastError(); free(h); return fail(nullptr, SE2GPU_ERR_CUDA, "no CUDA device"); }
@@ -578,8 +580,8 @@ extern "C" int se2gpu_create(const se2gpu_problem *P, int precision, int trace_c
     h->stream = h->own_stream;
   }
   {
-    // the tiled kernels serve FP64 and the FP32 internal-force entry point
-    cudaError_t e = (precision == SE2GPU_FP64) ? se2::prepare_f64(P->p) : se2::prepare_f32(P->p);
+    // (the tiled kernel of the FP32 internal-force entry point)
+    cudaError_t e = (precision == SE2GPU_FP64) ? cudaSuccess : se2::prepare_f32(P->p);
     if (e != cudaSuccess) { fail(h, SE2GPU_ERR_CUDA, "kernel set-up: %s", cudaGetErrorString(e)); TRY(SE2GPU_ERR_CUDA); }
   }
   TRY(upload(h, &h->lam, P->lambda, (size_t)ne));
@@ -605,8 +607,31 @@ extern "C" int se2gpu_create(const se2gpu_problem *P, int precision, int trace_c
   if (precision == SE2GPU_FP64) {
     const size_t vbytes = (size_t)nnodes * 2 * 8;
     for (int b = 0; b < 2; b++)
-      for (int f = 0; f < 3; f++) TRY(dzero(h, &h->f64[b][f], vbytes));
+      for (int f = 0; f < 2; f++) TRY(dzero(h, (void **)&h->f64[b][f], vbytes));
+    TRY(dzero(h, (void **)&h->a64, vbytes));
+    // element forces of a step, written before they are read
+    for (int b = 0; b < 2; b++) TRY(dalloc(h, (void **)&h->ef[b], (size_t)ne * npe * 16));
     TRY(upload(h, &h->mass, P->mass, (size_t)nnodes));   // the reference divides by M
+    TRY(dalloc(h, (void **)&h->rmass, (size_t)nnodes * 8));
+    if (se2::f64_launch_reciprocal((const double *)h->mass, h->rmass, (size_t)nnodes, h->nsm, h->stream) != cudaSuccess) {
+      cudaGetLastError();
+      fail(h, SE2GPU_ERR_CUDA, "1/M");
+      TRY(SE2GPU_ERR_CUDA);
+    }
+    // the reference's scaled derivatives dN/dx = (1/J00) dN/dxi per element column, dN/dy per row
+    std::vector<double> dx((size_t)P->mx * npe), dy((size_t)P->my * npe);
+    for (size_t i = 0; i < dx.size(); i++) dx[i] = P->iJ00[i / npe] * P->D[i % npe];
+    for (size_t i = 0; i < dy.size(); i++) dy[i] = P->iJ11[i / npe] * P->D[i % npe];
+    TRY(upload_d(h, &h->Dx, dx.data(), dx.size()));
+    TRY(upload_d(h, &h->Dy, dy.data(), dy.size()));
+    const double consts[2] = {1.0, -0.0};
+    TRY(upload_d(h, &h->f64_consts, consts, 2));
+    std::vector<int> sxy;
+    for (int s = 0; s < P->nsrc; s++) {
+      sxy.push_back(P->src_elem[s] % P->mx * P->p);
+      sxy.push_back(P->src_elem[s] / P->mx * P->p);
+    }
+    TRY(upload_i(h, (int **)&h->src_xy, sxy.data(), sxy.size()));
   } else {
     const bool kahan = is_kahan(h), df = is_df(h);
     h->pitch = (int)((nx_g + 1 + 15) / 16 * 16);   // >= 1 padding node: paired reads stay in the row
@@ -775,28 +800,23 @@ extern "C" int se2gpu_selftest_wait_expiry(se2gpu_solver *h, double *seconds)
 }
 
 // ---------------------------------------------------------------- FP64 (tiled, reference order)
-static se2::StepParams<double> f64_params(se2gpu_solver *h)
+static se2::F64Params f64_params(const se2gpu_solver *h)
 {
-  se2::StepParams<double> prm;
-  memset(&prm, 0, sizeof(prm));
-  prm.mx = h->mx; prm.my = h->my; prm.nx_g = h->nx_g; prm.ny_g = h->ny_g;
-  prm.ntx = h->ntx; prm.nty = h->nty;
-  prm.mass = (const double *)h->mass; prm.lam = (const double *)h->lam; prm.mu = (const double *)h->mu;
-  prm.J00 = (const double *)h->J00; prm.J11 = (const double *)h->J11;
-  prm.iJ00 = (const double *)h->iJ00; prm.iJ11 = (const double *)h->iJ11;
-  prm.D = (const double *)h->D; prm.wq = (const double *)h->wq;
+  se2::F64Params q;
+  memset(&q, 0, sizeof(q));
+  q.mx = h->mx; q.my = h->my; q.nx_g = h->nx_g; q.ny_g = h->ny_g;
+  q.mass = (const double *)h->mass; q.rmass = h->rmass;
+  q.lam = (const double *)h->lam; q.mu = (const double *)h->mu;
+  q.J00 = (const double *)h->J00; q.J11 = (const double *)h->J11;
+  q.Dx = h->Dx; q.Dy = h->Dy; q.wq = (const double *)h->wq;
+  q.constants = h->f64_consts;
   // coefficients exactly as the reference forms them: dt, 0.5*dt*dt, 0.5*dt
-  prm.c_dt = h->dt; prm.c_u = 0.5 * h->dt * h->dt; prm.c_v = 0.5 * h->dt;
-  prm.nsrc = h->nsrc; prm.src_elem = h->src_elem; prm.src_vals = (const double *)h->src_vals;
-  prm.nrec = h->nrec; prm.rec_node = h->rec_node; prm.rec_elem = h->rec_elem; prm.rec_gll = h->rec_gll;
-  prm.Dd = h->Dd; prm.iJ00d = h->iJ00d; prm.iJ11d = h->iJ11d;
-  return prm;
-}
-
-static void f64_bind(se2gpu_solver *h, se2::StepParams<double> &prm, int in, int outb)
-{
-  prm.u_in = (const double2 *)h->f64[in][0]; prm.v_in = (const double2 *)h->f64[in][1]; prm.a_in = (const double2 *)h->f64[in][2];
-  prm.u_out = (double2 *)h->f64[outb][0]; prm.v_out = (double2 *)h->f64[outb][1]; prm.a_out = (double2 *)h->f64[outb][2];
+  q.c_dt = h->dt; q.c_u = 0.5 * h->dt * h->dt; q.c_v = 0.5 * h->dt;
+  q.nsrc = h->nsrc; q.src_xy = h->src_xy; q.src_vals = (const double *)h->src_vals;
+  q.rec_elem = h->rec_elem; q.rec_gll = h->rec_gll;
+  q.Dd = h->Dd; q.iJ00d = h->iJ00d; q.iJ11d = h->iJ11d;
+  q.a_in = h->a64;
+  return q;
 }
 
 // ---------------------------------------------------------------- FP32 (persistent leapfrog)
@@ -832,11 +852,12 @@ static int flush_record(se2gpu_solver *h)
   h->launches++;
   double *row = h->traces + (size_t)h->rows_written * 7 * h->nrec;
   if (is_f64(h)) {
-    auto prm = f64_params(h);
-    f64_bind(h, prm, h->cur, h->cur);
-    prm.record = 1;
-    prm.trace_row = row;
-    e = se2::launch_record_f64(h->p, prm, h->stream);
+    auto q = f64_params(h);
+    q.mode = se2::F64_START;
+    q.u_in = h->f64[h->cur][0]; q.v_in = h->f64[h->cur][1];
+    q.nrec = h->nrec;
+    q.trace_row = row;
+    e = se2::f64_launch_record(h->p, q, h->stream);
   } else {
     auto prm = f32_params(h);
     prm.rbuf_in = h->rbuf[h->rlast];
@@ -850,22 +871,32 @@ static int flush_record(se2gpu_solver *h)
   return 0;
 }
 
+// n steps: START from (u, v, a), n - 1 MIDDLE launches that finish a step and begin the
+// next, and the last step's v and a.  A launch records the receivers of the step before
+// it; the last step's row stays pending.
 static int advance_f64(se2gpu_solver *h, int nsteps)
 {
-  auto prm = f64_params(h);
-  prm.mode = 0;
+  auto q = f64_params(h);
   for (int k = 0; k < nsteps; k++) {
-    f64_bind(h, prm, h->cur, 1 - h->cur);
-    prm.stf = h->stf_dev + (size_t)k * h->nsrc;
-    prm.record = h->pending_record ? 1 : 0;
-    prm.trace_row = h->traces + (size_t)h->rows_written * 7 * h->nrec;
+    const int in = h->cur, outb = 1 - h->cur;
+    q.mode = k ? se2::F64_MIDDLE : se2::F64_START;
+    q.u_in = h->f64[in][0]; q.v_in = h->f64[in][1]; q.ef_in = h->ef[in];
+    q.u_out = h->f64[outb][0]; q.v_out = h->f64[outb][1]; q.ef_out = h->ef[outb];
+    q.stf = k ? h->stf_dev + (size_t)(k - 1) * h->nsrc : nullptr;
+    q.nrec = h->pending_record ? h->nrec : 0;
+    q.trace_row = h->traces + (size_t)h->rows_written * 7 * h->nrec;
     h->launches++;
-    cudaError_t e = se2::launch_step_f64(h->p, prm, h->nblocks, h->stream);
+    cudaError_t e = se2::f64_launch_step(h->p, q, h->nsm, h->stream);
     if (e != cudaSuccess) return fail(h, SE2GPU_ERR_CUDA, "step kernel: %s", cudaGetErrorString(e));
     if (h->pending_record) { h->rows_written++; h->pending_record = false; }
-    h->cur = 1 - h->cur;
+    h->cur = outb;
     if (h->nrec > 0) h->pending_record = true;
   }
+  q.ef_in = h->ef[h->cur];
+  q.stf = h->stf_dev + (size_t)(nsteps - 1) * h->nsrc;
+  h->launches++;
+  cudaError_t e = se2::f64_launch_last(h->p, q, h->f64[h->cur][1], h->a64, h->stream);
+  if (e != cudaSuccess) return fail(h, SE2GPU_ERR_CUDA, "step kernel: %s", cudaGetErrorString(e));
   return 0;
 }
 
@@ -949,7 +980,7 @@ extern "C" int se2gpu_set_fields(se2gpu_solver *h, const double *u, const double
   if (is_f64(h)) {
     const double *src[3] = {u, v, a};
     for (int f = 0; f < 3; f++)
-      if (src[f] && (rc = copy_f64(h, (double *)h->f64[h->cur][f], src[f], n, cudaMemcpyHostToDevice))) return rc;
+      if (src[f] && (rc = copy_f64(h, f64_field(h, f), src[f], n, cudaMemcpyHostToDevice))) return rc;
     return 0;
   }
   // FP32: unspecified fields keep their current values
@@ -972,7 +1003,7 @@ extern "C" int se2gpu_get_fields(se2gpu_solver *h, double *u, double *v, double 
   if (is_f64(h)) {
     double *dst[3] = {u, v, a};
     for (int f = 0; f < 3; f++)
-      if (dst[f] && (rc = copy_f64(h, dst[f], (const double *)h->f64[h->cur][f], n, cudaMemcpyDeviceToHost))) return rc;
+      if (dst[f] && (rc = copy_f64(h, dst[f], f64_field(h, f), n, cudaMemcpyDeviceToHost))) return rc;
     return 0;
   }
   if (h->pageable) {
@@ -1021,7 +1052,7 @@ extern "C" int se2gpu_norms(se2gpu_solver *h, double out[6])
   const int nb = 1024;
   h->launches++;
   if (is_f64(h)) {
-    se2::norms_partial<double><<<nb, 256, 0, h->stream>>>((const double *)h->f64[h->cur][0], (const double *)h->f64[h->cur][1],
+    se2::norms_partial<<<nb, 256, 0, h->stream>>>(f64_field(h, 0), f64_field(h, 1),
                                                           h->nnodes * 2, h->norm_part);
     CK(h, cudaGetLastError());
   } else {
@@ -1047,22 +1078,31 @@ extern "C" int se2gpu_norms(se2gpu_solver *h, double out[6])
 }
 
 // ---------------------------------------------------------------- internal force (packed layout)
-template <typename T>
-static int force_t(se2gpu_solver *h, const void *u_dev, void *F_dev)
+static int force_f64(se2gpu_solver *h, const void *u_dev, void *F_dev)
 {
-  typedef typename se2::Vec2<T>::type T2;
-  se2::StepParams<T> prm;
+  auto q = f64_params(h);
+  q.mode = se2::F64_FORCE;
+  q.u_in = (const double2 *)u_dev;
+  q.ef_out = h->ef[0];
+  q.ef_in = h->ef[0];
+  h->launches += 2;
+  cudaError_t e = se2::f64_launch_step(h->p, q, h->nsm, h->stream);
+  if (e == cudaSuccess) e = se2::f64_launch_force(h->p, q, (double2 *)F_dev, h->stream);
+  if (e != cudaSuccess) return fail(h, SE2GPU_ERR_CUDA, "force kernel: %s", cudaGetErrorString(e));
+  return 0;
+}
+
+static int force_f32(se2gpu_solver *h, const void *u_dev, void *F_dev)
+{
+  se2::ForceParams prm;
   memset(&prm, 0, sizeof(prm));
-  prm.mx = h->mx; prm.my = h->my; prm.nx_g = h->nx_g; prm.ny_g = h->ny_g; prm.ntx = h->ntx; prm.nty = h->nty;
-  prm.lam = (const T *)h->lam; prm.mu = (const T *)h->mu; prm.J00 = (const T *)h->J00; prm.J11 = (const T *)h->J11;
-  prm.iJ00 = (const T *)h->iJ00; prm.iJ11 = (const T *)h->iJ11; prm.D = (const T *)h->D; prm.wq = (const T *)h->wq;
-  prm.mode = 1;
-  prm.u_in = (const T2 *)u_dev;
-  prm.f_out = (T2 *)F_dev;
+  prm.mx = h->mx; prm.my = h->my; prm.nx_g = h->nx_g; prm.ny_g = h->ny_g;
+  prm.lam = (const float *)h->lam; prm.mu = (const float *)h->mu; prm.J00 = (const float *)h->J00; prm.J11 = (const float *)h->J11;
+  prm.iJ00 = (const float *)h->iJ00; prm.iJ11 = (const float *)h->iJ11; prm.D = (const float *)h->D; prm.wq = (const float *)h->wq;
+  prm.u_in = (const float2 *)u_dev;
+  prm.f_out = (float2 *)F_dev;
   h->launches++;
-  cudaError_t e;
-  if constexpr (sizeof(T) == 8) e = se2::launch_step_f64(h->p, prm, h->nblocks - 1, h->stream);
-  else e = se2::launch_step_f32(h->p, prm, h->nblocks - 1, h->stream);
+  cudaError_t e = se2::launch_force_f32(h->p, prm, h->stream);
   if (e != cudaSuccess) return fail(h, SE2GPU_ERR_CUDA, "force kernel: %s", cudaGetErrorString(e));
   return 0;
 }
@@ -1071,7 +1111,7 @@ extern "C" int se2gpu_assemble_linear_form_device(se2gpu_solver *h, const void *
 {
   if (!h || !u_dev || !F_dev) return SE2GPU_ERR_ARG;
   CK(h, cudaSetDevice(h->device));
-  return (h->tsize == 8) ? force_t<double>(h, u_dev, F_dev) : force_t<float>(h, u_dev, F_dev);
+  return (h->tsize == 8) ? force_f64(h, u_dev, F_dev) : force_f32(h, u_dev, F_dev);
 }
 
 extern "C" int se2gpu_assemble_linear_form(se2gpu_solver *h, const double *u, double *F)
@@ -1115,9 +1155,9 @@ extern "C" int se2gpu_device_fields(const se2gpu_solver *h, void **u, void **v, 
 {
   if (!h) return SE2GPU_ERR_ARG;
   if (is_f64(h)) {
-    if (u) *u = h->f64[h->cur][0];
-    if (v) *v = h->f64[h->cur][1];
-    if (a) *a = h->f64[h->cur][2];
+    if (u) *u = f64_field(h, 0);
+    if (v) *v = f64_field(h, 1);
+    if (a) *a = f64_field(h, 2);
   } else {
     if (u) *u = h->pu[h->cur];
     if (v) *v = h->pw[h->cur];
@@ -1130,7 +1170,7 @@ extern "C" int se2gpu_tile_configs(const se2gpu_solver *h, int *edge, int *threa
 {
   if (!h) return SE2GPU_ERR_ARG;
   if (is_f64(h)) {
-    if (max_configs > 0 && edge && threads) { edge[0] = se2::tile_edge(h->p); threads[0] = 256; }
+    if (max_configs > 0 && edge && threads) { edge[0] = se2::f64_tile_edge(h->p); threads[0] = 256; }
     return 1;
   }
   const int n = se2p::num_configs(h->p);
@@ -1148,7 +1188,7 @@ extern "C" int se2gpu_tile_config_info(const se2gpu_solver *h, int config, int i
   if (!h || !info) return SE2GPU_ERR_ARG;
   if (is_f64(h)) {
     if (config != 0) return SE2GPU_ERR_ARG;
-    info[0] = se2::tile_edge(h->p); info[1] = 256; info[2] = 0; info[3] = 0;
+    info[0] = se2::f64_tile_edge(h->p); info[1] = 256; info[2] = 0; info[3] = 0;
     return 0;
   }
   se2p::TileShape ts;
@@ -1194,7 +1234,7 @@ std::vector<std::pair<void *, size_t>> state_arrays(se2gpu_solver *h)
   std::vector<std::pair<void *, size_t>> v;
   if (is_f64(h)) {
     const size_t b = (size_t)h->nnodes * 2 * 8;
-    for (int f = 0; f < 3; f++) v.push_back({h->f64[h->cur][f], b});
+    for (int f = 0; f < 3; f++) v.push_back({f64_field(h, f), b});
   } else {
     const size_t b = (size_t)h->ny_g * h->pitch * 8;
     v.push_back({h->pu[h->cur], b});

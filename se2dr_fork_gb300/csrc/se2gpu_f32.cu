@@ -9,14 +9,16 @@ namespace se2 {
 template <int P>
 static cudaError_t prep()
 {
-  return cudaFuncSetAttribute(step_kernel<P, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)smem_layout<P, float, false>().total);
+  return cudaFuncSetAttribute(force_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_layout<P>().total);
 }
 
 template <int P>
-static cudaError_t launch(const StepParams<float> &prm, int nblocks, cudaStream_t st)
+static cudaError_t launch(const ForceParams &prm, cudaStream_t st)
 {
-  step_kernel<P, float, false><<<nblocks, 256, smem_layout<P, float, false>().total, st>>>(prm);
+  ForceParams q = prm;
+  q.ntx = (q.mx + Tile<P>::TE - 1) / Tile<P>::TE;
+  q.nty = (q.my + Tile<P>::TE - 1) / Tile<P>::TE;
+  force_kernel<P><<<q.ntx * q.nty, 256, smem_layout<P>().total, st>>>(q);
   return cudaGetLastError();
 }
 
@@ -30,9 +32,9 @@ static cudaError_t launch(const StepParams<float> &prm, int nblocks, cudaStream_
   }
 
 cudaError_t prepare_f32(int p) { SE2_DISPATCH(prep) return cudaErrorInvalidValue; }
-cudaError_t launch_step_f32(int p, const StepParams<float> &prm, int nblocks, cudaStream_t st)
+cudaError_t launch_force_f32(int p, const ForceParams &prm, cudaStream_t st)
 {
-  SE2_DISPATCH(launch, prm, nblocks, st)
+  SE2_DISPATCH(launch, prm, st)
   return cudaErrorInvalidValue;
 }
 

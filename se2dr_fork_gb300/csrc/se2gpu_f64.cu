@@ -1,37 +1,10 @@
-// se2gpu_f64.cu -- FP64 (reference operation order) instantiations, degrees 1..8.
-#include "se2gpu_launch.h"
+// se2gpu_f64.cu -- FP64 (reference operation order) kernels, degrees 1..8, and their launches.
+#include <algorithm>
+
+#include "se2gpu_f64_launch.h"
+#include "se2gpu_f64.cuh"
 
 namespace se2 {
-
-int tile_edge(int p)
-{
-  switch (p) {
-    case 1: return Tile<1>::TE; case 2: return Tile<2>::TE; case 3: return Tile<3>::TE; case 4: return Tile<4>::TE;
-    case 5: return Tile<5>::TE; case 6: return Tile<6>::TE; case 7: return Tile<7>::TE; case 8: return Tile<8>::TE;
-    default: return 0;
-  }
-}
-
-template <int P>
-static cudaError_t prep()
-{
-  return cudaFuncSetAttribute(step_kernel<P, double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)smem_layout<P, double, false>().total);
-}
-
-template <int P>
-static cudaError_t launch(const StepParams<double> &prm, int nblocks, cudaStream_t st)
-{
-  step_kernel<P, double, false><<<nblocks, 256, smem_layout<P, double, false>().total, st>>>(prm);
-  return cudaGetLastError();
-}
-
-template <int P>
-static cudaError_t record(const StepParams<double> &prm, cudaStream_t st)
-{
-  record_kernel<P, double><<<1, 128, 0, st>>>(prm);
-  return cudaGetLastError();
-}
 
 #define SE2_DISPATCH(fn, ...)                                               \
   switch (p) {                                                              \
@@ -39,22 +12,109 @@ static cudaError_t record(const StepParams<double> &prm, cudaStream_t st)
     case 3: return fn<3>(__VA_ARGS__); case 4: return fn<4>(__VA_ARGS__);   \
     case 5: return fn<5>(__VA_ARGS__); case 6: return fn<6>(__VA_ARGS__);   \
     case 7: return fn<7>(__VA_ARGS__); case 8: return fn<8>(__VA_ARGS__);   \
-    default: return cudaErrorInvalidValue;                                  \
+    default: return {};                                                     \
   }
 
-cudaError_t prepare_f64(int p) { SE2_DISPATCH(prep) }
-cudaError_t launch_step_f64(int p, const StepParams<double> &prm, int nblocks, cudaStream_t st) { SE2_DISPATCH(launch, prm, nblocks, st) }
-cudaError_t launch_record_f64(int p, const StepParams<double> &prm, cudaStream_t st) { SE2_DISPATCH(record, prm, st) }
+template <int P>
+static int edge() { return F64Tile<P, 2>::TX; }
+int f64_tile_edge(int p) { SE2_DISPATCH(edge) }
 
-size_t smem_f64(int p)
+template <class A> struct arg { typedef A type; };   // (keeps A out of the deduction)
+// launch, beginning while the launch before it in the stream drains
+template <class... A>
+static cudaError_t launch_dependent(void (*fn)(A...), dim3 grid, int threads, cudaStream_t st, typename arg<A>::type... args)
 {
-  switch (p) {
-    case 1: return smem_layout<1, double, false>().total; case 2: return smem_layout<2, double, false>().total;
-    case 3: return smem_layout<3, double, false>().total; case 4: return smem_layout<4, double, false>().total;
-    case 5: return smem_layout<5, double, false>().total; case 6: return smem_layout<6, double, false>().total;
-    case 7: return smem_layout<7, double, false>().total; case 8: return smem_layout<8, double, false>().total;
-    default: return 0;
-  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, fn, args...);
+}
+
+template <int P, int SIZE>
+static long tiles(const F64Params &q)
+{
+  typedef F64Tile<P, SIZE> T;
+  return (long)((q.mx + T::TX - 1) / T::TX) * ((q.my + T::TY - 1) / T::TY);
+}
+
+// FP64 warp instructions of the busiest SM: a tile's element points (20 (p+1) each, strain
+// and divergence) and its nodes (about 40 each), in whole warps
+template <int P, int SIZE>
+static long cost(const F64Params &q, int nsm)
+{
+  typedef F64Tile<P, SIZE> T;
+  const long points = (T::TX * T::TY * (P + 1) * (P + 1) + 31) / 32;
+  const long nodes = ((T::TX * P + 1) * (T::TY * P + 1) + 31) / 32;
+  return ((tiles<P, SIZE>(q) + nsm - 1) / nsm) * (points * 20 * (P + 1) + nodes * 40);
+}
+
+template <int P, int SIZE>
+static cudaError_t step_t(F64Params &q, int nsm, cudaStream_t st)
+{
+  typedef F64Tile<P, SIZE> T;
+  q.ntx = (q.mx + T::TX - 1) / T::TX;
+  q.ntiles = (int)tiles<P, SIZE>(q);
+  const int per = T::NT / 32;   // receivers per sampling CTA and pass
+  q.nsamp = std::min((q.nrec + per - 1) / per, 256);
+  // A launch made while the one before it drains starts about 2 us sooner (100-step blocks:
+  // 9.9 -> 7.3 us per step at 300 nodes, 27.6 -> 25.8 at 60000).  Letting it begin before
+  // that one's last CTAs have ended gains another 0.5-1 us where every SM has at most one
+  // tile; with more, the early CTAs fill the SMs that are idle at that moment and
+  // unbalance the rest (13.5 -> 24 us at degree 4, 35 x 35 elements).
+  q.trigger = q.ntiles <= nsm;
+  if (q.mode == F64_MIDDLE) return launch_dependent(f64_step<P, SIZE>, dim3(q.ntiles + q.nsamp), T::NT, st, q);
+  f64_step<P, SIZE><<<q.ntiles + q.nsamp, T::NT, 0, st>>>(q);
+  return cudaGetLastError();
+}
+
+// The tile size with the least work on the busiest SM.  Over all degrees and 300 to 400000
+// nodes this is within 1 % (mean) and 11 % (worst) of the best of the three as timed; taking
+// always one size costs up to 3.5x (degree 6, 9 x 9 elements: 11.8, 16.1 or 38.1 us).
+template <int P>
+static cudaError_t step(const F64Params &prm, int nsm, cudaStream_t st)
+{
+  F64Params q = prm;
+  const long c0 = cost<P, 0>(q, nsm), c1 = cost<P, 1>(q, nsm), c2 = cost<P, 2>(q, nsm);
+  if (c0 < c1 && c0 < c2) return step_t<P, 0>(q, nsm, st);
+  return (c1 < c2) ? step_t<P, 1>(q, nsm, st) : step_t<P, 2>(q, nsm, st);
+}
+
+static dim3 node_grid(const F64Params &q) { return dim3((q.nx_g + 255) / 256, std::min(q.ny_g, 65535)); }
+
+template <int P>
+static cudaError_t last(const F64Params &q, double2 *v, double2 *a, cudaStream_t st)
+{
+  return launch_dependent(f64_last<P>, node_grid(q), 256, st, q, v, a);
+}
+
+template <int P>
+static cudaError_t force(const F64Params &q, double2 *f, cudaStream_t st)
+{
+  return launch_dependent(f64_force<P>, node_grid(q), 256, st, q, f);
+}
+
+template <int P>
+static cudaError_t record(const F64Params &q, cudaStream_t st)
+{
+  f64_record<P><<<std::min((q.nrec + 3) / 4, 256), 128, 0, st>>>(q);
+  return cudaGetLastError();
+}
+
+cudaError_t f64_launch_step(int p, const F64Params &q, int nsm, cudaStream_t st) { SE2_DISPATCH(step, q, nsm, st) }
+cudaError_t f64_launch_last(int p, const F64Params &q, double2 *v, double2 *a, cudaStream_t st) { SE2_DISPATCH(last, q, v, a, st) }
+cudaError_t f64_launch_force(int p, const F64Params &q, double2 *f, cudaStream_t st) { SE2_DISPATCH(force, q, f, st) }
+cudaError_t f64_launch_record(int p, const F64Params &q, cudaStream_t st) { SE2_DISPATCH(record, q, st) }
+
+cudaError_t f64_launch_reciprocal(const double *mass, double *r, size_t n, int nsm, cudaStream_t st)
+{
+  f64_reciprocal<<<8 * nsm, 256, 0, st>>>(mass, r, n);
+  return cudaGetLastError();
 }
 
 }  // namespace se2

@@ -20,8 +20,11 @@ struct se2gpu_solver {
   int device, nsm;
   cudaStream_t stream, own_stream;
   size_t tsize;                  // compute precision (4 or 8 bytes)
-  // FP64 state: two buffer sets of packed u, v, a
-  void *f64[2][3];
+  // FP64 state: two buffer sets of packed u, v; a of the last step; element forces of a step
+  // (written with the buffer set of the same index); 1/M; scaled derivative tables
+  double2 *f64[2][2], *a64, *ef[2];
+  double *rmass, *Dx, *Dy, *f64_consts;
+  int2 *src_xy;                  // first node of each source's element
   int cur;
   // FP32 leapfrog state (padded): u, w, cu, cw per buffer set, a of the last step
   int pitch;
@@ -44,7 +47,6 @@ struct se2gpu_solver {
   int *src_elem, *rec_node, *rec_elem, *rec_gll;
   void *scratch_u, *scratch_f;   // assemble_linear_form staging (packed)
   long launches;
-  int ntx, nty, nblocks;         // FP64 tiles
   char err[512];
 };
 
