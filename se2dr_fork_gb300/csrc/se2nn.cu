@@ -19,6 +19,7 @@
 
 #include "se2nn.h"
 #include "se2nn_gemm.cuh"
+#include "se2nn_rows.cuh"
 #include "se2nn_tc.cuh"
 
 using nnk::bf16;
@@ -96,15 +97,44 @@ __global__ void k_gelu_bwd(const bf16 *dpost, const bf16 *pre, bf16 *dpre, long 
 // column sums of X[M][N] (bf16): partial[chunk][N] over rows [chunk*rows, ...).  With N <= EW
 // the block's threads split into EW / N row lanes per column; each lane sums every
 // (EW / N)-th row of the chunk and the lanes are added in lane order (fixed partition).
-__global__ void k_colsum_partial(const bf16 *X, long M, int N, long rows, float *partial)
+// The rows pass through shared memory by 16-byte copies where N allows (a lane's own
+// 2-byte loads left the memory system idle: 36 us for 67 MB).
+constexpr int CSE = 4096;   // elements per stage
+__global__ void __launch_bounds__(EW) k_colsum_partial(const bf16 *X, long M, int N, long rows, float *partial)
 {
   __shared__ float s[EW];
+  __shared__ __align__(16) bf16 st[4 * CSE];
   const long r0 = blockIdx.y * rows, r1 = (r0 + rows < M) ? r0 + rows : M;
   if (N <= EW) {
     const int lanes = EW / N, c = threadIdx.x % N, lane = threadIdx.x / N;
     float v = 0.f;
-    if (lane < lanes)
+    if (N % 8 == 0) {
+      const int csr = CSE / N, nst = (int)((r1 - r0 + csr - 1) / csr), per = N / 8;   // rows per stage, stages
+      auto load = [&](int i) {
+        if (i < nst) {
+          const int n = (int)min((long)csr, r1 - r0 - (long)i * csr) * per;
+          const bf16 *src = X + (r0 + (long)i * csr) * N;
+          for (int e = threadIdx.x; e < n; e += EW) nnk::cp_async16(nnk::smem_addr(st + (i & 3) * CSE + e * 8), src + e * 8, 16);
+        }
+        nnk::cp_async_commit();
+      };
+      for (int i = 0; i < 3; i++) load(i);
+      int next = lane;   // this lane's next row of the chunk
+      for (int i = 0; i < nst; i++) {
+        nnk::cp_async_wait<2>();
+        __syncthreads();
+        load(i + 3);
+        const bf16 *t = st + (i & 3) * CSE;
+        const int end = (int)min((long)csr * (i + 1), r1 - r0);
+        if (lane < lanes) {
+#pragma unroll 8
+          for (; next < end; next += lanes) v += __bfloat162float(t[(next - csr * i) * N + c]);
+        }
+      }
+      nnk::cp_async_wait<0>();
+    } else if (lane < lanes) {
       for (long r = r0 + lane; r < r1; r += lanes) v += __bfloat162float(X[r * N + c]);
+    }
     s[threadIdx.x] = v;
     __syncthreads();
     if ((int)threadIdx.x < N) {
@@ -121,14 +151,35 @@ __global__ void k_colsum_partial(const bf16 *X, long M, int N, long rows, float 
   }
 }
 
-// out[i] = sum over k < nparts of partial[k][i], in order
-__global__ void k_sum_parts(const float *partial, int nparts, long n, float *out)
+// out[i] = sum over k < nparts of partial[k][i], in order.  A block takes 32 columns: all its
+// threads bring the partials into shared memory, many loads in flight, and one warp adds
+// them in order there (adding straight from global memory cost one L2 round trip after
+// another: 512 parts of 64 columns took 45 us)
+constexpr int SPC = 32, SPK = 256;   // columns, parts per pass
+__global__ void __launch_bounds__(EW) k_sum_parts(const float *partial, int nparts, long n, float *out)
 {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int k = 0; k < nparts; k++) s += partial[(long)k * n + i];
-    out[i] = s;
+  __shared__ float s[SPK][SPC];
+  const int c = threadIdx.x % SPC, lane = threadIdx.x / SPC;
+  const long i = (long)blockIdx.x * SPC + c;
+  float t = 0.f;
+  for (int k0 = 0; k0 < nparts; k0 += SPK) {
+    float v[SPK / (EW / SPC)];
+#pragma unroll
+    for (int u = 0; u < SPK / (EW / SPC); u++) {
+      const int k = k0 + lane + u * (EW / SPC);
+      v[u] = (k < nparts && i < n) ? partial[(long)k * n + i] : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < SPK / (EW / SPC); u++) s[lane + u * (EW / SPC)][c] = v[u];
+    __syncthreads();
+    if (lane == 0) {
+      const int m = min(SPK, nparts - k0);
+#pragma unroll 16
+      for (int k = 0; k < m; k++) t += s[k][c];
+    }
   }
+  if (lane == 0 && i < n) out[i] = t;
 }
 
 // D0[((b*nrec + r)*ny + row)] = H[b][row][rec_x[r]][0:w]: every row of each receiver's column
@@ -143,18 +194,24 @@ __global__ void k_decoder_gather(const bf16 *H, const int *rec_x, int B, int nre
   }
 }
 
-// dH[b][row][x][c] = sum over receivers r in column x of dD0[((b*nrec + r)*ny + row)][c]
+// dH[b][row][x][c] = sum over receivers r in column x of dD0[((b*nrec + r)*ny + row)][c],
+// eight channels a thread (w is a multiple of 16)
 __global__ void k_decoder_scatter(const bf16 *dD0, const int *rec_x, int B, int nrec, int ny, int nx, int w, bf16 *dH)
 {
-  const long n = (long)B * ny * nx * w;
+  const int w8 = w / 8;
+  const long n = (long)B * ny * nx * w8;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    const int c = (int)(i % w);
-    const long pix = i / w;
+    const int c = (int)(i % w8) * 8;
+    const long pix = i / w8;
     const int x = (int)(pix % nx), row = (int)((pix / nx) % ny), b = (int)(pix / ((long)nx * ny));
-    float v = 0.f;
+    float v[8] = {};
     for (int r = 0; r < nrec; r++)
-      if (rec_x[r] == x) v += __bfloat162float(dD0[(((long)b * nrec + r) * ny + row) * w + c]);
-    dH[i] = __float2bfloat16(v);
+      if (rec_x[r] == x) {
+        const bf16 *s = dD0 + (((long)b * nrec + r) * ny + row) * w + c;
+        for (int q = 0; q < 8; q++) v[q] += __bfloat162float(s[q]);
+      }
+    *reinterpret_cast<uint4 *>(dH + pix * w + c) =
+        make_uint4(nnk::pack_bf16(v[0], v[1]), nnk::pack_bf16(v[2], v[3]), nnk::pack_bf16(v[4], v[5]), nnk::pack_bf16(v[6], v[7]));
   }
 }
 
@@ -178,8 +235,9 @@ __global__ void k_mse(const float *out, const float *target, long n, double *par
   if (threadIdx.x == 0) partial[blockIdx.x] = s[0];
 }
 
-__global__ void k_adam(float *p, const float *g, float *m, float *v, long n, float lr, float b1, float b2, float eps,
-                       float wd, float c1, float c2)
+// (pb: the BF16 operand copy of the parameters)
+__global__ void k_adam(float *p, const float *g, float *m, float *v, bf16 *pb, long n, float lr, float b1, float b2,
+                       float eps, float wd, float c1, float c2)
 {
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     const float gi = g[i];
@@ -188,7 +246,9 @@ __global__ void k_adam(float *p, const float *g, float *m, float *v, long n, flo
     m[i] = mi;
     v[i] = vi;
     const float mh = mi / c1, vh = vi / c2;
-    p[i] = p[i] - lr * (mh / (sqrtf(vh) + eps) + wd * p[i]);
+    const float pi = p[i] - lr * (mh / (sqrtf(vh) + eps) + wd * p[i]);
+    p[i] = pi;
+    pb[i] = __float2bfloat16(pi);
   }
 }
 
@@ -234,11 +294,15 @@ struct se2nn {
   std::vector<long> oWre, oWim, oW, ob;
   float *params = nullptr, *grads = nullptr, *adam_m = nullptr, *adam_v = nullptr;
   long adam_t = 0;
-  // BF16 copies of the matrix parameters
-  bf16 *W0b = nullptr, *W1b = nullptr, *W2b = nullptr;
-  std::vector<bf16 *> Wb, Wblk;
-  // DFT matrices (BF16): Ex [2m][nx], My [4m][2ny], Myinv [2ny][4m], Exinv [nx][2m]
-  bf16 *Ex = nullptr, *My = nullptr, *Myinv = nullptr, *Exinv = nullptr;
+  // BF16 copy of all parameters, and into it the matrices the kernels read; the 2w x 2w mode
+  // blocks of the GEMM path are formed from the parameters when that path next runs
+  bf16 *Pb = nullptr, *W0b = nullptr, *W1b = nullptr, *W2b = nullptr;
+  std::vector<bf16 *> Wb, Wreb, Wimb, Wblk;
+  bool wblk_stale = true;
+  int nsm = 0, row_ctas[4] = {1, 1, 1, 1};   // SMs; the row kernels' resident CTAs per SM
+  // DFT matrices (BF16): Ex [2m][nx], My [4m][2ny], Myinv [2ny][4m] (= My^T), Exinv [nx][2m],
+  // and the transposes ExT [nx][2m], ExinvT [2m][nx]
+  bf16 *Ex = nullptr, *My = nullptr, *Myinv = nullptr, *Exinv = nullptr, *ExT = nullptr, *ExinvT = nullptr;
   int *rec_x = nullptr;
   // activations (max batch)
   std::vector<bf16 *> H, Apre, Zp;
@@ -313,7 +377,7 @@ int build_dft(se2nn *h)
   const int nx = h->c.nx, ny = h->c.ny, m = h->m;
   const double tau = 2.0 * M_PI;
   auto ky_of = [&](int j) { return j < m ? j : ny - 2 * m + j; };
-  std::vector<float> ex(2 * m * nx), my(4 * m * 2 * ny), myi(2 * ny * 4 * m), exi(nx * 2 * m);
+  std::vector<float> ex(2 * m * nx), my(4 * m * 2 * ny), myi(2 * ny * 4 * m), exi(nx * 2 * m), ext(nx * 2 * m), exit(2 * m * nx);
   for (int kx = 0; kx < m; kx++)
     for (int x = 0; x < nx; x++) {
       const double t = tau * kx * x / nx;
@@ -337,7 +401,14 @@ int build_dft(se2nn *h)
       myi[(y * 2 + 1) * 4 * m + j * 2 + 0] = (float)s;
       myi[(y * 2 + 1) * 4 * m + j * 2 + 1] = (float)c;
     }
+  for (int k = 0; k < 2 * m; k++)
+    for (int x = 0; x < nx; x++) {
+      ext[x * 2 * m + k] = ex[k * nx + x];
+      exit[k * nx + x] = exi[x * 2 * m + k];
+    }
   int rc;
+  if ((rc = nalloc(h, &h->ExT, ext.size())) || (rc = upload_bf16(h, h->ExT, ext))) return rc;
+  if ((rc = nalloc(h, &h->ExinvT, exit.size())) || (rc = upload_bf16(h, h->ExinvT, exit))) return rc;
   if ((rc = nalloc(h, &h->Ex, ex.size())) || (rc = upload_bf16(h, h->Ex, ex))) return rc;
   if ((rc = nalloc(h, &h->My, my.size())) || (rc = upload_bf16(h, h->My, my))) return rc;
   if ((rc = nalloc(h, &h->Myinv, myi.size())) || (rc = upload_bf16(h, h->Myinv, myi))) return rc;
@@ -345,18 +416,23 @@ int build_dft(se2nn *h)
   return 0;
 }
 
-// refresh the BF16 operand copies from the FP32 master parameters
+// refresh the BF16 operand copy from the FP32 master parameters
 int refresh_bf16(se2nn *h)
 {
-  const int w = h->w, cin = h->c.cin, hid = h->c.hidden, ns = h->nsub;
-  k_f32_to_bf16<<<nblk((long)cin * w), EW, 0, h->stream>>>(h->params + h->oW0, h->W0b, (long)cin * w);
-  k_f32_to_bf16<<<nblk((long)w * hid), EW, 0, h->stream>>>(h->params + h->oW1, h->W1b, (long)w * hid);
-  k_f32_to_bf16<<<nblk((long)hid * ns), EW, 0, h->stream>>>(h->params + h->oW2, h->W2b, (long)hid * ns);
-  for (int l = 0; l < h->L; l++) {
-    k_f32_to_bf16<<<nblk((long)w * w), EW, 0, h->stream>>>(h->params + h->oW[l], h->Wb[l], (long)w * w);
-    const long nb = (long)h->nmodes * 4 * w * w;
-    k_build_wblk<<<nblk(nb), EW, 0, h->stream>>>(h->params + h->oWre[l], h->params + h->oWim[l], h->Wblk[l], h->nmodes, w);
-  }
+  k_f32_to_bf16<<<nblk(h->P), EW, 0, h->stream>>>(h->params, h->Pb, h->P);
+  h->wblk_stale = true;
+  NCK(h, cudaGetLastError());
+  return 0;
+}
+
+// the mode blocks of the GEMM path
+int refresh_wblk(se2nn *h)
+{
+  if (!h->wblk_stale) return 0;
+  for (int l = 0; l < h->L; l++)
+    k_build_wblk<<<nblk((long)h->nmodes * 4 * h->w * h->w), EW, 0, h->stream>>>(h->params + h->oWre[l], h->params + h->oWim[l],
+                                                                                h->Wblk[l], h->nmodes, h->w);
+  h->wblk_stale = false;
   NCK(h, cudaGetLastError());
   return 0;
 }
@@ -461,7 +537,7 @@ int colsum(se2nn *h, const bf16 *X, long M, int N, long rows, float *out)
 {
   const int chunks = (int)((M + rows - 1) / rows);
   k_colsum_partial<<<dim3(1, chunks), EW, 0, h->stream>>>(X, M, N, rows, h->partial);
-  k_sum_parts<<<nblk(N), EW, 0, h->stream>>>(h->partial, chunks, N, out);
+  k_sum_parts<<<nblk(N, SPC), EW, 0, h->stream>>>(h->partial, chunks, N, out);
   NCK(h, cudaGetLastError());
   return 0;
 }
@@ -473,7 +549,7 @@ int weight_grad(se2nn *h, const bf16 *X, int rows, const bf16 *dY, int B, float 
   const long kc = h->npix / s;
   GemmArgs g = mk(X, rows, kc * rows, 1, dY, w, kc * w, 0, rows, w, (int)kc, B * s, h->partial, w, (long)rows * w, 1);
   GEMM(h, g);
-  k_sum_parts<<<nblk((long)rows * w), EW, 0, h->stream>>>(h->partial, B * s, (long)rows * w, out);
+  k_sum_parts<<<nblk((long)rows * w, SPC), EW, 0, h->stream>>>(h->partial, B * s, (long)rows * w, out);
   NCK(h, cudaGetLastError());
   return 0;
 }
@@ -484,7 +560,7 @@ int splitk_grad(se2nn *h, const bf16 *X, int M, const bf16 *dY, int N, long K, l
   const int parts = (int)(K / chunk);
   GemmArgs g = mk(X, M, chunk * M, 1, dY, N, chunk * N, 0, M, N, (int)chunk, parts, h->partial, N, (long)M * N, 1);
   GEMM(h, g);
-  k_sum_parts<<<nblk((long)M * N), EW, 0, h->stream>>>(h->partial, parts, (long)M * N, out);
+  k_sum_parts<<<nblk((long)M * N, SPC), EW, 0, h->stream>>>(h->partial, parts, (long)M * N, out);
   NCK(h, cudaGetLastError());
   return 0;
 }
@@ -527,16 +603,217 @@ int spectral_bwd(se2nn *h, int l, const bf16 *dS, int B, bf16 *dHacc)
   return 0;
 }
 
-int forward(se2nn *h, const bf16 *x, int B, float *out)
+// ---- the fused path (se2nn_rows.cuh): the default wherever its shapes allow; the GEMM path
+// serves the others and, with se2nn_set_tensor_path 0 or 2, every shape.  Same bits.
+bool fused_shape(const se2nn *h)
+{
+  const se2nn_config &c = h->c;
+  return (h->w == 16 || h->w == 32 || h->w == 48 || h->w == 64) && c.cin <= 64 && c.nx % 16 == 0 &&
+         c.nx <= nnk::RNX && c.ny % 8 == 0 && c.ny <= nnk::RNY && h->m <= nnk::RM;
+}
+bool fused_ok(const se2nn *h, const void *x)
+{
+  return g_tc_path == 1 && fused_shape(h) && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+}
+
+// Kernel set-up at create: shared-memory limits (at the largest size any network uses, so that
+// handles of different shapes agree on them) and the row kernels' resident CTAs.
+template <class F>
+cudaError_t allow_smem(F *fn, size_t smem)
+{
+  return (smem > 48 * 1024) ? cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : cudaSuccess;
+}
+
+template <int W, int KIND>
+cudaError_t row_setup(se2nn *h)
+{
+  typedef nnk::RowSmem<W, KIND> S;
+  cudaError_t e = allow_smem(nnk::row_kernel<W, KIND>, S::bytes(nnk::RNX, 64));
+  int n = 1;
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, nnk::row_kernel<W, KIND>, nnk::RT, S::bytes(h->c.nx, h->c.cin));
+  h->row_ctas[KIND] = std::max(1, n);
+  return e;
+}
+
+template <int W>
+int fused_setup_w(se2nn *h)
+{
+  cudaError_t e = row_setup<W, nnk::ROW_LIFT>(h);
+  if (e == cudaSuccess) e = row_setup<W, nnk::ROW_FWD>(h);
+  if (e == cudaSuccess) e = row_setup<W, nnk::ROW_BWD>(h);
+  if (e == cudaSuccess) e = row_setup<W, nnk::ROW_TOP>(h);
+  if (e == cudaSuccess) e = allow_smem(nnk::y_analysis, nnk::y_analysis_smem(nnk::RNY));
+  if (e == cudaSuccess) e = allow_smem(nnk::y_synthesis, nnk::y_synthesis_smem(nnk::RNY));
+  if (e == cudaSuccess) e = allow_smem(nnk::last_kernel<W>, nnk::last_smem<W>());
+  if (e == cudaSuccess) e = allow_smem(nnk::mode_mix<W>, nnk::mode_smem<W>());
+  if (e == cudaSuccess) e = allow_smem(nnk::mode_grad<W>, nnk::mode_grad_smem<W>());
+  if (e == cudaSuccess) e = allow_smem(nnk::weight_grad_partial<W>, nnk::wgrad_smem(64, W));
+  NCK(h, e);
+  return 0;
+}
+
+template <int W, int KIND>
+int row_launch(se2nn *h, const nnk::RowArgs &a)
+{
+  nnk::row_kernel<W, KIND><<<std::min(a.rows, h->row_ctas[KIND] * h->nsm), nnk::RT, nnk::RowSmem<W, KIND>::bytes(a.nx, a.cin), h->stream>>>(a);
+  NCK(h, cudaGetLastError());
+  return 0;
+}
+
+// f<W>(h, ...) for the network's width
+#define NN_WIDTH(f, ...)                       \
+  switch (h->w) {                              \
+    case 16: return f<16>(__VA_ARGS__);        \
+    case 32: return f<32>(__VA_ARGS__);        \
+    case 48: return f<48>(__VA_ARGS__);        \
+    default: return f<64>(__VA_ARGS__);        \
+  }
+
+int fused_setup(se2nn *h)
+{
+  if (!fused_shape(h)) return 0;
+  NN_WIDTH(fused_setup_w, h)
+}
+
+nnk::RowArgs row_args(se2nn *h, int B)
+{
+  nnk::RowArgs a;
+  memset(&a, 0, sizeof(a));
+  a.rows = B * h->c.ny; a.nx = h->c.nx; a.ny = h->c.ny; a.m2 = 2 * h->m; a.cin = h->c.cin;
+  a.nrec = h->c.nrec; a.rec_x = h->rec_x;
+  return a;
+}
+
+int y_analysis(se2nn *h, const bf16 *spec, bf16 *Zp, int B)
+{
+  const size_t smem = nnk::y_analysis_smem(h->c.ny);
+  nnk::y_analysis<<<dim3((h->m * h->w + 63) / 64, B), 128, smem, h->stream>>>(nnk::YArgs{h->My, spec, Zp, h->c.ny, h->m, h->w, B});
+  NCK(h, cudaGetLastError());
+  return 0;
+}
+
+int y_synthesis(se2nn *h, const bf16 *Y, bf16 *spec, int B)
+{
+  const size_t smem = nnk::y_synthesis_smem(h->c.ny);
+  nnk::y_synthesis<<<dim3((h->m * h->w + 63) / 64, B), 256, smem, h->stream>>>(nnk::YArgs{h->Myinv, Y, spec, h->c.ny, h->m, h->w, B});
+  NCK(h, cudaGetLastError());
+  return 0;
+}
+
+template <int W>
+int mode_mix(se2nn *h, int l, int B)
+{
+  constexpr size_t smem = nnk::mode_smem<W>();
+  nnk::mode_mix<W><<<h->nmodes, nnk::RT, smem, h->stream>>>(
+      nnk::ModeArgs{h->Zp[l], h->Wreb[l], h->Wimb[l], h->Y, nullptr, nullptr, nullptr, h->m, B});
+  NCK(h, cudaGetLastError());
+  return 0;
+}
+
+// from the spectrum rows Xf of H[l] to the spectrum rows Yy of the layer's spectral part
+int spectrum_fwd(se2nn *h, int l, int B)
+{
+  auto mix = [&]() -> int { NN_WIDTH(mode_mix, h, l, B) };
+  int rc;
+  if ((rc = y_analysis(h, h->Xf, h->Zp[l], B)) || (rc = mix()) || (rc = y_synthesis(h, h->Y, h->Yy, B))) return rc;
+  return 0;
+}
+
+template <int W>
+int last_rows(se2nn *h, int B)
+{
+  const int l = h->L - 1;
+  constexpr size_t smem = nnk::last_smem<W>();
+  nnk::LastArgs a{h->H[l], h->Yy, h->Wb[l], h->Exinv, h->params + h->ob[l], h->rec_x, h->D0, B * h->c.ny, h->c.nx, h->c.ny,
+                  2 * h->m, h->c.nrec};
+  nnk::last_kernel<W><<<(a.rows + 7) / 8, nnk::RT, smem, h->stream>>>(a);
+  NCK(h, cudaGetLastError());
+  return 0;
+}
+
+// the lift and the Fourier layers to the decoder's input D0; keep: store the pre-activations
+template <int W>
+int layers_fwd(se2nn *h, const bf16 *x, int B, bool keep)
+{
+  int rc;
+  nnk::RowArgs a = row_args(h, B);
+  a.in = x; a.wt = h->W0b; a.bias = h->params + h->ob0; a.efwd = h->Ex; a.out = h->H[0]; a.spec_out = h->Xf;
+  if ((rc = row_launch<W, nnk::ROW_LIFT>(h, a))) return rc;
+  for (int l = 0; l < h->L; l++) {
+    if ((rc = spectrum_fwd(h, l, B))) return rc;
+    if (l == h->L - 1) break;
+    a = row_args(h, B);
+    a.in = h->H[l]; a.spec = h->Yy; a.wt = h->Wb[l]; a.bias = h->params + h->ob[l]; a.einv = h->Exinv; a.efwd = h->Ex;
+    a.out = h->H[l + 1]; a.aux = keep ? h->Apre[l] : nullptr; a.spec_out = h->Xf;
+    if ((rc = row_launch<W, nnk::ROW_FWD>(h, a))) return rc;
+  }
+  return last_rows<W>(h, B);
+}
+
+int layers_fused(se2nn *h, const bf16 *x, int B, bool keep) { NN_WIDTH(layers_fwd, h, x, B, keep) }
+
+template <int W>
+int mode_grad(se2nn *h, int l, int B)
+{
+  constexpr size_t smem = nnk::mode_grad_smem<W>();
+  nnk::mode_grad<W><<<h->nmodes, nnk::RT, smem, h->stream>>>(
+      nnk::ModeArgs{h->Zp[l], h->Wreb[l], h->Wimb[l], h->Y, h->Yp, h->grads + h->oWre[l], h->grads + h->oWim[l], h->m, B});
+  NCK(h, cudaGetLastError());
+  return 0;
+}
+
+template <int W>
+int weight_grad_rows(se2nn *h, const bf16 *X, int R, const bf16 *dY, int B, float *out)
+{
+  nnk::weight_grad_partial<W><<<B * h->split, nnk::RT, nnk::wgrad_smem(R, W), h->stream>>>(X, R, dY, h->npix / h->split, h->partial);
+  k_sum_parts<<<nblk((long)R * W, SPC), EW, 0, h->stream>>>(h->partial, B * h->split, (long)R * W, out);
+  NCK(h, cudaGetLastError());
+  return 0;
+}
+
+// backward of the Fourier layers and the lift from dD0.  dHa and dHb take turns as the layers'
+// gradients: dA of layer l (below the first layer dH[0]) with its spectrum rows in Xf.
+template <int W>
+int layers_bwd(se2nn *h, const bf16 *x, int B)
+{
+  const long rows = (long)B * h->npix;
+  int rc;
+  nnk::RowArgs a = row_args(h, B);
+  a.dd0 = h->dD0; a.efwd = h->ExinvT; a.out = h->dHa; a.spec_out = h->Xf;
+  if ((rc = row_launch<W, nnk::ROW_TOP>(h, a))) return rc;
+  for (int l = h->L - 1; l >= 0; l--) {
+    if ((rc = weight_grad_rows<W>(h, h->H[l], W, h->dHa, B, h->grads + h->oW[l]))) return rc;
+    if ((rc = colsum(h, h->dHa, rows, W, 1024, h->grads + h->ob[l]))) return rc;
+    if ((rc = y_analysis(h, h->Xf, h->Yp, B)) || (rc = mode_grad<W>(h, l, B)) || (rc = y_synthesis(h, h->Y, h->Yy, B))) return rc;
+    a = row_args(h, B);
+    a.in = h->dHa; a.spec = h->Yy; a.wt = h->Wb[l]; a.einv = h->ExT; a.efwd = h->ExinvT; a.out = h->dHb;
+    a.pre = l ? h->Apre[l - 1] : nullptr;
+    a.spec_out = l ? h->Xf : nullptr;
+    if ((rc = row_launch<W, nnk::ROW_BWD>(h, a))) return rc;
+    std::swap(h->dHa, h->dHb);
+  }
+  if ((rc = weight_grad_rows<W>(h, x, h->c.cin, h->dHa, B, h->grads + h->oW0))) return rc;
+  return colsum(h, h->dHa, rows, W, 1024, h->grads + h->ob0);
+}
+
+int layers_bwd_fused(se2nn *h, const bf16 *x, int B) { NN_WIDTH(layers_bwd, h, x, B) }
+
+// keep: the pass is followed by backward (pre-activations are stored)
+int forward(se2nn *h, const bf16 *x, int B, float *out, bool keep)
 {
   const int w = h->w, L = h->L, nrec = h->c.nrec, hid = h->c.hidden;
   const long rows = (long)B * h->npix;
+  int rc;
+  const bool fused = fused_ok(h, x);
+  if (fused) {
+    if ((rc = layers_fused(h, x, B, keep))) return rc;
+  } else {
+  if ((rc = refresh_wblk(h))) return rc;
   {
     GemmArgs g = mk(x, h->c.cin, 0, 0, h->W0b, w, 0, 0, (int)rows, w, h->c.cin, 1, h->H[0], w, 0, 0);
     g.bias = h->params + h->ob0;
     GEMM(h, g);
   }
-  int rc;
   for (int l = 0; l < L; l++) {
     if ((rc = spectral_fwd(h, l, h->H[l], B, h->S))) return rc;
     GemmArgs g = mk(h->H[l], w, 0, 0, h->Wb[l], w, 0, 0, (int)rows, w, w, 1, h->H[l + 1], w, 0, 0);
@@ -545,9 +822,10 @@ int forward(se2nn *h, const bf16 *x, int B, float *out)
     if (l < L - 1) { g.act = 1; g.aux = h->Apre[l]; g.ldaux = w; }
     GEMM(h, g);
   }
+  }
   const bf16 *HL = h->H[L];
   const long drows = (long)B * nrec * h->c.ny;
-  k_decoder_gather<<<nblk(drows * w), EW, 0, h->stream>>>(HL, h->rec_x, B, nrec, h->c.ny, h->c.nx, w, h->D0);
+  if (!fused) k_decoder_gather<<<nblk(drows * w), EW, 0, h->stream>>>(HL, h->rec_x, B, nrec, h->c.ny, h->c.nx, w, h->D0);
   {
     GemmArgs g = mk(h->D0, w, 0, 0, h->W1b, hid, 0, 0, (int)drows, hid, w, 1, h->D1, hid, 0, 0);
     g.bias = h->params + h->oc1; g.act = 1; g.aux = h->D1pre; g.ldaux = hid;
@@ -575,7 +853,9 @@ int backward(se2nn *h, const bf16 *x, int B)
   if ((rc = splitk_grad(h, h->D0, w, h->dD1, hid, drows, h->c.ny, h->grads + h->oW1))) return rc;
   if ((rc = colsum(h, h->dD1, drows, hid, 256, h->grads + h->oc1))) return rc;
   GEMM(h, mk(h->dD1, hid, 0, 0, h->W1b, hid, 0, 1, (int)drows, w, hid, 1, h->dD0, w, 0, 0));
-  k_decoder_scatter<<<nblk(rows * w), EW, 0, h->stream>>>(h->dD0, h->rec_x, B, nrec, h->c.ny, h->c.nx, w, h->dHa);
+  if (fused_ok(h, x)) return layers_bwd_fused(h, x, B);
+  if ((rc = refresh_wblk(h))) return rc;
+  k_decoder_scatter<<<nblk(rows * w / 8), EW, 0, h->stream>>>(h->dD0, h->rec_x, B, nrec, h->c.ny, h->c.nx, w, h->dHa);
   // Fourier layers, last to first: dHa holds dL/dH[l+1]
   for (int l = L - 1; l >= 0; l--) {
     const bf16 *dA = h->dHa;
@@ -651,17 +931,28 @@ extern "C" int se2nn_create(const se2nn_config *cfg, unsigned long long seed, se
     delete h;
     return nfail(nullptr, -2, "cudaStreamCreate failed");
   }
+  {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+      cudaGetLastError();
+      nfail(h, -2, "device query failed");
+      TRY(-2);
+    }
+  }
   TRY(nalloc(h, &h->params, h->P));
   TRY(nalloc(h, &h->grads, h->P));
   TRY(nalloc(h, &h->adam_m, h->P));
   TRY(nalloc(h, &h->adam_v, h->P));
-  TRY(nalloc(h, &h->W0b, (size_t)c.cin * w));
-  TRY(nalloc(h, &h->W1b, (size_t)w * c.hidden));
-  TRY(nalloc(h, &h->W2b, (size_t)c.hidden * h->nsub));
-  h->Wb.assign(L, nullptr); h->Wblk.assign(L, nullptr); h->Zp.assign(L, nullptr);
+  TRY(nalloc(h, &h->Pb, h->P));
+  h->W0b = h->Pb + h->oW0; h->W1b = h->Pb + h->oW1; h->W2b = h->Pb + h->oW2;
+  for (int l = 0; l < L; l++) {
+    h->Wb.push_back(h->Pb + h->oW[l]);
+    h->Wreb.push_back(h->Pb + h->oWre[l]);
+    h->Wimb.push_back(h->Pb + h->oWim[l]);
+  }
+  h->Wblk.assign(L, nullptr); h->Zp.assign(L, nullptr);
   h->H.assign(L + 1, nullptr); h->Apre.assign(L > 1 ? L - 1 : 0, nullptr);
   for (int l = 0; l < L; l++) {
-    TRY(nalloc(h, &h->Wb[l], (size_t)w * w));
     TRY(nalloc(h, &h->Wblk[l], (size_t)nm * 4 * w * w));
     TRY(nalloc(h, &h->Zp[l], (size_t)nm * Bm * 2 * w));
   }
@@ -698,6 +989,7 @@ extern "C" int se2nn_create(const se2nn_config *cfg, unsigned long long seed, se
     TRY(nalloc(h, &h->partial, (size_t)h->partial_n));
   }
   TRY(build_dft(h));
+  TRY(fused_setup(h));
   // initial parameters (seeded)
   {
     std::vector<float> p(h->P, 0.f);
@@ -786,7 +1078,7 @@ extern "C" int se2nn_forward(se2nn *h, const void *x_dev, int batch, float *out_
   if (!h || !x_dev || !out_dev) return -1;
   int rc = check_batch(h, batch);
   if (rc) return rc;
-  return forward(h, static_cast<const bf16 *>(x_dev), batch, out_dev);
+  return forward(h, static_cast<const bf16 *>(x_dev), batch, out_dev, false);
 }
 
 extern "C" int se2nn_loss_grad(se2nn *h, const void *x_dev, int batch, const float *target_dev, double *loss,
@@ -797,7 +1089,7 @@ extern "C" int se2nn_loss_grad(se2nn *h, const void *x_dev, int batch, const flo
   if (rc) return rc;
   const bf16 *x = static_cast<const bf16 *>(x_dev);
   float *out = out_dev ? out_dev : h->out;
-  if ((rc = forward(h, x, batch, out))) return rc;
+  if ((rc = forward(h, x, batch, out, true))) return rc;
   const long n = (long)batch * h->c.nrec * h->c.nout;
   const int nb = (int)std::min<long>(1024, (n + EW - 1) / EW);
   k_mse<<<nb, EW, 0, h->stream>>>(out, target_dev, n, h->lpart, h->dpred);
@@ -817,10 +1109,11 @@ extern "C" int se2nn_adam_step(se2nn *h, float lr, float beta1, float beta2, flo
   if (!h) return -1;
   h->adam_t++;
   const float c1 = 1.f - powf(beta1, (float)h->adam_t), c2 = 1.f - powf(beta2, (float)h->adam_t);
-  k_adam<<<nblk(h->P), EW, 0, h->stream>>>(h->params, h->grads, h->adam_m, h->adam_v, h->P, lr, beta1, beta2, eps,
+  k_adam<<<nblk(h->P), EW, 0, h->stream>>>(h->params, h->grads, h->adam_m, h->adam_v, h->Pb, h->P, lr, beta1, beta2, eps,
                                             weight_decay, c1, c2);
+  h->wblk_stale = true;
   NCK(h, cudaGetLastError());
-  return refresh_bf16(h);
+  return 0;
 }
 
 extern "C" int se2nn_build_inputs(se2nn *h, const void *materials_dev, const float *src_dev, const int *idx_dev,

@@ -1,0 +1,706 @@
+// se2nn_rows.cuh -- the surrogate network's layers as fused kernels, for sm_103a.
+//
+// A Fourier layer is five contractions around one activation-sized array.  Run as one GEMM
+// launch each, every contraction moves that array through memory (67 MB at batch 32) for
+// a K of 32 to 128, so what bounds them is memory traffic and launch latency, not the tensor
+// pipe.  Fused along the image row -- the unit on which both x transforms and the 1x1
+// convolution act -- a layer reads and writes it once:
+//
+//   row_kernel    one image row (nx pixels x W channels) at a time: the inverse x transform of
+//                 the layer's spectrum row, the 1x1 convolution, bias, GELU, and the forward
+//                 x transform of the result for the next layer.  Backward: the adjoint of the
+//                 same chain with GELU' of the stored pre-activation.
+//   y_analysis    per sample: the forward y transform, stored mode-major
+//   mode_mix      per mode: the complex channel mixing from the two real weight matrices
+//   mode_grad     per mode: the adjoint of the mixing and both weight gradients
+//   y_synthesis   per sample: the inverse y transform
+//
+// Numbers.  Every contraction accumulates in FP32 over k in ascending steps of 16
+// (mma.m16n8k16, products of zero padding adding exact zeros), and every array that the
+// unfused kernels store in BF16 is rounded to BF16 at the same place, so the results
+// are the same bits as the GEMM kernels' (tests/test_nn_fused.py).
+//
+// Used for W = 16, 32, 48, 64, nx <= 128 a multiple of 16, ny <= 128 a multiple of 8 and up to
+// 16 modes (se2nn.cu, fused_ok); other shapes run the GEMM kernels.
+#pragma once
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "se2nn_gemm.cuh"
+
+namespace nnk {
+
+constexpr int RT = 256;                  // threads of the row kernels
+constexpr int RK = 32;                   // x modes (re, im) padded to two k steps
+constexpr int RNX = 128, RNY = 128, RM = 16;   // largest row, column, modes
+
+template <int LEFT> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
+
+// asynchronous copy of rows x cols (a multiple of 8) elements into shared memory
+__device__ __forceinline__ void copy_tile(bf16 *s, int lds, const bf16 *g, long ldg, int rows, int cols, int nt)
+{
+  const int per = cols / 8;
+  for (int e = threadIdx.x; e < rows * per; e += nt) {
+    const int r = e / per, c = (e - r * per) * 8;
+    cp_async16(smem_addr(s + r * lds + c), g + r * ldg + c, 16);
+  }
+}
+// the same for a whole tile of zero-padded rows, by plain stores
+__device__ __forceinline__ void zero_rows(bf16 *s, int lds, int r0, int r1, int nt)
+{
+  for (int e = threadIdx.x; e < (r1 - r0) * lds; e += nt) s[r0 * lds + e] = __float2bfloat16(0.f);
+}
+
+// fragments: A stored m-major (k contiguous) or k-major; B stored k-major (n contiguous) or n-major
+__device__ __forceinline__ void frag_a(uint32_t *f, const bf16 *s, int lds, int m0, int k0)
+{
+  const int lane = threadIdx.x & 31, mat = lane >> 3, r = lane & 7;
+  ldsm_x4(f, smem_addr(s + (m0 + (mat & 1) * 8 + r) * lds + k0 + (mat >> 1) * 8), false);
+}
+__device__ __forceinline__ void frag_at(uint32_t *f, const bf16 *s, int lds, int m0, int k0)
+{
+  const int lane = threadIdx.x & 31, mat = lane >> 3, r = lane & 7;
+  ldsm_x4(f, smem_addr(s + (k0 + (mat >> 1) * 8 + r) * lds + m0 + (mat & 1) * 8), true);
+}
+// two n tiles of 8: f[0..1] columns n0 .. n0 + 7, f[2..3] columns n0 + 8 .. n0 + 15
+__device__ __forceinline__ void frag_b(uint32_t *f, const bf16 *s, int lds, int n0, int k0)
+{
+  const int lane = threadIdx.x & 31, mat = lane >> 3, r = lane & 7;
+  ldsm_x4(f, smem_addr(s + (k0 + (mat & 1) * 8 + r) * lds + n0 + (mat >> 1) * 8), true);
+}
+__device__ __forceinline__ void frag_bt(uint32_t *f, const bf16 *s, int lds, int n0, int k0)
+{
+  const int lane = threadIdx.x & 31, mat = lane >> 3, r = lane & 7;
+  ldsm_x4(f, smem_addr(s + (n0 + (mat >> 1) * 8 + r) * lds + k0 + (mat & 1) * 8), false);
+}
+__device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16(x)); }
+__device__ __forceinline__ uint32_t pack_bf16(float x, float y)
+{
+  const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
+  return *reinterpret_cast<const uint32_t *>(&v);
+}
+__device__ __forceinline__ float2 unpack_bf16(uint32_t u)
+{
+  const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162 *>(&u);
+  return make_float2(__low2float(v), __high2float(v));
+}
+
+enum { ROW_LIFT = 0, ROW_FWD = 1, ROW_BWD = 2, ROW_TOP = 3 };
+
+struct RowArgs {
+  const bf16 *in;        // [rows][nx][W]: FWD H, BWD dA of the layer above (LIFT [rows][nx][cin])
+  const bf16 *spec;      // [rows][m2][W]: FWD the layer's spectrum after the inverse y transform, BWD its adjoint
+  const bf16 *wt;        // FWD, LIFT [K][W]; BWD [W][W], applied transposed
+  const float *bias;     // FWD, LIFT
+  const bf16 *einv;      // [nx][m2]: spectrum row -> pixels
+  const bf16 *efwd;      // [m2][nx]: pixels -> spectrum row
+  const bf16 *pre;       // BWD: pre-activation of the layer below (null: none)
+  bf16 *out;             // [rows][nx][W]: H, or dA (dH below the first layer)
+  bf16 *aux;             // FWD: pre-activation (null: not stored)
+  bf16 *spec_out;        // [rows][m2][W] (null: none)
+  int rows, nx, m2, cin;
+  // TOP: the decoder's data gradient [B][nrec][ny][W], summed into the receivers' columns
+  const bf16 *dd0;
+  const int *rec_x;
+  int nrec, ny;
+};
+
+template <int W, int KIND>
+struct RowSmem {
+  static constexpr int LW = W + 8, LE = RK + 8;
+  static constexpr int KIN = (KIND == ROW_LIFT) ? 64 : W;   // widest convolution input
+  static __host__ __device__ size_t wt() { return (KIND == ROW_TOP) ? 0 : (size_t)KIN * LW; }
+  static __host__ __device__ size_t einv(int nx) { return (KIND == ROW_FWD || KIND == ROW_BWD) ? (size_t)nx * LE : 0; }
+  static __host__ __device__ size_t efwd(int nx) { return (size_t)RK * (nx + 8); }
+  static __host__ __device__ size_t in(int nx, int cin) { return (size_t)nx * ((KIND == ROW_LIFT) ? cin + 8 : LW); }
+  static __host__ __device__ size_t spec() { return (KIND == ROW_FWD || KIND == ROW_BWD) ? (size_t)RK * LW : 0; }
+  static __host__ __device__ size_t pre(int nx) { return (KIND == ROW_BWD) ? (size_t)nx * LW : 0; }
+  static __host__ __device__ size_t stage(int nx, int cin) { return in(nx, cin) + spec() + pre(nx); }
+  static __host__ __device__ size_t out(int nx) { return (KIND == ROW_LIFT) ? (size_t)nx * LW : 0; }
+  static __host__ __device__ size_t bytes(int nx, int cin)
+  {
+    return 2 * (wt() + einv(nx) + efwd(nx) + (KIND == ROW_TOP ? 1 : 2) * stage(nx, cin) + out(nx)) + W * sizeof(float);
+  }
+};
+
+// rows [m0, m0 + 16) x W of a shared tile -> global memory, 16 bytes a lane, by one warp
+template <int W>
+__device__ __forceinline__ void store_rows16(bf16 *g, const bf16 *s, int m0)
+{
+  constexpr int PER = W / 8;
+  for (int e = threadIdx.x & 31; e < 16 * PER; e += 32) {
+    const int r = e / PER, c = (e - r * PER) * 8;
+    *reinterpret_cast<uint4 *>(g + (size_t)(m0 + r) * W + c) = *reinterpret_cast<const uint4 *>(s + (m0 + r) * (W + 8) + c);
+  }
+}
+
+// spectrum row [m2][W] of a row of pixels in shared memory: efwd (RK x nx, zero rows past m2)
+template <int W>
+__device__ __forceinline__ void x_analysis(const bf16 *sE, const bf16 *px, int nx, int m2, bf16 *out)
+{
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+  const int mt = warp & 1, np = warp >> 1;   // 16 spectrum rows x 16 channels per warp
+  if (np * 16 >= W || mt * 16 >= m2) return;
+  float acc[2][4] = {};
+  for (int k = 0; k < nx; k += 16) {
+    uint32_t a[4], b[4];
+    frag_a(a, sE, nx + 8, mt * 16, k);
+    frag_b(b, px, W + 8, np * 16, k);
+    mma_bf16(acc[0], a, b);
+    mma_bf16(acc[1], a, b + 2);
+  }
+#pragma unroll
+  for (int t = 0; t < 2; t++)
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int r = mt * 16 + gid + 8 * h;
+      if (r < m2) *reinterpret_cast<uint32_t *>(out + (size_t)r * W + np * 16 + t * 8 + tig * 2) = pack_bf16(acc[t][2 * h], acc[t][2 * h + 1]);
+    }
+}
+
+// Persistent over the image rows, two stages of asynchronous copies.  A warp owns 16 pixels
+// through the convolution and activation, so the results replace its input in shared memory
+// without a block barrier; the x transform at the end reads all pixels.
+template <int W, int KIND>
+__global__ void __launch_bounds__(RT, 2) row_kernel(const RowArgs a)
+{
+  typedef RowSmem<W, KIND> L;
+  constexpr int LW = L::LW, LE = L::LE, NT = W / 8;
+  extern __shared__ __align__(16) unsigned char rsm[];
+  bf16 *sW = reinterpret_cast<bf16 *>(rsm);
+  bf16 *sI = sW + L::wt();
+  bf16 *sE = sI + L::einv(a.nx);
+  bf16 *st0 = sE + L::efwd(a.nx);
+  bf16 *sO = st0 + (KIND == ROW_TOP ? 1 : 2) * L::stage(a.nx, a.cin);
+  float *sB = reinterpret_cast<float *>(sO + L::out(a.nx));
+  const int nx = a.nx, m2 = a.m2, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+  const int kin = (KIND == ROW_LIFT) ? a.cin : W, lin = (KIND == ROW_LIFT) ? a.cin + 8 : LW;
+  constexpr bool SPEC = KIND == ROW_FWD || KIND == ROW_BWD;
+
+  // tables, zero-padded to whole k steps
+  if (KIND != ROW_TOP) copy_tile(sW, LW, a.wt, W, kin, W, RT);
+  for (int e = threadIdx.x; e < RK * (nx + 8); e += RT) {
+    const int r = e / (nx + 8), c = e - r * (nx + 8);
+    sE[e] = (r < m2 && c < nx) ? a.efwd[r * nx + c] : __float2bfloat16(0.f);
+  }
+  if (SPEC) {
+    for (int e = threadIdx.x; e < nx * LE; e += RT) {
+      const int r = e / LE, c = e - r * LE;
+      sI[e] = (c < m2) ? a.einv[r * m2 + c] : __float2bfloat16(0.f);
+    }
+    for (int s = 0; s < 2; s++) zero_rows(st0 + s * L::stage(nx, a.cin) + L::in(nx, a.cin), LW, m2, RK, RT);
+  }
+  if (KIND == ROW_LIFT || KIND == ROW_FWD)
+    for (int e = threadIdx.x; e < W; e += RT) sB[e] = a.bias[e];
+
+  auto load = [&](int row, int s) {
+    bf16 *st = st0 + s * L::stage(nx, a.cin);
+    copy_tile(st, lin, a.in + (size_t)row * nx * kin, kin, nx, kin, RT);
+    if (SPEC) copy_tile(st + L::in(nx, a.cin), LW, a.spec + (size_t)row * m2 * W, W, m2, W, RT);
+    if (KIND == ROW_BWD && a.pre) copy_tile(st + L::in(nx, a.cin) + L::spec(), LW, a.pre + (size_t)row * nx * W, W, nx, W, RT);
+  };
+  if (KIND != ROW_TOP) {
+    if ((int)blockIdx.x < a.rows) load(blockIdx.x, 0);
+    cp_async_commit();
+  }
+  int s = 0;
+  for (int row = blockIdx.x; row < a.rows; row += gridDim.x, s ^= 1) {
+    bf16 *px = st0;   // the row's pixels [nx][LW], input and then result
+    if (KIND == ROW_TOP) {
+      const int b = row / a.ny, y = row - b * a.ny;
+      __syncthreads();   // (the previous row's x transform has read px)
+      for (int e = threadIdx.x; e < nx * NT; e += RT) {
+        const int x = e / NT, c = (e - x * NT) * 8;
+        float v[8] = {};
+        for (int r = 0; r < a.nrec; r++)
+          if (a.rec_x[r] == x) {
+            const uint4 q = *reinterpret_cast<const uint4 *>(a.dd0 + (((size_t)b * a.nrec + r) * a.ny + y) * W + c);
+            const uint32_t u[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+              const float2 f = unpack_bf16(u[i]);
+              v[2 * i] += f.x;
+              v[2 * i + 1] += f.y;
+            }
+          }
+        const uint4 o = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+        *reinterpret_cast<uint4 *>(px + x * LW + c) = o;
+        *reinterpret_cast<uint4 *>(a.out + ((size_t)row * nx + x) * W + c) = o;
+      }
+    } else {
+      bf16 *st = st0 + s * L::stage(nx, a.cin);
+      if (row + (int)gridDim.x < a.rows) load(row + gridDim.x, s ^ 1);   // (freed by the barrier that ended the previous row)
+      cp_async_commit();
+      cp_async_wait<1>();
+      __syncthreads();
+      px = (KIND == ROW_LIFT) ? sO : st;
+      const int m0 = warp * 16;
+      if (m0 < nx) {
+        // spectrum row -> pixels, and the 1x1 convolution
+        float sp[NT][4] = {}, cv[NT][4] = {};
+        if (SPEC) {
+          const bf16 *sS = st + L::in(nx, a.cin);
+#pragma unroll
+          for (int k = 0; k < RK; k += 16) {
+            uint32_t fa[4], fb[4];
+            frag_a(fa, sI, LE, m0, k);
+#pragma unroll
+            for (int n = 0; n < NT; n += 2) {
+              frag_b(fb, sS, LW, n * 8, k);
+              mma_bf16(sp[n], fa, fb);
+              mma_bf16(sp[n + 1], fa, fb + 2);
+            }
+          }
+        }
+        for (int k = 0; k < kin; k += 16) {
+          uint32_t fa[4], fb[4];
+          frag_a(fa, st, lin, m0, k);
+#pragma unroll
+          for (int n = 0; n < NT; n += 2) {
+            if (KIND == ROW_BWD) frag_bt(fb, sW, LW, n * 8, k);
+            else frag_b(fb, sW, LW, n * 8, k);
+            mma_bf16(cv[n], fa, fb);
+            mma_bf16(cv[n + 1], fa, fb + 2);
+          }
+        }
+        __syncwarp();   // the warp's pixels have been read
+        const bf16 *sP = st + L::in(nx, a.cin) + L::spec();
+        if (KIND == ROW_FWD && a.aux) {
+#pragma unroll
+          for (int n = 0; n < NT; n++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+              const int c = n * 8 + tig * 2, p = m0 + gid + 8 * h;
+              *reinterpret_cast<uint32_t *>(px + p * LW + c) =
+                  pack_bf16(cv[n][2 * h] + round_bf16(sp[n][2 * h]) + sB[c], cv[n][2 * h + 1] + round_bf16(sp[n][2 * h + 1]) + sB[c + 1]);
+            }
+          __syncwarp();
+          store_rows16<W>(a.aux + (size_t)row * nx * W, px, m0);
+          __syncwarp();
+        }
+#pragma unroll
+        for (int n = 0; n < NT; n++)
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const int c = n * 8 + tig * 2, p = m0 + gid + 8 * h;
+            float x = cv[n][2 * h], y = cv[n][2 * h + 1];
+            if (KIND == ROW_LIFT) {
+              x += sB[c];
+              y += sB[c + 1];
+            } else if (KIND == ROW_FWD) {
+              x = gelu_f(x + round_bf16(sp[n][2 * h]) + sB[c]);
+              y = gelu_f(y + round_bf16(sp[n][2 * h + 1]) + sB[c + 1]);
+            } else {
+              x = sp[n][2 * h] + round_bf16(x);
+              y = sp[n][2 * h + 1] + round_bf16(y);
+              if (a.pre) {
+                const float2 q = unpack_bf16(*reinterpret_cast<const uint32_t *>(sP + p * LW + c));
+                x = round_bf16(x) * gelu_grad_f(q.x);
+                y = round_bf16(y) * gelu_grad_f(q.y);
+              }
+            }
+            *reinterpret_cast<uint32_t *>(px + p * LW + c) = pack_bf16(x, y);
+          }
+        __syncwarp();
+        store_rows16<W>(a.out + (size_t)row * nx * W, px, m0);
+      }
+    }
+    if (a.spec_out) {
+      __syncthreads();
+      x_analysis<W>(sE, px, nx, m2, a.spec_out + (size_t)row * m2 * W);
+    }
+    if (KIND != ROW_TOP) __syncthreads();   // this stage is free for the row after the next
+  }
+}
+
+// The last layer at the receivers' pixels only (the decoder reads nothing else): one warp per
+// image row, 16 receivers at a time, D0[b][r][y][W] = bf16(conv + spectral + bias).
+struct LastArgs {
+  const bf16 *in, *spec, *wt, *einv;
+  const float *bias;
+  const int *rec_x;
+  bf16 *d0;
+  int rows, nx, ny, m2, nrec;
+};
+template <int W>
+constexpr size_t last_smem() { return 2 * ((size_t)W * (W + 8) + 8 * ((size_t)RK * (W + 8) + 16 * (W + 8) + 16 * (RK + 8))); }
+
+template <int W>
+__global__ void __launch_bounds__(RT) last_kernel(const LastArgs a)
+{
+  constexpr int LW = W + 8, LE = RK + 8, NT = W / 8;
+  extern __shared__ __align__(16) unsigned char rsm[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+  bf16 *sW = reinterpret_cast<bf16 *>(rsm);
+  bf16 *sS = sW + W * LW + warp * (RK * LW + 16 * LW + 16 * LE), *sH = sS + RK * LW, *sI = sH + 16 * LW;
+  copy_tile(sW, LW, a.wt, W, W, W, RT);
+  cp_async_commit();
+  const int row = blockIdx.x * 8 + warp;
+  const bool on = row < a.rows;
+  const int b = row / a.ny, y = row - b * a.ny;
+  if (on) {
+    for (int e = lane; e < a.m2 * NT; e += 32)
+      cp_async16(smem_addr(sS + (e / NT) * LW + (e % NT) * 8), a.spec + ((size_t)row * a.m2 + e / NT) * W + (e % NT) * 8, 16);
+    for (int e = lane; e < (RK - a.m2) * LW; e += 32) sS[a.m2 * LW + e] = __float2bfloat16(0.f);
+    cp_async_commit();
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+  if (!on) return;
+  for (int r0 = 0; r0 < a.nrec; r0 += 16) {
+    __syncwarp();
+    for (int e = lane; e < 16 * NT; e += 32) {
+      const int r = e / NT, x = (r0 + r < a.nrec) ? a.rec_x[r0 + r] : 0;
+      cp_async16(smem_addr(sH + r * LW + (e % NT) * 8), a.in + ((size_t)row * a.nx + x) * W + (e % NT) * 8, 16);
+    }
+    cp_async_commit();
+    for (int e = lane; e < 16 * LE; e += 32) {
+      const int r = e / LE, c = e - r * LE, x = (r0 + r < a.nrec) ? a.rec_x[r0 + r] : 0;
+      sI[e] = (c < a.m2) ? a.einv[x * a.m2 + c] : __float2bfloat16(0.f);
+    }
+    cp_async_wait<0>();
+    __syncwarp();
+    float sp[NT][4] = {}, cv[NT][4] = {};
+#pragma unroll
+    for (int k = 0; k < RK; k += 16) {
+      uint32_t fa[4], fb[4];
+      frag_a(fa, sI, LE, 0, k);
+#pragma unroll
+      for (int n = 0; n < NT; n += 2) {
+        frag_b(fb, sS, LW, n * 8, k);
+        mma_bf16(sp[n], fa, fb);
+        mma_bf16(sp[n + 1], fa, fb + 2);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < W; k += 16) {
+      uint32_t fa[4], fb[4];
+      frag_a(fa, sH, LW, 0, k);
+#pragma unroll
+      for (int n = 0; n < NT; n += 2) {
+        frag_b(fb, sW, LW, n * 8, k);
+        mma_bf16(cv[n], fa, fb);
+        mma_bf16(cv[n + 1], fa, fb + 2);
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < NT; n++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int c = n * 8 + tig * 2, r = r0 + gid + 8 * h;
+        if (r < a.nrec)
+          *reinterpret_cast<uint32_t *>(a.d0 + (((size_t)b * a.nrec + r) * a.ny + y) * W + c) =
+              pack_bf16(cv[n][2 * h] + round_bf16(sp[n][2 * h]) + a.bias[c], cv[n][2 * h + 1] + round_bf16(sp[n][2 * h + 1]) + a.bias[c + 1]);
+      }
+  }
+}
+
+// ---- y transforms: A [4m][2ny] (k contiguous) shared by the samples; 64 columns (kx, c) per CTA
+struct YArgs {
+  const bf16 *A;         // My [4m][2ny], or its transpose [2ny][4m] for the synthesis
+  const bf16 *B;         // analysis [b][2ny][m w]; synthesis [b][4m][m w]
+  bf16 *C;               // analysis: mode-major [(j, kx)][b][part][w]; synthesis [b][2ny][m w]
+  int ny, m, w, batch;
+};
+__host__ __device__ inline size_t y_analysis_smem(int ny) { return 2 * ((size_t)64 * (2 * ny + 8) + (size_t)2 * ny * 72); }
+__host__ __device__ inline size_t y_synthesis_smem(int ny) { return 2 * ((size_t)2 * ny * 72 + (size_t)64 * 72); }
+
+// copies of the 64 columns from n0 of rows k0 .. k1 (zero past column N)
+__device__ __forceinline__ void copy_cols(bf16 *s, const bf16 *g, long ldg, int k0, int k1, int n0, int N, int nt)
+{
+  for (int e = threadIdx.x; e < (k1 - k0) * 8; e += nt) {
+    const int r = k0 + e / 8, c = (e & 7) * 8;
+    const bool in = n0 + c < N;   // (N is a multiple of 16)
+    cp_async16(smem_addr(s + r * 72 + c), in ? g + r * ldg + n0 + c : g, in ? 16 : 0);
+  }
+}
+
+__global__ void __launch_bounds__(128) y_analysis(const YArgs a)
+{
+  extern __shared__ __align__(16) unsigned char rsm[];
+  const int K = 2 * a.ny, LA = K + 8, M = 4 * a.m, N = a.m * a.w, n0 = blockIdx.x * 64, b = blockIdx.y;
+  bf16 *sA = reinterpret_cast<bf16 *>(rsm), *sB = sA + 64 * LA;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+  // everything in flight at once, in four parts of k that are computed as they land
+  const int part = (K / 4 + 15) / 16 * 16;
+  for (int q = 0; q < 4; q++) {
+    const int k0 = min(q * part, K), k1 = min(k0 + part, K), per = (k1 - k0) / 8;
+    for (int e = threadIdx.x; e < M * per; e += 128) {
+      const int r = e / per, c = k0 + (e - r * per) * 8;
+      cp_async16(smem_addr(sA + r * LA + c), a.A + (size_t)r * K + c, 16);
+    }
+    copy_cols(sB, a.B + (size_t)b * K * N, N, k0, k1, n0, N, 128);
+    cp_async_commit();
+  }
+  zero_rows(sA, LA, M, 64, 128);
+  float acc[8][4] = {};
+  for (int q = 0; q < 4; q++) {
+    if (q == 0) cp_async_wait<3>();
+    else if (q == 1) cp_async_wait<2>();
+    else if (q == 2) cp_async_wait<1>();
+    else cp_async_wait<0>();
+    __syncthreads();
+    if (warp * 16 >= M) continue;
+    for (int k = min(q * part, K); k < min((q + 1) * part, K); k += 16) {
+      uint32_t fa[4], fb[4];
+      frag_a(fa, sA, LA, warp * 16, k);
+#pragma unroll
+      for (int n = 0; n < 8; n += 2) {
+        frag_b(fb, sB, 72, n * 8, k);
+        mma_bf16(acc[n], fa, fb);
+        mma_bf16(acc[n + 1], fa, fb + 2);
+      }
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < 8; n++)
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int r = warp * 16 + gid + 8 * h, col = n0 + n * 8 + tig * 2;
+      if (r >= M || col >= N) continue;
+      const int j = r >> 1, pt = r & 1, kx = col / a.w, c = col - kx * a.w;
+      *reinterpret_cast<uint32_t *>(a.C + (((size_t)(j * a.m + kx) * a.batch + b) * 2 + pt) * a.w + c) = pack_bf16(acc[n][2 * h], acc[n][2 * h + 1]);
+    }
+}
+
+__global__ void __launch_bounds__(256) y_synthesis(const YArgs a)
+{
+  extern __shared__ __align__(16) unsigned char rsm[];
+  const int K = 4 * a.m, K16 = (K + 15) / 16 * 16, M = 2 * a.ny, N = a.m * a.w, n0 = blockIdx.x * 64, b = blockIdx.y;
+  bf16 *sA = reinterpret_cast<bf16 *>(rsm), *sB = sA + M * 72;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+  copy_cols(sB, a.B + (size_t)b * K * N, N, 0, K, n0, N, 256);
+  zero_rows(sB, 72, K, K16, 256);
+  if (K % 8 == 0) {
+    copy_tile(sA, 72, a.A, K, M, K, 256);
+    if (K16 > K)
+      for (int e = threadIdx.x; e < M * (K16 - K); e += 256) sA[(e / (K16 - K)) * 72 + K + e % (K16 - K)] = __float2bfloat16(0.f);
+  } else {
+    for (int e = threadIdx.x; e < M * K16; e += 256) {
+      const int r = e / K16, c = e - r * K16;
+      sA[r * 72 + c] = (c < K) ? a.A[(size_t)r * K + c] : __float2bfloat16(0.f);
+    }
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  for (int m0 = warp * 16; m0 < M; m0 += 128) {
+    float acc[8][4] = {};
+    for (int k = 0; k < K16; k += 16) {
+      uint32_t fa[4], fb[4];
+      frag_a(fa, sA, 72, m0, k);
+#pragma unroll
+      for (int n = 0; n < 8; n += 2) {
+        frag_b(fb, sB, 72, n * 8, k);
+        mma_bf16(acc[n], fa, fb);
+        mma_bf16(acc[n + 1], fa, fb + 2);
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < 8; n++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int r = m0 + gid + 8 * h, col = n0 + n * 8 + tig * 2;
+        if (col < N) *reinterpret_cast<uint32_t *>(a.C + ((size_t)b * M + r) * N + col) = pack_bf16(acc[n][2 * h], acc[n][2 * h + 1]);
+      }
+  }
+}
+
+// ---- channel mixing of one mode: [Zre Zim] [[Wre Wim] [-Wim Wre]] per sample, k ascending over
+// (part, channel).  The block matrix is never formed: -Wim is Wim with its sign bits flipped.
+struct ModeArgs {
+  const bf16 *Z;           // [mode][b][2][w]
+  const bf16 *Wre, *Wim;   // [mode][w][w]
+  bf16 *Y;                 // [b][j][part][kx][w]
+  const bf16 *dY;          // mode_grad: [mode][b][2][w]
+  float *dWre, *dWim;      // mode_grad: [mode][w][w]
+  int m, batch;
+};
+constexpr int MB = 32;   // samples per pass
+template <int W> constexpr size_t mode_smem() { return 2 * ((size_t)2 * W * (W + 8) + (size_t)MB * (2 * W + 8)); }
+
+template <int W>
+__device__ __forceinline__ void mode_load_z(bf16 *s, const bf16 *g, int rows)
+{
+  constexpr int LZ = 2 * W + 8;
+  copy_tile(s, LZ, g, 2 * W, rows, 2 * W, RT);
+  zero_rows(s, LZ, rows, MB, RT);
+}
+
+// TRANS: the adjoint (dZ = dY Wblk^T)
+template <int W, bool TRANS>
+__device__ __forceinline__ void mode_product(const bf16 *sZ, const bf16 *sRe, const bf16 *sIm, bf16 *Y, int mode, int m, int b0, int batch)
+{
+  constexpr int LW = W + 8, LZ = 2 * W + 8, NP = 2 * W / 16;   // column pairs of tiles
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+  const int j = mode / m, kx = mode - j * m;
+  for (int u = warp; u < NP * (MB / 16); u += RT / 32) {
+    const int mt = u & 1, n0 = (u >> 1) * 16, po = n0 / W, co = n0 - po * W;
+    if (b0 + mt * 16 >= batch) continue;
+    float acc[2][4] = {};
+#pragma unroll
+    for (int pi = 0; pi < 2; pi++) {
+      // block (pi, po) of the mixing matrix, or (po, pi) of its transpose
+      const bf16 *w = (pi == po) ? sRe : sIm;
+      const uint32_t flip = (pi != po && (TRANS ? po == 1 : pi == 1)) ? 0x80008000u : 0u;
+#pragma unroll
+      for (int k = 0; k < W; k += 16) {
+        uint32_t fa[4], fb[4];
+        frag_a(fa, sZ, LZ, mt * 16, pi * W + k);
+        if (TRANS) frag_bt(fb, w, LW, co, k);
+        else frag_b(fb, w, LW, co, k);
+#pragma unroll
+        for (int i = 0; i < 4; i++) fb[i] ^= flip;
+        mma_bf16(acc[0], fa, fb);
+        mma_bf16(acc[1], fa, fb + 2);
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < 2; t++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int b = b0 + mt * 16 + gid + 8 * h;
+        if (b < batch)
+          *reinterpret_cast<uint32_t *>(Y + ((((size_t)b * 2 * m + j) * 2 + po) * m + kx) * W + co + t * 8 + tig * 2) =
+              pack_bf16(acc[t][2 * h], acc[t][2 * h + 1]);
+      }
+  }
+}
+
+template <int W>
+__global__ void __launch_bounds__(RT) mode_mix(const ModeArgs a)
+{
+  constexpr int LW = W + 8;
+  extern __shared__ __align__(16) unsigned char rsm[];
+  bf16 *sRe = reinterpret_cast<bf16 *>(rsm), *sIm = sRe + W * LW, *sZ = sIm + W * LW;
+  const int mode = blockIdx.x;
+  copy_tile(sRe, LW, a.Wre + (size_t)mode * W * W, W, W, W, RT);
+  copy_tile(sIm, LW, a.Wim + (size_t)mode * W * W, W, W, W, RT);
+  for (int b0 = 0; b0 < a.batch; b0 += MB) {
+    if (b0) __syncthreads();
+    mode_load_z<W>(sZ, a.Z + ((size_t)mode * a.batch + b0) * 2 * W, min(MB, a.batch - b0));
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    mode_product<W, false>(sZ, sRe, sIm, a.Y, mode, a.m, b0, a.batch);
+  }
+}
+
+// The adjoint of the mixing (dZ, stored like Y) and the gradients of Wre and Wim of one mode:
+// with d = [Zre Zim]^T [dYre dYim], k over the samples, dWre = d(re,re) + d(im,im) and
+// dWim = d(re,im) - d(im,re).
+template <int W> constexpr size_t mode_grad_smem() { return 2 * ((size_t)2 * W * (W + 8) + (size_t)2 * MB * (2 * W + 8)); }
+
+template <int W>
+__global__ void __launch_bounds__(RT) mode_grad(const ModeArgs a)
+{
+  constexpr int LW = W + 8, LZ = 2 * W + 8, T = W / 16, U = (T * T + 7) / 8;
+  extern __shared__ __align__(16) unsigned char rsm[];
+  bf16 *sRe = reinterpret_cast<bf16 *>(rsm), *sIm = sRe + W * LW, *sZ = sIm + W * LW, *sY = sZ + MB * LZ;
+  const int mode = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+  copy_tile(sRe, LW, a.Wre + (size_t)mode * W * W, W, W, W, RT);
+  copy_tile(sIm, LW, a.Wim + (size_t)mode * W * W, W, W, W, RT);
+  float acc[U][4][2][4] = {};   // re-re, im-im, re-im, im-re
+  for (int b0 = 0; b0 < a.batch; b0 += MB) {
+    if (b0) __syncthreads();
+    const int rows = min(MB, a.batch - b0);
+    mode_load_z<W>(sZ, a.Z + ((size_t)mode * a.batch + b0) * 2 * W, rows);
+    mode_load_z<W>(sY, a.dY + ((size_t)mode * a.batch + b0) * 2 * W, rows);
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    mode_product<W, true>(sY, sRe, sIm, a.Y, mode, a.m, b0, a.batch);
+    for (int k = 0; k < rows; k += 16)
+#pragma unroll
+      for (int i = 0; i < U; i++) {
+        const int u = warp + 8 * i, ci = (u / T) * 16, co = (u % T) * 16;
+        if (u >= T * T) break;
+        uint32_t zr[4], zi[4], yr[4], yi[4];
+        frag_at(zr, sZ, LZ, ci, k);
+        frag_at(zi, sZ, LZ, W + ci, k);
+        frag_b(yr, sY, LZ, co, k);
+        frag_b(yi, sY, LZ, W + co, k);
+#pragma unroll
+        for (int t = 0; t < 2; t++) {
+          mma_bf16(acc[i][0][t], zr, yr + 2 * t);
+          mma_bf16(acc[i][1][t], zi, yi + 2 * t);
+          mma_bf16(acc[i][2][t], zr, yi + 2 * t);
+          mma_bf16(acc[i][3][t], zi, yr + 2 * t);
+        }
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < U; i++) {
+    const int u = warp + 8 * i, ci = (u / T) * 16, co = (u % T) * 16;
+    if (u >= T * T) break;
+#pragma unroll
+    for (int t = 0; t < 2; t++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const size_t o = ((size_t)mode * W + ci + gid + 8 * h) * W + co + t * 8 + tig * 2;
+        *reinterpret_cast<float2 *>(a.dWre + o) =
+            make_float2(acc[i][0][t][2 * h] + acc[i][1][t][2 * h], acc[i][0][t][2 * h + 1] + acc[i][1][t][2 * h + 1]);
+        *reinterpret_cast<float2 *>(a.dWim + o) =
+            make_float2(acc[i][2][t][2 * h] - acc[i][3][t][2 * h], acc[i][2][t][2 * h + 1] - acc[i][3][t][2 * h + 1]);
+      }
+  }
+}
+
+// ---- weight gradient of a 1x1 convolution: partial[chunk] (R x W) = X^T dY over kc pixels, k
+// ascending; X [pixels][R], dY [pixels][W]
+constexpr int WGK = 64, WGS = 3;   // pixels per stage, stages
+inline size_t wgrad_smem(int R, int W) { return 2 * (size_t)WGS * WGK * (R + 8 + W + 8); }
+
+template <int W>
+__global__ void __launch_bounds__(RT) weight_grad_partial(const bf16 *X, int R, const bf16 *dY, int kc, float *partial)
+{
+  constexpr int LW = W + 8, NP = W / 16, U = 2;   // 16 x 16 tiles, at most 4 x 4 over 8 warps
+  extern __shared__ __align__(16) unsigned char rsm[];
+  const int LR = R + 8, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+  const size_t p0 = (size_t)blockIdx.x * kc;
+  bf16 *st = reinterpret_cast<bf16 *>(rsm);
+  const int stage = WGK * (LR + LW), nst = (kc + WGK - 1) / WGK, units = (R / 16) * NP;
+  auto load = [&](int i) {
+    if (i < nst) {
+      bf16 *s = st + (i % WGS) * stage;
+      const int n = min(WGK, kc - i * WGK);
+      copy_tile(s, LR, X + (p0 + (size_t)i * WGK) * R, R, n, R, RT);
+      copy_tile(s + WGK * LR, LW, dY + (p0 + (size_t)i * WGK) * W, W, n, W, RT);
+    }
+    cp_async_commit();
+  };
+  for (int i = 0; i < WGS - 1; i++) load(i);
+  float acc[U][2][4] = {};
+  for (int i = 0; i < nst; i++) {
+    cp_async_wait<WGS - 2>();
+    __syncthreads();
+    load(i + WGS - 1);
+    const bf16 *sX = st + (i % WGS) * stage, *sY = sX + WGK * LR;
+    for (int k = 0; k < min(WGK, kc - i * WGK); k += 16)
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int t = warp + 8 * u;
+        if (t >= units) break;
+        uint32_t fa[4], fb[4];
+        frag_at(fa, sX, LR, (t / NP) * 16, k);
+        frag_b(fb, sY, LW, (t % NP) * 16, k);
+        mma_bf16(acc[u][0], fa, fb);
+        mma_bf16(acc[u][1], fa, fb + 2);
+      }
+  }
+  cp_async_wait<0>();
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const int t = warp + 8 * u;
+    if (t >= units) break;
+#pragma unroll
+    for (int c = 0; c < 2; c++)
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+        *reinterpret_cast<float2 *>(partial + ((size_t)blockIdx.x * R + (t / NP) * 16 + gid + 8 * h) * W + (t % NP) * 16 + c * 8 + tig * 2) =
+            make_float2(acc[u][c][2 * h], acc[u][c][2 * h + 1]);
+  }
+}
+
+}  // namespace nnk
