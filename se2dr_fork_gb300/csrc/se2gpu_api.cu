@@ -368,9 +368,9 @@ extern "C" void se2gpu_destroy(se2gpu_solver *h)
     dfree(h, h->pu[b]); dfree(h, h->pw[b]); dfree(h, h->pcu[b]); dfree(h, h->pcw[b]); dfree(h, h->rbuf[b]);
   }
   void *ptrs[] = {h->a64, h->rmass, h->Dx, h->Dy, h->f64_consts, h->src_xy, h->pa, h->pminv, h->mass_bad, h->err_dev, h->mass, h->lam, h->mu, h->J00, h->J11, h->iJ00, h->iJ11, h->D, h->wq,
-                  h->src_vals, h->Dd, h->iJ00d, h->iJ11d, h->stf_dev, h->traces, h->norm_part, h->src_elem,
-                  h->rec_node, h->rec_elem, h->rec_gll, h->scratch_u, h->scratch_f, h->tile_src_off,
-                  h->tile_src_idx, h->tile_rec_off, h->tile_rec_idx, h->cellc, h->tile_bounds};
+                  h->src_vals, h->Dd, h->iJ00d, h->iJ11d, h->stf_dev, h->traces, h->norm_part,
+                  h->rec_node, h->rec_elem, h->rec_gll, h->scratch_u, h->scratch_f, h->tile_src,
+                  h->tile_rec, h->cellc, h->tile_bounds};
   for (void *p : ptrs) dfree(h, p);
   if (h->stream) cudaStreamSynchronize(h->stream);   // the frees are done before the stream goes
   delete h->src_elem_h;
@@ -469,7 +469,7 @@ static int setup_f32_config(se2gpu_solver *h, int config, bool in_create = false
   const int te = ts.tex, P = h->p;
   const int ntx = (h->mx + te - 1) / te, nty = (h->my + te - 1) / te, ntiles = ntx * nty;
   // tile lists: a source or receiver element appears in every tile whose owned nodes it touches
-  auto build = [&](const std::vector<int> &elems, std::vector<int> &off, std::vector<int> &idx) {
+  auto build = [&](const std::vector<int> &elems, std::vector<int> &off, std::vector<int> &ent) {
     std::vector<std::vector<int>> per(ntiles);
     for (int q = 0; q < (int)elems.size(); q++) {
       const int ex = elems[q] % h->mx, ey = elems[q] / h->mx;
@@ -482,8 +482,12 @@ static int setup_f32_config(se2gpu_solver *h, int config, bool in_create = false
     }
     off.assign(ntiles + 1, 0);
     for (int t = 0; t < ntiles; t++) off[t + 1] = off[t] + (int)per[t].size();
-    idx.clear();
-    for (int t = 0; t < ntiles; t++) idx.insert(idx.end(), per[t].begin(), per[t].end());
+    ent.clear();
+    for (int t = 0; t < ntiles; t++)
+      for (int q : per[t]) {
+        const int e[4] = {q, elems[q] % h->mx * P, elems[q] / h->mx * P, 0};
+        ent.insert(ent.end(), e, e + 4);
+      }
   };
   std::vector<int> so, si, ro, ri;
   build(*h->src_elem_h, so, si);
@@ -493,20 +497,16 @@ static int setup_f32_config(se2gpu_solver *h, int config, bool in_create = false
     tb[4 * (size_t)t] = so[t]; tb[4 * (size_t)t + 1] = so[t + 1];
     tb[4 * (size_t)t + 2] = ro[t]; tb[4 * (size_t)t + 3] = ro[t + 1];
   }
-  dfree(h, h->tile_src_off); dfree(h, h->tile_src_idx); dfree(h, h->tile_rec_off); dfree(h, h->tile_rec_idx);
-  dfree(h, h->tile_bounds);
-  h->tile_src_off = h->tile_src_idx = h->tile_rec_off = h->tile_rec_idx = nullptr;
-  h->tile_bounds = nullptr;
+  dfree(h, h->tile_src); dfree(h, h->tile_rec); dfree(h, h->tile_bounds);
+  h->tile_src = h->tile_rec = h->tile_bounds = nullptr;
   int rc;
   if ((rc = upload_i(h, (int **)&h->tile_bounds, tb.data(), tb.size()))) return rc;
-  if ((rc = upload_i(h, &h->tile_src_off, so.data(), so.size()))) return rc;
-  if ((rc = upload_i(h, &h->tile_src_idx, si.data(), si.size()))) return rc;
-  if ((rc = upload_i(h, &h->tile_rec_off, ro.data(), ro.size()))) return rc;
-  if ((rc = upload_i(h, &h->tile_rec_idx, ri.data(), ri.size()))) return rc;
+  if ((rc = upload_i(h, (int **)&h->tile_src, si.data(), si.size()))) return rc;
+  if ((rc = upload_i(h, (int **)&h->tile_rec, ri.data(), ri.size()))) return rc;
   h->pconfig = config;
   h->pntx = ntx;
   h->pnty = nty;
-  h->pgrid = std::min(ntiles, std::max(1, se2p::occupancy(P, config, mode)) * h->nsm);
+  h->pgrid = std::min(ntiles + 1, std::max(1, se2p::occupancy(P, config, mode)) * h->nsm);
   return 0;
 }
 
@@ -595,7 +595,6 @@ extern "C" int se2gpu_create(const se2gpu_problem *P, int precision, int trace_c
   TRY(upload_d(h, &h->Dd, P->D, (size_t)npe));
   TRY(upload_d(h, &h->iJ00d, P->iJ00, (size_t)P->mx));
   TRY(upload_d(h, &h->iJ11d, P->iJ11, (size_t)P->my));
-  TRY(upload_i(h, &h->src_elem, P->src_elem, (size_t)P->nsrc));
   if (P->nsrc) TRY(upload(h, &h->src_vals, P->src_vals, (size_t)P->nsrc * 2 * npe));
   TRY(upload_i(h, &h->rec_node, P->rec_node, (size_t)P->nrec));
   TRY(upload_i(h, &h->rec_elem, P->rec_elem, (size_t)P->nrec));
@@ -832,12 +831,11 @@ static se2p::Params f32_params(se2gpu_solver *h)
   prm.iJ00 = (const float *)h->iJ00; prm.iJ11 = (const float *)h->iJ11;
   prm.dt = (float)h->dt; prm.half_dt = (float)(0.5 * h->dt);
   prm.dt_lo = (float)(h->dt - (double)prm.dt); prm.half_dt_lo = (float)(0.5 * h->dt - (double)prm.half_dt);
-  prm.nsrc = h->nsrc; prm.src_elem = h->src_elem; prm.src_vals = (const float *)h->src_vals;
+  prm.nsrc = h->nsrc; prm.src_vals = (const float *)h->src_vals;
   prm.nrec = h->nrec; prm.rec_elem = h->rec_elem; prm.rec_gll = h->rec_gll;
   prm.Dd = h->Dd; prm.iJ00d = h->iJ00d; prm.iJ11d = h->iJ11d;
   prm.err = h->err_dev;
-  prm.tile_src_off = h->tile_src_off; prm.tile_src_idx = h->tile_src_idx;
-  prm.tile_rec_off = h->tile_rec_off; prm.tile_rec_idx = h->tile_rec_idx;
+  prm.tile_src = h->tile_src; prm.tile_rec = h->tile_rec;
   prm.cellc = h->cellc; prm.tile_bounds = h->tile_bounds;
   return prm;
 }
@@ -914,7 +912,7 @@ static int advance_f32(se2gpu_solver *h, int nsteps)
     prm.record = h->pending_record ? 1 : 0;
     prm.trace_row = h->traces + (size_t)h->rows_written * 7 * h->nrec;
     h->launches++;
-    cudaError_t e = se2p::launch_step(h->p, h->pconfig, mode, h->maps[in], prm, h->pgrid, h->stream);
+    cudaError_t e = se2p::launch_step(h->p, h->pconfig, mode, h->maps[in], prm, h->pgrid, k > 0, h->stream);
     if (e != cudaSuccess) return fail(h, SE2GPU_ERR_CUDA, "step kernel: %s", cudaGetErrorString(e));
     if (h->pending_record) { h->rows_written++; h->pending_record = false; }
     h->cur = outb;

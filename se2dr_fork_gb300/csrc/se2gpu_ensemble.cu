@@ -62,6 +62,11 @@ struct se2gpu_ensemble {
   double *stf_h[2] = {nullptr, nullptr}, *tr_h[2] = {nullptr, nullptr};   // pinned host staging
   cudaEvent_t ev_h2d[2] = {nullptr, nullptr}, ev_d2h[2] = {nullptr, nullptr};
   cudaStream_t stream = nullptr, own_stream = nullptr;
+  // the launch chains of a block: chunk i of the ensemble runs on chain i % chains, chain 0 being
+  // the block's own stream; `fork` and `joins` order the others behind and before it
+  std::vector<cudaStream_t> side;
+  cudaEvent_t fork = nullptr;
+  std::vector<cudaEvent_t> joins;
   cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};   // [input buffer][slot]
   int *err_dev = nullptr;
   long launches = 0, replays = 0;
@@ -131,6 +136,9 @@ extern "C" void se2gpu_ensemble_destroy(se2gpu_ensemble *e)
   }
   cudaFree(e->err_dev);
   for (se2gpu_solver *h : e->sol) se2gpu_destroy(h);
+  for (cudaStream_t s : e->side) cudaStreamDestroy(s);
+  for (cudaEvent_t ev : e->joins) cudaEventDestroy(ev);
+  if (e->fork) cudaEventDestroy(e->fork);
   if (e->own_stream) cudaStreamDestroy(e->own_stream);
   delete e;
 }
@@ -204,6 +212,24 @@ static int build_group(se2gpu_ensemble *e, Group &g)
   g.nitems = (int)items.size();
   int rc = dput(e, &g.items, items.data(), items.size());
   if (rc) return rc;
+  return 0;
+}
+
+// streams and events of the launch chains: one chain per chunk, at most ENS_CHAINS
+constexpr int ENS_CHAINS = 8;
+static int make_chains(se2gpu_ensemble *e)
+{
+  int chunks = 0;
+  for (const Group &g : e->groups) chunks += (int)g.chunks.size();
+  if (!e->fork) ECK(e, cudaEventCreateWithFlags(&e->fork, cudaEventDisableTiming));
+  while ((int)e->side.size() < std::min(chunks, ENS_CHAINS) - 1) {
+    cudaStream_t s = nullptr;
+    cudaEvent_t ev = nullptr;
+    ECK(e, cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    e->side.push_back(s);
+    ECK(e, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    e->joins.push_back(ev);
+  }
   return 0;
 }
 
@@ -284,6 +310,7 @@ extern "C" int se2gpu_ensemble_create(const se2gpu_problem *shots, int nshots, i
     }
     TRY(build_group(e, g));
   }
+  TRY(make_chains(e));
 #undef TRY
   *out = e;
   return 0;
@@ -330,11 +357,20 @@ extern "C" int se2gpu_ensemble_tile_config(const se2gpu_ensemble *e, int p)
   return SE2GPU_ERR_ARG;
 }
 
-// the launches of one block of n <= K steps starting from input buffer `cur`, slot sl
+// The launches of one block of n <= K steps starting from input buffer `cur`, slot sl.  The
+// chunks are independent of one another, so each walks its steps on a chain of its own
+// (streams, or branches of the captured graph): while the last CTAs of one chunk's step
+// drain, another chunk's fill the SMs, and small groups run side by side.
 static int enqueue_block(se2gpu_ensemble *e, int cur, int sl, int n, cudaStream_t st)
 {
+  const int chains = 1 + (int)e->side.size();
+  if (chains > 1) {
+    ECK(e, cudaEventRecord(e->fork, st));
+    for (cudaStream_t s : e->side) ECK(e, cudaStreamWaitEvent(s, e->fork, 0));
+  }
   for (int k = 0; k < n; k++) {
     const int cin = cur ^ (k & 1);
+    int chunk = 0;
     for (Group &g : e->groups)
       for (const Chunk &ch : g.chunks) {
         static thread_local se2p::BatchArgs ba;   // 28 KB: kept off the stack
@@ -346,10 +382,15 @@ static int enqueue_block(se2gpu_ensemble *e, int cur, int sl, int n, cudaStream_
         ba.write_a = (k == n - 1) ? 1 : 0;
         ba.err = e->err_dev;
         memcpy(ba.shots, g.htab[cin][sl].data() + ch.first, sizeof(se2p::Params) * ch.nshots);
-        cudaError_t r = se2p::launch_batch(g.p, g.config, e->kahan, ba, ch.grid, st);
+        const int c = chunk++ % chains;
+        cudaError_t r = se2p::launch_batch(g.p, g.config, e->kahan, ba, ch.grid, k > 0, c ? e->side[c - 1] : st);
         if (r != cudaSuccess)
           return efail(e, SE2GPU_ERR_CUDA, "batched step kernel (degree %d): %s", g.p, cudaGetErrorString(r));
       }
+  }
+  for (size_t s = 0; s < e->side.size(); s++) {
+    ECK(e, cudaEventRecord(e->joins[s], e->side[s]));
+    ECK(e, cudaStreamWaitEvent(st, e->joins[s], 0));
   }
   for (Group &g : e->groups) {
     cudaError_t r = se2p::launch_record_batch(g.p, g.tab[cur][sl], (int)g.shots.size(), n - 1, st);

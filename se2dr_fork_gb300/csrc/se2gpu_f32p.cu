@@ -3,6 +3,8 @@
 // their host-side helpers (tensor maps, constant tables, norms of the leapfrog state).
 #include <cudaTypedefs.h>
 
+#include <algorithm>
+
 #include "se2gpu_persist.cuh"
 #include "se2gpu_persist_launch.h"
 
@@ -139,11 +141,28 @@ int occupancy(int p, int config, int mode, bool batch)
     cudaGetLastError();
     return 1;
   }
-  return n;
+  return std::min(n, 3);   // the persistent grid's CTAs per SM: what the tile configurations are sized for
+}
+
+// a launch that may begin (its set-up before cudaGridDependencySynchronize) while the launch
+// before it on the stream drains: about 2 us of every short step
+static cudaError_t launch(const void *fn, int grid, int threads, void **args, size_t smem, bool dependent, cudaStream_t st)
+{
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = dependent ? 1 : 0;
+  return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
 cudaError_t launch_step(int p, int config, int mode, const CUtensorMap *maps, const Params &prm, int grid,
-                        cudaStream_t st)
+                        bool dependent, cudaStream_t st)
 {
   const Entry *e = find(p, config);
   if (!e) return cudaErrorInvalidValue;
@@ -154,16 +173,16 @@ cudaError_t launch_step(int p, int config, int mode, const CUtensorMap *maps, co
   Params pc = prm;
   CUtensorMap m0 = maps[0], m1 = maps[1], m2 = maps[2], m3 = maps[3], m4 = maps[4], m5 = maps[5];
   void *args[] = {&m0, &m1, &m2, &m3, &m4, &m5, &pc};
-  return cudaLaunchKernel(fn, dim3(grid), dim3(e->nt), args, smem, st);
+  return launch(fn, grid, e->nt, args, smem, dependent, st);
 }
 
-cudaError_t launch_batch(int p, int config, bool kahan, const BatchArgs &ba, int grid, cudaStream_t st)
+cudaError_t launch_batch(int p, int config, bool kahan, const BatchArgs &ba, int grid, bool dependent, cudaStream_t st)
 {
   const Entry *e = find(p, config);
   if (!e) return cudaErrorInvalidValue;
   BatchArgs a = ba;
   void *args[] = {&a};
-  return cudaLaunchKernel(e->bfn[kahan ? 1 : 0], dim3(grid), dim3(e->nt), args, e->bsmem[kahan ? 1 : 0], st);
+  return launch(e->bfn[kahan ? 1 : 0], grid, e->nt, args, e->bsmem[kahan ? 1 : 0], dependent, st);
 }
 
 template <int P>

@@ -37,14 +37,14 @@ struct se2gpu_solver {
   float4 *cellc;                 // plain and Kahan modes: (lam detJ, mu detJ, d xi/dx, d eta/dy) per cell
   int4 *tile_bounds;             // per tile: source and receiver list bounds
   int pgrid, pconfig, pntx, pnty;
-  int *tile_src_off, *tile_src_idx, *tile_rec_off, *tile_rec_idx;
+  int4 *tile_src, *tile_rec;     // per-tile list entries
   std::vector<int> *src_elem_h, *rec_elem_h;
   int *err_dev;
   // tables in compute precision
   void *mass, *lam, *mu, *J00, *J11, *iJ00, *iJ11, *D, *wq, *src_vals;
   double *Dd, *iJ00d, *iJ11d, *stf_dev, *traces, *norm_part;
   int stf_cap;
-  int *src_elem, *rec_node, *rec_elem, *rec_gll;
+  int *rec_node, *rec_elem, *rec_gll;
   void *scratch_u, *scratch_f;   // assemble_linear_form staging (packed)
   long launches;
   char err[512];

@@ -336,6 +336,16 @@ __device__ void sample_rows(const Params &prm, const float *rbuf_in, double *tra
   }
 }
 
+// an entry of a tile's source or receiver list; its loads stay inside the (rarely run, not
+// unrolled) loops, where they hold no registers of the node phase
+__device__ __forceinline__ int4 list_entry(const int4 *p)
+{
+  int4 v;
+  asm volatile("ld.global.nc.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+#define SE2P_COLD _Pragma("unroll 1")
+
 // the pointers of one step of a tile's shot: this step's source values, the receiver
 // side buffer it writes and the optional a_k output (null: not written)
 struct StepPtrs {
@@ -545,9 +555,9 @@ __device__ __forceinline__ bool tile_body(const Params &prm, const StepPtrs stp,
         if (lft && in_y) { const float2 fe = X1[own - XS + P]; fx += fe.x; fy += fe.y; }
         if (in_x && in_y) { const float2 fe = X1[own]; fx += fe.x; fy += fe.y; }
       }
-      for (int q = s0; q < s1; q++) {
-        const int sidx = prm.tile_src_idx[q], se = prm.src_elem[sidx], sx = se % prm.mx, sy = se / prm.mx;
-        const int a = X - sx * P, bb = Y - sy * P;
+      SE2P_COLD for (int q = s0; q < s1; q++) {
+        const int4 ent = list_entry(prm.tile_src + q);
+        const int sidx = ent.x, a = X - ent.y, bb = Y - ent.z;
         if (a >= 0 && a <= P && bb >= 0 && bb <= P) {
           const float val = (float)stp.stf[sidx];
           const float *sv = prm.src_vals + (size_t)sidx * 2 * NPE + 2 * (a + bb * N1);
@@ -560,9 +570,9 @@ __device__ __forceinline__ bool tile_body(const Params &prm, const StepPtrs stp,
       const int oi = oy * OBW + (X - b.OXa);
       float2 u = rU[ri], w = oW[oi];
       float2 cu = KAHAN ? rCU[ri] : make_float2(0.f, 0.f), cw = KAHAN ? oCW[oi] : make_float2(0.f, 0.f);
-      for (int q = r0; q < r1; q++) {
-        const int r = prm.tile_rec_idx[q], re = prm.rec_elem[r], rx = re % prm.mx, ry = re / prm.mx;
-        const int a = X - rx * P, bb = Y - ry * P;
+      SE2P_COLD for (int q = r0; q < r1; q++) {
+        const int4 ent = list_entry(prm.tile_rec + q);
+        const int r = ent.x, a = X - ent.y, bb = Y - ent.z;
         if (a >= 0 && a <= P && bb >= 0 && bb <= P) {
           float *rb = stp.rbuf_out + ((size_t)r * NPE + a + bb * N1) * 6;
           rb[0] = u.x; rb[1] = u.y; rb[2] = fmaf(half_dt, acc.x, w.x); rb[3] = fmaf(half_dt, acc.y, w.y);
@@ -609,9 +619,9 @@ __device__ __forceinline__ bool tile_body(const Params &prm, const StepPtrs stp,
       if (bot && in_x) { const float2 fe = X1[own - NEX * XS + P * RS]; f[h][0] += fe.x; f[h][1] += fe.y; }
       if (lft && in_y) { const float2 fe = X1[own - XS + P]; f[h][0] += fe.x; f[h][1] += fe.y; }
       if (in_x && in_y) { const float2 fe = X1[own]; f[h][0] += fe.x; f[h][1] += fe.y; }
-      for (int q = s0; q < s1; q++) {
-        const int sidx = prm.tile_src_idx[q], se = prm.src_elem[sidx], sx = se % prm.mx, sy = se / prm.mx;
-        const int a = X - sx * P, bb = Y - sy * P;
+      SE2P_COLD for (int q = s0; q < s1; q++) {
+        const int4 ent = list_entry(prm.tile_src + q);
+        const int sidx = ent.x, a = X - ent.y, bb = Y - ent.z;
         if (a >= 0 && a <= P && bb >= 0 && bb <= P) {
           const float val = (float)stp.stf[sidx];
           const float *sv = prm.src_vals + (size_t)sidx * 2 * NPE + 2 * (a + bb * N1);
@@ -634,9 +644,9 @@ __device__ __forceinline__ bool tile_body(const Params &prm, const StepPtrs stp,
         const int X = XA + h;
         const float ux = h ? u.z : u.x, uy = h ? u.w : u.y, wx = h ? w.z : w.x, wy = h ? w.w : w.y;
         const float ax = h ? acc.z : acc.x, ay = h ? acc.w : acc.y;
-        for (int q = r0; q < r1; q++) {
-          const int r = prm.tile_rec_idx[q], re = prm.rec_elem[r], rx = re % prm.mx, ry = re / prm.mx;
-          const int a = X - rx * P, bb = Y - ry * P;
+        SE2P_COLD for (int q = r0; q < r1; q++) {
+          const int4 ent = list_entry(prm.tile_rec + q);
+          const int r = ent.x, a = X - ent.y, bb = Y - ent.z;
           if (a >= 0 && a <= P && bb >= 0 && bb <= P) {
             float *rb = stp.rbuf_out + ((size_t)r * NPE + a + bb * N1) * 6;
             rb[0] = ux; rb[1] = uy; rb[2] = fmaf(half_dt, ax, wx); rb[3] = fmaf(half_dt, ay, wy);
@@ -768,8 +778,8 @@ __device__ __forceinline__ bool tile_body_df(const Params &prm, const StepPtrs s
     iy = tf{prm.iJ11[ey], prm.iJ11[prm.my + ey]};
     detJ = tf_mul(tf{prm.J00[ex], prm.J00[prm.mx + ex]}, tf{prm.J11[ey], prm.J11[prm.my + ey]});
   }
-  const int s0 = prm.tile_src_off[t], s1 = prm.tile_src_off[t + 1];
-  const int r0 = prm.tile_rec_off[t], r1 = prm.tile_rec_off[t + 1];
+  const int4 bnd = prm.tile_bounds[t];
+  const int s0 = bnd.x, s1 = bnd.y, r0 = bnd.z, r1 = bnd.w;
   // node phase: single nodes strided by NT; 1/M (both parts) loaded before the wait
   constexpr int NOWN = G::OWM * G::OWM;
   constexpr int MAXS = (NOWN + NT - 1) / NT;
@@ -925,9 +935,9 @@ __device__ __forceinline__ bool tile_body_df(const Params &prm, const StepPtrs s
       if (lft && in_y) add(X1[own - XS + P]);
       if (in_x && in_y) add(X1[own]);
     }
-    for (int q = s0; q < s1; q++) {
-      const int sidx = prm.tile_src_idx[q], se = prm.src_elem[sidx], sx = se % prm.mx, sy = se / prm.mx;
-      const int a = X - sx * P, bb = Y - sy * P;
+    SE2P_COLD for (int q = s0; q < s1; q++) {
+      const int4 ent = list_entry(prm.tile_src + q);
+      const int sidx = ent.x, a = X - ent.y, bb = Y - ent.z;
       if (a >= 0 && a <= P && bb >= 0 && bb <= P) {
         const tf val = tf_from_double(stp.stf[sidx]);
         const size_t vi = (size_t)sidx * 2 * NPE + 2 * (a + bb * N1);
@@ -940,9 +950,9 @@ __device__ __forceinline__ bool tile_body_df(const Params &prm, const StepPtrs s
     const int oi = oy * OBW + (X - b.OXa);
     const float2 u = rU[ri], cu = rCU[ri], w = oW[oi], cw = oCW[oi];
     const tf ux{u.x, -cu.x}, uy{u.y, -cu.y}, wx{w.x, -cw.x}, wy{w.y, -cw.y};
-    for (int q = r0; q < r1; q++) {
-      const int r = prm.tile_rec_idx[q], re = prm.rec_elem[r], rx = re % prm.mx, ry = re / prm.mx;
-      const int a = X - rx * P, bb = Y - ry * P;
+    SE2P_COLD for (int q = r0; q < r1; q++) {
+      const int4 ent = list_entry(prm.tile_rec + q);
+      const int r = ent.x, a = X - ent.y, bb = Y - ent.z;
       if (a >= 0 && a <= P && bb >= 0 && bb <= P) {
         float *rb = stp.rbuf_out + ((size_t)r * NPE + a + bb * N1) * 12;
         const tf vx = tf_add(wx, tf_mul(hdt, ax)), vy = tf_add(wy, tf_mul(hdt, ay));
@@ -1026,7 +1036,8 @@ persist_step(const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ C
     if (AC) { prefetch_map(&tm_c); prefetch_map(&tm_m); }
   }
   __syncthreads();
-  if (blockIdx.x == 0 && prm.record) sample_rows<P, DF>(prm, prm.rbuf_in, prm.trace_row);
+  // (programmatic dependent launch: the set-up above runs while the launch before this one drains)
+  cudaGridDependencySynchronize();
 
   int el, j;
   bool valid;
@@ -1088,6 +1099,9 @@ persist_step(const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ C
     tx = txn;
     ty = tyn;
   }
+  // receiver rows of the previous step, by the CTA with the fewest tiles (none, where the grid
+  // has room): at the head of CTA 0 they delayed its first tile by about 2 us a step
+  if (prm.record && blockIdx.x == gridDim.x - 1) sample_rows<P, DF>(prm, prm.rbuf_in, prm.trace_row);
 }
 
 // Many independent shots of one degree in one persistent launch.  The CTAs walk
@@ -1131,12 +1145,7 @@ persist_batch(const __grid_constant__ BatchArgs ba)
     fence_barrier_init();
   }
   __syncthreads();
-  // receivers of the previous step of this block, one CTA per shot
-  if (ba.kblk > 0)
-    for (int sh = blockIdx.x; sh < ba.nshots; sh += gridDim.x) {
-      const Params &q = ba.shots[sh];
-      if (q.nrec > 0) sample_rows<P>(q, batch_rbuf(q, ba.kblk - 1), q.trace_row + (size_t)(ba.kblk - 1) * 7 * q.nrec);
-    }
+  cudaGridDependencySynchronize();
 
   int el, j;
   bool valid;
@@ -1199,6 +1208,13 @@ persist_batch(const __grid_constant__ BatchArgs ba)
     cur = nxt;
     nxt = nn;
   }
+  // receivers of the previous step of this block, one CTA per shot, from the CTAs with the
+  // fewest tiles on
+  if (ba.kblk > 0)
+    for (int sh = gridDim.x - 1 - blockIdx.x; sh < ba.nshots; sh += gridDim.x) {
+      const Params &q = ba.shots[sh];
+      if (q.nrec > 0) sample_rows<P>(q, batch_rbuf(q, ba.kblk - 1), q.trace_row + (size_t)(ba.kblk - 1) * 7 * q.nrec);
+    }
 }
 
 // receivers of the last step (kblk) of a block of batched steps, one CTA per shot

@@ -48,8 +48,9 @@ int config_shape(int p, int config, int mode, TileShape *s);
 cudaError_t prepare(int p, int config, int mode);                     // dynamic shared-memory limit
 int occupancy(int p, int config, int mode, bool batch = false);       // resident CTAs per SM
 // maps: region u, region cu, owned w, owned cw of the input state, cell constants, 1/M
+// dependent: the launch may begin while the step launched before it on the stream drains
 cudaError_t launch_step(int p, int config, int mode, const CUtensorMap *maps, const Params &prm, int grid,
-                        cudaStream_t st);
+                        bool dependent, cudaStream_t st);
 cudaError_t launch_record(int p, const Params &prm, cudaStream_t st, bool df = false);
 
 // the two-float kernels (their own translation unit, with its own constant tables)
@@ -58,7 +59,7 @@ const void *df_kernel(int p, int config, size_t *smem);
 cudaError_t df_launch_record(int p, const Params &prm, cudaStream_t st);
 // batched step of many shots of degree p (tables in device memory), and the
 // receiver rows of a block's last step
-cudaError_t launch_batch(int p, int config, bool kahan, const BatchArgs &ba, int grid, cudaStream_t st);
+cudaError_t launch_batch(int p, int config, bool kahan, const BatchArgs &ba, int grid, bool dependent, cudaStream_t st);
 cudaError_t launch_record_batch(int p, const Params *shots, int nshots, int kblk, cudaStream_t st);
 int make_map(CUtensorMap *map, void *base, int nx, int ny, int pitch, int bw, int bh);      // float2 nodes
 int make_map_f32(CUtensorMap *map, void *base, int nx, int ny, int pitch, int bw, int bh);  // float nodes

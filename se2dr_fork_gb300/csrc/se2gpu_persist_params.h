@@ -25,7 +25,6 @@ struct Params {
   float dt, half_dt;
   float dt_lo, half_dt_lo;         // two-float mode: dt = dt + dt_lo, dt/2 = half_dt + half_dt_lo
   int nsrc;
-  const int *src_elem;
   const float *src_vals;           // [nsrc][2*npe]
   const double *stf;               // this step's values per source
   // receivers
@@ -39,9 +38,11 @@ struct Params {
   const double *Dd, *iJ00d, *iJ11d;
   double *trace_row;
   int *err;                        // error flag (bounded waits)
-  // per-tile lists (CSR over tiles) of the sources and receivers whose element
-  // touches the tile's owned nodes, built on the host
-  const int *tile_src_off, *tile_src_idx, *tile_rec_off, *tile_rec_idx;
+  // per-tile lists of the sources and receivers whose element touches the tile's owned
+  // nodes, built on the host: (index, first node column, first node row of the element, 0) --
+  // one load per entry (an index into the element table cost two dependent loads per entry
+  // and node)
+  const int4 *tile_src, *tile_rec;
   // per tile: (first source, end of sources, first receiver, end of receivers) in the lists
   const int4 *tile_bounds;
 };
