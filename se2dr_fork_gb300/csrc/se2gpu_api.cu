@@ -701,7 +701,7 @@ extern "C" int se2gpu_create(const se2gpu_problem *P, int precision, int trace_c
       if (e != cudaSuccess) { fail(h, SE2GPU_ERR_CUDA, "constant tables: %s", cudaGetErrorString(e)); TRY(SE2GPU_ERR_CUDA); }
       h->src_elem_h = new std::vector<int>(P->src_elem, P->src_elem + P->nsrc);
       h->rec_elem_h = new std::vector<int>(P->rec_elem, P->rec_elem + P->nrec);
-      TRY(setup_f32_config(h, df ? 0 : se2p::default_config(P->p), true));
+      TRY(setup_f32_config(h, se2p::default_config(P->p, pmode(h), P->mx, P->my, h->nsm), true));
     }
     for (cudaEvent_t &ev : h->side_done) {
       const cudaError_t e = cudaStreamWaitEvent(h->stream, ev, 0);

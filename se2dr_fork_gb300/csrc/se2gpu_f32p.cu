@@ -73,10 +73,13 @@ static const Entry *find(int p, int config)
   return nullptr;
 }
 
-// the configuration a handle starts with: per degree the one the autotuner measured
-// fastest on GB300 at about 16M nodes (and, at degree 4, at the 2048^2 workload)
-int default_config(int p)
+// the configuration a handle starts with.  Plain and Kahan: per degree the one the autotuner
+// measured fastest on GB300 at about 16M nodes (and, at degree 4, at the 2048^2 workload).
+// Two-float: 0, and at degree 7 its 5 x 5 tiles once they reach every SM (301 against 336 us
+// at 2.5M nodes, 43 against 47 at 262000; 26 against 19 at 20000)
+int default_config(int p, int mode, int mx, int my, int nsm)
 {
+  if (mode == MODE_DF) return (p == 7 && (long)((mx + 4) / 5) * ((my + 4) / 5) >= nsm) ? 1 : 0;
   static const int best[8] = {2, 0, 2, 1, 2, 0, 2, 1};
   return (p >= 1 && p <= 8 && best[p - 1] < num_configs(p)) ? best[p - 1] : 0;
 }
