@@ -121,6 +121,23 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity)
 // ---------------------------------------------------------------- geometry
 __host__ __device__ constexpr int round_up(int x, int m) { return (x + m - 1) / m * m; }
 
+// Exchange buffers of the plain and Kahan tile body: element stride XS and the stride RS of an
+// element's rows (point (a, b) at a + b RS), in float2.  Chosen with a count of the
+// wavefronts of every access of a tile (8-byte accesses, 16 lanes at a time, 16 bank pairs;
+// columns have stride 1 over an element's lines, rows RS), per degree the fewest that keep the
+// resident CTAs: against rows of p + 1 with a pad per element, 24 % fewer exchange wavefronts at
+// degree 1, 8 % at 2, 28 % at 3, 10 % at 4, 45 % at 5, 22 % at 6, 58 % at 7, 6 % at 8.
+// Measured at 5M nodes, Kahan, us per step: degree 1 138 -> 129, 2 103 -> 100, 3 89 -> 84,
+// 5 90 -> 85, 6 89 -> 85, 7 111 -> 98 (the two-float body keeps Geo's XS).
+template <int P, bool KAHAN>
+struct Xch {
+  // plain degree 5 and 6: the widest layout that leaves three CTAs per SM
+  static constexpr int RS = (P == 1) ? 3 : (P == 2) ? 4 : (P == 3) ? 5 : (P == 4) ? 6 : (P == 5) ? (KAHAN ? 9 : 7)
+                          : (P == 6) ? (KAHAN ? 10 : 9) : (P == 7) ? 9 : 10;
+  static constexpr int XS = (P == 1) ? 6 : (P == 2) ? 19 : (P == 3) ? 20 : (P == 4) ? 37 : (P == 5) ? (KAHAN ? 54 : 42)
+                          : (P == 6) ? (KAHAN ? 71 : 63) : (P == 7) ? 72 : 89;
+};
+
 template <int P, int TE>
 struct Geo {
   static constexpr int N1 = P + 1, NPE = N1 * N1;
@@ -129,12 +146,6 @@ struct Geo {
   // element would start on bank 0; pads chosen with a wavefront model of the kernel's
   // accesses)
   static constexpr int XS = NPE + (P == 1 ? 2 : P == 3 ? 3 : P == 6 ? 6 : P == 7 ? 7 : P == 8 ? 8 : 0);
-  // the plain and Kahan tile body's exchange buffers: element stride XSK and the stride RS of
-  // an element's rows (point (a, b) at a + b RS).  At degree 4 rows of 6 in elements of 37
-  // float2: the same wavefront count gives 9-10 % fewer exchange-buffer wavefronts than
-  // rows of 5 in elements of 25 for 6x6, 7x7 and 8x8 tiles (the two-float body keeps XS)
-  static constexpr int RS = (P == 4) ? 6 : N1;
-  static constexpr int XSK = (P == 4) ? 37 : XS;
   static constexpr int NEX = TE + 1, NE = NEX * NEX;      // elements incl. halo
   static constexpr int ITEMS = NE * N1;                   // (element, line) work items
   // warp-aligned mapping: EPW whole elements per warp (their N1 lines in consecutive
@@ -181,7 +192,7 @@ struct Layout {
   static constexpr size_t STAGE = REG * (KAHAN ? 2 : 1) + CELLB;
   static constexpr size_t OWNB = OWN * (KAHAN ? 2 : 1) + MINVB + BNDB;
   // exchange buffer: float2 per point, float4 (two-float x, y) in the two-float mode
-  static constexpr size_t XCH = al128(DF ? sizeof(float4) * G::NE * G::XS : sizeof(float2) * G::NE * G::XSK);
+  static constexpr size_t XCH = al128(DF ? sizeof(float4) * G::NE * G::XS : sizeof(float2) * G::NE * Xch<P, KAHAN>::XS);
   static constexpr size_t MISC = 64;
   static constexpr size_t TOTAL = 2 * STAGE + NOB * OWNB + 2 * XCH + MISC;
   static constexpr size_t BATCH_TOTAL = TOTAL;   // the batched kernel's shot parameters are a kernel parameter
@@ -366,7 +377,7 @@ __device__ __forceinline__ bool tile_body(const Params &prm, const StepPtrs stp,
 {
   typedef Geo<P, TE> G;
   typedef Layout<P, TE, KAHAN, 1, false, AC> L;
-  constexpr int N1 = G::N1, NPE = G::NPE, NEX = G::NEX, BXW = G::BXW, OBW = G::OBW, XS = G::XSK, RS = G::RS;
+  constexpr int N1 = G::N1, NPE = G::NPE, NEX = G::NEX, BXW = G::BXW, OBW = G::OBW, XS = Xch<P, KAHAN>::XS, RS = Xch<P, KAHAN>::RS;
   const float *D = c_D[P - 1];
   const float *W = c_w[P - 1];
   const TileBox b = tile_box<P, TE>(prm, tx, ty);
