@@ -235,20 +235,37 @@ __global__ void k_mse(const float *out, const float *target, long n, double *par
   if (threadIdx.x == 0) partial[blockIdx.x] = s[0];
 }
 
-// (pb: the BF16 operand copy of the parameters)
+__device__ __forceinline__ float adam_1(float p, float g, float &m, float &v, float lr, float b1, float b2, float eps, float wd,
+                                        float c1, float c2)
+{
+  // (the roundings are spelled out: they decide which operand copies change)
+  m = __fmaf_rn(1.f - b1, g, __fmul_rn(b1, m));
+  v = __fmaf_rn(__fmul_rn(1.f - b2, g), g, __fmul_rn(b2, v));
+  const float mh = m / c1, vh = v / c2;
+  return __fmaf_rn(-lr, __fmaf_rn(wd, p, mh / (sqrtf(vh) + eps)), p);
+}
+
+// four parameters a thread (16-byte accesses); pb: the BF16 operand copy of the parameters
 __global__ void k_adam(float *p, const float *g, float *m, float *v, bf16 *pb, long n, float lr, float b1, float b2,
                        float eps, float wd, float c1, float c2)
 {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.f - b1) * gi;
-    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float mh = mi / c1, vh = vi / c2;
-    const float pi = p[i] - lr * (mh / (sqrtf(vh) + eps) + wd * p[i]);
-    p[i] = pi;
-    pb[i] = __float2bfloat16(pi);
+  const long i = 4 * (blockIdx.x * (long)blockDim.x + threadIdx.x);
+  if (i + 4 <= n) {
+    float4 P = *reinterpret_cast<float4 *>(p + i), M = *reinterpret_cast<float4 *>(m + i), V = *reinterpret_cast<float4 *>(v + i);
+    const float4 G = *reinterpret_cast<const float4 *>(g + i);
+    P.x = adam_1(P.x, G.x, M.x, V.x, lr, b1, b2, eps, wd, c1, c2);
+    P.y = adam_1(P.y, G.y, M.y, V.y, lr, b1, b2, eps, wd, c1, c2);
+    P.z = adam_1(P.z, G.z, M.z, V.z, lr, b1, b2, eps, wd, c1, c2);
+    P.w = adam_1(P.w, G.w, M.w, V.w, lr, b1, b2, eps, wd, c1, c2);
+    *reinterpret_cast<float4 *>(p + i) = P;
+    *reinterpret_cast<float4 *>(m + i) = M;
+    *reinterpret_cast<float4 *>(v + i) = V;
+    *reinterpret_cast<uint2 *>(pb + i) = make_uint2(nnk::pack_bf16(P.x, P.y), nnk::pack_bf16(P.z, P.w));
+  } else {
+    for (long k = i; k < n; k++) {
+      p[k] = adam_1(p[k], g[k], m[k], v[k], lr, b1, b2, eps, wd, c1, c2);
+      pb[k] = __float2bfloat16(p[k]);
+    }
   }
 }
 
@@ -257,6 +274,7 @@ __global__ void k_build_inputs(const float *mat, const float *src, const int *id
                                float inv2s2, bf16 *x)
 {
   const long n = (long)B * ny * nx;
+  const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0;   // 16-byte stores: 51 -> 8 us for a batch of 32
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     const int cx = (int)(i % nx), cy = (int)((i / nx) % ny), b = (int)(i / ((long)nx * ny));
     const long s = idx[b];
@@ -271,7 +289,12 @@ __global__ void k_build_inputs(const float *mat, const float *src, const int *id
     ch[4] = (2.f * cx + 1.f) / nx - 1.f;
     ch[5] = (2.f * cy + 1.f) / ny - 1.f;
     bf16 *o = x + i * cin;
-    for (int c = 0; c < cin; c++) o[c] = __float2bfloat16(c < 6 ? ch[c] : 0.f);
+    if (vec) {   // (cin is a multiple of 16)
+      *reinterpret_cast<uint4 *>(o) = make_uint4(nnk::pack_bf16(ch[0], ch[1]), nnk::pack_bf16(ch[2], ch[3]), nnk::pack_bf16(ch[4], ch[5]), 0u);
+      for (int c = 8; c < cin; c += 8) *reinterpret_cast<uint4 *>(o + c) = make_uint4(0u, 0u, 0u, 0u);
+    } else {
+      for (int c = 0; c < cin; c++) o[c] = __float2bfloat16(c < 6 ? ch[c] : 0.f);
+    }
   }
 }
 
@@ -309,7 +332,7 @@ struct se2nn {
   bf16 *S = nullptr, *Xf = nullptr, *Z = nullptr, *Yp = nullptr, *Y = nullptr, *Yy = nullptr, *dZp = nullptr;
   bf16 *D0 = nullptr, *D1pre = nullptr, *D1 = nullptr, *dpred = nullptr;
   bf16 *dHa = nullptr, *dHb = nullptr, *dA = nullptr, *dD1 = nullptr, *dD0 = nullptr;
-  float *out = nullptr, *partial = nullptr, *dblk = nullptr;
+  float *out = nullptr, *partial = nullptr, *colpart = nullptr, *decpart = nullptr, *dblk = nullptr;
   double *lpart = nullptr;
   long partial_n = 0;
   int split = 1, nsub = 1;
@@ -609,7 +632,7 @@ bool fused_shape(const se2nn *h)
 {
   const se2nn_config &c = h->c;
   return (h->w == 16 || h->w == 32 || h->w == 48 || h->w == 64) && c.cin <= 64 && c.nx % 16 == 0 &&
-         c.nx <= nnk::RNX && c.ny % 8 == 0 && c.ny <= nnk::RNY && h->m <= nnk::RM;
+         c.nx <= nnk::RNX && c.ny % 8 == 0 && c.ny <= nnk::RNY && h->m <= nnk::RM && c.nrec <= nnk::RREC;
 }
 bool fused_ok(const se2nn *h, const void *x)
 {
@@ -648,6 +671,8 @@ int fused_setup_w(se2nn *h)
   if (e == cudaSuccess) e = allow_smem(nnk::mode_mix<W>, nnk::mode_smem<W>());
   if (e == cudaSuccess) e = allow_smem(nnk::mode_grad<W>, nnk::mode_grad_smem<W>());
   if (e == cudaSuccess) e = allow_smem(nnk::weight_grad_partial<W>, nnk::wgrad_smem(64, W));
+  if (e == cudaSuccess) e = allow_smem(nnk::dec_fwd<W>, nnk::dec_fwd_smem<W>(nnk::DH));
+  if (e == cudaSuccess) e = allow_smem(nnk::dec_bwd<W>, nnk::dec_bwd_smem<W>(nnk::DH));
   NCK(h, e);
   return 0;
 }
@@ -687,7 +712,7 @@ nnk::RowArgs row_args(se2nn *h, int B)
 int y_analysis(se2nn *h, const bf16 *spec, bf16 *Zp, int B)
 {
   const size_t smem = nnk::y_analysis_smem(h->c.ny);
-  nnk::y_analysis<<<dim3((h->m * h->w + 63) / 64, B), 128, smem, h->stream>>>(nnk::YArgs{h->My, spec, Zp, h->c.ny, h->m, h->w, B});
+  nnk::y_analysis<<<dim3((h->m * h->w + nnk::YN - 1) / nnk::YN, B), nnk::RT, smem, h->stream>>>(nnk::YArgs{h->My, spec, Zp, h->c.ny, h->m, h->w, B});
   NCK(h, cudaGetLastError());
   return 0;
 }
@@ -695,7 +720,7 @@ int y_analysis(se2nn *h, const bf16 *spec, bf16 *Zp, int B)
 int y_synthesis(se2nn *h, const bf16 *Y, bf16 *spec, int B)
 {
   const size_t smem = nnk::y_synthesis_smem(h->c.ny);
-  nnk::y_synthesis<<<dim3((h->m * h->w + 63) / 64, B), 256, smem, h->stream>>>(nnk::YArgs{h->Myinv, Y, spec, h->c.ny, h->m, h->w, B});
+  nnk::y_synthesis<<<dim3((h->m * h->w + nnk::YN - 1) / nnk::YN, B), nnk::RT, smem, h->stream>>>(nnk::YArgs{h->Myinv, Y, spec, h->c.ny, h->m, h->w, B});
   NCK(h, cudaGetLastError());
   return 0;
 }
@@ -762,13 +787,18 @@ int mode_grad(se2nn *h, int l, int B)
   return 0;
 }
 
+// weight and bias gradients of a 1x1 convolution: X^T dY and the column sums of dY
 template <int W>
-int weight_grad_rows(se2nn *h, const bf16 *X, int R, const bf16 *dY, int B, float *out)
+int conv_grads(se2nn *h, const bf16 *X, int R, const bf16 *dY, int B, float *dw, float *db)
 {
-  nnk::weight_grad_partial<W><<<B * h->split, nnk::RT, nnk::wgrad_smem(R, W), h->stream>>>(X, R, dY, h->npix / h->split, h->partial);
-  k_sum_parts<<<nblk((long)R * W, SPC), EW, 0, h->stream>>>(h->partial, B * h->split, (long)R * W, out);
+  const int kc = h->npix / h->split;
+  const long rows = (long)B * h->npix;
+  const bool sums = kc % nnk::CSP == 0;   // whole column sums per chunk; else a pass of their own
+  nnk::weight_grad_partial<W><<<B * h->split, nnk::RT, nnk::wgrad_smem(R, W), h->stream>>>(X, R, dY, kc, h->partial, sums ? h->colpart : nullptr);
+  k_sum_parts<<<nblk((long)R * W, SPC), EW, 0, h->stream>>>(h->partial, B * h->split, (long)R * W, dw);
+  if (sums) k_sum_parts<<<nblk(W, SPC), EW, 0, h->stream>>>(h->colpart, (int)(rows / nnk::CSP), W, db);
   NCK(h, cudaGetLastError());
-  return 0;
+  return sums ? 0 : colsum(h, dY, rows, W, nnk::CSP, db);
 }
 
 // backward of the Fourier layers and the lift from dD0.  dHa and dHb take turns as the layers'
@@ -776,14 +806,12 @@ int weight_grad_rows(se2nn *h, const bf16 *X, int R, const bf16 *dY, int B, floa
 template <int W>
 int layers_bwd(se2nn *h, const bf16 *x, int B)
 {
-  const long rows = (long)B * h->npix;
   int rc;
   nnk::RowArgs a = row_args(h, B);
   a.dd0 = h->dD0; a.efwd = h->ExinvT; a.out = h->dHa; a.spec_out = h->Xf;
   if ((rc = row_launch<W, nnk::ROW_TOP>(h, a))) return rc;
   for (int l = h->L - 1; l >= 0; l--) {
-    if ((rc = weight_grad_rows<W>(h, h->H[l], W, h->dHa, B, h->grads + h->oW[l]))) return rc;
-    if ((rc = colsum(h, h->dHa, rows, W, 1024, h->grads + h->ob[l]))) return rc;
+    if ((rc = conv_grads<W>(h, h->H[l], W, h->dHa, B, h->grads + h->oW[l], h->grads + h->ob[l]))) return rc;
     if ((rc = y_analysis(h, h->Xf, h->Yp, B)) || (rc = mode_grad<W>(h, l, B)) || (rc = y_synthesis(h, h->Y, h->Yy, B))) return rc;
     a = row_args(h, B);
     a.in = h->dHa; a.spec = h->Yy; a.wt = h->Wb[l]; a.einv = h->ExT; a.efwd = h->ExinvT; a.out = h->dHb;
@@ -792,11 +820,51 @@ int layers_bwd(se2nn *h, const bf16 *x, int B)
     if ((rc = row_launch<W, nnk::ROW_BWD>(h, a))) return rc;
     std::swap(h->dHa, h->dHb);
   }
-  if ((rc = weight_grad_rows<W>(h, x, h->c.cin, h->dHa, B, h->grads + h->oW0))) return rc;
-  return colsum(h, h->dHa, rows, W, 1024, h->grads + h->ob0);
+  return conv_grads<W>(h, x, h->c.cin, h->dHa, B, h->grads + h->oW0, h->grads + h->ob0);
 }
 
 int layers_bwd_fused(se2nn *h, const bf16 *x, int B) { NN_WIDTH(layers_bwd, h, x, B) }
+
+// ---- the fused decoder
+bool fused_decoder(const se2nn *h) { return h->c.hidden <= nnk::DH && h->nsub <= nnk::DN; }
+
+nnk::DecArgs dec_args(se2nn *h, int B)
+{
+  nnk::DecArgs a;
+  memset(&a, 0, sizeof(a));
+  a.d0 = h->D0; a.w1 = h->W1b; a.w2 = h->W2b; a.c1 = h->params + h->oc1; a.c2 = h->params + h->oc2;
+  a.rows = B * h->c.nrec * h->c.ny; a.hid = h->c.hidden; a.ns = h->nsub; a.ny = h->c.ny;
+  return a;
+}
+
+template <int W>
+int decoder_fwd_w(se2nn *h, int B, float *out, bool keep)
+{
+  nnk::DecArgs a = dec_args(h, B);
+  a.out = out;
+  if (keep) { a.d1pre = h->D1pre; a.d1 = h->D1; }
+  nnk::dec_fwd<W><<<std::min((a.rows + 127) / 128, 4 * h->nsm), nnk::RT, nnk::dec_fwd_smem<W>(a.hid), h->stream>>>(a);
+  NCK(h, cudaGetLastError());
+  return 0;
+}
+int decoder_fwd(se2nn *h, int B, float *out, bool keep) { NN_WIDTH(decoder_fwd_w, h, B, out, keep) }
+
+// weight gradients' partials (then summed), bias gradients, dD0
+template <int W>
+int decoder_bwd_w(se2nn *h, int B)
+{
+  nnk::DecArgs a = dec_args(h, B);
+  const int units = B * h->c.nrec;
+  a.d1pre = h->D1pre; a.d1 = h->D1; a.dout = h->dpred; a.dd1 = h->dD1; a.dd0 = h->dD0;
+  a.dw1 = h->partial; a.dw2 = h->decpart;
+  nnk::dec_bwd<W><<<std::min(units, 2 * h->nsm), nnk::RT, nnk::dec_bwd_smem<W>(a.hid), h->stream>>>(a);
+  k_sum_parts<<<nblk((long)W * a.hid, SPC), EW, 0, h->stream>>>(h->partial, units, (long)W * a.hid, h->grads + h->oW1);
+  k_sum_parts<<<nblk((long)a.hid * a.ns, SPC), EW, 0, h->stream>>>(h->decpart, units, (long)a.hid * a.ns, h->grads + h->oW2);
+  NCK(h, cudaGetLastError());
+  int rc = colsum(h, h->dpred, a.rows, a.ns, 256, h->grads + h->oc2);
+  return rc ? rc : colsum(h, h->dD1, a.rows, a.hid, 256, h->grads + h->oc1);
+}
+int decoder_bwd(se2nn *h, int B) { NN_WIDTH(decoder_bwd_w, h, B) }
 
 // keep: the pass is followed by backward (pre-activations are stored)
 int forward(se2nn *h, const bf16 *x, int B, float *out, bool keep)
@@ -825,6 +893,7 @@ int forward(se2nn *h, const bf16 *x, int B, float *out, bool keep)
   }
   const bf16 *HL = h->H[L];
   const long drows = (long)B * nrec * h->c.ny;
+  if (fused && fused_decoder(h)) return decoder_fwd(h, B, out, keep);
   if (!fused) k_decoder_gather<<<nblk(drows * w), EW, 0, h->stream>>>(HL, h->rec_x, B, nrec, h->c.ny, h->c.nx, w, h->D0);
   {
     GemmArgs g = mk(h->D0, w, 0, 0, h->W1b, hid, 0, 0, (int)drows, hid, w, 1, h->D1, hid, 0, 0);
@@ -845,6 +914,10 @@ int backward(se2nn *h, const bf16 *x, int B)
   const int w = h->w, npix = h->npix, L = h->L, nrec = h->c.nrec, hid = h->c.hidden, ns = h->nsub;
   const long rows = (long)B * npix, drows = (long)B * nrec * h->c.ny;
   int rc;
+  if (fused_ok(h, x) && fused_decoder(h)) {
+    if ((rc = decoder_bwd(h, B))) return rc;
+    return layers_bwd_fused(h, x, B);
+  }
   // decoder (pointwise MLP over the receivers' columns); drows is a multiple of ny
   if ((rc = splitk_grad(h, h->D1, hid, h->dpred, ns, drows, h->c.ny, h->grads + h->oW2))) return rc;
   if ((rc = colsum(h, h->dpred, drows, ns, 256, h->grads + h->oc2))) return rc;
@@ -987,6 +1060,8 @@ extern "C" int se2nn_create(const se2nn_config *cfg, unsigned long long seed, se
                               (((long)drows + 255) / 256) * std::max(h->nsub, c.hidden));
     h->partial_n = std::max(wg, std::max(cs1, cs2));
     TRY(nalloc(h, &h->partial, (size_t)h->partial_n));
+    TRY(nalloc(h, &h->colpart, (size_t)cs1));
+    TRY(nalloc(h, &h->decpart, (size_t)Bm * c.nrec * c.hidden * h->nsub));
   }
   TRY(build_dft(h));
   TRY(fused_setup(h));
@@ -1109,7 +1184,7 @@ extern "C" int se2nn_adam_step(se2nn *h, float lr, float beta1, float beta2, flo
   if (!h) return -1;
   h->adam_t++;
   const float c1 = 1.f - powf(beta1, (float)h->adam_t), c2 = 1.f - powf(beta2, (float)h->adam_t);
-  k_adam<<<nblk(h->P), EW, 0, h->stream>>>(h->params, h->grads, h->adam_m, h->adam_v, h->Pb, h->P, lr, beta1, beta2, eps,
+  k_adam<<<nblk((h->P + 3) / 4), EW, 0, h->stream>>>(h->params, h->grads, h->adam_m, h->adam_v, h->Pb, h->P, lr, beta1, beta2, eps,
                                             weight_decay, c1, c2);
   h->wblk_stale = true;
   NCK(h, cudaGetLastError());

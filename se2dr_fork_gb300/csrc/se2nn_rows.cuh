@@ -33,7 +33,7 @@ namespace nnk {
 
 constexpr int RT = 256;                  // threads of the row kernels
 constexpr int RK = 32;                   // x modes (re, im) padded to two k steps
-constexpr int RNX = 128, RNY = 128, RM = 16;   // largest row, column, modes
+constexpr int RNX = 128, RNY = 128, RM = 16, RREC = 128;   // largest row, column, modes, receivers
 
 template <int LEFT> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
 
@@ -175,6 +175,7 @@ __global__ void __launch_bounds__(RT, 2) row_kernel(const RowArgs a)
   bf16 *sO = st0 + (KIND == ROW_TOP ? 1 : 2) * L::stage(a.nx, a.cin);
   float *sB = reinterpret_cast<float *>(sO + L::out(a.nx));
   const int nx = a.nx, m2 = a.m2, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+  __shared__ int rec[KIND == ROW_TOP ? RNX : 1], more[KIND == ROW_TOP ? RREC : 1];   // TOP: a column's first receiver, the next of a receiver
   const int kin = (KIND == ROW_LIFT) ? a.cin : W, lin = (KIND == ROW_LIFT) ? a.cin + 8 : LW;
   constexpr bool SPEC = KIND == ROW_FWD || KIND == ROW_BWD;
 
@@ -193,6 +194,18 @@ __global__ void __launch_bounds__(RT, 2) row_kernel(const RowArgs a)
   }
   if (KIND == ROW_LIFT || KIND == ROW_FWD)
     for (int e = threadIdx.x; e < W; e += RT) sB[e] = a.bias[e];
+  if (KIND == ROW_TOP)
+    for (int x = threadIdx.x; x < nx; x += RT) {   // (one thread per column: its receivers in ascending order)
+      int first = -1, last = -1;
+      for (int r = 0; r < a.nrec; r++)
+        if (a.rec_x[r] == x) {
+          if (first < 0) first = r;
+          else more[last] = r;
+          last = r;
+          more[r] = -1;
+        }
+      rec[x] = first;
+    }
 
   auto load = [&](int row, int s) {
     bf16 *st = st0 + s * L::stage(nx, a.cin);
@@ -213,17 +226,16 @@ __global__ void __launch_bounds__(RT, 2) row_kernel(const RowArgs a)
       for (int e = threadIdx.x; e < nx * NT; e += RT) {
         const int x = e / NT, c = (e - x * NT) * 8;
         float v[8] = {};
-        for (int r = 0; r < a.nrec; r++)
-          if (a.rec_x[r] == x) {
-            const uint4 q = *reinterpret_cast<const uint4 *>(a.dd0 + (((size_t)b * a.nrec + r) * a.ny + y) * W + c);
-            const uint32_t u[4] = {q.x, q.y, q.z, q.w};
+        for (int r = rec[x]; r >= 0; r = more[r]) {
+          const uint4 q = *reinterpret_cast<const uint4 *>(a.dd0 + (((size_t)b * a.nrec + r) * a.ny + y) * W + c);
+          const uint32_t u[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-              const float2 f = unpack_bf16(u[i]);
-              v[2 * i] += f.x;
-              v[2 * i + 1] += f.y;
-            }
+          for (int i = 0; i < 4; i++) {
+            const float2 f = unpack_bf16(u[i]);
+            v[2 * i] += f.x;
+            v[2 * i + 1] += f.y;
           }
+        }
         const uint4 o = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
         *reinterpret_cast<uint4 *>(px + x * LW + c) = o;
         *reinterpret_cast<uint4 *>(a.out + ((size_t)row * nx + x) * W + c) = o;
@@ -396,44 +408,49 @@ __global__ void __launch_bounds__(RT) last_kernel(const LastArgs a)
   }
 }
 
-// ---- y transforms: A [4m][2ny] (k contiguous) shared by the samples; 64 columns (kx, c) per CTA
+// ---- y transforms: A [4m][2ny] (k contiguous) shared by the samples; 128 columns (kx, c) per
+// CTA, so that a batch of 32 is one wave at two CTAs per SM (64 columns: 512 CTAs of 70 KB in
+// 456 places, 18 us; 128 columns: see below)
+constexpr int YN = 128, YL = YN + 8;
 struct YArgs {
   const bf16 *A;         // My [4m][2ny], or its transpose [2ny][4m] for the synthesis
   const bf16 *B;         // analysis [b][2ny][m w]; synthesis [b][4m][m w]
   bf16 *C;               // analysis: mode-major [(j, kx)][b][part][w]; synthesis [b][2ny][m w]
   int ny, m, w, batch;
 };
-__host__ __device__ inline size_t y_analysis_smem(int ny) { return 2 * ((size_t)64 * (2 * ny + 8) + (size_t)2 * ny * 72); }
-__host__ __device__ inline size_t y_synthesis_smem(int ny) { return 2 * ((size_t)2 * ny * 72 + (size_t)64 * 72); }
+__host__ __device__ inline size_t y_analysis_smem(int ny) { return 2 * ((size_t)64 * (2 * ny + 8) + (size_t)2 * ny * YL); }
+__host__ __device__ inline size_t y_synthesis_smem(int ny) { return 2 * ((size_t)2 * ny * 72 + (size_t)64 * YL + (size_t)8 * 16 * YL); }
 
-// copies of the 64 columns from n0 of rows k0 .. k1 (zero past column N)
-__device__ __forceinline__ void copy_cols(bf16 *s, const bf16 *g, long ldg, int k0, int k1, int n0, int N, int nt)
+// copies of the YN columns from n0 of rows k0 .. k1 (zero past column N)
+__device__ __forceinline__ void copy_cols(bf16 *s, const bf16 *g, long ldg, int k0, int k1, int n0, int N)
 {
-  for (int e = threadIdx.x; e < (k1 - k0) * 8; e += nt) {
-    const int r = k0 + e / 8, c = (e & 7) * 8;
+  for (int e = threadIdx.x; e < (k1 - k0) * (YN / 8); e += RT) {
+    const int r = k0 + e / (YN / 8), c = (e % (YN / 8)) * 8;
     const bool in = n0 + c < N;   // (N is a multiple of 16)
-    cp_async16(smem_addr(s + r * 72 + c), in ? g + r * ldg + n0 + c : g, in ? 16 : 0);
+    cp_async16(smem_addr(s + r * YL + c), in ? g + r * ldg + n0 + c : g, in ? 16 : 0);
   }
 }
 
-__global__ void __launch_bounds__(128) y_analysis(const YArgs a)
+// warp w: rows 16 (w % 4) .., columns 64 (w / 4) ..
+__global__ void __launch_bounds__(RT, 2) y_analysis(const YArgs a)
 {
   extern __shared__ __align__(16) unsigned char rsm[];
-  const int K = 2 * a.ny, LA = K + 8, M = 4 * a.m, N = a.m * a.w, n0 = blockIdx.x * 64, b = blockIdx.y;
+  const int K = 2 * a.ny, LA = K + 8, M = 4 * a.m, N = a.m * a.w, n0 = blockIdx.x * YN, b = blockIdx.y;
   bf16 *sA = reinterpret_cast<bf16 *>(rsm), *sB = sA + 64 * LA;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+  const int m0 = (warp & 3) * 16, c0 = (warp >> 2) * 64;
   // everything in flight at once, in four parts of k that are computed as they land
   const int part = (K / 4 + 15) / 16 * 16;
   for (int q = 0; q < 4; q++) {
     const int k0 = min(q * part, K), k1 = min(k0 + part, K), per = (k1 - k0) / 8;
-    for (int e = threadIdx.x; e < M * per; e += 128) {
+    for (int e = threadIdx.x; e < M * per; e += RT) {
       const int r = e / per, c = k0 + (e - r * per) * 8;
       cp_async16(smem_addr(sA + r * LA + c), a.A + (size_t)r * K + c, 16);
     }
-    copy_cols(sB, a.B + (size_t)b * K * N, N, k0, k1, n0, N, 128);
+    copy_cols(sB, a.B + (size_t)b * K * N, N, k0, k1, n0, N);
     cp_async_commit();
   }
-  zero_rows(sA, LA, M, 64, 128);
+  zero_rows(sA, LA, M, 64, RT);
   float acc[8][4] = {};
   for (int q = 0; q < 4; q++) {
     if (q == 0) cp_async_wait<3>();
@@ -441,13 +458,13 @@ __global__ void __launch_bounds__(128) y_analysis(const YArgs a)
     else if (q == 2) cp_async_wait<1>();
     else cp_async_wait<0>();
     __syncthreads();
-    if (warp * 16 >= M) continue;
+    if (m0 >= M) continue;
     for (int k = min(q * part, K); k < min((q + 1) * part, K); k += 16) {
       uint32_t fa[4], fb[4];
-      frag_a(fa, sA, LA, warp * 16, k);
+      frag_a(fa, sA, LA, m0, k);
 #pragma unroll
       for (int n = 0; n < 8; n += 2) {
-        frag_b(fb, sB, 72, n * 8, k);
+        frag_b(fb, sB, YL, c0 + n * 8, k);
         mma_bf16(acc[n], fa, fb);
         mma_bf16(acc[n + 1], fa, fb + 2);
       }
@@ -457,27 +474,29 @@ __global__ void __launch_bounds__(128) y_analysis(const YArgs a)
   for (int n = 0; n < 8; n++)
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-      const int r = warp * 16 + gid + 8 * h, col = n0 + n * 8 + tig * 2;
+      const int r = m0 + gid + 8 * h, col = n0 + c0 + n * 8 + tig * 2;
       if (r >= M || col >= N) continue;
       const int j = r >> 1, pt = r & 1, kx = col / a.w, c = col - kx * a.w;
       *reinterpret_cast<uint32_t *>(a.C + (((size_t)(j * a.m + kx) * a.batch + b) * 2 + pt) * a.w + c) = pack_bf16(acc[n][2 * h], acc[n][2 * h + 1]);
     }
 }
 
-__global__ void __launch_bounds__(256) y_synthesis(const YArgs a)
+// warp w: rows 16 w, 16 w + 128, ..; its 16 x YN results leave through a patch of shared memory in
+// 16-byte stores
+__global__ void __launch_bounds__(RT, 2) y_synthesis(const YArgs a)
 {
   extern __shared__ __align__(16) unsigned char rsm[];
-  const int K = 4 * a.m, K16 = (K + 15) / 16 * 16, M = 2 * a.ny, N = a.m * a.w, n0 = blockIdx.x * 64, b = blockIdx.y;
-  bf16 *sA = reinterpret_cast<bf16 *>(rsm), *sB = sA + M * 72;
+  const int K = 4 * a.m, K16 = (K + 15) / 16 * 16, M = 2 * a.ny, N = a.m * a.w, n0 = blockIdx.x * YN, b = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
-  copy_cols(sB, a.B + (size_t)b * K * N, N, 0, K, n0, N, 256);
-  zero_rows(sB, 72, K, K16, 256);
+  bf16 *sA = reinterpret_cast<bf16 *>(rsm), *sB = sA + M * 72, *sO = sB + 64 * YL + warp * 16 * YL;
+  copy_cols(sB, a.B + (size_t)b * K * N, N, 0, K, n0, N);
+  zero_rows(sB, YL, K, K16, RT);
   if (K % 8 == 0) {
-    copy_tile(sA, 72, a.A, K, M, K, 256);
+    copy_tile(sA, 72, a.A, K, M, K, RT);
     if (K16 > K)
-      for (int e = threadIdx.x; e < M * (K16 - K); e += 256) sA[(e / (K16 - K)) * 72 + K + e % (K16 - K)] = __float2bfloat16(0.f);
+      for (int e = threadIdx.x; e < M * (K16 - K); e += RT) sA[(e / (K16 - K)) * 72 + K + e % (K16 - K)] = __float2bfloat16(0.f);
   } else {
-    for (int e = threadIdx.x; e < M * K16; e += 256) {
+    for (int e = threadIdx.x; e < M * K16; e += RT) {
       const int r = e / K16, c = e - r * K16;
       sA[r * 72 + c] = (c < K) ? a.A[(size_t)r * K + c] : __float2bfloat16(0.f);
     }
@@ -486,24 +505,31 @@ __global__ void __launch_bounds__(256) y_synthesis(const YArgs a)
   cp_async_wait<0>();
   __syncthreads();
   for (int m0 = warp * 16; m0 < M; m0 += 128) {
-    float acc[8][4] = {};
-    for (int k = 0; k < K16; k += 16) {
-      uint32_t fa[4], fb[4];
-      frag_a(fa, sA, 72, m0, k);
 #pragma unroll
-      for (int n = 0; n < 8; n += 2) {
-        frag_b(fb, sB, 72, n * 8, k);
-        mma_bf16(acc[n], fa, fb);
-        mma_bf16(acc[n + 1], fa, fb + 2);
+    for (int half = 0; half < 2; half++) {
+      float acc[8][4] = {};
+      for (int k = 0; k < K16; k += 16) {
+        uint32_t fa[4], fb[4];
+        frag_a(fa, sA, 72, m0, k);
+#pragma unroll
+        for (int n = 0; n < 8; n += 2) {
+          frag_b(fb, sB, YL, half * 64 + n * 8, k);
+          mma_bf16(acc[n], fa, fb);
+          mma_bf16(acc[n + 1], fa, fb + 2);
+        }
       }
+#pragma unroll
+      for (int n = 0; n < 8; n++)
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+          *reinterpret_cast<uint32_t *>(sO + (gid + 8 * h) * YL + half * 64 + n * 8 + tig * 2) = pack_bf16(acc[n][2 * h], acc[n][2 * h + 1]);
     }
-#pragma unroll
-    for (int n = 0; n < 8; n++)
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int r = m0 + gid + 8 * h, col = n0 + n * 8 + tig * 2;
-        if (col < N) *reinterpret_cast<uint32_t *>(a.C + ((size_t)b * M + r) * N + col) = pack_bf16(acc[n][2 * h], acc[n][2 * h + 1]);
-      }
+    __syncwarp();
+    for (int e = lane; e < 16 * (YN / 8); e += 32) {
+      const int r = e / (YN / 8), c = (e % (YN / 8)) * 8;
+      if (n0 + c < N) *reinterpret_cast<uint4 *>(a.C + ((size_t)b * M + m0 + r) * N + n0 + c) = *reinterpret_cast<const uint4 *>(sO + r * YL + c);
+    }
+    __syncwarp();
   }
 }
 
@@ -648,12 +674,14 @@ __global__ void __launch_bounds__(RT) mode_grad(const ModeArgs a)
 }
 
 // ---- weight gradient of a 1x1 convolution: partial[chunk] (R x W) = X^T dY over kc pixels, k
-// ascending; X [pixels][R], dY [pixels][W]
-constexpr int WGK = 64, WGS = 3;   // pixels per stage, stages
+// ascending; X [pixels][R], dY [pixels][W].  Where kc is a multiple of CSP, also the column sums of
+// dY over every CSP pixels (sums: [pixels / CSP][W]) while its rows are in shared memory: RT / W
+// lanes per column, each over every (RT / W)-th pixel, added in lane order.
+constexpr int WGK = 128, WGS = 2, CSP = 1024;   // pixels per stage, stages, pixels per column sum
 inline size_t wgrad_smem(int R, int W) { return 2 * (size_t)WGS * WGK * (R + 8 + W + 8); }
 
 template <int W>
-__global__ void __launch_bounds__(RT) weight_grad_partial(const bf16 *X, int R, const bf16 *dY, int kc, float *partial)
+__global__ void __launch_bounds__(RT) weight_grad_partial(const bf16 *X, int R, const bf16 *dY, int kc, float *partial, float *sums)
 {
   constexpr int LW = W + 8, NP = W / 16, U = 2;   // 16 x 16 tiles, at most 4 x 4 over 8 warps
   extern __shared__ __align__(16) unsigned char rsm[];
@@ -670,12 +698,17 @@ __global__ void __launch_bounds__(RT) weight_grad_partial(const bf16 *X, int R, 
     }
     cp_async_commit();
   };
-  for (int i = 0; i < WGS - 1; i++) load(i);
+  constexpr int LANES = RT / W;
+  __shared__ float sc[RT];
+  const int lane_c = threadIdx.x / W, col = threadIdx.x % W;
+  int next = lane_c;   // this lane's next pixel of the column sum
+  float csum = 0.f;
+  load(0);
   float acc[U][2][4] = {};
   for (int i = 0; i < nst; i++) {
-    cp_async_wait<WGS - 2>();
+    load(i + 1);   // (its stage was freed by the barrier that ended the previous pass)
+    cp_async_wait<1>();
     __syncthreads();
-    load(i + WGS - 1);
     const bf16 *sX = st + (i % WGS) * stage, *sY = sX + WGK * LR;
     for (int k = 0; k < min(WGK, kc - i * WGK); k += 16)
 #pragma unroll
@@ -688,6 +721,24 @@ __global__ void __launch_bounds__(RT) weight_grad_partial(const bf16 *X, int R, 
         mma_bf16(acc[u][0], fa, fb);
         mma_bf16(acc[u][1], fa, fb + 2);
       }
+    if (sums) {
+      const int at = (i * WGK) % CSP;   // this stage's first pixel within its column sum
+      if (lane_c < LANES)
+#pragma unroll 8
+        for (; next < at + WGK; next += LANES) csum += __bfloat162float(sY[(next - at) * LW + col]);
+      if (at + WGK == CSP) {
+        sc[threadIdx.x] = csum;
+        __syncthreads();
+        if (threadIdx.x < W) {
+          float t = 0.f;
+          for (int l = 0; l < LANES; l++) t += sc[l * W + threadIdx.x];
+          sums[((p0 + (size_t)i * WGK) / CSP) * W + threadIdx.x] = t;
+        }
+        next = lane_c;
+        csum = 0.f;
+      }
+    }
+    __syncthreads();
   }
   cp_async_wait<0>();
 #pragma unroll
@@ -700,6 +751,218 @@ __global__ void __launch_bounds__(RT) weight_grad_partial(const bf16 *X, int R, 
       for (int h = 0; h < 2; h++)
         *reinterpret_cast<float2 *>(partial + ((size_t)blockIdx.x * R + (t / NP) * 16 + gid + 8 * h) * W + (t % NP) * 16 + c * 8 + tig * 2) =
             make_float2(acc[u][c][2 * h], acc[u][c][2 * h + 1]);
+  }
+}
+
+// ---- the decoder, D1 = gelu(D0 W1 + c1), out = D1 W2 + c2, and its backward.  hidden a multiple
+// of 16 up to 128, nsub up to 16 (padded with zero columns).
+constexpr int DH = 128, DN = 16, DLN = DN + 8;
+struct DecArgs {
+  const bf16 *d0;              // [rows][W]
+  const bf16 *w1, *w2;         // [W][hid], [hid][ns]
+  const float *c1, *c2;
+  bf16 *d1pre, *d1;            // [rows][hid]: stored by the forward pass of training (null: not), read by the backward
+  float *out;                  // [rows][ns]
+  const bf16 *dout;            // backward: [rows][ns]
+  bf16 *dd1, *dd0;             // [rows][hid], [rows][W]
+  float *dw1, *dw2;            // partial gradients per chunk of ny rows: [W][hid], [hid][ns]
+  int rows, hid, ns, ny;
+};
+template <int W> __host__ __device__ constexpr size_t dec_fwd_smem(int hid) { return 2 * ((size_t)W * (hid + 8) + (size_t)hid * DLN + 8 * 16 * (W + 8)); }
+template <int W> __host__ __device__ constexpr size_t dec_bwd_smem(int hid)
+{
+  return 2 * ((size_t)W * (hid + 8) + (size_t)hid * DLN + RNY * ((size_t)W + 8 + hid + 8 + DLN));
+}
+
+template <int W>
+__device__ __forceinline__ void dec_weights(bf16 *sW1, bf16 *sW2, const DecArgs &a)
+{
+  copy_tile(sW1, a.hid + 8, a.w1, a.hid, W, a.hid, RT);
+  for (int e = threadIdx.x; e < a.hid * DN; e += RT) {
+    const int r = e / DN, c = e - r * DN;
+    sW2[r * DLN + c] = (c < a.ns) ? a.w2[r * a.ns + c] : __float2bfloat16(0.f);
+  }
+}
+
+// one warp per 16 rows: the hidden values of 16 channels at a time go from the first product's
+// accumulators through GELU straight into the second product's operand registers
+template <int W>
+__global__ void __launch_bounds__(RT, 2) dec_fwd(const DecArgs a)
+{
+  constexpr int LW = W + 8;
+  extern __shared__ __align__(16) unsigned char rsm[];
+  const int LH = a.hid + 8, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+  bf16 *sW1 = reinterpret_cast<bf16 *>(rsm), *sW2 = sW1 + W * LH, *sD = sW2 + a.hid * DLN + warp * 16 * LW;
+  dec_weights<W>(sW1, sW2, a);
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  const bool pair = a.ns % 2 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 7) == 0;
+  for (int r0 = (blockIdx.x * 8 + warp) * 16; r0 < a.rows; r0 += gridDim.x * 128) {
+    for (int e = lane; e < 16 * (W / 8); e += 32) {
+      const int r = min(r0 + e / (W / 8), a.rows - 1);
+      cp_async16(smem_addr(sD + (e / (W / 8)) * LW + (e % (W / 8)) * 8), a.d0 + (size_t)r * W + (e % (W / 8)) * 8, 16);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncwarp();
+    uint32_t fd[W / 16][4];
+#pragma unroll
+    for (int k = 0; k < W / 16; k++) frag_a(fd[k], sD, LW, 0, k * 16);
+    float o[2][4] = {};
+    for (int hc = 0; hc < a.hid; hc += 16) {
+      float acc[2][4] = {};
+#pragma unroll
+      for (int k = 0; k < W / 16; k++) {
+        uint32_t fb[4];
+        frag_b(fb, sW1, LH, hc, k * 16);
+        mma_bf16(acc[0], fd[k], fb);
+        mma_bf16(acc[1], fd[k], fb + 2);
+      }
+      uint32_t fa[4], fb[4];
+#pragma unroll
+      for (int t = 0; t < 2; t++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int c = hc + t * 8 + tig * 2, r = r0 + gid + 8 * h;
+          const float x = acc[t][2 * h] + a.c1[c], y = acc[t][2 * h + 1] + a.c1[c + 1];
+          fa[2 * t + h] = pack_bf16(gelu_f(x), gelu_f(y));
+          if (a.d1 && r < a.rows) {
+            *reinterpret_cast<uint32_t *>(a.d1pre + (size_t)r * a.hid + c) = pack_bf16(x, y);
+            *reinterpret_cast<uint32_t *>(a.d1 + (size_t)r * a.hid + c) = fa[2 * t + h];
+          }
+        }
+      frag_b(fb, sW2, DLN, 0, hc);
+      mma_bf16(o[0], fa, fb);
+      mma_bf16(o[1], fa, fb + 2);
+    }
+#pragma unroll
+    for (int t = 0; t < 2; t++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int c = t * 8 + tig * 2, r = r0 + gid + 8 * h;
+        if (r >= a.rows || c >= a.ns) continue;
+        float *p = a.out + (size_t)r * a.ns + c;
+        const float x = o[t][2 * h] + a.c2[c];
+        if (pair) *reinterpret_cast<float2 *>(p) = make_float2(x, o[t][2 * h + 1] + a.c2[c + 1]);
+        else {
+          p[0] = x;
+          if (c + 1 < a.ns) p[1] = o[t][2 * h + 1] + a.c2[c + 1];
+        }
+      }
+    __syncwarp();
+  }
+}
+
+// one chunk of ny rows (one receiver of one sample) at a time: both weight gradients' partials,
+// k over the chunk's rows ascending, and the data gradient
+template <int W>
+__global__ void __launch_bounds__(RT, 2) dec_bwd(const DecArgs a)
+{
+  constexpr int LW = W + 8;
+  extern __shared__ __align__(16) unsigned char rsm[];
+  const int LH = a.hid + 8, HT = a.hid / 16, rows = (a.ny + 15) / 16 * 16;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+  bf16 *sW1 = reinterpret_cast<bf16 *>(rsm), *sW2 = sW1 + W * LH, *sD0 = sW2 + a.hid * DLN, *sD1 = sD0 + RNY * LW, *sP = sD1 + RNY * LH;
+  dec_weights<W>(sW1, sW2, a);
+  zero_rows(sD0, LW, a.ny, rows, RT);
+  zero_rows(sD1, LH, a.ny, rows, RT);
+  zero_rows(sP, DLN, a.ny, rows, RT);
+  for (int u = blockIdx.x; u < a.rows / a.ny; u += gridDim.x) {
+    const size_t r0 = (size_t)u * a.ny;
+    copy_tile(sD0, LW, a.d0 + r0 * W, W, a.ny, W, RT);
+    copy_tile(sD1, LH, a.d1 + r0 * a.hid, a.hid, a.ny, a.hid, RT);
+    cp_async_commit();
+    for (int e = threadIdx.x; e < a.ny * DN; e += RT) {
+      const int r = e / DN, c = e - r * DN;
+      sP[r * DLN + c] = (c < a.ns) ? a.dout[(r0 + r) * a.ns + c] : __float2bfloat16(0.f);
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    // dW2 = D1^T dout
+    for (int t = warp; t < HT; t += 8) {
+      float acc[2][4] = {};
+      for (int k = 0; k < rows; k += 16) {
+        uint32_t fa[4], fb[4];
+        frag_at(fa, sD1, LH, t * 16, k);
+        frag_b(fb, sP, DLN, 0, k);
+        mma_bf16(acc[0], fa, fb);
+        mma_bf16(acc[1], fa, fb + 2);
+      }
+#pragma unroll
+      for (int v = 0; v < 2; v++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const int r = t * 16 + gid + 8 * (i >> 1), c = v * 8 + tig * 2 + (i & 1);
+          if (c < a.ns) a.dw2[((size_t)u * a.hid + r) * a.ns + c] = acc[v][i];
+        }
+    }
+    __syncthreads();   // D1 has been read: its place takes dD1
+    const int m0 = warp * 16;
+    if (m0 < rows) {
+      uint32_t fa[4];
+      frag_a(fa, sP, DLN, m0, 0);
+      for (int hc = 0; hc < a.hid; hc += 16) {
+        float acc[2][4] = {};
+        uint32_t fb[4];
+        frag_bt(fb, sW2, DLN, hc, 0);
+        mma_bf16(acc[0], fa, fb);
+        mma_bf16(acc[1], fa, fb + 2);
+#pragma unroll
+        for (int t = 0; t < 2; t++)
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const int c = hc + t * 8 + tig * 2, r = m0 + gid + 8 * h;
+            if (r >= a.ny) continue;
+            const size_t o = (r0 + r) * a.hid + c;
+            const float2 p = unpack_bf16(*reinterpret_cast<const uint32_t *>(a.d1pre + o));
+            const uint32_t d = pack_bf16(round_bf16(acc[t][2 * h]) * gelu_grad_f(p.x), round_bf16(acc[t][2 * h + 1]) * gelu_grad_f(p.y));
+            *reinterpret_cast<uint32_t *>(sD1 + r * LH + c) = d;
+            *reinterpret_cast<uint32_t *>(a.dd1 + o) = d;
+          }
+      }
+    }
+    __syncthreads();
+    // dW1 = D0^T dD1
+    for (int t = warp; t < (W / 16) * HT; t += 8) {
+      const int mt = t / HT, nt = t - mt * HT;
+      float acc[2][4] = {};
+      for (int k = 0; k < rows; k += 16) {
+        uint32_t fa[4], fb[4];
+        frag_at(fa, sD0, LW, mt * 16, k);
+        frag_b(fb, sD1, LH, nt * 16, k);
+        mma_bf16(acc[0], fa, fb);
+        mma_bf16(acc[1], fa, fb + 2);
+      }
+#pragma unroll
+      for (int v = 0; v < 2; v++)
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+          *reinterpret_cast<float2 *>(a.dw1 + ((size_t)u * W + mt * 16 + gid + 8 * h) * a.hid + nt * 16 + v * 8 + tig * 2) =
+              make_float2(acc[v][2 * h], acc[v][2 * h + 1]);
+    }
+    // dD0 = dD1 W1^T
+    if (m0 < rows) {
+      float acc[W / 8][4] = {};
+      for (int k = 0; k < a.hid; k += 16) {
+        uint32_t fa[4], fb[4];
+        frag_a(fa, sD1, LH, m0, k);
+#pragma unroll
+        for (int n = 0; n < W / 8; n += 2) {
+          frag_bt(fb, sW1, LH, n * 8, k);
+          mma_bf16(acc[n], fa, fb);
+          mma_bf16(acc[n + 1], fa, fb + 2);
+        }
+      }
+#pragma unroll
+      for (int n = 0; n < W / 8; n++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int r = m0 + gid + 8 * h;
+          if (r < a.ny) *reinterpret_cast<uint32_t *>(a.dd0 + (r0 + r) * W + n * 8 + tig * 2) = pack_bf16(acc[n][2 * h], acc[n][2 * h + 1]);
+        }
+    }
+    __syncthreads();   // the tiles are free for the next chunk
   }
 }
 

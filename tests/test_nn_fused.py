@@ -31,6 +31,9 @@ CASES = [
     (64, 112, 64, 64, 16, 2, 16, 16, 128, 2),
     (128, 128, 16, 64, 16, 4, 16, 16, 128, 3),
     (96, 96, 16, 48, 12, 3, 16, 16, 128, 34),
+    # the decoder not fused: outputs per row, hidden width
+    (16, 32, 16, 32, 4, 2, 4, 24, 32, 2),
+    (16, 32, 16, 32, 4, 2, 4, 4, 144, 2),
     # not fused: height, width of the row, channels
     (12, 32, 16, 32, 4, 2, 4, 4, 32, 2),
     (16, 144, 16, 16, 4, 2, 4, 4, 32, 2),
