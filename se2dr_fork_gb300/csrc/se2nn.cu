@@ -15,6 +15,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <vector>
 
 #include "se2nn.h"
@@ -156,11 +157,27 @@ __global__ void __launch_bounds__(EW) k_colsum_partial(const bf16 *X, long M, in
 // them in order there (adding straight from global memory cost one L2 round trip after
 // another: 512 parts of 64 columns took 45 us)
 constexpr int SPC = 32, SPK = 256;   // columns, parts per pass
-__global__ void __launch_bounds__(EW) k_sum_parts(const float *partial, int nparts, long n, float *out)
+// up to four sums in one launch
+struct SumJob {
+  const float *partial;
+  float *out;
+  int nparts;
+  long n;
+};
+struct SumJobs {
+  SumJob job[4];
+  int first[5];   // first block of each job, and the end
+};
+__global__ void __launch_bounds__(EW) k_sum_parts(const SumJobs jobs)
 {
   __shared__ float s[SPK][SPC];
+  int which = 0;
+  while ((int)blockIdx.x >= jobs.first[which + 1]) which++;
+  const float *partial = jobs.job[which].partial;
+  const int nparts = jobs.job[which].nparts;
+  const long n = jobs.job[which].n;
   const int c = threadIdx.x % SPC, lane = threadIdx.x / SPC;
-  const long i = (long)blockIdx.x * SPC + c;
+  const long i = (long)(blockIdx.x - jobs.first[which]) * SPC + c;
   float t = 0.f;
   for (int k0 = 0; k0 < nparts; k0 += SPK) {
     float v[SPK / (EW / SPC)];
@@ -179,7 +196,22 @@ __global__ void __launch_bounds__(EW) k_sum_parts(const float *partial, int npar
       for (int k = 0; k < m; k++) t += s[k][c];
     }
   }
-  if (lane == 0 && i < n) out[i] = t;
+  if (lane == 0 && i < n) jobs.job[which].out[i] = t;
+}
+
+cudaError_t sum_parts(cudaStream_t st, std::initializer_list<SumJob> list)
+{
+  SumJobs jobs;
+  memset(&jobs, 0, sizeof(jobs));
+  int k = 0, blocks = 0;
+  for (const SumJob &j : list) {
+    jobs.job[k] = j;
+    jobs.first[k++] = blocks;
+    blocks += (int)nblk(j.n, SPC);
+  }
+  for (; k < 5; k++) jobs.first[k] = blocks;
+  k_sum_parts<<<blocks, EW, 0, st>>>(jobs);
+  return cudaGetLastError();
 }
 
 // D0[((b*nrec + r)*ny + row)] = H[b][row][rec_x[r]][0:w]: every row of each receiver's column
@@ -327,6 +359,7 @@ struct se2nn {
   // and the transposes ExT [nx][2m], ExinvT [2m][nx]
   bf16 *Ex = nullptr, *My = nullptr, *Myinv = nullptr, *Exinv = nullptr, *ExT = nullptr, *ExinvT = nullptr;
   int *rec_x = nullptr;
+  float *lut = nullptr;   // GELU' at BF16 arguments
   // activations (max batch)
   std::vector<bf16 *> H, Apre, Zp;
   bf16 *S = nullptr, *Xf = nullptr, *Z = nullptr, *Yp = nullptr, *Y = nullptr, *Yy = nullptr, *dZp = nullptr;
@@ -560,8 +593,7 @@ int colsum(se2nn *h, const bf16 *X, long M, int N, long rows, float *out)
 {
   const int chunks = (int)((M + rows - 1) / rows);
   k_colsum_partial<<<dim3(1, chunks), EW, 0, h->stream>>>(X, M, N, rows, h->partial);
-  k_sum_parts<<<nblk(N, SPC), EW, 0, h->stream>>>(h->partial, chunks, N, out);
-  NCK(h, cudaGetLastError());
+  NCK(h, sum_parts(h->stream, {{h->partial, out, chunks, N}}));
   return 0;
 }
 
@@ -572,8 +604,7 @@ int weight_grad(se2nn *h, const bf16 *X, int rows, const bf16 *dY, int B, float 
   const long kc = h->npix / s;
   GemmArgs g = mk(X, rows, kc * rows, 1, dY, w, kc * w, 0, rows, w, (int)kc, B * s, h->partial, w, (long)rows * w, 1);
   GEMM(h, g);
-  k_sum_parts<<<nblk((long)rows * w, SPC), EW, 0, h->stream>>>(h->partial, B * s, (long)rows * w, out);
-  NCK(h, cudaGetLastError());
+  NCK(h, sum_parts(h->stream, {{h->partial, out, B * s, (long)rows * w}}));
   return 0;
 }
 
@@ -583,8 +614,7 @@ int splitk_grad(se2nn *h, const bf16 *X, int M, const bf16 *dY, int N, long K, l
   const int parts = (int)(K / chunk);
   GemmArgs g = mk(X, M, chunk * M, 1, dY, N, chunk * N, 0, M, N, (int)chunk, parts, h->partial, N, (long)M * N, 1);
   GEMM(h, g);
-  k_sum_parts<<<nblk((long)M * N, SPC), EW, 0, h->stream>>>(h->partial, parts, (long)M * N, out);
-  NCK(h, cudaGetLastError());
+  NCK(h, sum_parts(h->stream, {{h->partial, out, parts, (long)M * N}}));
   return 0;
 }
 
@@ -665,12 +695,14 @@ int fused_setup_w(se2nn *h)
   if (e == cudaSuccess) e = row_setup<W, nnk::ROW_FWD>(h);
   if (e == cudaSuccess) e = row_setup<W, nnk::ROW_BWD>(h);
   if (e == cudaSuccess) e = row_setup<W, nnk::ROW_TOP>(h);
-  if (e == cudaSuccess) e = allow_smem(nnk::y_analysis, nnk::y_analysis_smem(nnk::RNY));
-  if (e == cudaSuccess) e = allow_smem(nnk::y_synthesis, nnk::y_synthesis_smem(nnk::RNY));
+  if (e == cudaSuccess) e = allow_smem(nnk::y_analysis<W>, nnk::y_analysis_smem(nnk::RNY));
+  if (e == cudaSuccess) e = allow_smem(nnk::y_synthesis<W>, nnk::y_synthesis_smem(nnk::RNY));
   if (e == cudaSuccess) e = allow_smem(nnk::last_kernel<W>, nnk::last_smem<W>());
   if (e == cudaSuccess) e = allow_smem(nnk::mode_mix<W>, nnk::mode_smem<W>());
   if (e == cudaSuccess) e = allow_smem(nnk::mode_grad<W>, nnk::mode_grad_smem<W>());
-  if (e == cudaSuccess) e = allow_smem(nnk::weight_grad_partial<W>, nnk::wgrad_smem(64, W));
+  if (e == cudaSuccess) e = allow_smem(nnk::weight_grad_partial<W, 0, false>, nnk::wgrad_smem<W>(64));
+  if (e == cudaSuccess) e = allow_smem(nnk::weight_grad_partial<W, W, true>, nnk::wgrad_smem<W>(64));
+  if (e == cudaSuccess) e = allow_smem(nnk::weight_grad_partial<W, 0, true>, nnk::wgrad_smem<W>(64));
   if (e == cudaSuccess) e = allow_smem(nnk::dec_fwd<W>, nnk::dec_fwd_smem<W>(nnk::DH));
   if (e == cudaSuccess) e = allow_smem(nnk::dec_bwd<W>, nnk::dec_bwd_smem<W>(nnk::DH));
   NCK(h, e);
@@ -697,6 +729,10 @@ int row_launch(se2nn *h, const nnk::RowArgs &a)
 int fused_setup(se2nn *h)
 {
   if (!fused_shape(h)) return 0;
+  int rc = nalloc(h, &h->lut, nnk::GLUT);
+  if (rc) return rc;
+  nnk::gelu_lut_kernel<<<nblk(nnk::GLUT), EW, 0, h->stream>>>(h->lut);
+  NCK(h, cudaGetLastError());
   NN_WIDTH(fused_setup_w, h)
 }
 
@@ -705,25 +741,29 @@ nnk::RowArgs row_args(se2nn *h, int B)
   nnk::RowArgs a;
   memset(&a, 0, sizeof(a));
   a.rows = B * h->c.ny; a.nx = h->c.nx; a.ny = h->c.ny; a.m2 = 2 * h->m; a.cin = h->c.cin;
-  a.nrec = h->c.nrec; a.rec_x = h->rec_x;
+  a.nrec = h->c.nrec; a.rec_x = h->rec_x; a.lut = h->lut;
   return a;
 }
 
-int y_analysis(se2nn *h, const bf16 *spec, bf16 *Zp, int B)
+template <int W>
+int y_analysis_w(se2nn *h, const bf16 *spec, bf16 *Zp, int B)
 {
   const size_t smem = nnk::y_analysis_smem(h->c.ny);
-  nnk::y_analysis<<<dim3((h->m * h->w + nnk::YN - 1) / nnk::YN, B), nnk::RT, smem, h->stream>>>(nnk::YArgs{h->My, spec, Zp, h->c.ny, h->m, h->w, B});
+  nnk::y_analysis<W><<<dim3((h->m * W + nnk::YN - 1) / nnk::YN, B), nnk::RT, smem, h->stream>>>(nnk::YArgs{h->My, spec, Zp, h->c.ny, h->m, B});
   NCK(h, cudaGetLastError());
   return 0;
 }
+int y_analysis(se2nn *h, const bf16 *spec, bf16 *Zp, int B) { NN_WIDTH(y_analysis_w, h, spec, Zp, B) }
 
-int y_synthesis(se2nn *h, const bf16 *Y, bf16 *spec, int B)
+template <int W>
+int y_synthesis_w(se2nn *h, const bf16 *Y, bf16 *spec, int B)
 {
   const size_t smem = nnk::y_synthesis_smem(h->c.ny);
-  nnk::y_synthesis<<<dim3((h->m * h->w + nnk::YN - 1) / nnk::YN, B), nnk::RT, smem, h->stream>>>(nnk::YArgs{h->Myinv, Y, spec, h->c.ny, h->m, h->w, B});
+  nnk::y_synthesis<W><<<dim3((h->m * W + nnk::YN - 1) / nnk::YN, B), nnk::RT, smem, h->stream>>>(nnk::YArgs{h->Myinv, Y, spec, h->c.ny, h->m, B});
   NCK(h, cudaGetLastError());
   return 0;
 }
+int y_synthesis(se2nn *h, const bf16 *Y, bf16 *spec, int B) { NN_WIDTH(y_synthesis_w, h, Y, spec, B) }
 
 template <int W>
 int mode_mix(se2nn *h, int l, int B)
@@ -794,11 +834,18 @@ int conv_grads(se2nn *h, const bf16 *X, int R, const bf16 *dY, int B, float *dw,
   const int kc = h->npix / h->split;
   const long rows = (long)B * h->npix;
   const bool sums = kc % nnk::CSP == 0;   // whole column sums per chunk; else a pass of their own
-  nnk::weight_grad_partial<W><<<B * h->split, nnk::RT, nnk::wgrad_smem(R, W), h->stream>>>(X, R, dY, kc, h->partial, sums ? h->colpart : nullptr);
-  k_sum_parts<<<nblk((long)R * W, SPC), EW, 0, h->stream>>>(h->partial, B * h->split, (long)R * W, dw);
-  if (sums) k_sum_parts<<<nblk(W, SPC), EW, 0, h->stream>>>(h->colpart, (int)(rows / nnk::CSP), W, db);
+  auto fn = (kc % nnk::WGK) ? nnk::weight_grad_partial<W, 0, false>
+            : (R == W) ? nnk::weight_grad_partial<W, W, true>
+                       : nnk::weight_grad_partial<W, 0, true>;
+  fn<<<B * h->split, nnk::RT, nnk::wgrad_smem<W>(R), h->stream>>>(X, R, dY, kc, h->partial, sums ? h->colpart : nullptr);
   NCK(h, cudaGetLastError());
-  return sums ? 0 : colsum(h, dY, rows, W, nnk::CSP, db);
+  const SumJob w{h->partial, dw, B * h->split, (long)R * W};
+  if (sums) {
+    NCK(h, sum_parts(h->stream, {w, {h->colpart, db, (int)(rows / nnk::CSP), W}}));
+    return 0;
+  }
+  NCK(h, sum_parts(h->stream, {w}));
+  return colsum(h, dY, rows, W, nnk::CSP, db);
 }
 
 // backward of the Fourier layers and the lift from dD0.  dHa and dHb take turns as the layers'
@@ -858,11 +905,16 @@ int decoder_bwd_w(se2nn *h, int B)
   a.d1pre = h->D1pre; a.d1 = h->D1; a.dout = h->dpred; a.dd1 = h->dD1; a.dd0 = h->dD0;
   a.dw1 = h->partial; a.dw2 = h->decpart;
   nnk::dec_bwd<W><<<std::min(units, 2 * h->nsm), nnk::RT, nnk::dec_bwd_smem<W>(a.hid), h->stream>>>(a);
-  k_sum_parts<<<nblk((long)W * a.hid, SPC), EW, 0, h->stream>>>(h->partial, units, (long)W * a.hid, h->grads + h->oW1);
-  k_sum_parts<<<nblk((long)a.hid * a.ns, SPC), EW, 0, h->stream>>>(h->decpart, units, (long)a.hid * a.ns, h->grads + h->oW2);
+  const int chunks = (a.rows + 255) / 256;
+  float *c2 = h->decpart + (size_t)units * a.hid * a.ns, *c1 = c2 + (size_t)chunks * a.ns;
+  k_colsum_partial<<<dim3(1, chunks), EW, 0, h->stream>>>(h->dpred, a.rows, a.ns, 256, c2);
+  k_colsum_partial<<<dim3(1, chunks), EW, 0, h->stream>>>(h->dD1, a.rows, a.hid, 256, c1);
   NCK(h, cudaGetLastError());
-  int rc = colsum(h, h->dpred, a.rows, a.ns, 256, h->grads + h->oc2);
-  return rc ? rc : colsum(h, h->dD1, a.rows, a.hid, 256, h->grads + h->oc1);
+  NCK(h, sum_parts(h->stream, {{h->partial, h->grads + h->oW1, units, (long)W * a.hid},
+                               {h->decpart, h->grads + h->oW2, units, (long)a.hid * a.ns},
+                               {c2, h->grads + h->oc2, chunks, a.ns},
+                               {c1, h->grads + h->oc1, chunks, a.hid}}));
+  return 0;
 }
 int decoder_bwd(se2nn *h, int B) { NN_WIDTH(decoder_bwd_w, h, B) }
 
@@ -1061,7 +1113,7 @@ extern "C" int se2nn_create(const se2nn_config *cfg, unsigned long long seed, se
     h->partial_n = std::max(wg, std::max(cs1, cs2));
     TRY(nalloc(h, &h->partial, (size_t)h->partial_n));
     TRY(nalloc(h, &h->colpart, (size_t)cs1));
-    TRY(nalloc(h, &h->decpart, (size_t)Bm * c.nrec * c.hidden * h->nsub));
+    TRY(nalloc(h, &h->decpart, (size_t)Bm * c.nrec * c.hidden * h->nsub + (drows + 255) / 256 * (size_t)(h->nsub + c.hidden)));
   }
   TRY(build_dft(h));
   TRY(fused_setup(h));

@@ -37,10 +37,13 @@ constexpr int RNX = 128, RNY = 128, RM = 16, RREC = 128;   // largest row, colum
 
 template <int LEFT> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
 
-// asynchronous copy of rows x cols (a multiple of 8) elements into shared memory
+// asynchronous copy of rows x cols (a multiple of 8) elements into shared memory.  COLS: the row
+// length where it is known (the index then needs no division, a third of the small kernels'
+// instructions otherwise)
+template <int COLS = 0>
 __device__ __forceinline__ void copy_tile(bf16 *s, int lds, const bf16 *g, long ldg, int rows, int cols, int nt)
 {
-  const int per = cols / 8;
+  const int per = (COLS ? COLS : cols) / 8;
   for (int e = threadIdx.x; e < rows * per; e += nt) {
     const int r = e / per, c = (e - r * per) * 8;
     cp_async16(smem_addr(s + r * lds + c), g + r * ldg + c, 16);
@@ -86,6 +89,29 @@ __device__ __forceinline__ float2 unpack_bf16(uint32_t u)
   return make_float2(__low2float(v), __high2float(v));
 }
 
+// GELU' of a BF16 pre-activation from a table in shared memory: the values of gelu_grad_f at the
+// BF16 numbers of magnitude 2^-8 to 4 (10 binades, both signs: 10 KB), the function itself
+// outside.  The function costs some 45 instructions, the look-up 6 and one conflicted read.
+constexpr int GLUT_LO = (127 - 8) << 7, GLUT_N = 10 << 7, GLUT = 2 * GLUT_N;
+__device__ __forceinline__ float gelu_grad_lut(uint32_t bits, const float *lut)
+{
+  const uint32_t i = (bits & 0x7fffu) - GLUT_LO;
+  if (i < GLUT_N) return lut[i + ((bits & 0x8000u) ? GLUT_N : 0)];
+  return gelu_grad_f(__uint_as_float(bits << 16));
+}
+__device__ __forceinline__ void load_gelu_lut(float *s, const float *lut, int nt)
+{
+  for (int e = threadIdx.x; e < GLUT / 4; e += nt) reinterpret_cast<float4 *>(s)[e] = reinterpret_cast<const float4 *>(lut)[e];
+}
+__global__ void gelu_lut_kernel(float *lut)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < GLUT) {
+    const uint32_t bits = (uint32_t)(GLUT_LO + i % GLUT_N) | (i < GLUT_N ? 0u : 0x8000u);
+    lut[i] = gelu_grad_f(__uint_as_float(bits << 16));
+  }
+}
+
 enum { ROW_LIFT = 0, ROW_FWD = 1, ROW_BWD = 2, ROW_TOP = 3 };
 
 struct RowArgs {
@@ -96,6 +122,7 @@ struct RowArgs {
   const bf16 *einv;      // [nx][m2]: spectrum row -> pixels
   const bf16 *efwd;      // [m2][nx]: pixels -> spectrum row
   const bf16 *pre;       // BWD: pre-activation of the layer below (null: none)
+  const float *lut;      // BWD: GELU' table
   bf16 *out;             // [rows][nx][W]: H, or dA (dH below the first layer)
   bf16 *aux;             // FWD: pre-activation (null: not stored)
   bf16 *spec_out;        // [rows][m2][W] (null: none)
@@ -108,29 +135,28 @@ struct RowArgs {
 
 template <int W, int KIND>
 struct RowSmem {
-  static constexpr int LW = W + 8, LE = RK + 8;
+  static constexpr int LW = W + 8;
   static constexpr int KIN = (KIND == ROW_LIFT) ? 64 : W;   // widest convolution input
   static __host__ __device__ size_t wt() { return (KIND == ROW_TOP) ? 0 : (size_t)KIN * LW; }
-  static __host__ __device__ size_t einv(int nx) { return (KIND == ROW_FWD || KIND == ROW_BWD) ? (size_t)nx * LE : 0; }
   static __host__ __device__ size_t efwd(int nx) { return (size_t)RK * (nx + 8); }
   static __host__ __device__ size_t in(int nx, int cin) { return (size_t)nx * ((KIND == ROW_LIFT) ? cin + 8 : LW); }
   static __host__ __device__ size_t spec() { return (KIND == ROW_FWD || KIND == ROW_BWD) ? (size_t)RK * LW : 0; }
-  static __host__ __device__ size_t pre(int nx) { return (KIND == ROW_BWD) ? (size_t)nx * LW : 0; }
-  static __host__ __device__ size_t stage(int nx, int cin) { return in(nx, cin) + spec() + pre(nx); }
+  static __host__ __device__ size_t stage(int nx, int cin) { return in(nx, cin) + spec(); }
   static __host__ __device__ size_t out(int nx) { return (KIND == ROW_LIFT) ? (size_t)nx * LW : 0; }
   static __host__ __device__ size_t bytes(int nx, int cin)
   {
-    return 2 * (wt() + einv(nx) + efwd(nx) + (KIND == ROW_TOP ? 1 : 2) * stage(nx, cin) + out(nx)) + W * sizeof(float);
+    return 2 * (wt() + efwd(nx) + (KIND == ROW_TOP ? 1 : 2) * stage(nx, cin) + out(nx)) + (W + (KIND == ROW_BWD ? GLUT : 0)) * sizeof(float);
   }
 };
 
-// rows [m0, m0 + 16) x W of a shared tile -> global memory, 16 bytes a lane, by one warp
-template <int W>
-__device__ __forceinline__ void store_rows16(bf16 *g, const bf16 *s, int m0)
+// rows [m0, m0 + 16), channels [c0, c0 + CW) of a shared tile -> global memory, 16 bytes a lane, by
+// one warp
+template <int W, int CW>
+__device__ __forceinline__ void store_rows16(bf16 *g, const bf16 *s, int m0, int c0)
 {
-  constexpr int PER = W / 8;
+  constexpr int PER = CW / 8;
   for (int e = threadIdx.x & 31; e < 16 * PER; e += 32) {
-    const int r = e / PER, c = (e - r * PER) * 8;
+    const int r = e / PER, c = c0 + (e - r * PER) * 8;
     *reinterpret_cast<uint4 *>(g + (size_t)(m0 + r) * W + c) = *reinterpret_cast<const uint4 *>(s + (m0 + r) * (W + 8) + c);
   }
 }
@@ -160,38 +186,47 @@ __device__ __forceinline__ void x_analysis(const bf16 *sE, const bf16 *px, int n
 }
 
 // Persistent over the image rows, two stages of asynchronous copies.  A warp owns 16 pixels
-// through the convolution and activation, so the results replace its input in shared memory
-// without a block barrier; the x transform at the end reads all pixels.
+// through the convolution and activation: it holds them in operand registers, so results (and, on
+// their way, the pre-activations) replace them in shared memory without a block barrier; the
+// x transform at the end reads all pixels.  What bounds it is the activation's arithmetic (about
+// 50 instructions per value, erff most of them) at the warps that fit: 32 channels at a time
+// and no second stage for the pre-activations leave three CTAs per SM (85 registers, 74 KB).
 template <int W, int KIND>
-__global__ void __launch_bounds__(RT, 2) row_kernel(const RowArgs a)
+__global__ void __launch_bounds__(RT, 3) row_kernel(const RowArgs a)
 {
   typedef RowSmem<W, KIND> L;
-  constexpr int LW = L::LW, LE = L::LE, NT = W / 8;
+  constexpr int LW = L::LW, NT = W / 8;
   extern __shared__ __align__(16) unsigned char rsm[];
   bf16 *sW = reinterpret_cast<bf16 *>(rsm);
-  bf16 *sI = sW + L::wt();
-  bf16 *sE = sI + L::einv(a.nx);
+  bf16 *sE = sW + L::wt();
   bf16 *st0 = sE + L::efwd(a.nx);
   bf16 *sO = st0 + (KIND == ROW_TOP ? 1 : 2) * L::stage(a.nx, a.cin);
-  float *sB = reinterpret_cast<float *>(sO + L::out(a.nx));
+  float *sB = reinterpret_cast<float *>(sO + L::out(a.nx)), *sG = sB + W;
   const int nx = a.nx, m2 = a.m2, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
   __shared__ int rec[KIND == ROW_TOP ? RNX : 1], more[KIND == ROW_TOP ? RREC : 1];   // TOP: a column's first receiver, the next of a receiver
   const int kin = (KIND == ROW_LIFT) ? a.cin : W, lin = (KIND == ROW_LIFT) ? a.cin + 8 : LW;
   constexpr bool SPEC = KIND == ROW_FWD || KIND == ROW_BWD;
 
   // tables, zero-padded to whole k steps
-  if (KIND != ROW_TOP) copy_tile(sW, LW, a.wt, W, kin, W, RT);
+  if (KIND != ROW_TOP) copy_tile<W>(sW, LW, a.wt, W, kin, W, RT);
   for (int e = threadIdx.x; e < RK * (nx + 8); e += RT) {
     const int r = e / (nx + 8), c = e - r * (nx + 8);
     sE[e] = (r < m2 && c < nx) ? a.efwd[r * nx + c] : __float2bfloat16(0.f);
   }
+  // a warp's pixels are the same columns of every row: its part of the inverse x transform stays in
+  // operand registers (row gid + 8 (i % 2), k pair 2 tig + 8 (i / 2) of a k step)
+  uint32_t fe[RK / 16][4];
   if (SPEC) {
-    for (int e = threadIdx.x; e < nx * LE; e += RT) {
-      const int r = e / LE, c = e - r * LE;
-      sI[e] = (c < m2) ? a.einv[r * m2 + c] : __float2bfloat16(0.f);
-    }
+#pragma unroll
+    for (int k = 0; k < RK / 16; k++)
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const int r = warp * 16 + gid + 8 * (i & 1), c = k * 16 + tig * 2 + 8 * (i >> 1);
+        fe[k][i] = (r < nx && c < m2) ? *reinterpret_cast<const uint32_t *>(a.einv + r * m2 + c) : 0u;
+      }
     for (int s = 0; s < 2; s++) zero_rows(st0 + s * L::stage(nx, a.cin) + L::in(nx, a.cin), LW, m2, RK, RT);
   }
+  if (KIND == ROW_BWD && a.pre) load_gelu_lut(sG, a.lut, RT);
   if (KIND == ROW_LIFT || KIND == ROW_FWD)
     for (int e = threadIdx.x; e < W; e += RT) sB[e] = a.bias[e];
   if (KIND == ROW_TOP)
@@ -209,10 +244,11 @@ __global__ void __launch_bounds__(RT, 2) row_kernel(const RowArgs a)
 
   auto load = [&](int row, int s) {
     bf16 *st = st0 + s * L::stage(nx, a.cin);
-    copy_tile(st, lin, a.in + (size_t)row * nx * kin, kin, nx, kin, RT);
-    if (SPEC) copy_tile(st + L::in(nx, a.cin), LW, a.spec + (size_t)row * m2 * W, W, m2, W, RT);
-    if (KIND == ROW_BWD && a.pre) copy_tile(st + L::in(nx, a.cin) + L::spec(), LW, a.pre + (size_t)row * nx * W, W, nx, W, RT);
-  };
+    if (KIND != ROW_LIFT) copy_tile<W>(st, lin, a.in + (size_t)row * nx * kin, kin, nx, kin, RT);
+    else if (kin == 16) copy_tile<16>(st, lin, a.in + (size_t)row * nx * kin, kin, nx, kin, RT);
+    else copy_tile(st, lin, a.in + (size_t)row * nx * kin, kin, nx, kin, RT);
+    if (SPEC) copy_tile<W>(st + L::in(nx, a.cin), LW, a.spec + (size_t)row * m2 * W, W, m2, W, RT);
+      };
   if (KIND != ROW_TOP) {
     if ((int)blockIdx.x < a.rows) load(blockIdx.x, 0);
     cp_async_commit();
@@ -242,80 +278,99 @@ __global__ void __launch_bounds__(RT, 2) row_kernel(const RowArgs a)
       }
     } else {
       bf16 *st = st0 + s * L::stage(nx, a.cin);
-      if (row + (int)gridDim.x < a.rows) load(row + gridDim.x, s ^ 1);   // (freed by the barrier that ended the previous row)
-      cp_async_commit();
-      cp_async_wait<1>();
+      cp_async_wait<0>();
       __syncthreads();
       px = (KIND == ROW_LIFT) ? sO : st;
       const int m0 = warp * 16;
-      if (m0 < nx) {
-        // spectrum row -> pixels, and the 1x1 convolution
-        float sp[NT][4] = {}, cv[NT][4] = {};
-        if (SPEC) {
-          const bf16 *sS = st + L::in(nx, a.cin);
+      const bool on = m0 < nx, pre = KIND == ROW_BWD && a.pre;
+      uint32_t fp[L::KIN / 16][4];
+      if (on) {
 #pragma unroll
-          for (int k = 0; k < RK; k += 16) {
-            uint32_t fa[4], fb[4];
-            frag_a(fa, sI, LE, m0, k);
+        for (int k = 0; k < L::KIN / 16; k++)
+          if (k * 16 < kin) frag_a(fp[k], st, lin, m0, k * 16);
+        __syncwarp();   // the warp's pixels have been read
+        if (pre)        // the pre-activations take their place
+          for (int e = lane; e < 16 * NT; e += 32)
+            cp_async16(smem_addr(px + (m0 + e / NT) * LW + (e % NT) * 8), a.pre + ((size_t)row * nx + m0 + e / NT) * W + (e % NT) * 8, 16);
+      }
+      cp_async_commit();
+      if (row + (int)gridDim.x < a.rows) load(row + gridDim.x, s ^ 1);   // (freed by the barrier that ended the previous row)
+      cp_async_commit();
+      if (on) {
+        const bf16 *sS = st + L::in(nx, a.cin);
+        constexpr int CW = (W % 32 == 0) ? 32 : 16, CT = CW / 8;   // channels at a time
 #pragma unroll
-            for (int n = 0; n < NT; n += 2) {
-              frag_b(fb, sS, LW, n * 8, k);
-              mma_bf16(sp[n], fa, fb);
-              mma_bf16(sp[n + 1], fa, fb + 2);
+        for (int c0 = 0; c0 < W; c0 += CW) {
+          // spectrum row -> pixels, and the 1x1 convolution
+          float sp[CT][4] = {}, cv[CT][4] = {};
+          uint32_t fb[4];
+          if (SPEC)
+#pragma unroll
+            for (int k = 0; k < RK / 16; k++)
+#pragma unroll
+              for (int n = 0; n < CT; n += 2) {
+                frag_b(fb, sS, LW, c0 + n * 8, k * 16);
+                mma_bf16(sp[n], fe[k], fb);
+                mma_bf16(sp[n + 1], fe[k], fb + 2);
+              }
+#pragma unroll
+          for (int k = 0; k < L::KIN / 16; k++)
+            if (k * 16 < kin)
+#pragma unroll
+              for (int n = 0; n < CT; n += 2) {
+                if (KIND == ROW_BWD) frag_bt(fb, sW, LW, c0 + n * 8, k * 16);
+                else frag_b(fb, sW, LW, c0 + n * 8, k * 16);
+                mma_bf16(cv[n], fp[k], fb);
+                mma_bf16(cv[n + 1], fp[k], fb + 2);
+              }
+          if (pre && c0 == 0) {
+            cp_async_wait<1>();
+            __syncwarp();
+          }
+          if (KIND == ROW_FWD) {
+            // the pre-activation, through px to memory where it is kept
+#pragma unroll
+            for (int n = 0; n < CT; n++)
+#pragma unroll
+              for (int h = 0; h < 2; h++) {
+                const int c = c0 + n * 8 + tig * 2;
+                cv[n][2 * h] = cv[n][2 * h] + round_bf16(sp[n][2 * h]) + sB[c];
+                cv[n][2 * h + 1] = cv[n][2 * h + 1] + round_bf16(sp[n][2 * h + 1]) + sB[c + 1];
+                if (a.aux) *reinterpret_cast<uint32_t *>(px + (m0 + gid + 8 * h) * LW + c) = pack_bf16(cv[n][2 * h], cv[n][2 * h + 1]);
+              }
+            if (a.aux) {
+              __syncwarp();
+              store_rows16<W, CW>(a.aux + (size_t)row * nx * W, px, m0, c0);
+              __syncwarp();
             }
           }
-        }
-        for (int k = 0; k < kin; k += 16) {
-          uint32_t fa[4], fb[4];
-          frag_a(fa, st, lin, m0, k);
 #pragma unroll
-          for (int n = 0; n < NT; n += 2) {
-            if (KIND == ROW_BWD) frag_bt(fb, sW, LW, n * 8, k);
-            else frag_b(fb, sW, LW, n * 8, k);
-            mma_bf16(cv[n], fa, fb);
-            mma_bf16(cv[n + 1], fa, fb + 2);
-          }
-        }
-        __syncwarp();   // the warp's pixels have been read
-        const bf16 *sP = st + L::in(nx, a.cin) + L::spec();
-        if (KIND == ROW_FWD && a.aux) {
-#pragma unroll
-          for (int n = 0; n < NT; n++)
+          for (int n = 0; n < CT; n++)
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-              const int c = n * 8 + tig * 2, p = m0 + gid + 8 * h;
-              *reinterpret_cast<uint32_t *>(px + p * LW + c) =
-                  pack_bf16(cv[n][2 * h] + round_bf16(sp[n][2 * h]) + sB[c], cv[n][2 * h + 1] + round_bf16(sp[n][2 * h + 1]) + sB[c + 1]);
-            }
-          __syncwarp();
-          store_rows16<W>(a.aux + (size_t)row * nx * W, px, m0);
-          __syncwarp();
-        }
-#pragma unroll
-        for (int n = 0; n < NT; n++)
-#pragma unroll
-          for (int h = 0; h < 2; h++) {
-            const int c = n * 8 + tig * 2, p = m0 + gid + 8 * h;
-            float x = cv[n][2 * h], y = cv[n][2 * h + 1];
-            if (KIND == ROW_LIFT) {
-              x += sB[c];
-              y += sB[c + 1];
-            } else if (KIND == ROW_FWD) {
-              x = gelu_f(x + round_bf16(sp[n][2 * h]) + sB[c]);
-              y = gelu_f(y + round_bf16(sp[n][2 * h + 1]) + sB[c + 1]);
-            } else {
-              x = sp[n][2 * h] + round_bf16(x);
-              y = sp[n][2 * h + 1] + round_bf16(y);
-              if (a.pre) {
-                const float2 q = unpack_bf16(*reinterpret_cast<const uint32_t *>(sP + p * LW + c));
-                x = round_bf16(x) * gelu_grad_f(q.x);
-                y = round_bf16(y) * gelu_grad_f(q.y);
+              const int c = c0 + n * 8 + tig * 2;
+              uint32_t *at = reinterpret_cast<uint32_t *>(px + (m0 + gid + 8 * h) * LW + c);
+              float x = cv[n][2 * h], y = cv[n][2 * h + 1];
+              if (KIND == ROW_LIFT) {
+                x += sB[c];
+                y += sB[c + 1];
+              } else if (KIND == ROW_FWD) {
+                x = gelu_f(x);
+                y = gelu_f(y);
+              } else {
+                x = sp[n][2 * h] + round_bf16(x);
+                y = sp[n][2 * h + 1] + round_bf16(y);
+                if (pre) {
+                  const uint32_t q = *at;
+                  x = round_bf16(x) * gelu_grad_lut(q & 0xffffu, sG);
+                  y = round_bf16(y) * gelu_grad_lut(q >> 16, sG);
+                }
               }
+              *at = pack_bf16(x, y);
             }
-            *reinterpret_cast<uint32_t *>(px + p * LW + c) = pack_bf16(x, y);
-          }
+        }
         __syncwarp();
-        store_rows16<W>(a.out + (size_t)row * nx * W, px, m0);
+        store_rows16<W, W>(a.out + (size_t)row * nx * W, px, m0, 0);
       }
     }
     if (a.spec_out) {
@@ -346,7 +401,7 @@ __global__ void __launch_bounds__(RT) last_kernel(const LastArgs a)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
   bf16 *sW = reinterpret_cast<bf16 *>(rsm);
   bf16 *sS = sW + W * LW + warp * (RK * LW + 16 * LW + 16 * LE), *sH = sS + RK * LW, *sI = sH + 16 * LW;
-  copy_tile(sW, LW, a.wt, W, W, W, RT);
+  copy_tile<W>(sW, LW, a.wt, W, W, W, RT);
   cp_async_commit();
   const int row = blockIdx.x * 8 + warp;
   const bool on = row < a.rows;
@@ -416,7 +471,7 @@ struct YArgs {
   const bf16 *A;         // My [4m][2ny], or its transpose [2ny][4m] for the synthesis
   const bf16 *B;         // analysis [b][2ny][m w]; synthesis [b][4m][m w]
   bf16 *C;               // analysis: mode-major [(j, kx)][b][part][w]; synthesis [b][2ny][m w]
-  int ny, m, w, batch;
+  int ny, m, batch;
 };
 __host__ __device__ inline size_t y_analysis_smem(int ny) { return 2 * ((size_t)64 * (2 * ny + 8) + (size_t)2 * ny * YL); }
 __host__ __device__ inline size_t y_synthesis_smem(int ny) { return 2 * ((size_t)2 * ny * 72 + (size_t)64 * YL + (size_t)8 * 16 * YL); }
@@ -432,20 +487,21 @@ __device__ __forceinline__ void copy_cols(bf16 *s, const bf16 *g, long ldg, int 
 }
 
 // warp w: rows 16 (w % 4) .., columns 64 (w / 4) ..
+template <int W>
 __global__ void __launch_bounds__(RT, 2) y_analysis(const YArgs a)
 {
   extern __shared__ __align__(16) unsigned char rsm[];
-  const int K = 2 * a.ny, LA = K + 8, M = 4 * a.m, N = a.m * a.w, n0 = blockIdx.x * YN, b = blockIdx.y;
+  const int K = 2 * a.ny, LA = K + 8, M = 4 * a.m, N = a.m * W, n0 = blockIdx.x * YN, b = blockIdx.y;
   bf16 *sA = reinterpret_cast<bf16 *>(rsm), *sB = sA + 64 * LA;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
   const int m0 = (warp & 3) * 16, c0 = (warp >> 2) * 64;
   // everything in flight at once, in four parts of k that are computed as they land
-  const int part = (K / 4 + 15) / 16 * 16;
+  constexpr int part = 2 * RNY / 4;
   for (int q = 0; q < 4; q++) {
-    const int k0 = min(q * part, K), k1 = min(k0 + part, K), per = (k1 - k0) / 8;
-    for (int e = threadIdx.x; e < M * per; e += RT) {
-      const int r = e / per, c = k0 + (e - r * per) * 8;
-      cp_async16(smem_addr(sA + r * LA + c), a.A + (size_t)r * K + c, 16);
+    const int k0 = min(q * part, K), k1 = min(k0 + part, K);
+    for (int e = threadIdx.x; e < M * (part / 8); e += RT) {
+      const int r = e / (part / 8), c = k0 + (e % (part / 8)) * 8;
+      if (c < k1) cp_async16(smem_addr(sA + r * LA + c), a.A + (size_t)r * K + c, 16);
     }
     copy_cols(sB, a.B + (size_t)b * K * N, N, k0, k1, n0, N);
     cp_async_commit();
@@ -476,23 +532,25 @@ __global__ void __launch_bounds__(RT, 2) y_analysis(const YArgs a)
     for (int h = 0; h < 2; h++) {
       const int r = m0 + gid + 8 * h, col = n0 + c0 + n * 8 + tig * 2;
       if (r >= M || col >= N) continue;
-      const int j = r >> 1, pt = r & 1, kx = col / a.w, c = col - kx * a.w;
-      *reinterpret_cast<uint32_t *>(a.C + (((size_t)(j * a.m + kx) * a.batch + b) * 2 + pt) * a.w + c) = pack_bf16(acc[n][2 * h], acc[n][2 * h + 1]);
+      const int j = r >> 1, pt = r & 1, kx = col / W, c = col - kx * W;
+      *reinterpret_cast<uint32_t *>(a.C + (((size_t)(j * a.m + kx) * a.batch + b) * 2 + pt) * W + c) = pack_bf16(acc[n][2 * h], acc[n][2 * h + 1]);
     }
 }
 
 // warp w: rows 16 w, 16 w + 128, ..; its 16 x YN results leave through a patch of shared memory in
 // 16-byte stores
+template <int W>
 __global__ void __launch_bounds__(RT, 2) y_synthesis(const YArgs a)
 {
   extern __shared__ __align__(16) unsigned char rsm[];
-  const int K = 4 * a.m, K16 = (K + 15) / 16 * 16, M = 2 * a.ny, N = a.m * a.w, n0 = blockIdx.x * YN, b = blockIdx.y;
+  const int K = 4 * a.m, K16 = (K + 15) / 16 * 16, M = 2 * a.ny, N = a.m * W, n0 = blockIdx.x * YN, b = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
   bf16 *sA = reinterpret_cast<bf16 *>(rsm), *sB = sA + M * 72, *sO = sB + 64 * YL + warp * 16 * YL;
   copy_cols(sB, a.B + (size_t)b * K * N, N, 0, K, n0, N);
   zero_rows(sB, YL, K, K16, RT);
   if (K % 8 == 0) {
-    copy_tile(sA, 72, a.A, K, M, K, RT);
+    for (int e = threadIdx.x; e < M * 8; e += RT)
+      if ((e & 7) * 8 < K) cp_async16(smem_addr(sA + (e >> 3) * 72 + (e & 7) * 8), a.A + (size_t)(e >> 3) * K + (e & 7) * 8, 16);
     if (K16 > K)
       for (int e = threadIdx.x; e < M * (K16 - K); e += RT) sA[(e / (K16 - K)) * 72 + K + e % (K16 - K)] = __float2bfloat16(0.f);
   } else {
@@ -550,7 +608,7 @@ template <int W>
 __device__ __forceinline__ void mode_load_z(bf16 *s, const bf16 *g, int rows)
 {
   constexpr int LZ = 2 * W + 8;
-  copy_tile(s, LZ, g, 2 * W, rows, 2 * W, RT);
+  copy_tile<2 * W>(s, LZ, g, 2 * W, rows, 2 * W, RT);
   zero_rows(s, LZ, rows, MB, RT);
 }
 
@@ -601,8 +659,8 @@ __global__ void __launch_bounds__(RT) mode_mix(const ModeArgs a)
   extern __shared__ __align__(16) unsigned char rsm[];
   bf16 *sRe = reinterpret_cast<bf16 *>(rsm), *sIm = sRe + W * LW, *sZ = sIm + W * LW;
   const int mode = blockIdx.x;
-  copy_tile(sRe, LW, a.Wre + (size_t)mode * W * W, W, W, W, RT);
-  copy_tile(sIm, LW, a.Wim + (size_t)mode * W * W, W, W, W, RT);
+  copy_tile<W>(sRe, LW, a.Wre + (size_t)mode * W * W, W, W, W, RT);
+  copy_tile<W>(sIm, LW, a.Wim + (size_t)mode * W * W, W, W, W, RT);
   for (int b0 = 0; b0 < a.batch; b0 += MB) {
     if (b0) __syncthreads();
     mode_load_z<W>(sZ, a.Z + ((size_t)mode * a.batch + b0) * 2 * W, min(MB, a.batch - b0));
@@ -625,8 +683,8 @@ __global__ void __launch_bounds__(RT) mode_grad(const ModeArgs a)
   extern __shared__ __align__(16) unsigned char rsm[];
   bf16 *sRe = reinterpret_cast<bf16 *>(rsm), *sIm = sRe + W * LW, *sZ = sIm + W * LW, *sY = sZ + MB * LZ;
   const int mode = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
-  copy_tile(sRe, LW, a.Wre + (size_t)mode * W * W, W, W, W, RT);
-  copy_tile(sIm, LW, a.Wim + (size_t)mode * W * W, W, W, W, RT);
+  copy_tile<W>(sRe, LW, a.Wre + (size_t)mode * W * W, W, W, W, RT);
+  copy_tile<W>(sIm, LW, a.Wim + (size_t)mode * W * W, W, W, W, RT);
   float acc[U][4][2][4] = {};   // re-re, im-im, re-im, im-re
   for (int b0 = 0; b0 < a.batch; b0 += MB) {
     if (b0) __syncthreads();
@@ -677,13 +735,18 @@ __global__ void __launch_bounds__(RT) mode_grad(const ModeArgs a)
 // ascending; X [pixels][R], dY [pixels][W].  Where kc is a multiple of CSP, also the column sums of
 // dY over every CSP pixels (sums: [pixels / CSP][W]) while its rows are in shared memory: RT / W
 // lanes per column, each over every (RT / W)-th pixel, added in lane order.
-constexpr int WGK = 128, WGS = 2, CSP = 1024;   // pixels per stage, stages, pixels per column sum
-inline size_t wgrad_smem(int R, int W) { return 2 * (size_t)WGS * WGK * (R + 8 + W + 8); }
+// At batch 32 there are 256 chunks for 152 SMs: two stages of copies ahead of the one in use keep
+// enough bytes in flight (one ahead: 41 us; half the columns per CTA: 57).
+constexpr int WGK = 128, WGS = 3, CSP = 1024;   // pixels per stage, stages, pixels per column sum
+template <int W> size_t wgrad_smem(int R) { return 2 * (size_t)WGS * WGK * (R + 8 + W + 8); }
 
-template <int W>
-__global__ void __launch_bounds__(RT) weight_grad_partial(const bf16 *X, int R, const bf16 *dY, int kc, float *partial, float *sums)
+// (RC: R where it is known, else 0; WHOLE: kc is a multiple of WGK -- both let the inner loop unroll
+// with fixed addresses)
+template <int W, int RC, bool WHOLE>
+__global__ void __launch_bounds__(RT) weight_grad_partial(const bf16 *X, int r_dyn, const bf16 *dY, int kc, float *partial, float *sums)
 {
-  constexpr int LW = W + 8, NP = W / 16, U = 2;   // 16 x 16 tiles, at most 4 x 4 over 8 warps
+  constexpr int LW = W + 8, NP = W / 16, U = RC ? (RC / 16 * NP + 7) / 8 : 2;   // 16 x 16 tiles, at most 4 x 4 over 8 warps
+  const int R = RC ? RC : r_dyn;
   extern __shared__ __align__(16) unsigned char rsm[];
   const int LR = R + 8, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
   const size_t p0 = (size_t)blockIdx.x * kc;
@@ -693,41 +756,52 @@ __global__ void __launch_bounds__(RT) weight_grad_partial(const bf16 *X, int R, 
     if (i < nst) {
       bf16 *s = st + (i % WGS) * stage;
       const int n = min(WGK, kc - i * WGK);
-      copy_tile(s, LR, X + (p0 + (size_t)i * WGK) * R, R, n, R, RT);
-      copy_tile(s + WGK * LR, LW, dY + (p0 + (size_t)i * WGK) * W, W, n, W, RT);
+      copy_tile<RC>(s, LR, X + (p0 + (size_t)i * WGK) * R, R, n, R, RT);
+      copy_tile<W>(s + WGK * LR, LW, dY + (p0 + (size_t)i * WGK) * W, W, n, W, RT);
     }
     cp_async_commit();
   };
-  constexpr int LANES = RT / W;
+  constexpr int LANES = RT / W, W2 = W / 2;
   __shared__ float sc[RT];
-  const int lane_c = threadIdx.x / W, col = threadIdx.x % W;
+  const int lane_c = threadIdx.x / W2, col = (threadIdx.x % W2) * 2;   // two columns a thread
   int next = lane_c;   // this lane's next pixel of the column sum
-  float csum = 0.f;
-  load(0);
+  float csum0 = 0.f, csum1 = 0.f;
+  for (int i = 0; i < WGS - 1; i++) load(i);
   float acc[U][2][4] = {};
   for (int i = 0; i < nst; i++) {
-    load(i + 1);   // (its stage was freed by the barrier that ended the previous pass)
-    cp_async_wait<1>();
+    load(i + WGS - 1);   // (its stage was freed by the barrier that ended the previous pass)
+    cp_async_wait<WGS - 1>();
     __syncthreads();
     const bf16 *sX = st + (i % WGS) * stage, *sY = sX + WGK * LR;
-    for (int k = 0; k < min(WGK, kc - i * WGK); k += 16)
+    const int kn = WHOLE ? WGK : min(WGK, kc - i * WGK);
 #pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int t = warp + 8 * u;
-        if (t >= units) break;
-        uint32_t fa[4], fb[4];
-        frag_at(fa, sX, LR, (t / NP) * 16, k);
-        frag_b(fb, sY, LW, (t % NP) * 16, k);
-        mma_bf16(acc[u][0], fa, fb);
-        mma_bf16(acc[u][1], fa, fb + 2);
+    for (int u = 0; u < U; u++) {
+      const int t = warp + 8 * u;
+      if (t < units) {
+#pragma unroll(WHOLE ? WGK / 16 : 1)
+        for (int k = 0; k < kn; k += 16) {
+          uint32_t fa[4], fb[4];
+          frag_at(fa, sX, LR, (t / NP) * 16, k);
+          frag_b(fb, sY, LW, (t % NP) * 16, k);
+          mma_bf16(acc[u][0], fa, fb);
+          mma_bf16(acc[u][1], fa, fb + 2);
+        }
       }
+    }
     if (sums) {
       const int at = (i * WGK) % CSP;   // this stage's first pixel within its column sum
       if (lane_c < LANES)
 #pragma unroll 8
-        for (; next < at + WGK; next += LANES) csum += __bfloat162float(sY[(next - at) * LW + col]);
+        for (; next < at + WGK; next += LANES) {
+          const float2 v = unpack_bf16(*reinterpret_cast<const uint32_t *>(sY + (next - at) * LW + col));
+          csum0 += v.x;
+          csum1 += v.y;
+        }
       if (at + WGK == CSP) {
-        sc[threadIdx.x] = csum;
+        if (lane_c < LANES) {
+          sc[lane_c * W + col] = csum0;
+          sc[lane_c * W + col + 1] = csum1;
+        }
         __syncthreads();
         if (threadIdx.x < W) {
           float t = 0.f;
@@ -735,7 +809,7 @@ __global__ void __launch_bounds__(RT) weight_grad_partial(const bf16 *X, int R, 
           sums[((p0 + (size_t)i * WGK) / CSP) * W + threadIdx.x] = t;
         }
         next = lane_c;
-        csum = 0.f;
+        csum0 = csum1 = 0.f;
       }
     }
     __syncthreads();
@@ -777,7 +851,8 @@ template <int W> __host__ __device__ constexpr size_t dec_bwd_smem(int hid)
 template <int W>
 __device__ __forceinline__ void dec_weights(bf16 *sW1, bf16 *sW2, const DecArgs &a)
 {
-  copy_tile(sW1, a.hid + 8, a.w1, a.hid, W, a.hid, RT);
+  if (a.hid == DH) copy_tile<DH>(sW1, a.hid + 8, a.w1, a.hid, W, a.hid, RT);
+  else copy_tile(sW1, a.hid + 8, a.w1, a.hid, W, a.hid, RT);
   for (int e = threadIdx.x; e < a.hid * DN; e += RT) {
     const int r = e / DN, c = e - r * DN;
     sW2[r * DLN + c] = (c < a.ns) ? a.w2[r * a.ns + c] : __float2bfloat16(0.f);
@@ -870,8 +945,9 @@ __global__ void __launch_bounds__(RT, 2) dec_bwd(const DecArgs a)
   zero_rows(sP, DLN, a.ny, rows, RT);
   for (int u = blockIdx.x; u < a.rows / a.ny; u += gridDim.x) {
     const size_t r0 = (size_t)u * a.ny;
-    copy_tile(sD0, LW, a.d0 + r0 * W, W, a.ny, W, RT);
-    copy_tile(sD1, LH, a.d1 + r0 * a.hid, a.hid, a.ny, a.hid, RT);
+    copy_tile<W>(sD0, LW, a.d0 + r0 * W, W, a.ny, W, RT);
+    if (a.hid == DH) copy_tile<DH>(sD1, LH, a.d1 + r0 * a.hid, a.hid, a.ny, a.hid, RT);
+    else copy_tile(sD1, LH, a.d1 + r0 * a.hid, a.hid, a.ny, a.hid, RT);
     cp_async_commit();
     for (int e = threadIdx.x; e < a.ny * DN; e += RT) {
       const int r = e / DN, c = e - r * DN;
