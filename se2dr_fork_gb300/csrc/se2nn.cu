@@ -16,6 +16,8 @@
 #include <cstdlib>
 #include <cstring>
 #include <initializer_list>
+#include <thread>
+#include <unistd.h>
 #include <vector>
 
 #include "se2nn.h"
@@ -1157,12 +1159,58 @@ extern "C" int se2nn_set_stream(se2nn *h, void *stream)
   return 0;
 }
 
+// Device -> the caller's host array.  A device that reads and writes pageable host memory
+// (cudaDevAttrPageableMemoryAccess) stores straight into it, after the host threads have
+// faulted its pages in; a copy of 68 MB through the driver's staging buffers took 3.3 ms.
+__global__ void k_copy_out(const float *__restrict__ src, float *__restrict__ dst, long n)
+{
+  const long n4 = ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) ? n / 4 : 0;
+  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x, step = (long)gridDim.x * blockDim.x;
+  for (long i = t; i < n4; i += step) reinterpret_cast<float4 *>(dst)[i] = reinterpret_cast<const float4 *>(src)[i];
+  for (long i = 4 * n4 + t; i < n; i += step) dst[i] = src[i];
+}
+
+static int copy_out(se2nn *h, float *dst, const float *src, long n)
+{
+  int dev = 0, pageable = 0;
+  cudaPointerAttributes at;
+  if (n < (1L << 18) || cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type == cudaMemoryTypeDevice || cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, dev) != cudaSuccess || !pageable) {
+    cudaGetLastError();
+    NCK(h, cudaStreamSynchronize(h->stream));
+    NCK(h, cudaMemcpy(dst, src, n * 4, cudaMemcpyDeviceToHost));
+    return 0;
+  }
+  // one store per page, on up to 16 threads (this overlaps the kernels still in flight)
+  const long per = std::max(4096L, sysconf(_SC_PAGESIZE)) / (long)sizeof(float), pages = (n + per - 1) / per;
+  const int nt = (int)std::min<long>(std::max(1u, std::min(16u, std::thread::hardware_concurrency())), (pages + 63) / 64);
+  auto touch = [&](int k) {
+    volatile float *q = dst;
+    for (long i = pages * k / nt; i < pages * (k + 1) / nt; i++) q[i * per] = 0.f;
+  };
+  {
+    std::thread th[16];
+    for (int k = 1; k < nt; k++) {
+      try {
+        th[k] = std::thread(touch, k);
+      } catch (...) {   // (no more threads: this one does the part)
+        touch(k);
+      }
+    }
+    touch(0);
+    for (std::thread &t : th)
+      if (t.joinable()) t.join();
+  }
+  k_copy_out<<<4 * h->nsm, EW, 0, h->stream>>>(src, dst, n);
+  NCK(h, cudaGetLastError());
+  NCK(h, cudaStreamSynchronize(h->stream));
+  return 0;
+}
+
 extern "C" int se2nn_get_params(se2nn *h, float *p)
 {
   if (!h || !p) return -1;
-  NCK(h, cudaStreamSynchronize(h->stream));
-  NCK(h, cudaMemcpy(p, h->params, h->P * 4, cudaMemcpyDeviceToHost));
-  return 0;
+  return copy_out(h, p, h->params, h->P);
 }
 
 extern "C" int se2nn_set_params(se2nn *h, const float *p)
@@ -1179,9 +1227,7 @@ extern "C" int se2nn_set_params(se2nn *h, const float *p)
 extern "C" int se2nn_get_grads(se2nn *h, float *g)
 {
   if (!h || !g) return -1;
-  NCK(h, cudaStreamSynchronize(h->stream));
-  NCK(h, cudaMemcpy(g, h->grads, h->P * 4, cudaMemcpyDeviceToHost));
-  return 0;
+  return copy_out(h, g, h->grads, h->P);
 }
 
 extern "C" int se2nn_set_receivers(se2nn *h, const int *rec_x)
