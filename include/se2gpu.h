@@ -135,8 +135,7 @@ int se2gpu_device_fields(const se2gpu_solver *h, void **u, void **v, void **a);
    CTA) available for the handle's degree and precision, for the autotuner;
    returns how many exist.  se2gpu_set_tile_config selects one; se2gpu_tile_config
    returns the selected one (a new handle starts with the configuration measured
-   fastest for its degree on GB300 in the plain and Kahan modes; 0 in the FP64 mode and,
-   but for large meshes of degree 7, in the two-float mode). */
+   fastest for its degree and mesh size on GB300; 0 in the FP64 mode). */
 int se2gpu_tile_configs(const se2gpu_solver *h, int *edge, int *threads, int max_configs);
 int se2gpu_set_tile_config(se2gpu_solver *h, int config);
 int se2gpu_tile_config(const se2gpu_solver *h);

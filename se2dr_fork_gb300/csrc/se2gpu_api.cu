@@ -512,6 +512,11 @@ static int setup_f32_config(se2gpu_solver *h, int config, bool in_create = false
 
 extern "C" int se2gpu_create(const se2gpu_problem *P, int precision, int trace_capacity, se2gpu_solver **out)
 {
+  return se2gpu_internal_create(P, precision, trace_capacity, false, out);
+}
+
+int se2gpu_internal_create(const se2gpu_problem *P, int precision, int trace_capacity, bool in_ensemble, se2gpu_solver **out)
+{
   if (!out) return fail(nullptr, SE2GPU_ERR_ARG, "null output handle");
   *out = nullptr;
   if (!P) return fail(nullptr, SE2GPU_ERR_ARG, "null problem");
@@ -701,7 +706,7 @@ extern "C" int se2gpu_create(const se2gpu_problem *P, int precision, int trace_c
       if (e != cudaSuccess) { fail(h, SE2GPU_ERR_CUDA, "constant tables: %s", cudaGetErrorString(e)); TRY(SE2GPU_ERR_CUDA); }
       h->src_elem_h = new std::vector<int>(P->src_elem, P->src_elem + P->nsrc);
       h->rec_elem_h = new std::vector<int>(P->rec_elem, P->rec_elem + P->nrec);
-      TRY(setup_f32_config(h, se2p::default_config(P->p, pmode(h), P->mx, P->my, h->nsm), true));
+      TRY(setup_f32_config(h, se2p::default_config(P->p, pmode(h), in_ensemble ? 0 : P->mx, P->my, h->nsm), true));
     }
     for (cudaEvent_t &ev : h->side_done) {
       const cudaError_t e = cudaStreamWaitEvent(h->stream, ev, 0);

@@ -259,7 +259,7 @@ extern "C" int se2gpu_ensemble_create(const se2gpu_problem *shots, int nshots, i
   e->rec_off.assign(nshots + 1, 0);
   for (int s = 0; s < nshots; s++) {
     se2gpu_solver *h = nullptr;
-    if (se2gpu_create(&shots[s], precision, 0, &h) != 0) {
+    if (se2gpu_internal_create(&shots[s], precision, 0, true, &h) != 0) {
       efail(e, SE2GPU_ERR_ARG, "shot %d: %s", s, se2gpu_create_error());
       TRY(SE2GPU_ERR_ARG);
     }

@@ -74,14 +74,25 @@ static const Entry *find(int p, int config)
 }
 
 // the configuration a handle starts with.  Plain and Kahan: per degree the one the autotuner
-// measured fastest on GB300 at about 16M nodes (and, at degree 4, at the 2048^2 workload).
-// Two-float: 0, and at degree 7 its 5 x 5 tiles once they reach every SM (301 against 336 us
-// at 2.5M nodes, 43 against 47 at 262000; 26 against 19 at 20000)
+// measured fastest on GB300 at about 16M nodes (and, at degree 4, at the 2048^2 workload; the
+// plain mode at degree 8 runs 4 x 4 tiles: 83 against 93 us a step at 5M nodes, 7.0 against 9.6 at
+// 260000), and smaller tiles on meshes that these divide into about one per SM (us a step: degree
+// 1, 17 x 17 elements 3.55 -> 3.39; degree 2, 35 x 35 4.92 -> 4.21; degree 5, 28 x 28 6.23 ->
+// 5.53; degree 6, 12 x 12 5.96 -> 5.44, but 58 x 58 5.50 -> 6.24; plain degree 8, 31 x 31
+// 6.52 -> 5.60).  Two-float: 0, and at degree 7 its 5 x 5 tiles once they reach every SM (301
+// against 336 us at 2.5M nodes, 43 against 47 at 262000; 26 against 19 at 20000).
+// mx = 0: the large-mesh choice (the ensemble's, whose shots share one).
 int default_config(int p, int mode, int mx, int my, int nsm)
 {
-  if (mode == MODE_DF) return (p == 7 && (long)((mx + 4) / 5) * ((my + 4) / 5) >= nsm) ? 1 : 0;
-  static const int best[8] = {2, 0, 2, 1, 2, 0, 2, 1};
-  return (p >= 1 && p <= 8 && best[p - 1] < num_configs(p)) ? best[p - 1] : 0;
+  if (p < 1 || p > 8) return 0;
+  auto tiles = [&](int config) {
+    const Entry *e = find(p, config);
+    return (mx == 0 || !e) ? 1L << 40 : (long)((mx + e->te - 1) / e->te) * ((my + e->te - 1) / e->te);
+  };
+  if (mode == MODE_DF) return (p == 7 && tiles(1) >= nsm) ? 1 : 0;
+  static const int best[8] = {2, 0, 2, 1, 2, 0, 2, 1}, small[8] = {1, 2, 2, 1, 1, 1, 2, 1};
+  if (tiles(small[p - 1]) <= ((p == 2 || p == 8) ? 2 : 1) * (long)nsm) return small[p - 1];
+  return (p == 8 && mode == MODE_PLAIN) ? 0 : best[p - 1];
 }
 
 int num_configs(int p)

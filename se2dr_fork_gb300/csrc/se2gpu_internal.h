@@ -50,6 +50,9 @@ struct se2gpu_solver {
   char err[512];
 };
 
+// se2gpu_create; in_ensemble: the tile configuration that all shots of a degree share, whatever the
+// mesh size
+int se2gpu_internal_create(const se2gpu_problem *P, int precision, int trace_capacity, bool in_ensemble, se2gpu_solver **out);
 // FP32 persistent-kernel parameters of a handle (no per-step pointers set)
 se2p::Params se2gpu_internal_f32_params(se2gpu_solver *h);
 // set the thread's message returned by se2gpu_last_error(NULL)
