@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "se2gpu.h"
+#include "se2gpu_f32df_launch.h"
 #include "se2gpu_f64_launch.h"
 #include "se2gpu_internal.h"
 #include "se2gpu_launch.h"
@@ -454,7 +455,7 @@ static int setup_f32_config(se2gpu_solver *h, int config, bool in_create = false
     cudaError_t e = se2p::prepare(h->p, config, mode);
     if (e != cudaSuccess) return fail(h, SE2GPU_ERR_CUDA, "persistent kernel set-up: %s", cudaGetErrorString(e));
   }
-  for (int b = 0; b < 2; b++) {
+  for (int b = 0; b < 2 && ts.halo; b++) {
     void *bases[4] = {h->pu[b], kahan ? (void *)h->pcu[b] : (void *)h->pu[b], h->pw[b], kahan ? (void *)h->pcw[b] : (void *)h->pw[b]};
     for (int m = 0; m < 4; m++) {
       const int bw = (m < 2) ? ts.region_w : ts.own_w, bh = (m < 2) ? ts.region_h : ts.own_h;
@@ -468,7 +469,9 @@ static int setup_f32_config(se2gpu_solver *h, int config, bool in_create = false
   }
   const int te = ts.tex, P = h->p;
   const int ntx = (h->mx + te - 1) / te, nty = (h->my + te - 1) / te, ntiles = ntx * nty;
-  // tile lists: a source or receiver element appears in every tile whose owned nodes it touches
+  // tile lists: a source or receiver element appears in every tile whose owned nodes it touches, or
+  // whose nodes it touches where a tile finishes the node lines that it shares with the next ones
+  const int far = ts.halo ? 0 : 1;
   auto build = [&](const std::vector<int> &elems, std::vector<int> &off, std::vector<int> &ent) {
     std::vector<std::vector<int>> per(ntiles);
     for (int q = 0; q < (int)elems.size(); q++) {
@@ -477,7 +480,7 @@ static int setup_f32_config(se2gpu_solver *h, int config, bool in_create = false
         for (int tx = std::max(0, (ex - 1) / te); tx <= std::min(ntx - 1, (ex + 1) / te); tx++) {
           const int X0 = tx * te * P, X1 = std::min((tx + 1) * te, h->mx) * P + (((tx + 1) * te >= h->mx) ? 1 : 0);
           const int Y0 = ty * te * P, Y1 = std::min((ty + 1) * te, h->my) * P + (((ty + 1) * te >= h->my) ? 1 : 0);
-          if (ex * P <= X1 - 1 && ex * P + P >= X0 && ey * P <= Y1 - 1 && ey * P + P >= Y0) per[ty * ntx + tx].push_back(q);
+          if (ex * P <= X1 - 1 + far && ex * P + P >= X0 && ey * P <= Y1 - 1 + far && ey * P + P >= Y0) per[ty * ntx + tx].push_back(q);
         }
     }
     off.assign(ntiles + 1, 0);
@@ -504,6 +507,7 @@ static int setup_f32_config(se2gpu_solver *h, int config, bool in_create = false
   if ((rc = upload_i(h, (int **)&h->tile_src, si.data(), si.size()))) return rc;
   if ((rc = upload_i(h, (int **)&h->tile_rec, ri.data(), ri.size()))) return rc;
   h->pconfig = config;
+  h->df_no_halo = !ts.halo;
   h->pntx = ntx;
   h->pnty = nty;
   h->pgrid = std::min(ntiles + 1, std::max(1, se2p::occupancy(P, config, mode)) * h->nsm);
@@ -647,6 +651,7 @@ int se2gpu_internal_create(const se2gpu_problem *P, int precision, int trace_cap
       TRY(dzero(h, (void **)&h->rbuf[b], (size_t)P->nrec * npe * rbuf_values(h) * 4));
     }
     TRY(dalloc(h, (void **)&h->pa, np * 8 * (df ? 2 : 1)));   // two-float mode: low parts after the high
+    for (int b = 0; b < 2 && df; b++) TRY(dalloc(h, (void **)&h->ef[b], (size_t)ne * npe * 16));   // element forces
     if (!df) {
       TRY(dalloc(h, (void **)&h->cellc, (size_t)ne * sizeof(float4)));
       k_cell_consts<<<(int)std::min<long>((ne + 255) / 256, 8L * h->nsm), 256, 0, h->stream>>>(
@@ -903,6 +908,36 @@ static int advance_f64(se2gpu_solver *h, int nsteps)
   return 0;
 }
 
+// two-float steps without a halo: START, MIDDLE per step but the last, LAST (se2gpu_f32df.cuh); a launch
+// that finishes a step records its receivers' elements and samples those of the step before
+static int advance_df(se2gpu_solver *h, int nsteps)
+{
+  se2p::DfParams q;
+  q.p = f32_params(h);
+  for (int k = 0; k <= nsteps; k++) {
+    const int in = h->cur, outb = 1 - h->cur;
+    q.mode = (k == 0) ? se2p::DF_START : (k == nsteps) ? se2p::DF_LAST : se2p::DF_MIDDLE;
+    q.u_in = h->pu[in]; q.w_in = h->pw[in]; q.cu_in = h->pcu[in]; q.cw_in = h->pcw[in];
+    q.ef_in = (const float4 *)h->ef[(k + 1) & 1]; q.ef_out = (float4 *)h->ef[k & 1];
+    q.p.u_out = h->pu[outb]; q.p.w_out = h->pw[outb]; q.p.cu_out = h->pcu[outb]; q.p.cw_out = h->pcw[outb];
+    q.p.a_out = h->pa;
+    q.p.stf = k ? h->stf_dev + (size_t)(k - 1) * h->nsrc : nullptr;
+    q.p.rbuf_in = h->rbuf[h->rlast];
+    q.p.rbuf_out = h->rbuf[1 - h->rlast];
+    q.p.record = h->pending_record ? 1 : 0;
+    q.p.trace_row = h->traces + (size_t)h->rows_written * 7 * h->nrec;
+    h->launches++;
+    cudaError_t e = se2p::df_launch(h->p, h->pconfig, q, k > 0, h->stream);
+    if (e != cudaSuccess) return fail(h, SE2GPU_ERR_CUDA, "step kernel: %s", cudaGetErrorString(e));
+    if (h->pending_record) { h->rows_written++; h->pending_record = false; }
+    if (k == 0) continue;   // (no step is finished yet)
+    h->cur = outb;
+    h->rlast = 1 - h->rlast;
+    if (h->nrec > 0) h->pending_record = true;
+  }
+  return 0;
+}
+
 static int advance_f32(se2gpu_solver *h, int nsteps)
 {
   auto prm = f32_params(h);
@@ -949,7 +984,7 @@ extern "C" int se2gpu_advance(se2gpu_solver *h, int nsteps, const double *stf)
     // the previous block may still read stf_dev: order the copy on the stream
     CK(h, cudaMemcpyAsync(h->stf_dev, stf, (size_t)nsteps * h->nsrc * 8, cudaMemcpyHostToDevice, h->stream));
   }
-  return is_f64(h) ? advance_f64(h, nsteps) : advance_f32(h, nsteps);
+  return is_f64(h) ? advance_f64(h, nsteps) : h->df_no_halo ? advance_df(h, nsteps) : advance_f32(h, nsteps);
 }
 
 extern "C" int se2gpu_traces(se2gpu_solver *h, double *out, int max_rows)

@@ -1,10 +1,8 @@
-// se2gpu_f32df.cu -- the persistent step kernel in the two-float mode (every value of a
-// step carried as a float pair, about 48 significant bits), degrees 1..8, over the same
-// tile configurations as the plain and Kahan modes.  A translation unit of its own:
-// the kernels are large and compile in parallel with the others, and this unit's
-// constant tables (high and low parts of D and the GLL weights) are set here.
-#include "se2gpu_persist.cuh"
-#include "se2gpu_persist_launch.h"
+// se2gpu_f32df.cu -- the two-float step kernels (every value of a step carried as a float pair,
+// about 48 significant bits), degrees 1..8.  A translation unit of its own: the kernels are
+// large and compile in parallel with the others, and this unit's constant tables (high and
+// low parts of D and the GLL weights) are set here.
+#include "se2gpu_f32df.cuh"
 
 namespace se2p {
 
@@ -30,30 +28,22 @@ cudaError_t df_set_tables(int p, const double *D, const double *w1d)
 
 namespace {
 
-struct DfEntry {
-  int p, te, nt;
-  size_t smem;
-  const void *fn;
-};
+template <int P, int TE, int NT>
+DfShape df_entry()
+{
+  static_assert(NT >= DfGeo<P, TE>::NE * (P + 1), "one (element, line) item per thread");
+  return DfShape{P, TE, NT, DfGeo<P, TE>::SMEM, (const void *)df_step<P, TE, NT>, false};
+}
 
-// registers sized for 2 CTAs per SM at most (1 with 384 threads or more): the pairs
+// with a halo: registers sized for 2 CTAs per SM at most (1 with 384 threads or more): the pairs
 // double most live values
-template <int P, int TE, int NT, bool WE>
-DfEntry df_entry()
+template <int P, int TE, int NT>
+DfShape halo_entry()
 {
   typedef Layout<P, TE, true, 1, true> L;
   constexpr int MS = min_blocks(L::TOTAL);
   constexpr int M = (NT >= 384) ? 1 : (MS < 2 ? MS : 2);
-  return DfEntry{P, TE, NT, L::TOTAL, (const void *)persist_step<P, TE, NT, true, 1, M, true, WE>};
-}
-
-const DfEntry *df_table(int *n)
-{
-#define SE2P_DF_ENTRY(P, TE, NT, NOB, MINB, WE) df_entry<P, TE, NT, (WE) != 0>(),
-  static DfEntry t[] = {SE2P_CONFIGS(SE2P_DF_ENTRY)};
-#undef SE2P_DF_ENTRY
-  *n = (int)(sizeof(t) / sizeof(t[0]));
-  return t;
+  return DfShape{P, TE, NT, L::TOTAL, (const void *)persist_step<P, TE, NT, true, 1, M, true, false>, true};
 }
 
 template <int P>
@@ -65,19 +55,39 @@ cudaError_t record_t(const Params &prm, cudaStream_t st)
 
 }  // namespace
 
-const void *df_kernel(int p, int config, size_t *smem)
+bool df_shape(int p, int config, DfShape *s)
 {
-  int n, k = 0;
-  const DfEntry *t = df_table(&n);
-  for (int i = 0; i < n; i++)
-    if (t[i].p == p) {
-      if (k == config) {
-        if (smem) *smem = t[i].smem;
-        return t[i].fn;
-      }
-      k++;
+#define SE2P_DF_ENTRY(P, TE, NT) df_entry<P, TE, NT>(),
+#define SE2P_HALO_ENTRY(P, TE, NT) halo_entry<P, TE, NT>(),
+  static const DfShape t[] = {SE2P_DF_CONFIGS(SE2P_DF_ENTRY, SE2P_HALO_ENTRY)};
+#undef SE2P_HALO_ENTRY
+#undef SE2P_DF_ENTRY
+  int k = 0;
+  for (const DfShape &e : t)
+    if (e.p == p && k++ == config) {
+      *s = e;
+      return true;
     }
-  return nullptr;
+  return false;
+}
+
+cudaError_t df_launch(int p, int config, const DfParams &q, bool dependent, cudaStream_t st)
+{
+  DfShape s;
+  if (!df_shape(p, config, &s) || s.halo) return cudaErrorInvalidValue;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(q.p.ntiles + (q.p.record ? 1 : 0));
+  cfg.blockDim = dim3(s.nt);
+  cfg.dynamicSmemBytes = s.smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = dependent ? 1 : 0;
+  DfParams a = q;
+  void *args[] = {&a};
+  return cudaLaunchKernelExC(&cfg, s.fn, args);
 }
 
 cudaError_t df_launch_record(int p, const Params &prm, cudaStream_t st)

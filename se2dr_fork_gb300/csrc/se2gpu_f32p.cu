@@ -5,6 +5,7 @@
 
 #include <algorithm>
 
+#include "se2gpu_f32df_launch.h"
 #include "se2gpu_persist.cuh"
 #include "se2gpu_persist_launch.h"
 
@@ -79,17 +80,36 @@ static const Entry *find(int p, int config)
 // 260000), and smaller tiles on meshes that these divide into about one per SM (us a step: degree
 // 1, 17 x 17 elements 3.55 -> 3.39; degree 2, 35 x 35 4.92 -> 4.21; degree 5, 28 x 28 6.23 ->
 // 5.53; degree 6, 12 x 12 5.96 -> 5.44, but 58 x 58 5.50 -> 6.24; plain degree 8, 31 x 31
-// 6.52 -> 5.60).  Two-float: 0, and at degree 7 its 5 x 5 tiles once they reach every SM (301
-// against 336 us at 2.5M nodes, 43 against 47 at 262000; 26 against 19 at 20000).
+// 6.52 -> 5.60).  Two-float: small tiles with a thread per node while a few of them fill an SM, then those
+// with the fewest idle threads, then (degrees 2 and 3) the halo kernel; the lines lie where the
+// times cross (us a step at 20000 / 80000 / 260000 / 1M nodes, chosen one first): degree 2 6 x 6 5.1 / 8.7
+// / 20.6 / 81, 8 x 8 6.8 / 10.1 / 20.2 / 78, halo 8.6 / 9.1 / 25.4 / 75; 3 5.6 / 8.1 / 20.5 / 78, 7.7 /
+// 9.0 / 19.5 / 72, 7.7 / 9.9 / 22.0 / 69; 4 3 x 3 7.8 / 9.2 / 25 / 96, 5 x 5 10.6 / 11.1 / 20 / 70; 5 2 x 2
+// 8.6 / 10.8 / 24.6 / 95, 4 x 4 12.7 / 12.8 / 22.1 / 74; 6 2 x 2 10.2 / 18.1 / 51 / 196, 3 x 3 14.2 /
+// 13.4 / 21.4 / 82, 6 x 6 19.1 / 17.9 / 24.9 / 79; 7 2 x 2 11.9 / 20.2 / 48 / 177, 4 x 4 18.4 / 17.5 / 24.9
+// / 81; 8 1 x 1 12.4 / 23.5 / 69 / 247, 3 x 3 17.5 / 17.0 / 29 / 100, 5 x 5 24 / 24 / 34 / 92.
 // mx = 0: the large-mesh choice (the ensemble's, whose shots share one).
 int default_config(int p, int mode, int mx, int my, int nsm)
 {
   if (p < 1 || p > 8) return 0;
   auto tiles = [&](int config) {
     const Entry *e = find(p, config);
-    return (mx == 0 || !e) ? 1L << 40 : (long)((mx + e->te - 1) / e->te) * ((my + e->te - 1) / e->te);
+    DfShape df;
+    const int te = (mode == MODE_DF && df_shape(p, config, &df)) ? df.te : e ? e->te : 0;
+    return (mx == 0 || !te) ? 1L << 40 : (long)((mx + te - 1) / te) * ((my + te - 1) / te);
   };
-  if (mode == MODE_DF) return (p == 7 && tiles(1) >= nsm) ? 1 : 0;
+  if (mode == MODE_DF) {
+    switch (p) {
+      case 1: return tiles(1) <= nsm ? 1 : 0;
+      case 2: return tiles(2) <= 4L * nsm ? 2 : tiles(1) <= 16L * nsm ? 1 : 0;
+      case 3: return tiles(2) <= 4L * nsm ? 2 : tiles(1) <= 28L * nsm ? 1 : 0;
+      case 4: return tiles(0) <= 4L * nsm ? 0 : 1;
+      case 5: return tiles(1) <= 6L * nsm ? 1 : 0;
+      case 6: return tiles(2) <= 2L * nsm ? 2 : tiles(0) < 4L * nsm ? 1 : 0;
+      case 7: return tiles(1) <= 2L * nsm ? 1 : 0;
+      default: return tiles(2) <= 5L * nsm ? 2 : tiles(0) < 2L * nsm ? 1 : 0;
+    }
+  }
   static const int best[8] = {2, 0, 2, 1, 2, 0, 2, 1}, small[8] = {1, 2, 2, 1, 1, 1, 2, 1};
   if (tiles(small[p - 1]) <= ((p == 2 || p == 8) ? 2 : 1) * (long)nsm) return small[p - 1];
   return (p == 8 && mode == MODE_PLAIN) ? 0 : best[p - 1];
@@ -106,19 +126,28 @@ int num_configs(int p)
 int config_shape(int p, int config, int mode, TileShape *s)
 {
   const Entry *e = find(p, config);
-  if (!e) return -1;
-  size_t df_smem = 0;
-  if (mode == MODE_DF && !df_kernel(p, config, &df_smem)) return -1;
-  s->tex = s->tey = e->te;
-  s->nt = e->nt;
-  s->region_w = round_up((e->te + 1) * p + 2 + ((p & 1) ? 2 : 0), 2);
-  s->region_h = (e->te + 1) * p + 1;
-  s->own_w = round_up(e->te * p + 2, 2);
-  s->own_h = e->te * p + 1;
-  s->cell_box = e->te + 1;
-  s->minv_w = round_up(e->te * p + 1 + 4, 4);
+  DfShape df;
+  if (!e || (mode == MODE_DF && !df_shape(p, config, &df))) return -1;
+  if (mode == MODE_DF && !df.halo) {
+    *s = TileShape{};   // (no tensor maps; the state of the tile is held once)
+    s->owned_buffers = 1;
+    s->tex = s->tey = df.te;
+    s->nt = df.nt;
+    s->smem = df.smem;
+    return 0;
+  }
+  const int te = (mode == MODE_DF) ? df.te : e->te;
+  s->halo = true;
+  s->tex = s->tey = te;
+  s->nt = (mode == MODE_DF) ? df.nt : e->nt;
+  s->region_w = round_up((te + 1) * p + 2 + ((p & 1) ? 2 : 0), 2);
+  s->region_h = (te + 1) * p + 1;
+  s->own_w = round_up(te * p + 2, 2);
+  s->own_h = te * p + 1;
+  s->cell_box = te + 1;
+  s->minv_w = round_up(te * p + 1 + 4, 4);
   s->owned_buffers = (mode == MODE_DF) ? 1 : e->nob;
-  s->smem = (mode == MODE_DF) ? df_smem : e->smem[mode ? 1 : 0];
+  s->smem = (mode == MODE_DF) ? df.smem : e->smem[mode ? 1 : 0];
   return 0;
 }
 
@@ -127,11 +156,10 @@ cudaError_t prepare(int p, int config, int mode)
   const Entry *e = find(p, config);
   if (!e) return cudaErrorInvalidValue;
   const int k = mode ? 1 : 0;
-  size_t df_smem = 0;
-  const void *dfn = (mode == MODE_DF) ? df_kernel(p, config, &df_smem) : nullptr;
-  if (mode == MODE_DF && !dfn) return cudaErrorInvalidValue;
-  const void *fns[2] = {dfn ? dfn : e->fn[k], e->bfn[k]};
-  const size_t sizes[2] = {dfn ? df_smem : e->smem[k], e->bsmem[k]};
+  DfShape df = {};
+  if (mode == MODE_DF && !df_shape(p, config, &df)) return cudaErrorInvalidValue;
+  const void *fns[2] = {df.fn ? df.fn : e->fn[k], e->bfn[k]};
+  const size_t sizes[2] = {df.fn ? df.smem : e->smem[k], e->bsmem[k]};
   for (int i = 0; i < 2; i++) {
     const void *fn = fns[i];
     cudaError_t r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizes[i]);
@@ -148,10 +176,9 @@ int occupancy(int p, int config, int mode, bool batch)
   int n = 0;
   if (!e) return 1;
   const int k = mode ? 1 : 0;
-  const void *fn = (batch ? e->bfn : e->fn)[k];
-  size_t smem = (batch ? e->bsmem : e->smem)[k];
-  if (mode == MODE_DF && !batch) fn = df_kernel(p, config, &smem);
-  if (!fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, e->nt, smem) != cudaSuccess) {
+  DfShape s{p, e->te, e->nt, (batch ? e->bsmem : e->smem)[k], (batch ? e->bfn : e->fn)[k], true};
+  if (mode == MODE_DF && !batch) df_shape(p, config, &s);
+  if (!s.fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, s.fn, s.nt, s.smem) != cudaSuccess) {
     cudaGetLastError();
     return 1;
   }
@@ -180,14 +207,12 @@ cudaError_t launch_step(int p, int config, int mode, const CUtensorMap *maps, co
 {
   const Entry *e = find(p, config);
   if (!e) return cudaErrorInvalidValue;
-  const void *fn = e->fn[mode ? 1 : 0];
-  size_t smem = e->smem[mode ? 1 : 0];
-  if (mode == MODE_DF) fn = df_kernel(p, config, &smem);
-  if (!fn) return cudaErrorInvalidValue;
+  DfShape s{p, e->te, e->nt, e->smem[mode ? 1 : 0], e->fn[mode ? 1 : 0], true};
+  if (mode == MODE_DF && (!df_shape(p, config, &s) || !s.halo)) return cudaErrorInvalidValue;   // (df_launch)
   Params pc = prm;
   CUtensorMap m0 = maps[0], m1 = maps[1], m2 = maps[2], m3 = maps[3], m4 = maps[4], m5 = maps[5];
   void *args[] = {&m0, &m1, &m2, &m3, &m4, &m5, &pc};
-  return launch(fn, grid, e->nt, args, smem, dependent, st);
+  return launch(s.fn, grid, s.nt, args, s.smem, dependent, st);
 }
 
 cudaError_t launch_batch(int p, int config, bool kahan, const BatchArgs &ba, int grid, bool dependent, cudaStream_t st)

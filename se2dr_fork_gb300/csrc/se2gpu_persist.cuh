@@ -815,14 +815,6 @@ __device__ __forceinline__ bool tile_body_df(const Params &prm, const StepPtrs s
   // ---- 1. derivatives along row j (registers) and column j (to X1), of the
   // displacement relative to the line's first node: (u_k - u_0) + (c_0 - c_k) with the
   // first difference split exactly by TwoSum
-  // From degree 6 on the loops over the output index are rolled (three at a time): unrolled, the
-  // two-float code of one item passes 100 KB and instruction fetch bounds the kernel, and
-  // its registers allow one CTA per SM.  What the rolled loops index goes through the thread's own
-  // exchange rows instead of registers.  Unrolled against rolled, ps per node and step at
-  // 2.5 to 4M nodes: degree 8 238 / 110, 7 175 / 121, 6 86 / 87 (261000 nodes: 99 / 93);
-  // 5 80 / 88, 4 65 / 67.
-  constexpr bool ROLL = P >= 6;
-  constexpr int DU = ROLL ? 3 : N1;
   tf gxr[N1], gyr[N1], Fx[N1], Fy[N1];
   const int base = (ecy * P) * BXW + ecx * P + xoff;
   if (active) {
@@ -839,7 +831,7 @@ __device__ __forceinline__ bool tile_body_df(const Params &prm, const StepPtrs s
         dy[k] = tf_two_sum(uk.y, -u0.y);
         dy[k].l = __fsub_rn(dy[k].l, __fsub_rn(ck.y, c0.y));
       }
-#pragma unroll DU
+#pragma unroll
       for (int q = 0; q < N1; q++) {
         tf sx{0.f, 0.f}, sy{0.f, 0.f};
 #pragma unroll
@@ -851,32 +843,21 @@ __device__ __forceinline__ bool tile_body_df(const Params &prm, const StepPtrs s
         sy = tf_norm(sy);
         const float4 g = make_float4(sx.h, sy.h, sx.l, sy.l);
         if (dir == 1) X1[el * XS + j + q * N1] = g;          // d/deta at (j, q)
-        else if (ROLL) X2[el * XS + q + j * N1] = g;         // d/dxi at (q, j): read back by this thread alone
         else { gxr[q] = sx; gyr[q] = sy; }
       }
     }
   }
   if constexpr (WE) __syncwarp(); else __syncthreads();
 
-  // ---- 2. stress at the row's points; xi divergence; eta fluxes to X2 (rolled: the xi fluxes
-  // take the place of the eta derivatives, which this thread alone reads, the eta fluxes
-  // that of the xi derivatives)
+  // ---- 2. stress at the row's points; xi divergence; eta fluxes to X2
   if (active) {
     const tf c11 = tf_add(tf_add(mu, mu), lam);
     const tf nfj = tf_neg(tf_mul(detJ, tf{c_w[P - 1][j], c_wl[P - 1][j]}));
-#pragma unroll DU
+#pragma unroll
     for (int q = 0; q < N1; q++) {
       const int at = el * XS + q + j * N1;
       const float4 g4 = X1[at];   // d/deta at (q, j)
-      tf gx, gy;
-      if constexpr (ROLL) {
-        const float4 x4 = X2[at];
-        gx = tf{x4.x, x4.z};
-        gy = tf{x4.y, x4.w};
-      } else {
-        gx = gxr[q];
-        gy = gyr[q];
-      }
+      const tf gx = gxr[q], gy = gyr[q];
       const tf gex{g4.x, g4.z}, gey{g4.y, g4.w};
       const tf e0 = tf_mul(ix, gx), e1 = tf_mul(iy, gey);
       const tf e2 = tf_add(tf_mul(ix, gy), tf_mul(iy, gex));
@@ -887,20 +868,12 @@ __device__ __forceinline__ bool tile_body_df(const Params &prm, const StepPtrs s
       const tf sxy = tf_mul(mu, e2);
       const tf Fxq = tf_mul(fx_, sxx), Fyq = tf_mul(fx_, sxy);
       const tf hx = tf_mul(fy_, sxy), hy = tf_mul(fy_, syy);
-      if constexpr (ROLL) X1[at] = make_float4(Fxq.h, Fyq.h, Fxq.l, Fyq.l);
-      else { Fx[q] = Fxq; Fy[q] = Fyq; }
+      Fx[q] = Fxq;
+      Fy[q] = Fyq;
       X2[at] = make_float4(hx.h, hy.h, hx.l, hy.l);
     }
-    if constexpr (ROLL) {
-#pragma unroll
-      for (int q = 0; q < N1; q++) {
-        const float4 f4 = X1[el * XS + q + j * N1];
-        Fx[q] = tf{f4.x, f4.z};
-        Fy[q] = tf{f4.y, f4.w};
-      }
-    }
     // xi part of the divergence for the row's nodes, to X1
-#pragma unroll DU
+#pragma unroll
     for (int a = 0; a < N1; a++) {
       tf rx{0.f, 0.f}, ry{0.f, 0.f};
 #pragma unroll
@@ -924,7 +897,7 @@ __device__ __forceinline__ bool tile_body_df(const Params &prm, const StepPtrs s
       fcx[q] = tf{f4.x, f4.z};
       fcy[q] = tf{f4.y, f4.w};
     }
-#pragma unroll DU
+#pragma unroll
     for (int bq = 0; bq < N1; bq++) {
       const float4 r = X1[el * XS + j + bq * N1];
       tf cx{r.x, r.z}, cy{r.y, r.w};

@@ -15,7 +15,7 @@ namespace se2p {
 // synchronise within the warp, threads = 32 x warps)).  Degree 4: 7x7 at 2 CTAs per SM
 // (92-96 registers) is the fastest, with two owned buffers; sized for 3 CTAs it is capped
 // at 64 registers and runs slower.  default_config gives each degree's fastest.  The
-// two-float mode uses the same list with one owned buffer.  New configurations go at the
+// two-float mode has a list of its own (se2gpu_f32df_launch.h).  New configurations go at the
 // end of their degree's list: the autotuner's cache and default_config refer to them by
 // position.
 #define SE2P_CONFIGS(X)                                                                      \
@@ -38,6 +38,7 @@ struct TileShape {
   int cell_box;        // cell-constant box edge (elements, float4 each)
   int minv_w;          // 1/M box width (floats; the box is own_h high)
   size_t smem;
+  bool halo;           // recomputes a halo of elements and loads by tensor maps (all but most two-float ones)
 };
 
 cudaError_t set_tables(int p, const double *D, const double *w1d);   // constant-memory D, w (current device)
@@ -55,7 +56,6 @@ cudaError_t launch_record(int p, const Params &prm, cudaStream_t st, bool df = f
 
 // the two-float kernels (their own translation unit, with its own constant tables)
 cudaError_t df_set_tables(int p, const double *D, const double *w1d);
-const void *df_kernel(int p, int config, size_t *smem);
 cudaError_t df_launch_record(int p, const Params &prm, cudaStream_t st);
 // batched step of many shots of degree p (tables in device memory), and the
 // receiver rows of a block's last step
