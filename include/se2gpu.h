@@ -134,8 +134,10 @@ int se2gpu_device_fields(const se2gpu_solver *h, void **u, void **v, void **a);
 /* Tile configurations of the step kernel (elements per tile edge, threads per
    CTA) available for the handle's degree and precision, for the autotuner;
    returns how many exist.  se2gpu_set_tile_config selects one; se2gpu_tile_config
-   returns the selected one (a new handle starts with the configuration measured
-   fastest for its degree and mesh size on GB300; 0 in the FP64 mode). */
+   returns the selected one (before a selection the one measured fastest for the
+   handle's degree and mesh size on GB300 among those for many tiles; a plain or Kahan
+   handle on a small mesh then runs the last one, which keeps element forces in
+   memory; 0 in the FP64 mode). */
 int se2gpu_tile_configs(const se2gpu_solver *h, int *edge, int *threads, int max_configs);
 int se2gpu_set_tile_config(se2gpu_solver *h, int config);
 int se2gpu_tile_config(const se2gpu_solver *h);

@@ -26,7 +26,6 @@
 #include <vector>
 
 #include "se2gpu.h"
-#include "se2gpu_f32df_launch.h"
 #include "se2gpu_f64_launch.h"
 #include "se2gpu_internal.h"
 #include "se2gpu_launch.h"
@@ -431,7 +430,7 @@ static int upload_leapfrog(se2gpu_solver *h, const double *u, const double *v, c
 static int make_const_maps(se2gpu_solver *h, const se2p::TileShape &ts)
 {
   for (int b = 0; b < 2; b++) memset(&h->maps[b][4], 0, 2 * sizeof(CUtensorMap));
-  if (pmode(h) == se2p::MODE_DF) return 0;
+  if (pmode(h) == se2p::MODE_DF || !ts.halo) return 0;
   int r = se2p::make_map_cells(&h->maps[0][4], h->cellc, h->mx, h->my, ts.cell_box);
   if (!r) r = se2p::make_map_f32(&h->maps[0][5], h->pminv, h->pitch, h->ny_g, h->pitch, ts.minv_w, ts.own_h);
   if (r) return fail(h, SE2GPU_ERR_CUDA, "cuTensorMapEncodeTiled failed for the tile constants (%d)", r);
@@ -466,6 +465,10 @@ static int setup_f32_config(se2gpu_solver *h, int config, bool in_create = false
   if (h->pminv) {   // (in se2gpu_create the 1/M map follows once 1/M is allocated)
     int r = make_const_maps(h, ts);
     if (r) return r;
+  }
+  for (int b = 0; b < 2 && !ts.halo && !h->ef[b]; b++) {   // element forces
+    const int rc = dalloc(h, (void **)&h->ef[b], (size_t)h->mx * h->my * h->npe * (is_df(h) ? 16 : 8));
+    if (rc) return rc;
   }
   const int te = ts.tex, P = h->p;
   const int ntx = (h->mx + te - 1) / te, nty = (h->my + te - 1) / te, ntiles = ntx * nty;
@@ -507,7 +510,7 @@ static int setup_f32_config(se2gpu_solver *h, int config, bool in_create = false
   if ((rc = upload_i(h, (int **)&h->tile_src, si.data(), si.size()))) return rc;
   if ((rc = upload_i(h, (int **)&h->tile_rec, ri.data(), ri.size()))) return rc;
   h->pconfig = config;
-  h->df_no_halo = !ts.halo;
+  h->no_halo = !ts.halo;
   h->pntx = ntx;
   h->pnty = nty;
   h->pgrid = std::min(ntiles + 1, std::max(1, se2p::occupancy(P, config, mode)) * h->nsm);
@@ -651,7 +654,6 @@ int se2gpu_internal_create(const se2gpu_problem *P, int precision, int trace_cap
       TRY(dzero(h, (void **)&h->rbuf[b], (size_t)P->nrec * npe * rbuf_values(h) * 4));
     }
     TRY(dalloc(h, (void **)&h->pa, np * 8 * (df ? 2 : 1)));   // two-float mode: low parts after the high
-    for (int b = 0; b < 2 && df; b++) TRY(dalloc(h, (void **)&h->ef[b], (size_t)ne * npe * 16));   // element forces
     if (!df) {
       TRY(dalloc(h, (void **)&h->cellc, (size_t)ne * sizeof(float4)));
       k_cell_consts<<<(int)std::min<long>((ne + 255) / 256, 8L * h->nsm), 256, 0, h->stream>>>(
@@ -711,7 +713,9 @@ int se2gpu_internal_create(const se2gpu_problem *P, int precision, int trace_cap
       if (e != cudaSuccess) { fail(h, SE2GPU_ERR_CUDA, "constant tables: %s", cudaGetErrorString(e)); TRY(SE2GPU_ERR_CUDA); }
       h->src_elem_h = new std::vector<int>(P->src_elem, P->src_elem + P->nsrc);
       h->rec_elem_h = new std::vector<int>(P->rec_elem, P->rec_elem + P->nrec);
-      TRY(setup_f32_config(h, se2p::default_config(P->p, pmode(h), in_ensemble ? 0 : P->mx, P->my, h->nsm), true));
+      const int mesh_x = in_ensemble ? 0 : P->mx;
+      TRY(setup_f32_config(h, se2p::first_config(P->p, pmode(h), mesh_x, P->my, h->nsm), true));
+      h->reported_config = se2p::default_config(P->p, pmode(h), mesh_x, P->my, h->nsm);
     }
     for (cudaEvent_t &ev : h->side_done) {
       const cudaError_t e = cudaStreamWaitEvent(h->stream, ev, 0);
@@ -908,17 +912,17 @@ static int advance_f64(se2gpu_solver *h, int nsteps)
   return 0;
 }
 
-// two-float steps without a halo: START, MIDDLE per step but the last, LAST (se2gpu_f32df.cuh); a launch
-// that finishes a step records its receivers' elements and samples those of the step before
-static int advance_df(se2gpu_solver *h, int nsteps)
+// steps without a halo: START, MIDDLE per step but the last, LAST (se2gpu_f32ef.cuh); a launch that
+// finishes a step records its receivers' elements and samples those of the step before
+static int advance_no_halo(se2gpu_solver *h, int nsteps)
 {
-  se2p::DfParams q;
+  se2p::EfParams q;
   q.p = f32_params(h);
   for (int k = 0; k <= nsteps; k++) {
     const int in = h->cur, outb = 1 - h->cur;
-    q.mode = (k == 0) ? se2p::DF_START : (k == nsteps) ? se2p::DF_LAST : se2p::DF_MIDDLE;
+    q.mode = (k == 0) ? se2p::EF_START : (k == nsteps) ? se2p::EF_LAST : se2p::EF_MIDDLE;
     q.u_in = h->pu[in]; q.w_in = h->pw[in]; q.cu_in = h->pcu[in]; q.cw_in = h->pcw[in];
-    q.ef_in = (const float4 *)h->ef[(k + 1) & 1]; q.ef_out = (float4 *)h->ef[k & 1];
+    q.ef_in = h->ef[(k + 1) & 1]; q.ef_out = h->ef[k & 1];
     q.p.u_out = h->pu[outb]; q.p.w_out = h->pw[outb]; q.p.cu_out = h->pcu[outb]; q.p.cw_out = h->pcw[outb];
     q.p.a_out = h->pa;
     q.p.stf = k ? h->stf_dev + (size_t)(k - 1) * h->nsrc : nullptr;
@@ -927,7 +931,7 @@ static int advance_df(se2gpu_solver *h, int nsteps)
     q.p.record = h->pending_record ? 1 : 0;
     q.p.trace_row = h->traces + (size_t)h->rows_written * 7 * h->nrec;
     h->launches++;
-    cudaError_t e = se2p::df_launch(h->p, h->pconfig, q, k > 0, h->stream);
+    cudaError_t e = se2p::launch_no_halo(h->p, h->pconfig, pmode(h), q, k > 0, h->stream);
     if (e != cudaSuccess) return fail(h, SE2GPU_ERR_CUDA, "step kernel: %s", cudaGetErrorString(e));
     if (h->pending_record) { h->rows_written++; h->pending_record = false; }
     if (k == 0) continue;   // (no step is finished yet)
@@ -984,7 +988,7 @@ extern "C" int se2gpu_advance(se2gpu_solver *h, int nsteps, const double *stf)
     // the previous block may still read stf_dev: order the copy on the stream
     CK(h, cudaMemcpyAsync(h->stf_dev, stf, (size_t)nsteps * h->nsrc * 8, cudaMemcpyHostToDevice, h->stream));
   }
-  return is_f64(h) ? advance_f64(h, nsteps) : h->df_no_halo ? advance_df(h, nsteps) : advance_f32(h, nsteps);
+  return is_f64(h) ? advance_f64(h, nsteps) : h->no_halo ? advance_no_halo(h, nsteps) : advance_f32(h, nsteps);
 }
 
 extern "C" int se2gpu_traces(se2gpu_solver *h, double *out, int max_rows)
@@ -1211,7 +1215,7 @@ extern "C" int se2gpu_tile_configs(const se2gpu_solver *h, int *edge, int *threa
     if (max_configs > 0 && edge && threads) { edge[0] = se2::f64_tile_edge(h->p); threads[0] = 256; }
     return 1;
   }
-  const int n = se2p::num_configs(h->p);
+  const int n = se2p::num_configs(h->p, pmode(h));
   for (int c = 0; c < n && c < max_configs; c++) {
     se2p::TileShape ts;
     se2p::config_shape(h->p, c, pmode(h), &ts);
@@ -1244,17 +1248,21 @@ extern "C" int se2gpu_tile_config_info(const se2gpu_solver *h, int config, int i
 extern "C" int se2gpu_tile_config(const se2gpu_solver *h)
 {
   if (!h) return SE2GPU_ERR_ARG;
-  return is_f64(h) ? 0 : h->pconfig;
+  return is_f64(h) ? 0 : h->reported_config;
 }
 
 extern "C" int se2gpu_set_tile_config(se2gpu_solver *h, int config)
 {
   if (!h) return SE2GPU_ERR_ARG;
   if (is_f64(h)) return (config == 0) ? 0 : fail(h, SE2GPU_ERR_ARG, "FP64 mode has a single tile configuration");
-  if (config < 0 || config >= se2p::num_configs(h->p)) return fail(h, SE2GPU_ERR_ARG, "tile configuration %d out of range", config);
+  if (config < 0 || config >= se2p::num_configs(h->p, pmode(h))) return fail(h, SE2GPU_ERR_ARG, "tile configuration %d out of range", config);
   CK(h, cudaSetDevice(h->device));
-  if (config == h->pconfig) return 0;   // already selected: tables, maps and grid are current
-  return setup_f32_config(h, config);
+  if (config != h->pconfig) {   // (else tables, maps and grid are current)
+    const int rc = setup_f32_config(h, config);
+    if (rc) return rc;
+  }
+  h->reported_config = config;
+  return 0;
 }
 
 // ---------------------------------------------------------------- checkpoint / resume

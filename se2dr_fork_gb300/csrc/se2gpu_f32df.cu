@@ -71,7 +71,7 @@ bool df_shape(int p, int config, DfShape *s)
   return false;
 }
 
-cudaError_t df_launch(int p, int config, const DfParams &q, bool dependent, cudaStream_t st)
+cudaError_t df_launch(int p, int config, const EfParams &q, bool dependent, cudaStream_t st)
 {
   DfShape s;
   if (!df_shape(p, config, &s) || s.halo) return cudaErrorInvalidValue;
@@ -85,7 +85,7 @@ cudaError_t df_launch(int p, int config, const DfParams &q, bool dependent, cuda
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = dependent ? 1 : 0;
-  DfParams a = q;
+  EfParams a = q;
   void *args[] = {&a};
   return cudaLaunchKernelExC(&cfg, s.fn, args);
 }

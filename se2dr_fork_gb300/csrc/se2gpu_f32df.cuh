@@ -10,8 +10,8 @@
 // about 50 B per node and step at degree 4.  3.53M nodes, degree 4, 6 steps: 1313 -> 1243 us; degree 7
 // at 2.5M nodes 304 -> 176 us a step, 20000 nodes 19.4 -> 11.9 (every size: se2gpu_f32df_launch.h).
 //
-// A block of n steps: one DF_START launch (element forces of the state), n - 1 DF_MIDDLE
-// launches, and DF_LAST, which finishes the last step and stores its a.
+// A block of n steps: one EF_START launch (element forces of the state), n - 1 EF_MIDDLE
+// launches, and EF_LAST, which finishes the last step and stores its a.
 #pragma once
 #include "se2gpu_persist.cuh"
 #include "se2gpu_f32df_launch.h"
@@ -37,19 +37,8 @@ struct DfNode {
   float4 g[4];
 };
 
-template <int P>
-struct DfPos {   // which of the four elements exist
-  int ex, ey, ix, iy;
-  bool in_x, in_y, lft, bot;
-  __device__ __forceinline__ DfPos(int mx, int my, int X, int Y)
-  {
-    ex = X / P; ey = Y / P; ix = X - ex * P; iy = Y - ey * P;
-    in_x = ex < mx; in_y = ey < my; lft = ix == 0 && ex > 0; bot = iy == 0 && ey > 0;
-  }
-};
-
 template <int P, int TE, int NT>
-__global__ void __launch_bounds__(NT, df_min_blocks(P, TE, NT)) df_step(const DfParams dp)
+__global__ void __launch_bounds__(NT, df_min_blocks(P, TE, NT)) df_step(const EfParams dp)
 {
   typedef DfGeo<P, TE> G;
   constexpr int N1 = G::N1, NPE = G::NPE, RW = G::RW, RP = G::RP, XS = G::XS;
@@ -81,13 +70,13 @@ __global__ void __launch_bounds__(NT, df_min_blocks(P, TE, NT)) df_step(const Df
     const size_t n = (size_t)Y * pitch + X;
     d.u = dp.u_in[n];
     d.cu = dp.cu_in[n];
-    if (dp.mode == DF_START) return;
+    if (dp.mode == EF_START) return;
     d.w = dp.w_in[n];
     d.cw = dp.cw_in[n];
     d.minv_h = prm.minv[n];
     d.minv_l = minv_lo[n];
-    const DfPos<P> c(prm.mx, prm.my, X, Y);
-    const float4 *ef = dp.ef_in + ((ptrdiff_t)c.ey * prm.mx + c.ex) * NPE + c.ix + c.iy * N1;
+    const NodePos<P> c(prm.mx, prm.my, X, Y);
+    const float4 *ef = static_cast<const float4 *>(dp.ef_in) + ((ptrdiff_t)c.ey * prm.mx + c.ex) * NPE + c.ix + c.iy * N1;
     if (c.bot && c.lft) d.g[0] = ef[-(ptrdiff_t)(prm.mx + 1) * NPE + P + P * N1];
     if (c.bot && c.in_x) d.g[1] = ef[-(ptrdiff_t)prm.mx * NPE + P * N1];
     if (c.lft && c.in_y) d.g[2] = ef[-(ptrdiff_t)NPE + P];
@@ -101,18 +90,18 @@ __global__ void __launch_bounds__(NT, df_min_blocks(P, TE, NT)) df_step(const Df
     load(i + NT, next);
     const int ry = i / RW, rx = i - ry * RW;
     const bool own = rx < own_w && ry < own_h;
-    if (rx > nex * P || ry > ney * P || (dp.mode == DF_LAST && !own)) continue;
+    if (rx > nex * P || ry > ney * P || (dp.mode == EF_LAST && !own)) continue;
     const int X = X0 + rx, Y = Y0 + ry;
     const size_t n = (size_t)Y * pitch + X;
     const float2 u = d.u, cu = d.cu, w = d.w, cw = d.cw;
-    if (dp.mode == DF_START) {
+    if (dp.mode == EF_START) {
       sU[i] = make_float4(u.x, u.y, cu.x, cu.y);
       continue;
     }
     const tf minv{d.minv_h, d.minv_l};
     tf fx{0.f, 0.f}, fy{0.f, 0.f};
     {
-      const DfPos<P> c(prm.mx, prm.my, X, Y);
+      const NodePos<P> c(prm.mx, prm.my, X, Y);
       const bool have[4] = {c.bot && c.lft, c.bot && c.in_x, c.lft && c.in_y, c.in_x && c.in_y};
 #pragma unroll
       for (int k = 0; k < 4; k++)
@@ -153,13 +142,13 @@ __global__ void __launch_bounds__(NT, df_min_blocks(P, TE, NT)) df_step(const Df
       prm.w_out[n] = make_float2(wxn.h, wyn.h);
       prm.cu_out[n] = make_float2(-uxn.l, -uyn.l);
       prm.cw_out[n] = make_float2(-wxn.l, -wyn.l);
-      if (dp.mode == DF_LAST) {
+      if (dp.mode == EF_LAST) {
         prm.a_out[n] = make_float2(ax.h, ay.h);
         prm.a_out[(size_t)prm.ny_g * pitch + n] = make_float2(ax.l, ay.l);   // low parts after the high parts
       }
     }
   }
-  if (dp.mode == DF_LAST) return;
+  if (dp.mode == EF_LAST) return;
 
   // ---- the element forces: one thread per (element, line j)
   const int el = threadIdx.x / N1, j = threadIdx.x - el * N1, ecy = el / TE, ecx = el - ecy * TE;
@@ -268,7 +257,7 @@ __global__ void __launch_bounds__(NT, df_min_blocks(P, TE, NT)) df_step(const Df
 
   // ---- 3. eta part of the divergence along column j, added to the xi part: the element's forces
   if (active) {
-    float4 *ef = dp.ef_out + ((size_t)ey * prm.mx + ex) * NPE;
+    float4 *ef = static_cast<float4 *>(dp.ef_out) + ((size_t)ey * prm.mx + ex) * NPE;
     tf fcx[N1], fcy[N1];
 #pragma unroll
     for (int q = 0; q < N1; q++) {

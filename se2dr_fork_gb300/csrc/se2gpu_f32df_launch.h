@@ -6,16 +6,6 @@
 
 namespace se2p {
 
-enum { DF_START = 0, DF_MIDDLE = 1, DF_LAST = 2 };
-
-struct DfParams {
-  Params p;                                          // outputs, tables, lists, receivers
-  const float2 *u_in, *w_in, *cu_in, *cw_in;
-  const float4 *ef_in;                               // element forces (x.h, y.h, x.l, y.l) of the step to finish
-  float4 *ef_out;
-  int mode;
-};
-
 // Tile configurations of the two-float mode, X(degree, elements per tile edge, threads) for the step
 // without a halo (threads >= edge^2 (degree + 1), whole warps) and H(degree, edge, threads) for the
 // one that recomputes a halo of elements (se2gpu_persist.cuh), as many per degree as the other FP32
@@ -62,6 +52,6 @@ struct DfShape {
 // configuration of degree p, with or without a halo; false: no such configuration
 bool df_shape(int p, int config, DfShape *s);
 // the step without a halo (the other one: launch_step)
-cudaError_t df_launch(int p, int config, const DfParams &q, bool dependent, cudaStream_t st);
+cudaError_t df_launch(int p, int config, const EfParams &q, bool dependent, cudaStream_t st);
 
 }  // namespace se2p

@@ -6,6 +6,7 @@
 #include <algorithm>
 
 #include "se2gpu_f32df_launch.h"
+#include "se2gpu_f32ef_launch.h"
 #include "se2gpu_persist.cuh"
 #include "se2gpu_persist_launch.h"
 
@@ -21,7 +22,8 @@ cudaError_t set_tables(int p, const double *D, const double *w1d)
   if (e != cudaSuccess) return e;
   e = cudaMemcpyToSymbol(c_w, w, sizeof(w), sizeof(w) * (p - 1));
   if (e != cudaSuccess) return e;
-  return df_set_tables(p, D, w1d);
+  e = df_set_tables(p, D, w1d);
+  return e != cudaSuccess ? e : ef_set_tables(p, D, w1d);
 }
 
 // ---- one configuration = (degree, elements per tile edge, threads) ----------
@@ -77,17 +79,18 @@ static const Entry *find(int p, int config)
 // the configuration a handle starts with.  Plain and Kahan: per degree the one the autotuner
 // measured fastest on GB300 at about 16M nodes (and, at degree 4, at the 2048^2 workload; the
 // plain mode at degree 8 runs 4 x 4 tiles: 83 against 93 us a step at 5M nodes, 7.0 against 9.6 at
-// 260000), and smaller tiles on meshes that these divide into about one per SM (us a step: degree
-// 1, 17 x 17 elements 3.55 -> 3.39; degree 2, 35 x 35 4.92 -> 4.21; degree 5, 28 x 28 6.23 ->
-// 5.53; degree 6, 12 x 12 5.96 -> 5.44, but 58 x 58 5.50 -> 6.24; plain degree 8, 31 x 31
-// 6.52 -> 5.60).  Two-float: small tiles with a thread per node while a few of them fill an SM, then those
-// with the fewest idle threads, then (degrees 2 and 3) the halo kernel; the lines lie where the
-// times cross (us a step at 20000 / 80000 / 260000 / 1M nodes, chosen one first): degree 2 6 x 6 5.1 / 8.7
-// / 20.6 / 81, 8 x 8 6.8 / 10.1 / 20.2 / 78, halo 8.6 / 9.1 / 25.4 / 75; 3 5.6 / 8.1 / 20.5 / 78, 7.7 /
-// 9.0 / 19.5 / 72, 7.7 / 9.9 / 22.0 / 69; 4 3 x 3 7.8 / 9.2 / 25 / 96, 5 x 5 10.6 / 11.1 / 20 / 70; 5 2 x 2
-// 8.6 / 10.8 / 24.6 / 95, 4 x 4 12.7 / 12.8 / 22.1 / 74; 6 2 x 2 10.2 / 18.1 / 51 / 196, 3 x 3 14.2 /
-// 13.4 / 21.4 / 82, 6 x 6 19.1 / 17.9 / 24.9 / 79; 7 2 x 2 11.9 / 20.2 / 48 / 177, 4 x 4 18.4 / 17.5 / 24.9
-// / 81; 8 1 x 1 12.4 / 23.5 / 69 / 247, 3 x 3 17.5 / 17.0 / 29 / 100, 5 x 5 24 / 24 / 34 / 92.
+// 260000), and smaller tiles on meshes that these divide into about one per SM (us a step: degree 6,
+// 47 x 47 elements 6.43 -> 5.91; plain degree 8, 31 x 31 6.52 -> 5.60).  On still smaller ones
+// first_config goes over to the step without a halo (se2gpu_f32ef.cuh; Kahan, 80000 nodes, halo / not:
+// degree 1 5.2 / 6.9, 2 5.3 / 5.4, 3 5.2 / 5.2, 4 5.8 / 5.5, 5 5.9 / 6.3, 6 5.9 / 6.1, 7 7.2 / 5.9, 8
+// 6.5 / 7.6).  Two-float: small tiles with a thread per node while a few of them fill an SM, then
+// those with the fewest idle threads, then (degrees 2 and 3) the halo kernel; the lines lie where
+// the times cross (us a step at 20000 / 80000 / 260000 / 1M nodes): degree 2 6 x 6 5.1 / 8.7 / 20.6 / 81,
+// 8 x 8 6.8 / 10.1 / 20.2 / 78, halo 8.6 / 9.1 / 25.4 / 75; 3 4 x 4 with 192 threads 5.6 / 8.1 / 20.5 / 78,
+// with 64 7.7 / 9.0 / 19.5 / 72, halo 7.7 / 9.9 / 22.0 / 69; 4 3 x 3 7.8 / 9.2 / 25 / 96, 5 x 5 10.6 / 11.1 /
+// 20 / 70; 5 2 x 2 8.6 / 10.8 / 24.6 / 95, 4 x 4 12.7 / 12.8 / 22.1 / 74; 6 2 x 2 10.2 / 18.1 / 51 / 196, 3 x 3
+// 14.2 / 13.4 / 21.4 / 82, 6 x 6 19.1 / 17.9 / 24.9 / 79; 7 2 x 2 11.9 / 20.2 / 48 / 177, 4 x 4 18.4 / 17.5 /
+// 24.9 / 81; 8 1 x 1 12.4 / 23.5 / 69 / 247, 3 x 3 17.5 / 17.0 / 29 / 100, 5 x 5 24 / 24 / 34 / 92.
 // mx = 0: the large-mesh choice (the ensemble's, whose shots share one).
 int default_config(int p, int mode, int mx, int my, int nsm)
 {
@@ -123,12 +126,48 @@ int num_configs(int p)
   return k;
 }
 
+// what a handle on which no configuration was chosen runs: without a halo on a small mesh, up to so
+// many tiles per SM
+int first_config(int p, int mode, int mx, int my, int nsm)
+{
+  static const int few[8] = {3, 2, 2, 4, 3, 2, 3, 3};
+  EfShape ef;
+  if (mode != MODE_DF && mx && ef_shape(p, 0, &ef) &&
+      (long)((mx + ef.te - 1) / ef.te) * ((my + ef.te - 1) / ef.te) <= few[p - 1] * (long)nsm)
+    return num_configs(p);
+  return default_config(p, mode, mx, my, nsm);
+}
+
+int num_configs(int p, int mode)
+{
+  EfShape s;
+  int k = num_configs(p), n = 0;
+  while (mode != MODE_DF && ef_shape(p, n, &s)) n++;
+  return k + n;
+}
+
+// a configuration without a halo, of any mode
+static bool no_halo(int p, int config, int mode, DfShape *s)
+{
+  if (mode == MODE_DF) return df_shape(p, config, s) && !s->halo;
+  EfShape e;
+  if (config < num_configs(p) || !ef_shape(p, config - num_configs(p), &e)) return false;
+  const int k = mode ? 1 : 0;
+  *s = DfShape{p, e.te, e.nt, e.smem[k], e.fn[k], false};
+  return true;
+}
+
+cudaError_t launch_no_halo(int p, int config, int mode, const EfParams &q, bool dependent, cudaStream_t st)
+{
+  if (mode == MODE_DF) return df_launch(p, config, q, dependent, st);
+  return ef_launch(p, config - num_configs(p), mode == MODE_KAHAN, q, dependent, st);
+}
+
 int config_shape(int p, int config, int mode, TileShape *s)
 {
   const Entry *e = find(p, config);
   DfShape df;
-  if (!e || (mode == MODE_DF && !df_shape(p, config, &df))) return -1;
-  if (mode == MODE_DF && !df.halo) {
+  if (no_halo(p, config, mode, &df)) {
     *s = TileShape{};   // (no tensor maps; the state of the tile is held once)
     s->owned_buffers = 1;
     s->tex = s->tey = df.te;
@@ -136,6 +175,7 @@ int config_shape(int p, int config, int mode, TileShape *s)
     s->smem = df.smem;
     return 0;
   }
+  if (!e || (mode == MODE_DF && !df_shape(p, config, &df))) return -1;
   const int te = (mode == MODE_DF) ? df.te : e->te;
   s->halo = true;
   s->tex = s->tey = te;
@@ -151,33 +191,32 @@ int config_shape(int p, int config, int mode, TileShape *s)
   return 0;
 }
 
+static cudaError_t prepare_kernel(const void *fn, size_t smem)
+{
+  const cudaError_t r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  return r != cudaSuccess ? r : cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+}
+
 cudaError_t prepare(int p, int config, int mode)
 {
   const Entry *e = find(p, config);
-  if (!e) return cudaErrorInvalidValue;
   const int k = mode ? 1 : 0;
-  DfShape df = {};
-  if (mode == MODE_DF && !df_shape(p, config, &df)) return cudaErrorInvalidValue;
-  const void *fns[2] = {df.fn ? df.fn : e->fn[k], e->bfn[k]};
-  const size_t sizes[2] = {df.fn ? df.smem : e->smem[k], e->bsmem[k]};
-  for (int i = 0; i < 2; i++) {
-    const void *fn = fns[i];
-    cudaError_t r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizes[i]);
-    if (r != cudaSuccess) return r;
-    r = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    if (r != cudaSuccess) return r;
-  }
-  return cudaSuccess;
+  DfShape s = {};
+  if (no_halo(p, config, mode, &s) || (mode == MODE_DF && df_shape(p, config, &s))) return prepare_kernel(s.fn, s.smem);
+  if (!e || mode == MODE_DF) return cudaErrorInvalidValue;
+  const cudaError_t r = prepare_kernel(e->fn[k], e->smem[k]);
+  return r != cudaSuccess ? r : prepare_kernel(e->bfn[k], e->bsmem[k]);
 }
 
 int occupancy(int p, int config, int mode, bool batch)
 {
   const Entry *e = find(p, config);
   int n = 0;
-  if (!e) return 1;
   const int k = mode ? 1 : 0;
-  DfShape s{p, e->te, e->nt, (batch ? e->bsmem : e->smem)[k], (batch ? e->bfn : e->fn)[k], true};
-  if (mode == MODE_DF && !batch) df_shape(p, config, &s);
+  DfShape s = {};
+  if (e) s = DfShape{p, e->te, e->nt, (batch ? e->bsmem : e->smem)[k], (batch ? e->bfn : e->fn)[k], true};
+  if (!batch && mode == MODE_DF) df_shape(p, config, &s);
+  if (!batch) no_halo(p, config, mode, &s);
   if (!s.fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, s.fn, s.nt, s.smem) != cudaSuccess) {
     cudaGetLastError();
     return 1;

@@ -21,7 +21,7 @@ struct se2gpu_solver {
   cudaStream_t stream, own_stream;
   size_t tsize;                  // compute precision (4 or 8 bytes)
   // FP64 state: two buffer sets of packed u, v; a of the last step; element forces of a step
-  // (the two-float mode's too: 16 bytes per element node); 1/M; scaled derivative tables
+  // (FP32 steps without a halo too: 8 bytes per element node, two-float 16); 1/M; scaled derivative tables
   double2 *f64[2][2], *a64, *ef[2];
   double *rmass, *Dx, *Dy, *f64_consts;
   int2 *src_xy;                  // first node of each source's element
@@ -37,7 +37,8 @@ struct se2gpu_solver {
   float4 *cellc;                 // plain and Kahan modes: (lam detJ, mu detJ, d xi/dx, d eta/dy) per cell
   int4 *tile_bounds;             // per tile: source and receiver list bounds
   int pgrid, pconfig, pntx, pnty;
-  bool df_no_halo;               // two-float mode: the configuration's step is df_step (se2gpu_f32df.cuh)
+  int reported_config;           // pconfig once one was chosen; before that, the degree's default
+  bool no_halo;                  // FP32: the configuration's step keeps element forces (se2gpu_f32ef.cuh)
   int4 *tile_src, *tile_rec;     // per-tile list entries
   std::vector<int> *src_elem_h, *rec_elem_h;
   int *err_dev;

@@ -324,6 +324,19 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float inc)
   s = t;
 }
 
+// node (X, Y) of a mesh: its own element, its place in that, and which of the four elements around it
+// exist (a node line shared by two elements belongs to the right, upper one)
+template <int P>
+struct NodePos {
+  int ex, ey, ix, iy;
+  bool in_x, in_y, lft, bot;
+  __device__ __forceinline__ NodePos(int mx, int my, int X, int Y)
+  {
+    ex = X / P; ey = Y / P; ix = X - ex * P; iy = Y - ey * P;
+    in_x = ex < mx; in_y = ey < my; lft = ix == 0 && ex > 0; bot = iy == 0 && ey > 0;
+  }
+};
+
 // receiver rows of the previous step from the side buffer (u, v, a per element node)
 // (two-float mode: 12 values per node, the value being high + low)
 template <int P, bool DF = false>

@@ -42,8 +42,10 @@ struct TileShape {
 };
 
 cudaError_t set_tables(int p, const double *D, const double *w1d);   // constant-memory D, w (current device)
-int num_configs(int p);                                               // tile configurations for degree p
-int default_config(int p, int mode, int mx, int my, int nsm);             // a new handle's
+int num_configs(int p);                                               // tile configurations for degree p (ensembles)
+int num_configs(int p, int mode);                                     // of a handle: those without a halo follow
+int default_config(int p, int mode, int mx, int my, int nsm);         // the one a new handle reports
+int first_config(int p, int mode, int mx, int my, int nsm);           // and the one that it runs
 // mode: MODE_PLAIN, MODE_KAHAN or MODE_DF (the batched kernel: plain or Kahan)
 int config_shape(int p, int config, int mode, TileShape *s);
 cudaError_t prepare(int p, int config, int mode);                     // dynamic shared-memory limit
@@ -52,6 +54,8 @@ int occupancy(int p, int config, int mode, bool batch = false);       // residen
 // dependent: the launch may begin while the step launched before it on the stream drains
 cudaError_t launch_step(int p, int config, int mode, const CUtensorMap *maps, const Params &prm, int grid,
                         bool dependent, cudaStream_t st);
+// the step of a configuration without a halo (TileShape::halo false)
+cudaError_t launch_no_halo(int p, int config, int mode, const EfParams &q, bool dependent, cudaStream_t st);
 cudaError_t launch_record(int p, const Params &prm, cudaStream_t st, bool df = false);
 
 // the two-float kernels (their own translation unit, with its own constant tables)

@@ -65,4 +65,16 @@ struct BatchArgs {
 };
 static_assert(sizeof(BatchArgs) <= 32764, "a kernel parameter holds at most 32764 bytes");
 
+// a launch of a step kernel without a halo of elements (two-float: se2gpu_f32df.cuh; plain and Kahan:
+// se2gpu_f32ef.cuh): it finishes the previous step at its tile's nodes from the element forces
+// ef_in, and leaves the element forces of the new state in ef_out
+enum { EF_START = 0, EF_MIDDLE = 1, EF_LAST = 2 };   // no step to finish; both; no forces to leave
+struct EfParams {
+  Params p;                                          // outputs, tables, lists, receivers
+  const float2 *u_in, *w_in, *cu_in, *cw_in;
+  const void *ef_in;                                 // per cell and GLL point: float2 (x, y), two-float mode
+  void *ef_out;                                      // float4 (x.h, y.h, x.l, y.l)
+  int mode;
+};
+
 }  // namespace se2p
