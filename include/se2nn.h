@@ -92,15 +92,19 @@ int se2nn_gather_targets(se2nn *h, const float *targets_dev, const int *idx_dev,
 int se2nn_gemm(const void *A_dev, const void *B_dev, float *C_dev, int M, int N, int K, int batch, long lda, long ldb,
                long ldc, long sA, long sB, long sC, int transA, int transB, float alpha, float beta, void *stream);
 
-/* Tensor-core path of the row GEMMs (no counterpart in the reference).  Row GEMMs --
-   one batch, k-contiguous A, at least 128 rows, K and N multiples of 16 up to 128: the
-   lift, the 1x1 convolutions, the decoder and their data gradients -- can run on the
-   5th-generation tensor cores (tcgen05.mma, accumulators in tensor memory), the others
-   run on the mma.sync kernel.  mode 0: every GEMM on mma.sync; 1 (default): the row
-   GEMMs on tcgen05 except those with N <= 64 and 32 < K <= 64 (the 1x1 convolutions,
-   where mma.sync measured faster); 2: every row GEMM on tcgen05.  Process-wide.  se2nn_tensor_path_info: out[0] = tcgen05 GEMM launches,
-   out[1] = mma.sync GEMM launches, out[2] = 1 if a tcgen05 GEMM's bounded wait ever
-   expired. */
+/* Which kernels carry the contractions (no counterpart in the reference); the results
+   have the same bits in every mode.  mode 1 (default): the Fourier layers and the
+   decoder as kernels fused along the image row where the shapes allow (width 16, 32,
+   48 or 64, nx <= 128 a multiple of 16, ny <= 128 a multiple of 8, up to 16 modes), and
+   GEMMs for the rest.  mode 0 and 2: one GEMM launch per contraction, as for other shapes.
+   Row GEMMs -- one batch, k-contiguous A, at least 128 rows, K and N multiples of 16 up
+   to 128 -- can run on the 5th-generation tensor cores (tcgen05.mma, accumulators in
+   tensor memory), the others run on the mma.sync kernel.  Mode 0: every GEMM on mma.sync;
+   1: the row GEMMs on tcgen05 except those with N <= 64 and 32 < K <= 64 (where mma.sync
+   measured faster); 2: every row GEMM on tcgen05.  Process-wide.
+   se2nn_tensor_path_info: out[0] = tcgen05 GEMM launches, out[1] = mma.sync GEMM
+   launches (fused kernels count in neither), out[2] = 1 if a tcgen05 GEMM's bounded wait
+   ever expired. */
 int se2nn_set_tensor_path(int mode);
 int se2nn_tensor_path_info(long out[3]);
 

@@ -1,7 +1,6 @@
-// se2gpu_f32.cu -- FP32 instantiations of the tiled step kernel, degrees 1..8.  They
-// serve the FP32 internal-force entry point (se2gpu_assemble_linear_form[_device] on
-// an FP32 handle, plain arithmetic); FP32 time stepping runs the persistent kernels of
-// se2gpu_f32p.cu.
+// se2gpu_f32.cu -- the internal force in plain FP32, degrees 1..8: the entry point
+// se2gpu_assemble_linear_form[_device] on an FP32 handle.  FP32 time stepping runs the
+// kernels of se2gpu_f32p.cu, se2gpu_f32ef.cu and se2gpu_f32df.cu.
 #include "se2gpu_launch.h"
 
 namespace se2 {

@@ -2,7 +2,7 @@
 //
 // The same leapfrog as se2gpu_persist.cuh (state u, w with their low parts stored as Kahan terms:
 // value = hi - c) with every value of a step an unevaluated sum of two floats.  What bounds it on
-// large meshes is instruction issue (69 % of the issue slots busy, FP32 pipe 58 %, memory a sixth), so
+// large meshes is instruction issue (73 % of the issue slots busy, memory a quarter), so
 // no element is evaluated twice: as in the FP64 step (se2gpu_f64.cuh) a launch finishes the previous
 // step at the nodes of its tile, from the element forces in memory, and then leaves this step's
 // element forces there.  Only the nodes on tile edges are finished twice, where a halo of elements

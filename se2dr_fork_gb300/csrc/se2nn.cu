@@ -1,8 +1,10 @@
 // se2nn.cu -- the surrogate network runtime (include/se2nn.h): parameter and
 // activation buffers, forward and backward passes as sequences of hand-written
-// kernels, Adam, data-set gathers.  Every contraction runs through the BF16
-// tensor-core GEMM of se2nn_gemm.cuh; everything else is a small elementwise,
-// permutation or fixed-order reduction kernel below.  Results do not depend on
+// kernels, Adam, data-set gathers.  The Fourier layers and the decoder run as the fused
+// kernels of se2nn_rows.cuh where their shapes allow (fused_ok); otherwise, and in the
+// other tensor-path modes, every contraction runs through the BF16 tensor-core GEMMs of
+// se2nn_gemm.cuh and se2nn_tc.cuh, with the same bits.  Everything else is a small
+// elementwise, permutation or fixed-order reduction kernel below.  Results do not depend on
 // scheduling: reductions are two-stage with fixed partitions, no atomics.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

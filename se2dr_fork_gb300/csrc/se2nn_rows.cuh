@@ -464,8 +464,8 @@ __global__ void __launch_bounds__(RT) last_kernel(const LastArgs a)
 }
 
 // ---- y transforms: A [4m][2ny] (k contiguous) shared by the samples; 128 columns (kx, c) per
-// CTA, so that a batch of 32 is one wave at two CTAs per SM (64 columns: 512 CTAs of 70 KB in
-// 456 places, 18 us; 128 columns: see below)
+// CTA, so that a batch of 32 is one wave at two CTAs per SM (batch 32, analysis and
+// synthesis: 64 columns, 512 CTAs of 70 KB in 456 places, 18 and 15 us; 128 columns 10 and 10)
 constexpr int YN = 128, YL = YN + 8;
 struct YArgs {
   const bf16 *A;         // My [4m][2ny], or its transpose [2ny][4m] for the synthesis

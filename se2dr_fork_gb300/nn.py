@@ -89,15 +89,17 @@ class NnError(RuntimeError):
 
 
 def set_tensor_path(mode: int):
-    """Which GEMMs run on the tcgen05 tensor-core kernel (process-wide): 0 none (every GEMM on
-    the mma.sync kernel), 1 the row GEMMs except the 1x1 convolutions' shape (N <= 64,
-    32 < K <= 64), where mma.sync measured faster (default), 2 every qualifying row GEMM."""
+    """Which kernels carry the contractions (process-wide; the same bits in every mode): 1
+    (default) the fused layer kernels where the shapes allow, otherwise GEMMs with the row
+    GEMMs on tcgen05 except N <= 64, 32 < K <= 64, where mma.sync measured faster; 0 every
+    contraction a GEMM on the mma.sync kernel; 2 every contraction a GEMM, every qualifying
+    row GEMM on tcgen05."""
     if lib().se2nn_set_tensor_path(int(mode)) != 0:
         raise NnError(f"tensor path mode {mode} is not 0, 1 or 2")
 
 
 def tensor_path_info() -> dict:
-    """GEMM launches so far by kernel, and whether a tcgen05 GEMM's bounded wait expired."""
+    """GEMM launches so far by kernel (the fused layer kernels count in neither), and whether a tcgen05 GEMM's bounded wait expired."""
     out = (C.c_long * 3)()
     if lib().se2nn_tensor_path_info(out) != 0:
         raise NnError("se2nn_tensor_path_info failed")
