@@ -35,7 +35,7 @@ struct Entry {
   const void *bfn[2];             // persist_batch<...> [kahan]
 };
 
-template <int P, int TE, int NT, int NOB = owned_buffers(P), int MINB = 0, bool WE = false>
+template <int P, int TE, int NT, int NOB = owned_buffers(P), int MINB = 0, bool WE = false, int NST = 2>
 static Entry entry()
 {
   constexpr int M0 = MINB ? MINB : min_blocks(Layout<P, TE, false, NOB, false, true>::TOTAL);
@@ -44,12 +44,12 @@ static Entry entry()
   constexpr int B1 = MINB ? MINB : min_blocks(Layout<P, TE, true, NOB>::BATCH_TOTAL);
   Entry e;
   e.p = P; e.te = TE; e.nt = NT; e.nob = NOB;
-  e.smem[0] = Layout<P, TE, false, NOB, false, true>::TOTAL;
-  e.smem[1] = Layout<P, TE, true, NOB, false, true>::TOTAL;
+  e.smem[0] = NST == 2 ? Layout<P, TE, false, NOB, false, true>::TOTAL : Layout<P, TE, false, NOB, false, true>::TOTAL1;
+  e.smem[1] = NST == 2 ? Layout<P, TE, true, NOB, false, true>::TOTAL : Layout<P, TE, true, NOB, false, true>::TOTAL1;
   e.bsmem[0] = Layout<P, TE, false, NOB>::BATCH_TOTAL;
   e.bsmem[1] = Layout<P, TE, true, NOB>::BATCH_TOTAL;
-  e.fn[0] = (const void *)persist_step<P, TE, NT, false, NOB, M0, false, WE>;
-  e.fn[1] = (const void *)persist_step<P, TE, NT, true, NOB, M1, false, WE>;
+  e.fn[0] = (const void *)persist_step<P, TE, NT, false, NOB, M0, false, WE, NST>;
+  e.fn[1] = (const void *)persist_step<P, TE, NT, true, NOB, M1, false, WE, NST>;
   e.bfn[0] = (const void *)persist_batch<P, TE, NT, false, NOB, B0, WE>;
   e.bfn[1] = (const void *)persist_batch<P, TE, NT, true, NOB, B1, WE>;
   return e;
@@ -57,7 +57,7 @@ static Entry entry()
 
 static const Entry *table(int *n)
 {
-#define SE2P_ENTRY(P, TE, NT, NOB, MINB, WE) entry<P, TE, NT, (NOB) ? (NOB) : owned_buffers(P), MINB, (WE) != 0>(),
+#define SE2P_ENTRY(P, TE, NT, NOB, MINB, WE) entry<P, TE, NT, (NOB) ? (NOB) : owned_buffers(P), MINB, (WE) == 1, (WE) == 2 ? 1 : 2>(),
   static Entry t[] = {SE2P_CONFIGS(SE2P_ENTRY)};
 #undef SE2P_ENTRY
   *n = (int)(sizeof(t) / sizeof(t[0]));
@@ -126,24 +126,43 @@ int num_configs(int p)
   return k;
 }
 
-// what a handle on which no configuration was chosen runs: without a halo on a small mesh, up to so
-// many tiles per SM
+// What a handle on which no configuration was chosen runs: the step without a halo on a small mesh, up
+// to few[] of its tiles per SM, and at two degrees other tiles than default_config's where the rounds
+// that the resident CTAs need, times the elements of a tile with its halo, say that these take less.
+// us a step, Kahan / plain.  Degree 4: 6 x 6 while one per SM holds the mesh (71 x 71 elements 6.0 ->
+// 5.3 / 5.5 -> 5.0); 8 x 8 with one region stage, two CTAs per SM, in up to two rounds (128 x 128 8.7 -> 7.5
+// / 8.0 -> 6.6; 177 x 177 13.0 -> 12.2 / 11.5 -> 10.6; but 500 x 500 68 / 76: nothing is copied ahead).
+// Degree 7: 5 x 5 with one region stage, which leaves two (plain: three) CTAs per SM instead of one
+// (85 x 85 10.7 -> 9.1 / 10.7 -> 8.1; 143 x 143 22.5 -> 19.5 / 18.3 -> 15.9; 571 x 571 280 -> 266 / 220 -> 197).
 int first_config(int p, int mode, int mx, int my, int nsm)
 {
   static const int few[8] = {3, 2, 2, 4, 3, 2, 3, 3};
+  if (mode == MODE_DF || mx == 0) return default_config(p, mode, mx, my, nsm);
+  auto tiles = [&](int te) { return (long)((mx + te - 1) / te) * ((my + te - 1) / te); };
+  auto cost = [&](int te, int per_sm) {
+    const long slots = (long)per_sm * nsm;
+    return (tiles(te) + slots - 1) / slots * (te + 1) * (te + 1);
+  };
   EfShape ef;
-  if (mode != MODE_DF && mx && ef_shape(p, 0, &ef) &&
-      (long)((mx + ef.te - 1) / ef.te) * ((my + ef.te - 1) / ef.te) <= few[p - 1] * (long)nsm)
-    return num_configs(p);
+  if (ef_shape(p, 0, &ef) && tiles(ef.te) <= few[p - 1] * (long)nsm) return num_configs(p);
+  if (p == 4 && tiles(6) <= nsm) return 2;
+  if (p == 4 && tiles(8) <= 4L * nsm && cost(8, 2) < cost(7, 2)) return 6;
+  const int per_sm = (mode == MODE_KAHAN) ? 2 : 3;
+  if (p == 7 && 10 * cost(5, per_sm) <= 11 * cost(4, per_sm)) return 3;   // (5 x 5 has the smaller halo)
   return default_config(p, mode, mx, my, nsm);
 }
 
 int num_configs(int p, int mode)
 {
-  EfShape s;
-  int k = num_configs(p), n = 0;
-  while (mode != MODE_DF && ef_shape(p, n, &s)) n++;
-  return k + n;
+  EfShape e;
+  DfShape d;
+  int n = 0;
+  if (mode == MODE_DF) {
+    while (df_shape(p, n, &d)) n++;
+    return n;
+  }
+  while (ef_shape(p, n, &e)) n++;
+  return num_configs(p) + n;
 }
 
 // a configuration without a halo, of any mode

@@ -195,6 +195,7 @@ struct Layout {
   static constexpr size_t XCH = al128(DF ? sizeof(float4) * G::NE * G::XS : sizeof(float2) * G::NE * Xch<P, KAHAN>::XS);
   static constexpr size_t MISC = 64;
   static constexpr size_t TOTAL = 2 * STAGE + NOB * OWNB + 2 * XCH + MISC;
+  static constexpr size_t TOTAL1 = TOTAL - STAGE;   // with one region stage (more CTAs per SM, no copy a tile ahead)
   static constexpr size_t BATCH_TOTAL = TOTAL;   // the batched kernel's shot parameters are a kernel parameter
   static constexpr uint32_t TX_REGION =
       (uint32_t)((KAHAN ? 2 : 1) * sizeof(float2) * G::BXW * G::BXH + (AC ? sizeof(float4) * G::NEX * G::NEX : 0));
@@ -1021,11 +1022,12 @@ __device__ __forceinline__ void item_of(int &el, int &j, bool &valid)
 // DF: the two-float mode (KAHAN storage, tile_body_df); WE: the warp-aligned item mapping.
 // Thread 0 issues, at the start of each tile, the next tile's region (and owned boxes,
 // NOB = 2) or this tile's owned boxes (NOB = 1, on their own barrier), into the buffers
-// the previous tile freed.  Except in the two-float mode the per-tile constants come with
+// the previous tile freed; with one region stage (NST = 1) the next tile's region at the end of
+// this tile.  Except in the two-float mode the per-tile constants come with
 // the copies (AC): the cell constants with the region, 1/M and the tile's source/receiver
 // bounds with the owned boxes.
 template <int P, int TE, int NT, bool KAHAN, int NOB = owned_buffers(P),
-          int MINB = min_blocks(Layout<P, TE, KAHAN, NOB>::TOTAL), bool DF = false, bool WE = false>
+          int MINB = min_blocks(Layout<P, TE, KAHAN, NOB>::TOTAL), bool DF = false, bool WE = false, int NST = 2>
 __global__ void __launch_bounds__(NT, MINB)
 persist_step(const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ CUtensorMap tm_cu,
              const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_cw,
@@ -1037,16 +1039,17 @@ persist_step(const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ C
   constexpr int NEX = G::NEX;
   static_assert(WE ? NT >= 32 * G::NW : NT >= G::ITEMS, "one (element, line) item per thread");
   static_assert(NOB == 1 || NOB == 2, "one or two owned-box buffers");
+  static_assert(NST == 2 || NOB == 1, "one region stage goes with one owned buffer");
   static_assert(!DF || (KAHAN && NOB == 1), "the two-float mode keeps the Kahan storage and one owned buffer");
   const float *W = c_w[P - 1];
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned char *stage0 = smem;
-  unsigned char *stage1 = smem + L::STAGE;
-  unsigned char *ob0 = smem + 2 * L::STAGE;                                             // owned w (cw)
+  unsigned char *stage1 = smem + (NST - 1) * L::STAGE;
+  unsigned char *ob0 = smem + NST * L::STAGE;                                           // owned w (cw)
   unsigned char *ob1 = ob0 + (NOB - 1) * L::OWNB;
-  float2 *X1 = reinterpret_cast<float2 *>(smem + 2 * L::STAGE + NOB * L::OWNB);          // eta derivatives, then element forces
-  float2 *X2 = reinterpret_cast<float2 *>(smem + 2 * L::STAGE + NOB * L::OWNB + L::XCH); // eta fluxes
-  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + 2 * L::STAGE + NOB * L::OWNB + 2 * L::XCH);
+  float2 *X1 = reinterpret_cast<float2 *>(smem + NST * L::STAGE + NOB * L::OWNB);          // eta derivatives, then element forces
+  float2 *X2 = reinterpret_cast<float2 *>(smem + NST * L::STAGE + NOB * L::OWNB + L::XCH); // eta fluxes
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + NST * L::STAGE + NOB * L::OWNB + 2 * L::XCH);
   const uint32_t bar0 = smem_u32(&bars[0]), bar1 = smem_u32(&bars[1]), bo0 = smem_u32(&bars[2]);
 
   if (threadIdx.x == 0) {
@@ -1078,9 +1081,9 @@ persist_step(const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ C
     else issue_region<P, TE, KAHAN, AC>(tx, ty, stage0, bar0, &tm_u, &tm_cu, &tm_c);
   }
   for (int it = 0; t < prm.ntiles; it++, t += gridDim.x) {
-    const int s = it & 1;
+    const int s = (NST == 2) ? it & 1 : 0;
     const uint32_t bar = s ? bar1 : bar0;
-    const uint32_t parity = (it >> 1) & 1;
+    const uint32_t parity = (NST == 2) ? (it >> 1) & 1 : it & 1;
     int txn = tx + dtx, tyn = ty + dty;
     if (txn >= prm.ntx) { txn -= prm.ntx; tyn++; }
     // this tile's owned w (cw) with one owned buffer, the next tile's with two, and the
@@ -1092,7 +1095,7 @@ persist_step(const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ C
     if (threadIdx.x == 0) {
       fence_proxy_async();
       if (NOB == 1) issue_owned<P, TE, KAHAN, AC>(tx, ty, ob0, bo0, &tm_w, &tm_cw, &tm_m, bnd(tx, ty));
-      if (tn < prm.ntiles) {
+      if (NST == 2 && tn < prm.ntiles) {
         if (NOB == 2)
           issue_both<P, TE, KAHAN, AC>(txn, tyn, s ? stage0 : stage1, s ? ob0 : ob1, s ? bar0 : bar1, &tm_u, &tm_cu, &tm_w,
                                        &tm_cw, &tm_c, &tm_m, bnd(txn, tyn));
@@ -1115,12 +1118,16 @@ persist_step(const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ C
         // let this CTA's copies in flight land before the shared memory is released
         mbar_wait_bounded(bar, parity);
         if (NOB == 1) mbar_wait_bounded(bo0, par_o);
-        if (tn < prm.ntiles) mbar_wait_bounded(s ? bar0 : bar1, ((it + 1) >> 1) & 1);
+        if (NST == 2 && tn < prm.ntiles) mbar_wait_bounded(s ? bar0 : bar1, ((it + 1) >> 1) & 1);
       }
       return;
     }
     tx = txn;
     ty = tyn;
+    if (NST == 1 && tn < prm.ntiles && threadIdx.x == 0) {   // (the barrier that ended the tile freed the stage)
+      fence_proxy_async();
+      issue_region<P, TE, KAHAN, AC>(tx, ty, stage0, bar0, &tm_u, &tm_cu, &tm_c);
+    }
   }
   // receiver rows of the previous step, by the CTA with the fewest tiles (none, where the grid
   // has room): at the head of CTA 0 they delayed its first tile by about 2 us a step

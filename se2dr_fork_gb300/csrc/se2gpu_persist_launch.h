@@ -12,21 +12,20 @@ namespace se2p {
 // sized for (0: as many as the shared memory allows, up to 3), item mapping (0: one
 // thread per (element, line) in order, threads >= (edge + 1)^2 (degree + 1); 1:
 // warp-aligned, 32 / (degree + 1) whole elements per warp, whose three element phases
-// synchronise within the warp, threads = 32 x warps)).  Degree 4: 7x7 at 2 CTAs per SM
-// (92-96 registers) is the fastest, with two owned buffers; sized for 3 CTAs it is capped
-// at 64 registers and runs slower.  default_config gives each degree's fastest.  The
-// two-float mode has a list of its own (se2gpu_f32df_launch.h).  New configurations go at the
-// end of their degree's list: the autotuner's cache and default_config refer to them by
-// position.
+// synchronise within the warp, threads = 32 x warps; 2: as 0, with one region stage:
+// nothing is copied a tile ahead, but more CTAs fit an SM)).  default_config and
+// first_config choose.  The two-float mode has a list of its own (se2gpu_f32df_launch.h).
+// New configurations go at the end of their degree's list: the autotuner's cache and
+// default_config refer to them by position.
 #define SE2P_CONFIGS(X)                                                                      \
   X(1, 15, 512, 0, 0, 0) X(1, 11, 288, 0, 0, 0) X(1, 15, 512, 0, 0, 1)                       \
   X(2, 12, 512, 2, 2, 0) X(2, 10, 384, 0, 0, 0) X(2, 8, 256, 0, 0, 0) X(2, 10, 416, 0, 0, 1) \
   X(3, 7, 256, 0, 0, 0) X(3, 8, 352, 0, 0, 0) X(3, 7, 256, 0, 0, 1)                          \
   X(4, 7, 320, 1, 2, 0) X(4, 7, 320, 2, 0, 0) X(4, 6, 256, 2, 0, 0) X(4, 8, 416, 0, 0, 0)    \
-  X(4, 7, 352, 1, 2, 1) X(4, 6, 288, 2, 0, 1)                                                \
+  X(4, 7, 352, 1, 2, 1) X(4, 6, 288, 2, 0, 1) X(4, 8, 416, 1, 2, 2)                          \
   X(5, 6, 320, 0, 0, 0) X(5, 5, 224, 0, 0, 0) X(5, 6, 320, 0, 0, 1)                          \
   X(6, 5, 256, 0, 0, 0) X(6, 4, 192, 0, 0, 0) X(6, 5, 288, 0, 0, 1)                          \
-  X(7, 4, 224, 0, 0, 0) X(7, 5, 288, 0, 0, 0) X(7, 4, 224, 0, 0, 1)                          \
+  X(7, 4, 224, 0, 0, 0) X(7, 5, 288, 0, 0, 0) X(7, 4, 224, 0, 0, 1) X(7, 5, 288, 1, 2, 2)    \
   X(8, 4, 256, 0, 0, 0) X(8, 3, 160, 0, 0, 0) X(8, 4, 288, 0, 0, 1)
 
 // arithmetic modes of the persistent step kernel
