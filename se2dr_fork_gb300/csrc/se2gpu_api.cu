@@ -427,49 +427,44 @@ static int upload_leapfrog(se2gpu_solver *h, const double *u, const double *v, c
 // the step kernel's tensor maps of the per-tile constants (plain and Kahan modes): the
 // cell box and the 1/M box, the same for both buffer sets (the two-float mode reads its
 // constants with loads and has neither)
-static int make_const_maps(se2gpu_solver *h, const se2p::TileShape &ts)
+static int make_const_maps(se2gpu_solver *h, const se2p::TileShape &ts, CUtensorMap (*maps)[6])
 {
-  for (int b = 0; b < 2; b++) memset(&h->maps[b][4], 0, 2 * sizeof(CUtensorMap));
+  for (int b = 0; b < 2; b++) memset(&maps[b][4], 0, 2 * sizeof(CUtensorMap));
   if (pmode(h) == se2p::MODE_DF || !ts.halo) return 0;
-  int r = se2p::make_map_cells(&h->maps[0][4], h->cellc, h->mx, h->my, ts.cell_box);
-  if (!r) r = se2p::make_map_f32(&h->maps[0][5], h->pminv, h->pitch, h->ny_g, h->pitch, ts.minv_w, ts.own_h);
+  int r = se2p::make_map_cells(&maps[0][4], h->cellc, h->mx, h->my, ts.cell_box);
+  if (!r) r = se2p::make_map_f32(&maps[0][5], h->pminv, h->pitch, h->ny_g, h->pitch, ts.minv_w, ts.own_h);
   if (r) return fail(h, SE2GPU_ERR_CUDA, "cuTensorMapEncodeTiled failed for the tile constants (%d)", r);
-  h->maps[1][4] = h->maps[0][4];
-  h->maps[1][5] = h->maps[0][5];
+  maps[1][4] = maps[0][4];
+  maps[1][5] = maps[0][5];
   return 0;
 }
 
-// select one of the persistent kernel's tile configurations: kernel attributes,
-// tensor-map boxes, per-tile source/receiver lists and the persistent grid
-// (in_create: the handle has run no step yet, so nothing in flight reads the tile lists
-// and the host work here overlaps the set-up kernels still reading the caller's arrays)
-static int setup_f32_config(se2gpu_solver *h, int config, bool in_create = false)
+// what a tile configuration needs besides the state, complete before the handle takes it over
+struct TileSetup {
+  CUtensorMap maps[2][6];
+  int4 *src = nullptr, *rec = nullptr, *bounds = nullptr;
+  void *ef[2] = {nullptr, nullptr};   // element forces, where the handle has none yet
+  int ntx = 0, nty = 0;
+};
+
+// tensor maps, element-force buffers and per-tile source/receiver lists of a configuration, into t;
+// nothing of the handle changes
+static int build_tiles(se2gpu_solver *h, const se2p::TileShape &ts, TileSetup &t)
 {
   const bool kahan = is_kahan(h);
-  const int mode = pmode(h);
-  se2p::TileShape ts;
-  if (se2p::config_shape(h->p, config, mode, &ts)) return fail(h, SE2GPU_ERR_ARG, "no tile configuration %d for degree %d", config, h->p);
-  if (!in_create) CK(h, cudaStreamSynchronize(h->stream));
-  {
-    cudaError_t e = se2p::prepare(h->p, config, mode);
-    if (e != cudaSuccess) return fail(h, SE2GPU_ERR_CUDA, "persistent kernel set-up: %s", cudaGetErrorString(e));
-  }
+  memset(t.maps, 0, sizeof(t.maps));
   for (int b = 0; b < 2 && ts.halo; b++) {
     void *bases[4] = {h->pu[b], kahan ? (void *)h->pcu[b] : (void *)h->pu[b], h->pw[b], kahan ? (void *)h->pcw[b] : (void *)h->pw[b]};
     for (int m = 0; m < 4; m++) {
       const int bw = (m < 2) ? ts.region_w : ts.own_w, bh = (m < 2) ? ts.region_h : ts.own_h;
-      const int r = se2p::make_map(&h->maps[b][m], bases[m], h->nx_g, h->ny_g, h->pitch, bw, bh);
+      const int r = se2p::make_map(&t.maps[b][m], bases[m], h->nx_g, h->ny_g, h->pitch, bw, bh);
       if (r) return fail(h, SE2GPU_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", r);
     }
   }
-  if (h->pminv) {   // (in se2gpu_create the 1/M map follows once 1/M is allocated)
-    int r = make_const_maps(h, ts);
-    if (r) return r;
-  }
-  for (int b = 0; b < 2 && !ts.halo && !h->ef[b]; b++) {   // element forces
-    const int rc = dalloc(h, (void **)&h->ef[b], (size_t)h->mx * h->my * h->npe * (is_df(h) ? 16 : 8));
-    if (rc) return rc;
-  }
+  int rc;
+  if (h->pminv && (rc = make_const_maps(h, ts, t.maps))) return rc;   // (in se2gpu_create they follow once 1/M is allocated)
+  for (int b = 0; b < 2 && !ts.halo; b++)
+    if (!h->ef[b] && (rc = dalloc(h, &t.ef[b], (size_t)h->mx * h->my * h->npe * (is_df(h) ? 16 : 8)))) return rc;
   const int te = ts.tex, P = h->p;
   const int ntx = (h->mx + te - 1) / te, nty = (h->my + te - 1) / te, ntiles = ntx * nty;
   // tile lists: a source or receiver element appears in every tile whose owned nodes it touches, or
@@ -503,17 +498,50 @@ static int setup_f32_config(se2gpu_solver *h, int config, bool in_create = false
     tb[4 * (size_t)t] = so[t]; tb[4 * (size_t)t + 1] = so[t + 1];
     tb[4 * (size_t)t + 2] = ro[t]; tb[4 * (size_t)t + 3] = ro[t + 1];
   }
+  if ((rc = upload_i(h, (int **)&t.bounds, tb.data(), tb.size()))) return rc;
+  if ((rc = upload_i(h, (int **)&t.src, si.data(), si.size()))) return rc;
+  if ((rc = upload_i(h, (int **)&t.rec, ri.data(), ri.size()))) return rc;
+  t.ntx = ntx;
+  t.nty = nty;
+  return 0;
+}
+
+// select one of the persistent kernel's tile configurations: kernel attributes,
+// tensor-map boxes, per-tile source/receiver lists and the persistent grid.  The handle changes
+// only after everything that can fail has succeeded: on an error it runs on as it was.
+// (in_create: the handle has run no step yet, so nothing in flight reads the tile lists
+// and the host work here overlaps the set-up kernels still reading the caller's arrays)
+static int setup_f32_config(se2gpu_solver *h, int config, bool in_create = false)
+{
+  const int mode = pmode(h);
+  se2p::TileShape ts;
+  if (se2p::config_shape(h->p, config, mode, &ts)) return fail(h, SE2GPU_ERR_ARG, "no tile configuration %d for degree %d", config, h->p);
+  if (!in_create) CK(h, cudaStreamSynchronize(h->stream));
+  {
+    cudaError_t e = se2p::prepare(h->p, config, mode);
+    if (e != cudaSuccess) return fail(h, SE2GPU_ERR_CUDA, "persistent kernel set-up: %s", cudaGetErrorString(e));
+  }
+  TileSetup t;
+  const int rc = build_tiles(h, ts, t);
+  if (rc) {
+    for (void *p : {(void *)t.src, (void *)t.rec, (void *)t.bounds, t.ef[0], t.ef[1]}) dfree(h, p);
+    return rc;
+  }
+  memcpy(h->maps, t.maps, sizeof(h->maps));
   dfree(h, h->tile_src); dfree(h, h->tile_rec); dfree(h, h->tile_bounds);
-  h->tile_src = h->tile_rec = h->tile_bounds = nullptr;
-  int rc;
-  if ((rc = upload_i(h, (int **)&h->tile_bounds, tb.data(), tb.size()))) return rc;
-  if ((rc = upload_i(h, (int **)&h->tile_src, si.data(), si.size()))) return rc;
-  if ((rc = upload_i(h, (int **)&h->tile_rec, ri.data(), ri.size()))) return rc;
+  h->tile_src = t.src; h->tile_rec = t.rec; h->tile_bounds = t.bounds;
+  for (int b = 0; b < 2; b++) {
+    if (t.ef[b]) h->ef[b] = static_cast<double2 *>(t.ef[b]);
+    if (ts.halo) {   // (16 (p+1)^2 bytes per element, two-float 32: not kept by a configuration that has no use for them)
+      dfree(h, h->ef[b]);
+      h->ef[b] = nullptr;
+    }
+  }
   h->pconfig = config;
   h->no_halo = !ts.halo;
-  h->pntx = ntx;
-  h->pnty = nty;
-  h->pgrid = std::min(ntiles + 1, std::max(1, se2p::occupancy(P, config, mode)) * h->nsm);
+  h->pntx = t.ntx;
+  h->pnty = t.nty;
+  h->pgrid = std::min(t.ntx * t.nty + 1, std::max(1, se2p::occupancy(h->p, config, mode)) * h->nsm);
   return 0;
 }
 
@@ -750,7 +778,7 @@ int se2gpu_internal_create(const se2gpu_problem *P, int precision, int trace_cap
     }
     se2p::TileShape ts;
     if (se2p::config_shape(h->p, h->pconfig, pmode(h), &ts)) { fail(h, SE2GPU_ERR_ARG, "tile configuration"); TRY(SE2GPU_ERR_ARG); }
-    TRY(make_const_maps(h, ts));
+    TRY(make_const_maps(h, ts, h->maps));
   }
   {
     // one wait for everything queued above (kernels that read the caller's arrays included),

@@ -121,7 +121,14 @@ def _p(a: Optional[np.ndarray], t=_dp):
 
 
 class GpuError(RuntimeError):
-    pass
+    """A failed library call; `code` is its status (SE2GPU_ERR_*)."""
+
+    def __init__(self, message: str, code: int = 0):
+        super().__init__(message)
+        self.code = code
+
+
+ERR_NOMEM = -3   # SE2GPU_ERR_NOMEM
 
 
 def _problem(s: Setup):
@@ -166,7 +173,7 @@ class Solver:
 
     def _check(self, rc: int, what: str) -> int:
         if rc < 0:
-            raise GpuError(f"{what} failed ({rc}): {lib().se2gpu_last_error(self._h).decode()}")
+            raise GpuError(f"{what} failed ({rc}): {lib().se2gpu_last_error(self._h).decode()}", rc)
         return rc
 
     def close(self):
@@ -334,7 +341,7 @@ class Ensemble:
 
     def _check(self, rc: int, what: str) -> int:
         if rc < 0:
-            raise GpuError(f"{what} failed ({rc}): {lib().se2gpu_ensemble_last_error(self._h).decode()}")
+            raise GpuError(f"{what} failed ({rc}): {lib().se2gpu_ensemble_last_error(self._h).decode()}", rc)
         return rc
 
     def close(self):

@@ -1,0 +1,83 @@
+"""Device calls that fail on the host: the handle stays usable, nothing is left half changed.
+
+A preloaded library stands in for the runtime's allocation and launch calls and returns their
+error codes on request, so no allocation is driven to its limit and no kernel fails on the device.
+"""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+FAKE = r"""
+#define _GNU_SOURCE
+#include <dlfcn.h>
+#include <stddef.h>
+/* the runtime's own call (its library is not in the global scope: RTLD_NEXT does not see it) */
+static void *real_call(const char *name) { return dlsym(dlopen("libcudart.so.13", RTLD_LAZY | RTLD_NOLOAD), name); }
+static int alloc_in = -1;   /* calls until allocations fail; -1: never */
+void fake_alloc(int n) { alloc_in = n; }
+int cudaMallocFromPoolAsync(void **p, size_t n, void *pool, void *stream)
+{
+  static int (*real)(void **, size_t, void *, void *);
+  if (!real) real = (int (*)(void **, size_t, void *, void *))real_call("cudaMallocFromPoolAsync");
+  if (alloc_in == 0) return 2;   /* cudaErrorMemoryAllocation */
+  if (alloc_in > 0) alloc_in--;
+  return real(p, n, pool, stream);
+}
+"""
+
+PRELUDE = """
+import ctypes, sys
+import numpy as np
+from se2dr_fork_gb300 import gpu as G, host as H, spec as S
+fake = ctypes.CDLL(sys.argv[1])
+"""
+
+
+@pytest.fixture(scope="module")
+def run_with_fake(gpu_lib, tmp_path_factory):
+    d = tmp_path_factory.mktemp("fake")
+    src, lib = d / "fake.c", d / "libfake.so"
+    src.write_text(FAKE)
+    subprocess.run(["gcc", "-O1", "-shared", "-fPIC", "-o", str(lib), str(src), "-ldl"], check=True)
+
+    def run(code):
+        env = dict(os.environ, LD_PRELOAD=str(lib), PYTHONPATH=ROOT)
+        r = subprocess.run([sys.executable, "-c", PRELUDE + code, str(lib)], cwd=ROOT, env=env, timeout=300,
+                           capture_output=True, text=True)
+        assert r.returncode == 0, r.stdout + r.stderr
+    return run
+
+
+@pytest.mark.parametrize("precision", ["fp32_kahan", "fp32", "fp32_df"])
+def test_failed_tile_configuration_leaves_the_handle_as_it_was(run_with_fake, precision):
+    """Whatever allocation of se2gpu_set_tile_config fails, the handle goes on with the
+    configuration it had: same getter, same bits."""
+    run_with_fake(f"""
+su = H.Setup(S.demo(19, 17, p=3, tmax=1e30).replace(nt=1000))
+ref = G.Solver(su, "{precision}")
+n = len(ref.tile_configs())
+sol, rows, failures = G.Solver(su, "{precision}"), [], 0
+for start in range(n):
+    for c in range(n):
+        for k in range(6):
+            sol.set_tile_config(start)
+            fake.fake_alloc(k)
+            try:
+                sol.set_tile_config(c)
+            except G.GpuError as e:
+                assert e.code == G.ERR_NOMEM
+                failures += 1
+                assert sol.tile_config == start and G.lib().se2gpu_tile_config(sol._h) == start
+            fake.fake_alloc(-1)
+            rows.append(sol.run(2))
+want = ref.run(2 * len(rows))
+assert np.array_equal(np.concatenate(rows), want)
+assert all(np.array_equal(x, y) for x, y in zip(sol.fields(), ref.fields()))
+assert failures >= 3 * n * (n - 1), failures
+""")
