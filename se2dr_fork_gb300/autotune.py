@@ -15,7 +15,7 @@ import math
 import os
 from typing import Dict, Optional
 
-from .gpu import PRECISIONS, Solver
+from .gpu import ERR_NOMEM, PRECISIONS, GpuError, Solver
 
 CACHE = os.environ.get("SE2GPU_TUNING", os.path.join(os.path.dirname(os.path.abspath(__file__)), "tuning.json"))
 
@@ -67,13 +67,22 @@ def time_config(sol: Solver, config: int, steps: int, warmup: int = 2) -> float:
 
 
 def tune(setup, precision: str = "fp32_kahan", steps: int = 10, write: bool = True) -> dict:
-    """Measure every configuration on `setup`; return {config, edge, threads, seconds, all}."""
+    """Measure every configuration on `setup`; return {config, edge, threads, seconds, all}.
+    A configuration whose buffers the device cannot hold beside the handle is left out (its
+    seconds are None)."""
     sol = Solver(setup, precision, trace_capacity=2 * steps + 8)
     configs = sol.tile_configs()
     infos = [sol.tile_config_info(c) for c in range(len(configs))]
-    times = [time_config(sol, c, steps) for c in range(len(configs))]
+    times = []
+    for c in range(len(configs)):
+        try:
+            times.append(time_config(sol, c, steps))
+        except GpuError as e:
+            if e.code != ERR_NOMEM:
+                raise
+            times.append(None)
     sol.close()
-    best = min(range(len(times)), key=lambda c: times[c])
+    best = min((c for c in range(len(times)) if times[c] is not None), key=lambda c: times[c])
     res = {"config": best, "edge": configs[best][0], "threads": configs[best][1], "seconds": times[best],
            "all": [dict(info, seconds=s) for info, s in zip(infos, times)]}
     if write:
