@@ -357,17 +357,31 @@ extern "C" int se2gpu_ensemble_tile_config(const se2gpu_ensemble *e, int p)
   return SE2GPU_ERR_ARG;
 }
 
-// The launches of one block of n <= K steps starting from input buffer `cur`, slot sl.  The
-// chunks are independent of one another, so each walks its steps on a chain of its own
-// (streams, or branches of the captured graph): while the last CTAs of one chunk's step
-// drain, another chunk's fill the SMs, and small groups run side by side.
-static int enqueue_block(se2gpu_ensemble *e, int cur, int sl, int n, cudaStream_t st)
+// the side chains begin behind st's work so far ...
+static int fork_chains(se2gpu_ensemble *e, cudaStream_t st)
+{
+  if (e->side.empty()) return 0;
+  ECK(e, cudaEventRecord(e->fork, st));
+  for (cudaStream_t s : e->side) ECK(e, cudaStreamWaitEvent(s, e->fork, 0));
+  return 0;
+}
+
+// ... and st waits for them
+static int join_chains(se2gpu_ensemble *e, cudaStream_t st)
+{
+  for (size_t s = 0; s < e->side.size(); s++) {
+    ECK(e, cudaEventRecord(e->joins[s], e->side[s]));
+    ECK(e, cudaStreamWaitEvent(st, e->joins[s], 0));
+  }
+  return 0;
+}
+
+// The steps of a block.  The chunks are independent of one another, so each walks its steps on a
+// chain of its own (streams, or branches of the captured graph): while the last CTAs of one chunk's
+// step drain, another chunk's fill the SMs, and small groups run side by side.
+static int enqueue_steps(se2gpu_ensemble *e, int cur, int sl, int n, cudaStream_t st)
 {
   const int chains = 1 + (int)e->side.size();
-  if (chains > 1) {
-    ECK(e, cudaEventRecord(e->fork, st));
-    for (cudaStream_t s : e->side) ECK(e, cudaStreamWaitEvent(s, e->fork, 0));
-  }
   for (int k = 0; k < n; k++) {
     const int cin = cur ^ (k & 1);
     int chunk = 0;
@@ -388,10 +402,17 @@ static int enqueue_block(se2gpu_ensemble *e, int cur, int sl, int n, cudaStream_
           return efail(e, SE2GPU_ERR_CUDA, "batched step kernel (degree %d): %s", g.p, cudaGetErrorString(r));
       }
   }
-  for (size_t s = 0; s < e->side.size(); s++) {
-    ECK(e, cudaEventRecord(e->joins[s], e->side[s]));
-    ECK(e, cudaStreamWaitEvent(st, e->joins[s], 0));
-  }
+  return 0;
+}
+
+// The launches of one block of n <= K steps starting from input buffer `cur`, slot sl.  The chains
+// are joined also when a launch has failed: st then waits for all that was launched.
+static int enqueue_block(se2gpu_ensemble *e, int cur, int sl, int n, cudaStream_t st)
+{
+  int rc = fork_chains(e, st);
+  if (!rc) rc = enqueue_steps(e, cur, sl, n, st);
+  const int rj = join_chains(e, st);
+  if (rc || rj) return rc ? rc : rj;
   for (Group &g : e->groups) {
     cudaError_t r = se2p::launch_record_batch(g.p, g.tab[cur][sl], (int)g.shots.size(), n - 1, st);
     if (r != cudaSuccess) return efail(e, SE2GPU_ERR_CUDA, "receiver kernel (degree %d): %s", g.p, cudaGetErrorString(r));

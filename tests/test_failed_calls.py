@@ -29,6 +29,32 @@ int cudaMallocFromPoolAsync(void **p, size_t n, void *pool, void *stream)
   if (alloc_in > 0) alloc_in--;
   return real(p, n, pool, stream);
 }
+static int launch_in = -1, records, waits;
+void fake_launch(int n) { launch_in = n; records = waits = 0; }
+int fake_records(void) { return records; }
+int fake_waits(void) { return waits; }
+int cudaLaunchKernelExC(const void *cfg, const void *fn, void **args)
+{
+  static int (*real)(const void *, const void *, void **);
+  if (!real) real = (int (*)(const void *, const void *, void **))real_call("cudaLaunchKernelExC");
+  if (launch_in == 0) return 701;   /* cudaErrorLaunchOutOfResources */
+  if (launch_in > 0) launch_in--;
+  return real(cfg, fn, args);
+}
+int cudaEventRecord(void *event, void *stream)
+{
+  static int (*real)(void *, void *);
+  if (!real) real = (int (*)(void *, void *))real_call("cudaEventRecord");
+  records++;
+  return real(event, stream);
+}
+int cudaStreamWaitEvent(void *stream, void *event, unsigned flags)
+{
+  static int (*real)(void *, void *, unsigned);
+  if (!real) real = (int (*)(void *, void *, unsigned))real_call("cudaStreamWaitEvent");
+  waits++;
+  return real(stream, event, flags);
+}
 """
 
 PRELUDE = """
@@ -80,4 +106,37 @@ want = ref.run(2 * len(rows))
 assert np.array_equal(np.concatenate(rows), want)
 assert all(np.array_equal(x, y) for x, y in zip(sol.fields(), ref.fields()))
 assert failures >= 3 * n * (n - 1), failures
+""")
+
+
+@pytest.mark.parametrize("graphs", [False, True])
+def test_failed_ensemble_launch_joins_its_chains(run_with_fake, graphs):
+    """A block whose n-th launch fails leaves no chain running beside the ensemble's stream: each
+    side chain is recorded and waited for, captured or not, and the ensemble can be set and run
+    again."""
+    run_with_fake(f"""
+setups = [H.Setup(S.shot(7, i, size=(20 + i, 18), p=p, nt=64)) for i, p in enumerate((3, 4, 6, 3))]
+def new():
+    e = G.Ensemble(setups, "fp32_kahan", block=4)
+    e.set_graphs({graphs})
+    return e
+ref = new()
+want = ref.advance(8)
+ens = new()
+for n in range(12):   # 3 groups, one launch each per step
+    fake.fake_launch(n)
+    try:
+        ens.advance(4, traces=False)
+        raise SystemExit("the launch did not fail")
+    except G.GpuError as e:
+        assert e.code == -2, e
+    fork, joins = 1, 2   # (the upload's event is recorded besides)
+    assert fake.fake_waits() == 2 * joins and fake.fake_records() == fork + joins + 1, (fake.fake_waits(), fake.fake_records())
+    fake.fake_launch(-1)
+for i, su in enumerate(setups):
+    ens.set_fields(i, *(np.zeros(su.ndof) for _ in range(3)))
+got = ens.advance(8)
+assert all(np.array_equal(x, y) for x, y in zip(got, want))
+for i in range(len(setups)):
+    assert all(np.array_equal(x, y) for x, y in zip(ens.fields(i), ref.fields(i)))
 """)
