@@ -47,6 +47,7 @@ struct Group {
   std::vector<se2p::Params> htab[2][2];                                // the same, host (launch arguments)
   CUtensorMap *maps[2] = {nullptr, nullptr};                           // [input buffer], device [shot][4]
   int2 *items = nullptr;                                               // device (shot in its chunk, ty << 16 | tx)
+  bool ready = false;                      // the tables name the shots' current tile lists
 };
 
 }  // namespace
@@ -212,6 +213,7 @@ static int build_group(se2gpu_ensemble *e, Group &g)
   g.nitems = (int)items.size();
   int rc = dput(e, &g.items, items.data(), items.size());
   if (rc) return rc;
+  g.ready = true;
   return 0;
 }
 
@@ -342,6 +344,7 @@ extern "C" int se2gpu_ensemble_set_tile_config(se2gpu_ensemble *e, int p, int co
   if (config < 0 || config >= se2p::num_configs(p)) return efail(e, SE2GPU_ERR_ARG, "no tile configuration %d for degree %d", config, p);
   ECK(e, cudaStreamSynchronize(e->stream));
   drop_graphs(e);
+  it->ready = false;   // (from here on until the tables are built again: no block runs on freed lists)
   for (int s : it->shots)
     if (se2gpu_set_tile_config(e->sol[s], config) != 0)
       return efail(e, SE2GPU_ERR_CUDA, "shot %d: %s", s, se2gpu_last_error(e->sol[s]));
@@ -430,6 +433,8 @@ static int launches_per_block(const se2gpu_ensemble *e, int n)
 static int run_block(se2gpu_ensemble *e, int sl, int n)
 {
   const int cur = e->cur;
+  for (const Group &g : e->groups)
+    if (!g.ready) return efail(e, SE2GPU_ERR_STATE, "the tile configuration of degree %d could not be set: set one first", g.p);
   if (e->use_graphs && n == e->block) {
     if (!e->graph[cur][sl]) {
       cudaGraph_t graph = nullptr;

@@ -140,3 +140,31 @@ assert all(np.array_equal(x, y) for x, y in zip(got, want))
 for i in range(len(setups)):
     assert all(np.array_equal(x, y) for x, y in zip(ens.fields(i), ref.fields(i)))
 """)
+
+
+def test_failed_ensemble_tile_configuration_is_refused_until_one_is_set(run_with_fake):
+    """A tile configuration that fails for the second shot of its group leaves the group's tables
+    behind: no block runs until one has been set."""
+    run_with_fake("""
+setups = [H.Setup(S.shot(7, i, size=(20 + i, 18), p=p, nt=64)) for i, p in enumerate((3, 4, 3))]
+ref, ens = G.Ensemble(setups, "fp32_kahan", block=4), G.Ensemble(setups, "fp32_kahan", block=4)
+want = [ref.advance(8), ref.advance(8)]
+got = [ens.advance(8)]
+for k in (0, 4):
+    fake.fake_alloc(k)
+    try:
+        ens.set_tile_config(3, 1)
+        raise SystemExit("the allocation did not fail")
+    except G.GpuError:
+        pass
+    fake.fake_alloc(-1)
+    try:
+        ens.advance(8)
+        raise SystemExit("a block ran")
+    except G.GpuError as e:
+        assert e.code == -4, e   # SE2GPU_ERR_STATE
+ens.set_tile_config(3, 1)
+got.append(ens.advance(8))
+for g, w in zip(got, want):
+    assert all(np.array_equal(x, y) for x, y in zip(g, w))
+""")
