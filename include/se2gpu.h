@@ -134,10 +134,12 @@ int se2gpu_device_fields(const se2gpu_solver *h, void **u, void **v, void **a);
 /* Tile configurations of the step kernel (elements per tile edge, threads per
    CTA) available for the handle's degree and precision, for the autotuner;
    returns how many exist.  se2gpu_set_tile_config selects one; se2gpu_tile_config
-   returns the selected one (before a selection the one measured fastest for the
-   handle's degree and mesh size on GB300 among those for many tiles; a plain or Kahan
-   handle on a small mesh then runs the last one, which keeps element forces in
-   memory; 0 in the FP64 mode). */
+   returns the selected one.  A new handle has the number of its degree's tiles for large
+   meshes; on a mesh for which others measured faster on GB300 that number names these, so
+   it always is the fastest known choice and its entry in the list is what runs.  The other
+   numbers name the same tiles on every mesh.  FP64 has the one number 0, whose entry is
+   what runs on the handle's mesh (edge: elements along x).
+   A failed selection leaves the handle as it was. */
 int se2gpu_tile_configs(const se2gpu_solver *h, int *edge, int *threads, int max_configs);
 int se2gpu_set_tile_config(se2gpu_solver *h, int config);
 int se2gpu_tile_config(const se2gpu_solver *h);

@@ -742,8 +742,9 @@ int se2gpu_internal_create(const se2gpu_problem *P, int precision, int trace_cap
       h->src_elem_h = new std::vector<int>(P->src_elem, P->src_elem + P->nsrc);
       h->rec_elem_h = new std::vector<int>(P->rec_elem, P->rec_elem + P->nrec);
       const int mesh_x = in_ensemble ? 0 : P->mx;
-      TRY(setup_f32_config(h, se2p::first_config(P->p, pmode(h), mesh_x, P->my, h->nsm), true));
-      h->reported_config = se2p::default_config(P->p, pmode(h), mesh_x, P->my, h->nsm);
+      h->config = h->auto_config = se2p::auto_config(P->p, pmode(h));
+      h->auto_tiles = se2p::first_config(P->p, pmode(h), mesh_x, P->my, h->nsm);
+      TRY(setup_f32_config(h, h->auto_tiles, true));
     }
     for (cudaEvent_t &ev : h->side_done) {
       const cudaError_t e = cudaStreamWaitEvent(h->stream, ev, 0);
@@ -1236,6 +1237,9 @@ extern "C" int se2gpu_device_fields(const se2gpu_solver *h, void **u, void **v, 
   return 0;
 }
 
+// the tiles that a configuration number stands for on this handle
+static int tiles_of(const se2gpu_solver *h, int config) { return config == h->auto_config ? h->auto_tiles : config; }
+
 extern "C" int se2gpu_tile_configs(const se2gpu_solver *h, int *edge, int *threads, int max_configs)
 {
   if (!h) return SE2GPU_ERR_ARG;
@@ -1246,7 +1250,7 @@ extern "C" int se2gpu_tile_configs(const se2gpu_solver *h, int *edge, int *threa
   const int n = se2p::num_configs(h->p, pmode(h));
   for (int c = 0; c < n && c < max_configs; c++) {
     se2p::TileShape ts;
-    se2p::config_shape(h->p, c, pmode(h), &ts);
+    se2p::config_shape(h->p, tiles_of(h, c), pmode(h), &ts);
     if (edge) edge[c] = ts.tex;
     if (threads) threads[c] = ts.nt;
   }
@@ -1262,7 +1266,9 @@ extern "C" int se2gpu_tile_config_info(const se2gpu_solver *h, int config, int i
     return 0;
   }
   se2p::TileShape ts;
-  if (config < 0 || se2p::config_shape(h->p, config, pmode(h), &ts)) return SE2GPU_ERR_ARG;
+  if (config < 0 || config >= se2p::num_configs(h->p, pmode(h))) return SE2GPU_ERR_ARG;
+  config = tiles_of(h, config);
+  if (se2p::config_shape(h->p, config, pmode(h), &ts)) return SE2GPU_ERR_ARG;
   info[0] = ts.tex; info[1] = ts.nt; info[2] = ts.owned_buffers;
   // the occupancy query needs the kernel's dynamic shared-memory limit raised first
   if (cudaSetDevice(h->device) != cudaSuccess || se2p::prepare(h->p, config, pmode(h)) != cudaSuccess) {
@@ -1276,7 +1282,7 @@ extern "C" int se2gpu_tile_config_info(const se2gpu_solver *h, int config, int i
 extern "C" int se2gpu_tile_config(const se2gpu_solver *h)
 {
   if (!h) return SE2GPU_ERR_ARG;
-  return is_f64(h) ? 0 : h->reported_config;
+  return is_f64(h) ? 0 : h->config;
 }
 
 extern "C" int se2gpu_set_tile_config(se2gpu_solver *h, int config)
@@ -1285,11 +1291,11 @@ extern "C" int se2gpu_set_tile_config(se2gpu_solver *h, int config)
   if (is_f64(h)) return (config == 0) ? 0 : fail(h, SE2GPU_ERR_ARG, "FP64 mode has a single tile configuration");
   if (config < 0 || config >= se2p::num_configs(h->p, pmode(h))) return fail(h, SE2GPU_ERR_ARG, "tile configuration %d out of range", config);
   CK(h, cudaSetDevice(h->device));
-  if (config != h->pconfig) {   // (else tables, maps and grid are current)
-    const int rc = setup_f32_config(h, config);
+  if (tiles_of(h, config) != h->pconfig) {   // (else tables, maps and grid are current)
+    const int rc = setup_f32_config(h, tiles_of(h, config));
     if (rc) return rc;
   }
-  h->reported_config = config;
+  h->config = config;
   return 0;
 }
 

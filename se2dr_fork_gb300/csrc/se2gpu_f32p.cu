@@ -76,7 +76,7 @@ static const Entry *find(int p, int config)
   return nullptr;
 }
 
-// the configuration a handle starts with.  Plain and Kahan: per degree the one the autotuner
+// the tiles for meshes of many tiles.  Plain and Kahan: per degree the one the autotuner
 // measured fastest on GB300 at about 16M nodes (and, at degree 4, at the 2048^2 workload; the
 // plain mode at degree 8 runs 4 x 4 tiles: 83 against 93 us a step at 5M nodes, 7.0 against 9.6 at
 // 260000), and smaller tiles on meshes that these divide into about one per SM (us a step: degree 6,
@@ -126,7 +126,9 @@ int num_configs(int p)
   return k;
 }
 
-// What a handle on which no configuration was chosen runs: the step without a halo on a small mesh, up
+int auto_config(int p, int mode) { return mode == MODE_DF ? 0 : default_config(p, mode, 0, 0, 1); }
+
+// The tiles of a new handle (and of the number auto_config): the step without a halo on a small mesh, up
 // to few[] of its tiles per SM, and at two degrees other tiles than default_config's where the rounds
 // that the resident CTAs need, times the elements of a tile with its halo, say that these take less.
 // us a step, Kahan / plain.  Degree 4: 6 x 6 while one per SM holds the mesh (71 x 71 elements 6.0 ->

@@ -37,7 +37,8 @@ struct se2gpu_solver {
   float4 *cellc;                 // plain and Kahan modes: (lam detJ, mu detJ, d xi/dx, d eta/dy) per cell
   int4 *tile_bounds;             // per tile: source and receiver list bounds
   int pgrid, pconfig, pntx, pnty;
-  int reported_config;           // pconfig once one was chosen; before that, the degree's default
+  int config;                    // selected configuration number; pconfig: the tiles that it stands for
+  int auto_config, auto_tiles;   // the number of the mesh's own choice, and its tiles (se2p::first_config)
   bool no_halo;                  // FP32: the configuration's step keeps element forces (se2gpu_f32ef.cuh)
   int4 *tile_src, *tile_rec;     // per-tile list entries
   std::vector<int> *src_elem_h, *rec_elem_h;

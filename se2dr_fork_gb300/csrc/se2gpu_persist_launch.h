@@ -43,8 +43,11 @@ struct TileShape {
 cudaError_t set_tables(int p, const double *D, const double *w1d);   // constant-memory D, w (current device)
 int num_configs(int p);                                               // tile configurations for degree p (ensembles)
 int num_configs(int p, int mode);                                     // of a handle: those without a halo follow
-int default_config(int p, int mode, int mx, int my, int nsm);         // the one a new handle reports
-int first_config(int p, int mode, int mx, int my, int nsm);           // and the one that it runs
+int default_config(int p, int mode, int mx, int my, int nsm);         // the tiles for meshes of many tiles
+int first_config(int p, int mode, int mx, int my, int nsm);           // the tiles that a new handle runs
+// the number that a new handle has: on its mesh it stands for first_config's tiles (on a large one
+// these are the tiles of that number in the list)
+int auto_config(int p, int mode);
 // mode: MODE_PLAIN, MODE_KAHAN or MODE_DF (the batched kernel: plain or Kahan)
 int config_shape(int p, int config, int mode, TileShape *s);
 cudaError_t prepare(int p, int config, int mode);                     // dynamic shared-memory limit

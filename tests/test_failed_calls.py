@@ -105,7 +105,7 @@ for start in range(n):
 want = ref.run(2 * len(rows))
 assert np.array_equal(np.concatenate(rows), want)
 assert all(np.array_equal(x, y) for x, y in zip(sol.fields(), ref.fields()))
-assert failures >= 3 * n * (n - 1), failures
+assert failures >= 3 * (n - 1) * (n - 2), failures   # (two numbers may name the same tiles)
 """)
 
 
