@@ -99,11 +99,16 @@ def lookup(setup, precision: str) -> Optional[int]:
 
 def apply(sol: Solver, precision: Optional[str] = None) -> int:
     """Select the cached best configuration for this solver (configuration 0 if none).
-    `precision` defaults to the solver's own."""
+    `precision` defaults to the solver's own.  A cached number that names other tiles than when
+    it was measured is not used."""
     if precision is None:
         precision = {v: k for k, v in PRECISIONS.items()}[sol.precision]
-    c = lookup(sol.setup, precision)
-    if c is not None and c < len(sol.tile_configs()):
-        sol.set_tile_config(c)
-        return c
+    ent = load().get(key(sol.setup, precision))
+    configs = sol.tile_configs()
+    if ent is not None and int(ent["config"]) < len(configs):
+        c = int(ent["config"])
+        edge, threads = configs[c]
+        if (ent.get("edge", edge), ent.get("threads", threads)) == (edge, threads):
+            sol.set_tile_config(c)
+            return c
     return 0

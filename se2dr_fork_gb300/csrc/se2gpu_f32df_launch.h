@@ -8,8 +8,9 @@ namespace se2p {
 
 // Tile configurations of the two-float mode, X(degree, elements per tile edge, threads) for the step
 // without a halo (threads >= edge^2 (degree + 1), whole warps) and H(degree, edge, threads) for the
-// one that recomputes a halo of elements (se2gpu_persist.cuh), as many per degree as the other FP32
-// modes have.  The halo is kept where it was faster: large meshes of degrees 2 and 3, whose
+// one that recomputes a halo of elements (se2gpu_persist.cuh).  Per degree the tile for large meshes
+// comes first and those for small meshes last: a number kept from a list of other tiles then
+// selects one that a large mesh can run on.  The halo is kept where it was faster: large meshes of degrees 2 and 3, whose
 // elements are cheap against the node part and the forces' traffic (a million nodes: 75 against 78
 // us a step, 69 against 72).  Everywhere else it lost: at 2.5M nodes 257 against 234 us (degree 1),
 // 163 / 153 (4), 200 / 160 (5), 219 / 169 (6), 304 / 176 (7), 276 / 196 (8).  Small tiles with
@@ -20,10 +21,10 @@ namespace se2p {
   X(1, 12, 288) X(1, 8, 320) X(1, 6, 192)                                                   \
   H(2, 12, 512) X(2, 8, 192) X(2, 6, 192) X(2, 4, 96)                                       \
   H(3, 7, 256) X(3, 4, 64) X(3, 4, 192)                                                     \
-  X(4, 3, 192) X(4, 5, 128) X(4, 2, 96) X(4, 3, 64) X(4, 6, 192) X(4, 7, 256)               \
-  X(5, 4, 96) X(5, 2, 128) X(5, 6, 224)                                                     \
+  X(4, 5, 128) X(4, 7, 256) X(4, 6, 192) X(4, 3, 64) X(4, 3, 192) X(4, 2, 96)               \
+  X(5, 4, 96) X(5, 6, 224) X(5, 2, 128)                                                     \
   X(6, 6, 256) X(6, 3, 64) X(6, 2, 192)                                                     \
-  X(7, 4, 128) X(7, 2, 256) X(7, 3, 96)                                                     \
+  X(7, 4, 128) X(7, 3, 96) X(7, 2, 256)                                                     \
   X(8, 5, 256) X(8, 3, 96) X(8, 1, 96)
 
 // exchange rows: float4 between rows and between elements

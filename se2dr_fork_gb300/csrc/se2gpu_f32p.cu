@@ -106,10 +106,10 @@ int default_config(int p, int mode, int mx, int my, int nsm)
       case 1: return tiles(1) <= nsm ? 1 : 0;
       case 2: return tiles(2) <= 4L * nsm ? 2 : tiles(1) <= 16L * nsm ? 1 : 0;
       case 3: return tiles(2) <= 4L * nsm ? 2 : tiles(1) <= 28L * nsm ? 1 : 0;
-      case 4: return tiles(0) <= 4L * nsm ? 0 : 1;
-      case 5: return tiles(1) <= 6L * nsm ? 1 : 0;
+      case 4: return tiles(4) <= 4L * nsm ? 4 : 0;
+      case 5: return tiles(2) <= 6L * nsm ? 2 : 0;
       case 6: return tiles(2) <= 2L * nsm ? 2 : tiles(0) < 4L * nsm ? 1 : 0;
-      case 7: return tiles(1) <= 2L * nsm ? 1 : 0;
+      case 7: return tiles(2) <= 2L * nsm ? 2 : 0;
       default: return tiles(2) <= 5L * nsm ? 2 : tiles(0) < 2L * nsm ? 1 : 0;
     }
   }
@@ -126,7 +126,7 @@ int num_configs(int p)
   return k;
 }
 
-int auto_config(int p, int mode) { return mode == MODE_DF ? 0 : default_config(p, mode, 0, 0, 1); }
+int auto_config(int p, int mode) { return default_config(p, mode, 0, 0, 1); }
 
 // The tiles of a new handle (and of the number auto_config): the step without a halo on a small mesh, up
 // to few[] of its tiles per SM, and at two degrees other tiles than default_config's where the rounds

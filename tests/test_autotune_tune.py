@@ -43,3 +43,13 @@ def test_another_failure_is_raised(monkeypatch):
     with pytest.raises(G.GpuError) as e:
         _tune(monkeypatch, {0: -2})
     assert e.value.code == -2
+
+
+def test_a_cached_number_of_other_tiles_is_not_used(tmp_path, monkeypatch):
+    monkeypatch.setattr(A, "CACHE", str(tmp_path / "tuning.json"))
+    sol = FakeSolver(H.Setup(S.explosion64(16, 12, p=4)), "fp32_df")
+    sol.selected = None
+    sol.set_tile_config = lambda c: setattr(sol, "selected", c)
+    for edge, threads, want in [(5, 128, None), (6, 224, None), (6, 256, 2)]:
+        A.save({A.key(sol.setup, "fp32_df"): {"config": 2, "edge": edge, "threads": threads}})
+        assert A.apply(sol) == (want or 0) and sol.selected == want

@@ -49,3 +49,12 @@ def test_new_handle_reports_the_tiles_it_runs(precision, p, m, edge, threads, ow
     before = sol.info()["launches"]
     sol.advance(5)
     assert sol.info()["launches"] - before == n
+
+
+@pytest.mark.parametrize("p", range(1, 9))
+def test_two_float_numbers_of_small_tiles_come_last(p):
+    """A two-float number kept from another list of tiles selects one that a large mesh can run on:
+    the tiles of small meshes are the last ones."""
+    m = 1000 // p
+    edges = [e for e, _ in _solver(m, m, p, "fp32_df").tile_configs()]
+    assert min(edges) not in edges[:len(edges) // 2] and max(edges) in edges[:2]
