@@ -354,10 +354,11 @@ struct se2nn {
   float *params = nullptr, *grads = nullptr, *adam_m = nullptr, *adam_v = nullptr;
   long adam_t = 0;
   // BF16 copy of all parameters, and into it the matrices the kernels read; the 2w x 2w mode
-  // blocks of the GEMM path are formed from the parameters when that path next runs
+  // blocks of the GEMM path are formed when that path next runs or, once it has been captured,
+  // with every change of the parameters (the captured pass reads them when it is replayed)
   bf16 *Pb = nullptr, *W0b = nullptr, *W1b = nullptr, *W2b = nullptr;
   std::vector<bf16 *> Wb, Wreb, Wimb, Wblk;
-  bool wblk_stale = true;
+  bool wblk_stale = true, wblk_captured = false;
   int nsm = 0, row_ctas[4] = {1, 1, 1, 1};   // SMs; the row kernels' resident CTAs per SM
   // DFT matrices (BF16): Ex [2m][nx], My [4m][2ny], Myinv [2ny][4m] (= My^T), Exinv [nx][2m],
   // and the transposes ExT [nx][2m], ExinvT [2m][nx]
@@ -476,25 +477,50 @@ int build_dft(se2nn *h)
   return 0;
 }
 
-// refresh the BF16 operand copy from the FP32 master parameters
-int refresh_bf16(se2nn *h)
+bool capturing(const se2nn *h)
 {
-  k_f32_to_bf16<<<nblk(h->P), EW, 0, h->stream>>>(h->params, h->Pb, h->P);
-  h->wblk_stale = true;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(h->stream, &st) != cudaSuccess) cudaGetLastError();
+  return st != cudaStreamCaptureStatusNone;
+}
+
+// the mode blocks of the GEMM path, from the parameters
+int build_wblk(se2nn *h)
+{
+  for (int l = 0; l < h->L; l++)
+    k_build_wblk<<<nblk((long)h->nmodes * 4 * h->w * h->w), EW, 0, h->stream>>>(h->params + h->oWre[l], h->params + h->oWim[l],
+                                                                                h->Wblk[l], h->nmodes, h->w);
   NCK(h, cudaGetLastError());
   return 0;
 }
 
-// the mode blocks of the GEMM path
-int refresh_wblk(se2nn *h)
+// after each change of the parameters.  What is captured has not run: it takes the blocks along and
+// leaves the flag.
+int params_changed(se2nn *h)
 {
+  const bool cap = capturing(h), build = h->wblk_captured || cap;
+  if (!cap) h->wblk_stale = !build;
+  return build ? build_wblk(h) : 0;
+}
+
+// before the GEMM path reads the blocks
+int need_wblk(se2nn *h)
+{
+  if (capturing(h)) {
+    h->wblk_captured = true;
+    return h->wblk_stale ? build_wblk(h) : 0;
+  }
   if (!h->wblk_stale) return 0;
-  for (int l = 0; l < h->L; l++)
-    k_build_wblk<<<nblk((long)h->nmodes * 4 * h->w * h->w), EW, 0, h->stream>>>(h->params + h->oWre[l], h->params + h->oWim[l],
-                                                                                h->Wblk[l], h->nmodes, h->w);
   h->wblk_stale = false;
+  return build_wblk(h);
+}
+
+// refresh the BF16 operand copy from the FP32 master parameters
+int refresh_bf16(se2nn *h)
+{
+  k_f32_to_bf16<<<nblk(h->P), EW, 0, h->stream>>>(h->params, h->Pb, h->P);
   NCK(h, cudaGetLastError());
-  return 0;
+  return params_changed(h);
 }
 
 }  // namespace
@@ -932,7 +958,7 @@ int forward(se2nn *h, const bf16 *x, int B, float *out, bool keep)
   if (fused) {
     if ((rc = layers_fused(h, x, B, keep))) return rc;
   } else {
-  if ((rc = refresh_wblk(h))) return rc;
+  if ((rc = need_wblk(h))) return rc;
   {
     GemmArgs g = mk(x, h->c.cin, 0, 0, h->W0b, w, 0, 0, (int)rows, w, h->c.cin, 1, h->H[0], w, 0, 0);
     g.bias = h->params + h->ob0;
@@ -983,7 +1009,7 @@ int backward(se2nn *h, const bf16 *x, int B)
   if ((rc = colsum(h, h->dD1, drows, hid, 256, h->grads + h->oc1))) return rc;
   GEMM(h, mk(h->dD1, hid, 0, 0, h->W1b, hid, 0, 1, (int)drows, w, hid, 1, h->dD0, w, 0, 0));
   if (fused_ok(h, x)) return layers_bwd_fused(h, x, B);
-  if ((rc = refresh_wblk(h))) return rc;
+  if ((rc = need_wblk(h))) return rc;
   k_decoder_scatter<<<nblk(rows * w / 8), EW, 0, h->stream>>>(h->dD0, h->rec_x, B, nrec, h->c.ny, h->c.nx, w, h->dHa);
   // Fourier layers, last to first: dHa holds dL/dH[l+1]
   for (int l = L - 1; l >= 0; l--) {
@@ -1286,9 +1312,8 @@ extern "C" int se2nn_adam_step(se2nn *h, float lr, float beta1, float beta2, flo
   const float c1 = 1.f - powf(beta1, (float)h->adam_t), c2 = 1.f - powf(beta2, (float)h->adam_t);
   k_adam<<<nblk((h->P + 3) / 4), EW, 0, h->stream>>>(h->params, h->grads, h->adam_m, h->adam_v, h->Pb, h->P, lr, beta1, beta2, eps,
                                             weight_decay, c1, c2);
-  h->wblk_stale = true;
   NCK(h, cudaGetLastError());
-  return 0;
+  return params_changed(h);
 }
 
 extern "C" int se2nn_build_inputs(se2nn *h, const void *materials_dev, const float *src_dev, const int *idx_dev,
