@@ -1244,7 +1244,9 @@ extern "C" int se2gpu_tile_configs(const se2gpu_solver *h, int *edge, int *threa
 {
   if (!h) return SE2GPU_ERR_ARG;
   if (is_f64(h)) {
-    if (max_configs > 0 && edge && threads) { edge[0] = se2::f64_tile_edge(h->p); threads[0] = 256; }
+    const se2::F64TileShape t = se2::f64_tile(h->p, f64_params(h), h->nsm);
+    if (max_configs > 0 && edge) edge[0] = t.ex;
+    if (max_configs > 0 && threads) threads[0] = t.threads;
     return 1;
   }
   const int n = se2p::num_configs(h->p, pmode(h));
@@ -1262,7 +1264,8 @@ extern "C" int se2gpu_tile_config_info(const se2gpu_solver *h, int config, int i
   if (!h || !info) return SE2GPU_ERR_ARG;
   if (is_f64(h)) {
     if (config != 0) return SE2GPU_ERR_ARG;
-    info[0] = se2::f64_tile_edge(h->p); info[1] = 256; info[2] = 0; info[3] = 0;
+    const se2::F64TileShape t = se2::f64_tile(h->p, f64_params(h), h->nsm);
+    info[0] = t.ex; info[1] = t.threads; info[2] = 0; info[3] = 0;
     return 0;
   }
   se2p::TileShape ts;

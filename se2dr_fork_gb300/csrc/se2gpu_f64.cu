@@ -15,10 +15,6 @@ namespace se2 {
     default: return {};                                                     \
   }
 
-template <int P>
-static int edge() { return F64Tile<P, 2>::TX; }
-int f64_tile_edge(int p) { SE2_DISPATCH(edge) }
-
 template <class A> struct arg { typedef A type; };   // (keeps A out of the deduction)
 // launch, beginning while the launch before it in the stream drains
 template <class... A>
@@ -77,13 +73,32 @@ static cudaError_t step_t(F64Params &q, int nsm, cudaStream_t st)
 // nodes this is within 1 % (mean) and 11 % (worst) of the best of the three as timed; taking
 // always one size costs up to 3.5x (degree 6, 9 x 9 elements: 11.8, 16.1 or 38.1 us).
 template <int P>
+static int pick(const F64Params &q, int nsm)
+{
+  const long c0 = cost<P, 0>(q, nsm), c1 = cost<P, 1>(q, nsm), c2 = cost<P, 2>(q, nsm);
+  return (c0 < c1 && c0 < c2) ? 0 : (c1 < c2) ? 1 : 2;
+}
+
+template <int P>
 static cudaError_t step(const F64Params &prm, int nsm, cudaStream_t st)
 {
   F64Params q = prm;
-  const long c0 = cost<P, 0>(q, nsm), c1 = cost<P, 1>(q, nsm), c2 = cost<P, 2>(q, nsm);
-  if (c0 < c1 && c0 < c2) return step_t<P, 0>(q, nsm, st);
-  return (c1 < c2) ? step_t<P, 1>(q, nsm, st) : step_t<P, 2>(q, nsm, st);
+  switch (pick<P>(q, nsm)) {
+    case 0: return step_t<P, 0>(q, nsm, st);
+    case 1: return step_t<P, 1>(q, nsm, st);
+    default: return step_t<P, 2>(q, nsm, st);
+  }
 }
+
+template <int P>
+static F64TileShape shape(const F64Params &q, int nsm)
+{
+  static const F64TileShape t[3] = {{F64Tile<P, 0>::TX, F64Tile<P, 0>::TY, F64Tile<P, 0>::NT},
+                                    {F64Tile<P, 1>::TX, F64Tile<P, 1>::TY, F64Tile<P, 1>::NT},
+                                    {F64Tile<P, 2>::TX, F64Tile<P, 2>::TY, F64Tile<P, 2>::NT}};
+  return t[pick<P>(q, nsm)];
+}
+F64TileShape f64_tile(int p, const F64Params &q, int nsm) { SE2_DISPATCH(shape, q, nsm) }
 
 static dim3 node_grid(const F64Params &q) { return dim3((q.nx_g + 255) / 256, std::min(q.ny_g, 65535)); }
 

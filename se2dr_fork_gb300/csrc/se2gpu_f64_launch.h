@@ -31,7 +31,8 @@ struct F64Params {
 
 enum { F64_START = 0, F64_MIDDLE = 1, F64_FORCE = 2 };
 
-int f64_tile_edge(int p);   // elements along x of the wide tiles
+struct F64TileShape { int ex, ey, threads; };   // elements along x and y
+F64TileShape f64_tile(int p, const F64Params &q, int nsm);   // what f64_launch_step runs on the mesh of q
 // one START, MIDDLE or FORCE launch (q.mode); fills in the tile grid
 cudaError_t f64_launch_step(int p, const F64Params &q, int nsm, cudaStream_t st);
 // v and a of the block's last step from the element forces q.ef_in (v in place)
