@@ -46,6 +46,14 @@ DfShape halo_entry()
   return DfShape{P, TE, NT, L::TOTAL, (const void *)persist_step<P, TE, NT, true, 1, M, true, false>, true};
 }
 
+const void *last_fn(int p)
+{
+  static const void *t[8] = {(const void *)df_last<1>, (const void *)df_last<2>, (const void *)df_last<3>,
+                             (const void *)df_last<4>, (const void *)df_last<5>, (const void *)df_last<6>,
+                             (const void *)df_last<7>, (const void *)df_last<8>};
+  return t[p - 1];
+}
+
 template <int P>
 cudaError_t record_t(const Params &prm, cudaStream_t st)
 {
@@ -75,19 +83,21 @@ cudaError_t df_launch(int p, int config, const EfParams &q, bool dependent, cuda
 {
   DfShape s;
   if (!df_shape(p, config, &s) || s.halo) return cudaErrorInvalidValue;
+  EfParams a = q;
+  const int te = s.te * p, nbx = (q.p.nx_g + DF_LX - 1) / DF_LX, nblocks = nbx * ((q.p.ny_g + DF_LY - 1) / DF_LY);
+  const bool last = q.mode == EF_LAST;
+  void *step_args[] = {&a}, *last_args[] = {&a, (void *)&te, (void *)&nbx, (void *)&nblocks};
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(q.p.ntiles + (q.p.record ? 1 : 0));
-  cfg.blockDim = dim3(s.nt);
-  cfg.dynamicSmemBytes = s.smem;
+  cfg.gridDim = dim3((last ? nblocks : q.p.ntiles) + (q.p.record ? 1 : 0));
+  cfg.blockDim = dim3(last ? DF_LX * DF_LY : s.nt);
+  cfg.dynamicSmemBytes = last ? 0 : s.smem;
   cfg.stream = st;
   cudaLaunchAttribute at = {};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = dependent ? 1 : 0;
-  EfParams a = q;
-  void *args[] = {&a};
-  return cudaLaunchKernelExC(&cfg, s.fn, args);
+  return last ? cudaLaunchKernelExC(&cfg, last_fn(p), last_args) : cudaLaunchKernelExC(&cfg, s.fn, step_args);
 }
 
 cudaError_t df_launch_record(int p, const Params &prm, cudaStream_t st)

@@ -11,7 +11,7 @@
 // at 2.5M nodes 304 -> 176 us a step, 20000 nodes 19.4 -> 11.9 (every size: se2gpu_f32df_launch.h).
 //
 // A block of n steps: one EF_START launch (element forces of the state), n - 1 EF_MIDDLE
-// launches, and EF_LAST, which finishes the last step and stores its a.
+// launches, and EF_LAST, which finishes the last step at every node and stores its a (df_last).
 #pragma once
 #include "se2gpu_persist.cuh"
 #include "se2gpu_f32df_launch.h"
@@ -37,6 +37,115 @@ struct DfNode {
   float4 g[4];
 };
 
+template <int P>
+__device__ __forceinline__ void df_load(const EfParams &dp, int X, int Y, DfNode &d)
+{
+  constexpr int N1 = P + 1, NPE = N1 * N1;
+  const Params &prm = dp.p;
+  const size_t n = (size_t)Y * prm.pitch + X;
+  d.u = dp.u_in[n];
+  d.cu = dp.cu_in[n];
+  if (dp.mode == EF_START) return;
+  d.w = dp.w_in[n];
+  d.cw = dp.cw_in[n];
+  d.minv_h = prm.minv[n];
+  d.minv_l = prm.minv[(size_t)prm.ny_g * prm.pitch + n];
+  const NodePos<P> c(prm.mx, prm.my, X, Y);
+  const float4 *ef = static_cast<const float4 *>(dp.ef_in) + ((ptrdiff_t)c.ey * prm.mx + c.ex) * NPE + c.ix + c.iy * N1;
+  if (c.bot && c.lft) d.g[0] = ef[-(ptrdiff_t)(prm.mx + 1) * NPE + P + P * N1];
+  if (c.bot && c.in_x) d.g[1] = ef[-(ptrdiff_t)prm.mx * NPE + P * N1];
+  if (c.lft && c.in_y) d.g[2] = ef[-(ptrdiff_t)NPE + P];
+  if (c.in_x && c.in_y) d.g[3] = ef[0];
+}
+
+// the step of node (X, Y): a, then w and u, in the state's arithmetic; receivers' values where this
+// thread owns the node.  bnd: source and receiver list bounds of the node's tile
+struct DfStep {
+  tf ax, ay, wx, wy, ux, uy;
+};
+template <int P>
+__device__ __forceinline__ DfStep df_finish(const EfParams &dp, const DfNode &d, int X, int Y, const int4 bnd, bool own)
+{
+  constexpr int N1 = P + 1, NPE = N1 * N1;
+  const Params &prm = dp.p;
+  const tf dt{prm.dt, prm.dt_lo}, hdt{prm.half_dt, prm.half_dt_lo};
+  const float *src_lo = prm.src_vals + (size_t)prm.nsrc * 2 * NPE;
+  tf fx{0.f, 0.f}, fy{0.f, 0.f};
+  {
+    const NodePos<P> c(prm.mx, prm.my, X, Y);
+    const bool have[4] = {c.bot && c.lft, c.bot && c.in_x, c.lft && c.in_y, c.in_x && c.in_y};
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (have[k]) {
+        fx = tf_add(fx, tf{d.g[k].x, d.g[k].z});
+        fy = tf_add(fy, tf{d.g[k].y, d.g[k].w});
+      }
+  }
+  SE2P_COLD for (int q = bnd.x; q < bnd.y; q++) {
+    const int4 ent = list_entry(prm.tile_src + q);
+    const int sidx = ent.x, a = X - ent.y, bb = Y - ent.z;
+    if (a >= 0 && a <= P && bb >= 0 && bb <= P) {
+      const tf val = tf_from_double(prm.stf[sidx]);
+      const size_t vi = (size_t)sidx * 2 * NPE + 2 * (a + bb * N1);
+      fx = tf_add(fx, tf_mul(val, tf{prm.src_vals[vi], src_lo[vi]}));
+      fy = tf_add(fy, tf_mul(val, tf{prm.src_vals[vi + 1], src_lo[vi + 1]}));
+    }
+  }
+  const tf minv{d.minv_h, d.minv_l};
+  const tf ax = tf_mul(fx, minv), ay = tf_mul(fy, minv);
+  const tf ux{d.u.x, -d.cu.x}, uy{d.u.y, -d.cu.y}, wx{d.w.x, -d.cw.x}, wy{d.w.y, -d.cw.y};
+  if (own)
+    SE2P_COLD for (int q = bnd.z; q < bnd.w; q++) {
+      const int4 ent = list_entry(prm.tile_rec + q);
+      const int r = ent.x, a = X - ent.y, bb = Y - ent.z;
+      if (a >= 0 && a <= P && bb >= 0 && bb <= P) {
+        float *rb = prm.rbuf_out + ((size_t)r * NPE + a + bb * N1) * 12;
+        const tf vx = tf_add(wx, tf_mul(hdt, ax)), vy = tf_add(wy, tf_mul(hdt, ay));
+        const tf uxn = tf_norm(ux), uyn = tf_norm(uy);
+        rb[0] = uxn.h; rb[1] = uyn.h; rb[2] = vx.h; rb[3] = vy.h; rb[4] = ax.h; rb[5] = ay.h;
+        rb[6] = uxn.l; rb[7] = uyn.l; rb[8] = vx.l; rb[9] = vy.l; rb[10] = ax.l; rb[11] = ay.l;
+      }
+    }
+  const tf wxn = tf_add(wx, tf_mul(dt, ax)), wyn = tf_add(wy, tf_mul(dt, ay));
+  return DfStep{ax, ay, wxn, wyn, tf_add(ux, tf_mul(dt, wxn)), tf_add(uy, tf_mul(dt, wyn))};
+}
+__device__ __forceinline__ void df_store(const EfParams &dp, size_t n, const DfStep &r)
+{
+  dp.p.u_out[n] = make_float2(r.ux.h, r.uy.h);
+  dp.p.w_out[n] = make_float2(r.wx.h, r.wy.h);
+  dp.p.cu_out[n] = make_float2(-r.ux.l, -r.uy.l);
+  dp.p.cw_out[n] = make_float2(-r.wx.l, -r.wy.l);
+}
+
+// EF_LAST: the last step of a block at every node, and its a: one thread per node, each read once,
+// whatever the tiles (tile_nodes: nodes of a tile along an edge, for the lists).  It moves memory
+// only.  Walking the element kernel's tiles (a node of a CTA's region after the other, nodes on tile
+// edges idle) took 81 us at 2.5M nodes, degree 4, which made a block of a single step slower than
+// the step with a halo (160 -> 180 us); this takes 40 (single step 139).
+constexpr int DF_LX = 32, DF_LY = 8;   // nodes of a CTA along x and y
+template <int P>
+__global__ void __launch_bounds__(DF_LX * DF_LY) df_last(const EfParams dp, int tile_nodes, int nbx, int nblocks)
+{
+  const Params &prm = dp.p;
+  cudaGridDependencySynchronize();
+  if ((int)blockIdx.x >= nblocks) {   // (one more CTA: the receivers of the step before)
+    sample_rows<P, true>(prm, prm.rbuf_in, prm.trace_row);
+    return;
+  }
+  const int by = blockIdx.x / nbx, bx = blockIdx.x - by * nbx;
+  const int X = bx * DF_LX + threadIdx.x % DF_LX, Y = by * DF_LY + threadIdx.x / DF_LX;
+  if (X >= prm.nx_g || Y >= prm.ny_g) return;
+  DfNode d;
+  df_load<P>(dp, X, Y, d);
+  const int nty = prm.ntiles / prm.ntx;
+  const int tx = min(X / tile_nodes, prm.ntx - 1), ty = min(Y / tile_nodes, nty - 1);
+  const DfStep r = df_finish<P>(dp, d, X, Y, prm.tile_bounds[ty * prm.ntx + tx], true);
+  const size_t n = (size_t)Y * prm.pitch + X;
+  df_store(dp, n, r);
+  prm.a_out[n] = make_float2(r.ax.h, r.ay.h);
+  prm.a_out[(size_t)prm.ny_g * prm.pitch + n] = make_float2(r.ax.l, r.ay.l);   // low parts after the high parts
+}
+
 template <int P, int TE, int NT>
 __global__ void __launch_bounds__(NT, df_min_blocks(P, TE, NT)) df_step(const EfParams dp)
 {
@@ -54,33 +163,15 @@ __global__ void __launch_bounds__(NT, df_min_blocks(P, TE, NT)) df_step(const Ef
   }
   const int ty = blockIdx.x / prm.ntx, tx = blockIdx.x - ty * prm.ntx;
   const int ex0 = tx * TE, ey0 = ty * TE, nex = min(TE, prm.mx - ex0), ney = min(TE, prm.my - ey0);
-  const int X0 = ex0 * P, Y0 = ey0 * P, pitch = prm.pitch;
+  const int X0 = ex0 * P, Y0 = ey0 * P;
 
   // ---- the tile's nodes: finish the previous step (a node line shared with the next tile belongs to
   // that one, which writes it)
   const int own_w = nex * P + (ex0 + nex == prm.mx ? 1 : 0), own_h = ney * P + (ey0 + ney == prm.my ? 1 : 0);
   const int4 bnd = prm.tile_bounds[blockIdx.x];
-  const int s0 = bnd.x, s1 = bnd.y, r0 = bnd.z, r1 = bnd.w;
-  const tf dt{prm.dt, prm.dt_lo}, hdt{prm.half_dt, prm.half_dt_lo};
-  const float *src_lo = prm.src_vals + (size_t)prm.nsrc * 2 * NPE, *minv_lo = prm.minv + (size_t)prm.ny_g * pitch;
   auto load = [&](int i, DfNode &d) {
     const int ry = i / RW, rx = i - ry * RW;
-    if (i >= RW * RW || rx > nex * P || ry > ney * P) return;
-    const int X = X0 + rx, Y = Y0 + ry;
-    const size_t n = (size_t)Y * pitch + X;
-    d.u = dp.u_in[n];
-    d.cu = dp.cu_in[n];
-    if (dp.mode == EF_START) return;
-    d.w = dp.w_in[n];
-    d.cw = dp.cw_in[n];
-    d.minv_h = prm.minv[n];
-    d.minv_l = minv_lo[n];
-    const NodePos<P> c(prm.mx, prm.my, X, Y);
-    const float4 *ef = static_cast<const float4 *>(dp.ef_in) + ((ptrdiff_t)c.ey * prm.mx + c.ex) * NPE + c.ix + c.iy * N1;
-    if (c.bot && c.lft) d.g[0] = ef[-(ptrdiff_t)(prm.mx + 1) * NPE + P + P * N1];
-    if (c.bot && c.in_x) d.g[1] = ef[-(ptrdiff_t)prm.mx * NPE + P * N1];
-    if (c.lft && c.in_y) d.g[2] = ef[-(ptrdiff_t)NPE + P];
-    if (c.in_x && c.in_y) d.g[3] = ef[0];
+    if (i < RW * RW && rx <= nex * P && ry <= ney * P) df_load<P>(dp, X0 + rx, Y0 + ry, d);
   };
   DfNode next;
   load(threadIdx.x, next);
@@ -89,66 +180,16 @@ __global__ void __launch_bounds__(NT, df_min_blocks(P, TE, NT)) df_step(const Ef
     const DfNode d = next;
     load(i + NT, next);
     const int ry = i / RW, rx = i - ry * RW;
-    const bool own = rx < own_w && ry < own_h;
-    if (rx > nex * P || ry > ney * P || (dp.mode == EF_LAST && !own)) continue;
-    const int X = X0 + rx, Y = Y0 + ry;
-    const size_t n = (size_t)Y * pitch + X;
-    const float2 u = d.u, cu = d.cu, w = d.w, cw = d.cw;
+    if (rx > nex * P || ry > ney * P) continue;
     if (dp.mode == EF_START) {
-      sU[i] = make_float4(u.x, u.y, cu.x, cu.y);
+      sU[i] = make_float4(d.u.x, d.u.y, d.cu.x, d.cu.y);
       continue;
     }
-    const tf minv{d.minv_h, d.minv_l};
-    tf fx{0.f, 0.f}, fy{0.f, 0.f};
-    {
-      const NodePos<P> c(prm.mx, prm.my, X, Y);
-      const bool have[4] = {c.bot && c.lft, c.bot && c.in_x, c.lft && c.in_y, c.in_x && c.in_y};
-#pragma unroll
-      for (int k = 0; k < 4; k++)
-        if (have[k]) {
-          fx = tf_add(fx, tf{d.g[k].x, d.g[k].z});
-          fy = tf_add(fy, tf{d.g[k].y, d.g[k].w});
-        }
-    }
-    SE2P_COLD for (int q = s0; q < s1; q++) {
-      const int4 ent = list_entry(prm.tile_src + q);
-      const int sidx = ent.x, a = X - ent.y, bb = Y - ent.z;
-      if (a >= 0 && a <= P && bb >= 0 && bb <= P) {
-        const tf val = tf_from_double(prm.stf[sidx]);
-        const size_t vi = (size_t)sidx * 2 * NPE + 2 * (a + bb * N1);
-        fx = tf_add(fx, tf_mul(val, tf{prm.src_vals[vi], src_lo[vi]}));
-        fy = tf_add(fy, tf_mul(val, tf{prm.src_vals[vi + 1], src_lo[vi + 1]}));
-      }
-    }
-    const tf ax = tf_mul(fx, minv), ay = tf_mul(fy, minv);
-    const tf ux{u.x, -cu.x}, uy{u.y, -cu.y}, wx{w.x, -cw.x}, wy{w.y, -cw.y};
-    if (own)
-      SE2P_COLD for (int q = r0; q < r1; q++) {
-        const int4 ent = list_entry(prm.tile_rec + q);
-        const int r = ent.x, a = X - ent.y, bb = Y - ent.z;
-        if (a >= 0 && a <= P && bb >= 0 && bb <= P) {
-          float *rb = prm.rbuf_out + ((size_t)r * NPE + a + bb * N1) * 12;
-          const tf vx = tf_add(wx, tf_mul(hdt, ax)), vy = tf_add(wy, tf_mul(hdt, ay));
-          const tf uxn = tf_norm(ux), uyn = tf_norm(uy);
-          rb[0] = uxn.h; rb[1] = uyn.h; rb[2] = vx.h; rb[3] = vy.h; rb[4] = ax.h; rb[5] = ay.h;
-          rb[6] = uxn.l; rb[7] = uyn.l; rb[8] = vx.l; rb[9] = vy.l; rb[10] = ax.l; rb[11] = ay.l;
-        }
-      }
-    const tf wxn = tf_add(wx, tf_mul(dt, ax)), wyn = tf_add(wy, tf_mul(dt, ay));
-    const tf uxn = tf_add(ux, tf_mul(dt, wxn)), uyn = tf_add(uy, tf_mul(dt, wyn));
-    sU[i] = make_float4(uxn.h, uyn.h, -uxn.l, -uyn.l);
-    if (own) {
-      prm.u_out[n] = make_float2(uxn.h, uyn.h);
-      prm.w_out[n] = make_float2(wxn.h, wyn.h);
-      prm.cu_out[n] = make_float2(-uxn.l, -uyn.l);
-      prm.cw_out[n] = make_float2(-wxn.l, -wyn.l);
-      if (dp.mode == EF_LAST) {
-        prm.a_out[n] = make_float2(ax.h, ay.h);
-        prm.a_out[(size_t)prm.ny_g * pitch + n] = make_float2(ax.l, ay.l);   // low parts after the high parts
-      }
-    }
+    const bool own = rx < own_w && ry < own_h;
+    const DfStep r = df_finish<P>(dp, d, X0 + rx, Y0 + ry, bnd, own);
+    sU[i] = make_float4(r.ux.h, r.uy.h, -r.ux.l, -r.uy.l);
+    if (own) df_store(dp, (size_t)(Y0 + ry) * prm.pitch + X0 + rx, r);
   }
-  if (dp.mode == EF_LAST) return;
 
   // ---- the element forces: one thread per (element, line j)
   const int el = threadIdx.x / N1, j = threadIdx.x - el * N1, ecy = el / TE, ecx = el - ecy * TE;
