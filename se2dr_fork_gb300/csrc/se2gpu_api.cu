@@ -363,14 +363,12 @@ extern "C" void se2gpu_destroy(se2gpu_solver *h)
     if (ev) { cudaEventSynchronize(ev); cudaEventDestroy(ev); ev = nullptr; }
   if (h->stream) cudaStreamSynchronize(h->stream);
   for (int b = 0; b < 2; b++) {
-    for (int f = 0; f < 2; f++) dfree(h, h->f64[b][f]);
-    dfree(h, h->ef[b]);
     dfree(h, h->pu[b]); dfree(h, h->pw[b]); dfree(h, h->pcu[b]); dfree(h, h->pcw[b]); dfree(h, h->rbuf[b]);
   }
-  void *ptrs[] = {h->a64, h->rmass, h->Dx, h->Dy, h->f64_consts, h->src_xy, h->pa, h->pminv, h->mass_bad, h->err_dev, h->mass, h->lam, h->mu, h->J00, h->J11, h->iJ00, h->iJ11, h->D, h->wq,
+  void *ptrs[] = {h->f64[0][0], h->ef[0], h->Dx, h->pa, h->pminv, h->mass_bad, h->err_dev, h->mass, h->lam, h->mu, h->J00, h->J11, h->iJ00, h->iJ11, h->D, h->wq,
                   h->src_vals, h->Dd, h->iJ00d, h->iJ11d, h->stf_dev, h->traces, h->norm_part,
-                  h->rec_node, h->rec_elem, h->rec_gll, h->scratch_u, h->scratch_f, h->tile_src,
-                  h->tile_rec, h->cellc, h->tile_bounds};
+                  h->rec_node, h->rec_elem, h->rec_gll, h->scratch_u, h->scratch_f, h->cellc,
+                  h->tiles.bounds};
   for (void *p : ptrs) dfree(h, p);
   if (h->stream) cudaStreamSynchronize(h->stream);   // the frees are done before the stream goes
   delete h->src_elem_h;
@@ -439,20 +437,20 @@ static int make_const_maps(se2gpu_solver *h, const se2p::TileShape &ts, CUtensor
   return 0;
 }
 
-// what a tile configuration needs besides the state, complete before the handle takes it over
-struct TileSetup {
-  CUtensorMap maps[2][6];
-  int4 *src = nullptr, *rec = nullptr, *bounds = nullptr;
-  void *ef[2] = {nullptr, nullptr};   // element forces, where the handle has none yet
-  int ntx = 0, nty = 0;
-};
+static void free_tiles(se2gpu_solver *h, se2gpu_tiles &t)
+{
+  dfree(h, t.bounds);
+  t.src = t.rec = t.bounds = nullptr;
+}
 
-// tensor maps, element-force buffers and per-tile source/receiver lists of a configuration, into t;
+// a configuration's kernel attributes, tensor maps, per-tile source/receiver lists and grid, into t;
 // nothing of the handle changes
-static int build_tiles(se2gpu_solver *h, const se2p::TileShape &ts, TileSetup &t)
+static int build_tiles(se2gpu_solver *h, int config, const se2p::TileShape &ts, se2gpu_tiles &t)
 {
   const bool kahan = is_kahan(h);
-  memset(t.maps, 0, sizeof(t.maps));
+  memset(&t, 0, sizeof(t));
+  const cudaError_t e = se2p::prepare(h->p, config, pmode(h));
+  if (e != cudaSuccess) return fail(h, SE2GPU_ERR_CUDA, "persistent kernel set-up: %s", cudaGetErrorString(e));
   for (int b = 0; b < 2 && ts.halo; b++) {
     void *bases[4] = {h->pu[b], kahan ? (void *)h->pcu[b] : (void *)h->pu[b], h->pw[b], kahan ? (void *)h->pcw[b] : (void *)h->pw[b]};
     for (int m = 0; m < 4; m++) {
@@ -463,52 +461,56 @@ static int build_tiles(se2gpu_solver *h, const se2p::TileShape &ts, TileSetup &t
   }
   int rc;
   if (h->pminv && (rc = make_const_maps(h, ts, t.maps))) return rc;   // (in se2gpu_create they follow once 1/M is allocated)
-  for (int b = 0; b < 2 && !ts.halo; b++)
-    if (!h->ef[b] && (rc = dalloc(h, &t.ef[b], (size_t)h->mx * h->my * h->npe * (is_df(h) ? 16 : 8)))) return rc;
   const int te = ts.tex, P = h->p;
   const int ntx = (h->mx + te - 1) / te, nty = (h->my + te - 1) / te, ntiles = ntx * nty;
   // tile lists: a source or receiver element appears in every tile whose owned nodes it touches, or
   // whose nodes it touches where a tile finishes the node lines that it shares with the next ones
   const int far = ts.halo ? 0 : 1;
   auto build = [&](const std::vector<int> &elems, std::vector<int> &off, std::vector<int> &ent) {
-    std::vector<std::vector<int>> per(ntiles);
-    for (int q = 0; q < (int)elems.size(); q++) {
-      const int ex = elems[q] % h->mx, ey = elems[q] / h->mx;
-      for (int ty = std::max(0, (ey - 1) / te); ty <= std::min(nty - 1, (ey + 1) / te); ty++)
-        for (int tx = std::max(0, (ex - 1) / te); tx <= std::min(ntx - 1, (ex + 1) / te); tx++) {
-          const int X0 = tx * te * P, X1 = std::min((tx + 1) * te, h->mx) * P + (((tx + 1) * te >= h->mx) ? 1 : 0);
-          const int Y0 = ty * te * P, Y1 = std::min((ty + 1) * te, h->my) * P + (((ty + 1) * te >= h->my) ? 1 : 0);
-          if (ex * P <= X1 - 1 + far && ex * P + P >= X0 && ey * P <= Y1 - 1 + far && ey * P + P >= Y0) per[ty * ntx + tx].push_back(q);
-        }
-    }
-    off.assign(ntiles + 1, 0);
-    for (int t = 0; t < ntiles; t++) off[t + 1] = off[t] + (int)per[t].size();
-    ent.clear();
-    for (int t = 0; t < ntiles; t++)
-      for (int q : per[t]) {
-        const int e[4] = {q, elems[q] % h->mx * P, elems[q] / h->mx * P, 0};
-        ent.insert(ent.end(), e, e + 4);
+    auto each = [&](auto f) {   // f(tile, element index), elements ascending
+      for (int q = 0; q < (int)elems.size(); q++) {
+        const int ex = elems[q] % h->mx, ey = elems[q] / h->mx;
+        for (int ty = std::max(0, (ey - 1) / te); ty <= std::min(nty - 1, (ey + 1) / te); ty++)
+          for (int tx = std::max(0, (ex - 1) / te); tx <= std::min(ntx - 1, (ex + 1) / te); tx++) {
+            const int X0 = tx * te * P, X1 = std::min((tx + 1) * te, h->mx) * P + (((tx + 1) * te >= h->mx) ? 1 : 0);
+            const int Y0 = ty * te * P, Y1 = std::min((ty + 1) * te, h->my) * P + (((ty + 1) * te >= h->my) ? 1 : 0);
+            if (ex * P <= X1 - 1 + far && ex * P + P >= X0 && ey * P <= Y1 - 1 + far && ey * P + P >= Y0) f(ty * ntx + tx, q);
+          }
       }
+    };
+    off.assign(ntiles + 1, 0);
+    each([&](int t, int) { off[t + 1]++; });
+    for (int t = 0; t < ntiles; t++) off[t + 1] += off[t];
+    ent.assign(4 * (size_t)off[ntiles], 0);
+    std::vector<int> at(off.begin(), off.end() - 1);
+    each([&](int t, int q) {
+      int *e = &ent[4 * (size_t)at[t]++];
+      e[0] = q; e[1] = elems[q] % h->mx * P; e[2] = elems[q] / h->mx * P;
+    });
   };
   std::vector<int> so, si, ro, ri;
   build(*h->src_elem_h, so, si);
   build(*h->rec_elem_h, ro, ri);
-  std::vector<int> tb(4 * (size_t)ntiles);
+  std::vector<int> tb(4 * (size_t)ntiles);   // (one table, one upload: an allocation costs about 0.1 ms)
   for (int t = 0; t < ntiles; t++) {
     tb[4 * (size_t)t] = so[t]; tb[4 * (size_t)t + 1] = so[t + 1];
     tb[4 * (size_t)t + 2] = ro[t]; tb[4 * (size_t)t + 3] = ro[t + 1];
   }
+  tb.insert(tb.end(), si.begin(), si.end());
+  tb.insert(tb.end(), ri.begin(), ri.end());
   if ((rc = upload_i(h, (int **)&t.bounds, tb.data(), tb.size()))) return rc;
-  if ((rc = upload_i(h, (int **)&t.src, si.data(), si.size()))) return rc;
-  if ((rc = upload_i(h, (int **)&t.rec, ri.data(), ri.size()))) return rc;
+  t.src = t.bounds + ntiles;
+  t.rec = t.src + si.size() / 4;
+  t.config = config;
+  t.halo = ts.halo;
   t.ntx = ntx;
   t.nty = nty;
+  t.grid = std::min(ntiles + 1, std::max(1, se2p::occupancy(P, config, pmode(h))) * h->nsm);
   return 0;
 }
 
-// select one of the persistent kernel's tile configurations: kernel attributes,
-// tensor-map boxes, per-tile source/receiver lists and the persistent grid.  The handle changes
-// only after everything that can fail has succeeded: on an error it runs on as it was.
+// Select one of the step kernels' tile configurations.  The handle changes only after everything
+// that can fail has succeeded: on an error it runs on as it was.
 // (in_create: the handle has run no step yet, so nothing in flight reads the tile lists
 // and the host work here overlaps the set-up kernels still reading the caller's arrays)
 static int setup_f32_config(se2gpu_solver *h, int config, bool in_create = false)
@@ -517,31 +519,26 @@ static int setup_f32_config(se2gpu_solver *h, int config, bool in_create = false
   se2p::TileShape ts;
   if (se2p::config_shape(h->p, config, mode, &ts)) return fail(h, SE2GPU_ERR_ARG, "no tile configuration %d for degree %d", config, h->p);
   if (!in_create) CK(h, cudaStreamSynchronize(h->stream));
-  {
-    cudaError_t e = se2p::prepare(h->p, config, mode);
-    if (e != cudaSuccess) return fail(h, SE2GPU_ERR_CUDA, "persistent kernel set-up: %s", cudaGetErrorString(e));
-  }
-  TileSetup t;
-  const int rc = build_tiles(h, ts, t);
+  se2gpu_tiles t;
+  const size_t ef_bytes = ((size_t)h->mx * h->my * h->npe * (is_df(h) ? 16 : 8) + 15) / 16 * 16;
+  void *ef = nullptr;   // element forces, where the handle has none yet
+  int rc = build_tiles(h, config, ts, t);
+  if (!rc && !ts.halo && !h->ef[0]) rc = dalloc(h, &ef, 2 * ef_bytes);
   if (rc) {
-    for (void *p : {(void *)t.src, (void *)t.rec, (void *)t.bounds, t.ef[0], t.ef[1]}) dfree(h, p);
+    free_tiles(h, t);
+    dfree(h, ef);
     return rc;
   }
-  memcpy(h->maps, t.maps, sizeof(h->maps));
-  dfree(h, h->tile_src); dfree(h, h->tile_rec); dfree(h, h->tile_bounds);
-  h->tile_src = t.src; h->tile_rec = t.rec; h->tile_bounds = t.bounds;
-  for (int b = 0; b < 2; b++) {
-    if (t.ef[b]) h->ef[b] = static_cast<double2 *>(t.ef[b]);
-    if (ts.halo) {   // (16 (p+1)^2 bytes per element, two-float 32: not kept by a configuration that has no use for them)
-      dfree(h, h->ef[b]);
-      h->ef[b] = nullptr;
-    }
+  free_tiles(h, h->tiles);
+  h->tiles = t;
+  if (ef) {
+    h->ef[0] = static_cast<double2 *>(ef);
+    h->ef[1] = h->ef[0] + ef_bytes / 16;
   }
-  h->pconfig = config;
-  h->no_halo = !ts.halo;
-  h->pntx = t.ntx;
-  h->pnty = t.nty;
-  h->pgrid = std::min(t.ntx * t.nty + 1, std::max(1, se2p::occupancy(h->p, config, mode)) * h->nsm);
+  if (ts.halo) {   // (16 (p+1)^2 bytes per element, two-float 32: not kept by a configuration that has no use for them)
+    dfree(h, h->ef[0]);
+    h->ef[0] = h->ef[1] = nullptr;
+  }
   return 0;
 }
 
@@ -645,32 +642,36 @@ int se2gpu_internal_create(const se2gpu_problem *P, int precision, int trace_cap
 
   if (precision == SE2GPU_FP64) {
     const size_t vbytes = (size_t)nnodes * 2 * 8;
-    for (int b = 0; b < 2; b++)
-      for (int f = 0; f < 2; f++) TRY(dzero(h, (void **)&h->f64[b][f], vbytes));
-    TRY(dzero(h, (void **)&h->a64, vbytes));
-    // element forces of a step, written before they are read
-    for (int b = 0; b < 2; b++) TRY(dalloc(h, (void **)&h->ef[b], (size_t)ne * npe * 16));
+    TRY(dzero(h, (void **)&h->f64[0][0], 5 * vbytes));   // (one allocation of all five)
+    for (int k = 1; k < 4; k++) h->f64[k / 2][k % 2] = h->f64[0][0] + (size_t)k * nnodes;
+    h->a64 = h->f64[0][0] + 4 * (size_t)nnodes;
+    // element forces of a step, written before they are read, and 1/M
+    const size_t nef = (size_t)ne * npe;
+    TRY(dalloc(h, (void **)&h->ef[0], nef * 32 + (size_t)nnodes * 8));
+    h->ef[1] = h->ef[0] + nef;
+    h->rmass = reinterpret_cast<double *>(h->ef[1] + nef);
     TRY(upload(h, &h->mass, P->mass, (size_t)nnodes));   // the reference divides by M
-    TRY(dalloc(h, (void **)&h->rmass, (size_t)nnodes * 8));
     if (se2::f64_launch_reciprocal((const double *)h->mass, h->rmass, (size_t)nnodes, h->nsm, h->stream) != cudaSuccess) {
       cudaGetLastError();
       fail(h, SE2GPU_ERR_CUDA, "1/M");
       TRY(SE2GPU_ERR_CUDA);
     }
-    // the reference's scaled derivatives dN/dx = (1/J00) dN/dxi per element column, dN/dy per row
-    std::vector<double> dx((size_t)P->mx * npe), dy((size_t)P->my * npe);
-    for (size_t i = 0; i < dx.size(); i++) dx[i] = P->iJ00[i / npe] * P->D[i % npe];
-    for (size_t i = 0; i < dy.size(); i++) dy[i] = P->iJ11[i / npe] * P->D[i % npe];
-    TRY(upload_d(h, &h->Dx, dx.data(), dx.size()));
-    TRY(upload_d(h, &h->Dy, dy.data(), dy.size()));
-    const double consts[2] = {1.0, -0.0};
-    TRY(upload_d(h, &h->f64_consts, consts, 2));
-    std::vector<int> sxy;
+    // the reference's scaled derivatives dN/dx = (1/J00) dN/dxi per element column, dN/dy per row; the
+    // kernels' constants; the first node of each source's element
+    const size_t ndx = (size_t)P->mx * npe, ndy = (size_t)P->my * npe;
+    std::vector<double> tab(ndx + ndy + 2 + P->nsrc);
+    for (size_t i = 0; i < ndx; i++) tab[i] = P->iJ00[i / npe] * P->D[i % npe];
+    for (size_t i = 0; i < ndy; i++) tab[ndx + i] = P->iJ11[i / npe] * P->D[i % npe];
+    tab[ndx + ndy] = 1.0;
+    tab[ndx + ndy + 1] = -0.0;
     for (int s = 0; s < P->nsrc; s++) {
-      sxy.push_back(P->src_elem[s] % P->mx * P->p);
-      sxy.push_back(P->src_elem[s] / P->mx * P->p);
+      const int xy[2] = {P->src_elem[s] % P->mx * P->p, P->src_elem[s] / P->mx * P->p};
+      memcpy(&tab[ndx + ndy + 2 + s], xy, 8);
     }
-    TRY(upload_i(h, (int **)&h->src_xy, sxy.data(), sxy.size()));
+    TRY(upload_d(h, &h->Dx, tab.data(), tab.size()));
+    h->Dy = h->Dx + ndx;
+    h->f64_consts = h->Dy + ndy;
+    h->src_xy = reinterpret_cast<int2 *>(h->f64_consts + 2);
   } else {
     const bool kahan = is_kahan(h), df = is_df(h);
     h->pitch = (int)((nx_g + 1 + 15) / 16 * 16);   // >= 1 padding node: paired reads stay in the row
@@ -778,8 +779,8 @@ int se2gpu_internal_create(const se2gpu_problem *P, int precision, int trace_cap
       if (cudaMemcpyAsync(h->pminv, minv.get(), nm * 4, cudaMemcpyHostToDevice, h->stream) != cudaSuccess) { fail(h, SE2GPU_ERR_CUDA, "upload 1/M"); TRY(SE2GPU_ERR_CUDA); }
     }
     se2p::TileShape ts;
-    if (se2p::config_shape(h->p, h->pconfig, pmode(h), &ts)) { fail(h, SE2GPU_ERR_ARG, "tile configuration"); TRY(SE2GPU_ERR_ARG); }
-    TRY(make_const_maps(h, ts, h->maps));
+    if (se2p::config_shape(h->p, h->tiles.config, pmode(h), &ts)) { fail(h, SE2GPU_ERR_ARG, "tile configuration"); TRY(SE2GPU_ERR_ARG); }
+    TRY(make_const_maps(h, ts, h->tiles.maps));
   }
   {
     // one wait for everything queued above (kernels that read the caller's arrays included),
@@ -862,12 +863,12 @@ static se2::F64Params f64_params(const se2gpu_solver *h)
 }
 
 // ---------------------------------------------------------------- FP32 (persistent leapfrog)
-static se2p::Params f32_params(se2gpu_solver *h)
+static se2p::Params f32_params(const se2gpu_solver *h, const se2gpu_tiles &t)
 {
   se2p::Params prm;
   memset(&prm, 0, sizeof(prm));
   prm.mx = h->mx; prm.my = h->my; prm.nx_g = h->nx_g; prm.ny_g = h->ny_g; prm.pitch = h->pitch;
-  prm.ntx = h->pntx; prm.nty = h->pnty; prm.ntiles = h->pntx * h->pnty;
+  prm.ntx = t.ntx; prm.nty = t.nty; prm.ntiles = t.ntx * t.nty;
   prm.minv = h->pminv;
   prm.lam = (const float *)h->lam; prm.mu = (const float *)h->mu;
   prm.J00 = (const float *)h->J00; prm.J11 = (const float *)h->J11;
@@ -878,12 +879,12 @@ static se2p::Params f32_params(se2gpu_solver *h)
   prm.nrec = h->nrec; prm.rec_elem = h->rec_elem; prm.rec_gll = h->rec_gll;
   prm.Dd = h->Dd; prm.iJ00d = h->iJ00d; prm.iJ11d = h->iJ11d;
   prm.err = h->err_dev;
-  prm.tile_src = h->tile_src; prm.tile_rec = h->tile_rec;
-  prm.cellc = h->cellc; prm.tile_bounds = h->tile_bounds;
+  prm.tile_src = t.src; prm.tile_rec = t.rec;
+  prm.cellc = h->cellc; prm.tile_bounds = t.bounds;
   return prm;
 }
 
-se2p::Params se2gpu_internal_f32_params(se2gpu_solver *h) { return f32_params(h); }
+se2p::Params se2gpu_internal_f32_params(se2gpu_solver *h) { return f32_params(h, h->tiles); }
 
 // record the receivers of the last step if its row is still pending
 static int flush_record(se2gpu_solver *h)
@@ -900,7 +901,7 @@ static int flush_record(se2gpu_solver *h)
     q.trace_row = row;
     e = se2::f64_launch_record(h->p, q, h->stream);
   } else {
-    auto prm = f32_params(h);
+    auto prm = f32_params(h, h->tiles);
     prm.rbuf_in = h->rbuf[h->rlast];
     prm.record = 1;
     prm.trace_row = row;
@@ -946,7 +947,7 @@ static int advance_f64(se2gpu_solver *h, int nsteps)
 static int advance_no_halo(se2gpu_solver *h, int nsteps)
 {
   se2p::EfParams q;
-  q.p = f32_params(h);
+  q.p = f32_params(h, h->tiles);
   for (int k = 0; k <= nsteps; k++) {
     const int in = h->cur, outb = 1 - h->cur;
     q.mode = (k == 0) ? se2p::EF_START : (k == nsteps) ? se2p::EF_LAST : se2p::EF_MIDDLE;
@@ -960,7 +961,7 @@ static int advance_no_halo(se2gpu_solver *h, int nsteps)
     q.p.record = h->pending_record ? 1 : 0;
     q.p.trace_row = h->traces + (size_t)h->rows_written * 7 * h->nrec;
     h->launches++;
-    cudaError_t e = se2p::launch_no_halo(h->p, h->pconfig, pmode(h), q, k > 0, h->stream);
+    cudaError_t e = se2p::launch_no_halo(h->p, h->tiles.config, pmode(h), q, k > 0, h->stream);
     if (e != cudaSuccess) return fail(h, SE2GPU_ERR_CUDA, "step kernel: %s", cudaGetErrorString(e));
     if (h->pending_record) { h->rows_written++; h->pending_record = false; }
     if (k == 0) continue;   // (no step is finished yet)
@@ -973,7 +974,8 @@ static int advance_no_halo(se2gpu_solver *h, int nsteps)
 
 static int advance_f32(se2gpu_solver *h, int nsteps)
 {
-  auto prm = f32_params(h);
+  const se2gpu_tiles &t = h->tiles;
+  auto prm = f32_params(h, t);
   const int mode = pmode(h);
   for (int k = 0; k < nsteps; k++) {
     const int in = h->cur, outb = 1 - h->cur;
@@ -985,7 +987,7 @@ static int advance_f32(se2gpu_solver *h, int nsteps)
     prm.record = h->pending_record ? 1 : 0;
     prm.trace_row = h->traces + (size_t)h->rows_written * 7 * h->nrec;
     h->launches++;
-    cudaError_t e = se2p::launch_step(h->p, h->pconfig, mode, h->maps[in], prm, h->pgrid, k > 0, h->stream);
+    cudaError_t e = se2p::launch_step(h->p, t.config, mode, t.maps[in], prm, t.grid, k > 0, h->stream);
     if (e != cudaSuccess) return fail(h, SE2GPU_ERR_CUDA, "step kernel: %s", cudaGetErrorString(e));
     if (h->pending_record) { h->rows_written++; h->pending_record = false; }
     h->cur = outb;
@@ -1017,7 +1019,8 @@ extern "C" int se2gpu_advance(se2gpu_solver *h, int nsteps, const double *stf)
     // the previous block may still read stf_dev: order the copy on the stream
     CK(h, cudaMemcpyAsync(h->stf_dev, stf, (size_t)nsteps * h->nsrc * 8, cudaMemcpyHostToDevice, h->stream));
   }
-  return is_f64(h) ? advance_f64(h, nsteps) : h->no_halo ? advance_no_halo(h, nsteps) : advance_f32(h, nsteps);
+  if (is_f64(h)) return advance_f64(h, nsteps);
+  return h->tiles.halo ? advance_f32(h, nsteps) : advance_no_halo(h, nsteps);
 }
 
 extern "C" int se2gpu_traces(se2gpu_solver *h, double *out, int max_rows)
@@ -1294,7 +1297,7 @@ extern "C" int se2gpu_set_tile_config(se2gpu_solver *h, int config)
   if (is_f64(h)) return (config == 0) ? 0 : fail(h, SE2GPU_ERR_ARG, "FP64 mode has a single tile configuration");
   if (config < 0 || config >= se2p::num_configs(h->p, pmode(h))) return fail(h, SE2GPU_ERR_ARG, "tile configuration %d out of range", config);
   CK(h, cudaSetDevice(h->device));
-  if (tiles_of(h, config) != h->pconfig) {   // (else tables, maps and grid are current)
+  if (tiles_of(h, config) != h->tiles.config) {   // (else tables, maps and grid are current)
     const int rc = setup_f32_config(h, tiles_of(h, config));
     if (rc) return rc;
   }

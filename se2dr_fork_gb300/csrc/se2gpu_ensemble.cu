@@ -190,11 +190,11 @@ static int build_group(se2gpu_ensemble *e, Group &g)
     }
   for (int c = 0; c < 2; c++) {
     for (int i = 0; i < ns; i++)
-      for (int m = 0; m < 4; m++) maps[4 * (size_t)i + m] = e->sol[g.shots[i]]->maps[c][m];
+      for (int m = 0; m < 4; m++) maps[4 * (size_t)i + m] = e->sol[g.shots[i]]->tiles.maps[c][m];
     int rc = dput(e, &g.maps[c], maps.data(), maps.size());
     if (rc) return rc;
   }
-  g.config = e->sol[g.shots[0]]->pconfig;
+  g.config = e->sol[g.shots[0]]->tiles.config;
   const int occ = std::max(1, se2p::occupancy(g.p, g.config, e->kahan, true));
   for (int f = 0; f < ns; f += SE2P_BATCH_SHOTS) {
     Chunk ch;
@@ -203,8 +203,8 @@ static int build_group(se2gpu_ensemble *e, Group &g)
     ch.item_off = (int)items.size();
     for (int i = f; i < f + ch.nshots; i++) {
       se2gpu_solver *h = e->sol[g.shots[i]];
-      if (h->pntx >= 32768 || h->pnty >= 32768) return efail(e, SE2GPU_ERR_ARG, "shot %d: more than 32767 tiles along an axis", g.shots[i]);
-      for (int t = 0; t < h->pntx * h->pnty; t++) items.push_back(make_int2(i - f, ((t / h->pntx) << 16) | (t % h->pntx)));
+      if (h->tiles.ntx >= 32768 || h->tiles.nty >= 32768) return efail(e, SE2GPU_ERR_ARG, "shot %d: more than 32767 tiles along an axis", g.shots[i]);
+      for (int t = 0; t < h->tiles.ntx * h->tiles.nty; t++) items.push_back(make_int2(i - f, ((t / h->tiles.ntx) << 16) | (t % h->tiles.ntx)));
     }
     ch.nitems = (int)items.size() - ch.item_off;
     ch.grid = std::max(1, std::min(ch.nitems, occ * e->nsm));
@@ -306,7 +306,7 @@ extern "C" int se2gpu_ensemble_create(const se2gpu_problem *shots, int nshots, i
   }
   for (se2gpu_solver *h : e->sol) h->stream = e->stream;
   for (Group &g : e->groups) {
-    if (se2p::prepare(g.p, e->sol[g.shots[0]]->pconfig, e->kahan) != cudaSuccess) {
+    if (se2p::prepare(g.p, e->sol[g.shots[0]]->tiles.config, e->kahan) != cudaSuccess) {
       efail(e, SE2GPU_ERR_CUDA, "batched kernel set-up for degree %d", g.p);
       TRY(SE2GPU_ERR_CUDA);
     }

@@ -10,6 +10,15 @@
 #include "se2gpu.h"
 #include "se2gpu_persist_params.h"
 
+// a tile configuration of the FP32 modes, set up on a handle
+struct se2gpu_tiles {
+  CUtensorMap maps[2][6];        // per input buffer set: region u, cu, owned w, cw; cell constants, 1/M
+  int4 *bounds;                  // per tile: source and receiver list bounds (the allocation, with src and rec)
+  int4 *src, *rec;               // per-tile list entries
+  int config, ntx, nty, grid;
+  bool halo;                     // else its step keeps element forces (se2gpu_f32ef.cuh, se2gpu_f32df.cuh)
+};
+
 struct se2gpu_solver {
   int pageable;      // the device reads and writes pageable host memory (cudaDevAttrPageableMemoryAccess)
   int mx, my, p, n1, npe, nx_g, ny_g, precision;
@@ -20,8 +29,9 @@ struct se2gpu_solver {
   int device, nsm;
   cudaStream_t stream, own_stream;
   size_t tsize;                  // compute precision (4 or 8 bytes)
-  // FP64 state: two buffer sets of packed u, v; a of the last step; element forces of a step
-  // (FP32 steps without a halo too: 8 bytes per element node, two-float 16); 1/M; scaled derivative tables
+  // FP64 state: two buffer sets of packed u, v; a of the last step (f64[0][0] the allocation of all); element forces of a step
+  // (FP32 steps without a halo too: 8 bytes per element node, two-float 16; ef[0] is the allocation of both
+  // and of 1/M); scaled derivative tables (Dx the allocation of all that follow)
   double2 *f64[2][2], *a64, *ef[2];
   double *rmass, *Dx, *Dy, *f64_consts;
   int2 *src_xy;                  // first node of each source's element
@@ -33,14 +43,10 @@ struct se2gpu_solver {
   unsigned long long *mass_bad;  // first node with a mass that is not positive (device check at create)
   cudaEvent_t side_done[2];      // se2gpu_create: set-up work on side streams not yet joined
   int rlast;
-  CUtensorMap maps[2][6];        // per input buffer set: region u, cu, owned w, cw; cell constants, 1/M
   float4 *cellc;                 // plain and Kahan modes: (lam detJ, mu detJ, d xi/dx, d eta/dy) per cell
-  int4 *tile_bounds;             // per tile: source and receiver list bounds
-  int pgrid, pconfig, pntx, pnty;
-  int config;                    // selected configuration number; pconfig: the tiles that it stands for
+  se2gpu_tiles tiles;
+  int config;                    // selected configuration number (tiles.config: the tiles that it stands for)
   int auto_config, auto_tiles;   // the number of the mesh's own choice, and its tiles (se2p::first_config)
-  bool no_halo;                  // FP32: the configuration's step keeps element forces (se2gpu_f32ef.cuh)
-  int4 *tile_src, *tile_rec;     // per-tile list entries
   std::vector<int> *src_elem_h, *rec_elem_h;
   int *err_dev;
   // tables in compute precision

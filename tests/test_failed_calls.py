@@ -105,7 +105,7 @@ for start in range(n):
 want = ref.run(2 * len(rows))
 assert np.array_equal(np.concatenate(rows), want)
 assert all(np.array_equal(x, y) for x, y in zip(sol.fields(), ref.fields()))
-assert failures >= 3 * (n - 1) * (n - 2), failures   # (two numbers may name the same tiles)
+assert failures >= (n - 1) * (n - 2), failures   # (two numbers may name the same tiles)
 """)
 
 
@@ -150,7 +150,7 @@ setups = [H.Setup(S.shot(7, i, size=(20 + i, 18), p=p, nt=64)) for i, p in enume
 ref, ens = G.Ensemble(setups, "fp32_kahan", block=4), G.Ensemble(setups, "fp32_kahan", block=4)
 want = [ref.advance(8), ref.advance(8)]
 got = [ens.advance(8)]
-for k in (0, 4):
+for k in (0, 1):   # of the first shot, of the second
     fake.fake_alloc(k)
     try:
         ens.set_tile_config(3, 1)
