@@ -44,7 +44,7 @@ struct se2gpu_solver {
   cudaEvent_t side_done[2];      // se2gpu_create: set-up work on side streams not yet joined
   int rlast;
   float4 *cellc;                 // plain and Kahan modes: (lam detJ, mu detJ, d xi/dx, d eta/dy) per cell
-  se2gpu_tiles tiles;
+  se2gpu_tiles tiles, single;    // what blocks run; what a block of one step runs, where that is another (bounds set)
   int config;                    // selected configuration number (tiles.config: the tiles that it stands for)
   int auto_config, auto_tiles;   // the number of the mesh's own choice, and its tiles (se2p::first_config)
   std::vector<int> *src_elem_h, *rec_elem_h;

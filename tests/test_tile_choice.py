@@ -1,4 +1,5 @@
 """Which tiles a new handle runs, and that its configuration number names them."""
+import numpy as np
 import pytest
 
 from se2dr_fork_gb300 import gpu as G
@@ -58,3 +59,25 @@ def test_two_float_numbers_of_small_tiles_come_last(p):
     m = 1000 // p
     edges = [e for e, _ in _solver(m, m, p, "fp32_df").tile_configs()]
     assert min(edges) not in edges[:len(edges) // 2] and max(edges) in edges[:2]
+
+
+@pytest.mark.parametrize("precision", ["fp32_kahan", "fp32"])
+@pytest.mark.parametrize("p", range(1, 9))
+def test_block_of_one_step_is_one_launch(p, precision):
+    """On a small mesh a block of one step runs the tiles with a halo, unless the step without one
+    was selected by its own number; the states and rows are those of any other block length."""
+    m = 60 // p
+    sol, ref, own = (_solver(m, m, p, precision) for _ in range(3))
+    own.set_tile_config(len(own.tile_configs()) - 1)
+    for s, launches in ((sol, 1), (own, 2)):
+        before = s.info()["launches"]
+        s.advance(1)
+        assert s.info()["launches"] - before == launches
+    sol.advance(3)
+    for _ in range(3):
+        sol.advance(1)
+    own.advance(6)
+    ref.advance(7)
+    want = [ref.traces(), *ref.fields()]
+    for s in (sol, own):
+        assert all(np.array_equal(x, y) for x, y in zip([s.traces(), *s.fields()], want))
