@@ -1207,7 +1207,7 @@ static void touch_absent_pages(float *p, size_t bytes)
   }
   if (absent * 2 < pages) return;
   auto touch = [=](long i0, long i1) {
-    for (long i = i0; i < i1; i++) *reinterpret_cast<volatile float *>(std::max(a + i * page, (uintptr_t)p)) = 0.f;
+    for (long i = i0; i < i1; i++) *reinterpret_cast<volatile char *>(std::max(a + i * page, (uintptr_t)p)) = 0;
   };
   const long nt = std::max(1L, std::min((long)std::min(16u, std::thread::hardware_concurrency()), (long)bytes / TOUCH_BYTES));
   std::thread th[16];
@@ -1226,7 +1226,9 @@ static void touch_absent_pages(float *p, size_t bytes)
 static int copy_out(se2nn *h, float *dst, const float *src, long n)
 {
   NCK(h, cudaStreamSynchronize(h->stream));   // (earlier work may still read the array)
-  touch_absent_pages(dst, (size_t)n * sizeof(float));
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) cudaGetLastError();
+  else if (at.type != cudaMemoryTypeDevice) touch_absent_pages(dst, (size_t)n * sizeof(float));   // (the host cannot store there)
   NCK(h, cudaMemcpy(dst, src, n * 4, cudaMemcpyDeviceToHost));
   return 0;
 }

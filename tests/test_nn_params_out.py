@@ -58,3 +58,13 @@ def test_copies_queued_before_read_the_array_as_it_was(net):
     torch.cuda.synchronize()
     assert torch.equal(dev.cpu(), before)
     assert np.array_equal(pin.numpy(), want)
+
+
+@pytest.mark.parametrize("call", ["se2nn_get_params", "se2nn_get_grads"])
+def test_device_memory_is_not_stored_to_by_the_host(net, call):
+    """A device pointer is the copy's to refuse or to serve: the host threads leave it alone."""
+    dev = torch.full((net.nparams,), 5.0, device="cuda")
+    torch.cuda.synchronize()
+    rc = getattr(N.lib(), call)(net._h, C.cast(dev.data_ptr(), C.POINTER(C.c_float)))
+    want = net.params() if call == "se2nn_get_params" else net.grads()
+    assert np.array_equal(dev.cpu().numpy(), want if rc == 0 else np.full(net.nparams, 5.0, np.float32))
