@@ -237,12 +237,12 @@ int occupancy(int p, int config, int mode, bool batch)
   DfShape s = {};
   if (e) s = DfShape{p, e->te, e->nt, (batch ? e->bsmem : e->smem)[k], (batch ? e->bfn : e->fn)[k], true};
   if (!batch && mode == MODE_DF) df_shape(p, config, &s);
-  const bool per_tile = !batch && no_halo(p, config, mode, &s);   // (a CTA per tile)
+  if (!batch) no_halo(p, config, mode, &s);
   if (!s.fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, s.fn, s.nt, s.smem) != cudaSuccess) {
     cudaGetLastError();
     return 1;
   }
-  return per_tile ? n : std::min(n, 3);   // the persistent grid's CTAs per SM: what the tile configurations are sized for
+  return std::min(n, 3);   // the persistent grid's CTAs per SM: what the tile configurations are sized for
 }
 
 // a launch that may begin (its set-up before cudaGridDependencySynchronize) while the launch

@@ -81,16 +81,3 @@ def test_block_of_one_step_is_one_launch(p, precision):
     want = [ref.traces(), *ref.fields()]
     for s in (sol, own):
         assert all(np.array_equal(x, y) for x, y in zip([s.traces(), *s.fields()], want))
-
-
-@pytest.mark.parametrize("precision", ["fp32", "fp32_kahan"])
-@pytest.mark.parametrize("p", range(1, 9))
-def test_resident_ctas_of_tiles_without_a_halo(p, precision):
-    """Their registers are sized for 32 warps an SM up to degree 5 and 24 above; the cap of three
-    CTAs belongs to the persistent grid of the other tiles."""
-    sol = _solver(9, 7, p, precision)
-    n = len(sol.tile_configs())
-    info = sol.tile_config_info(n - 1)
-    assert info["ctas_per_sm"] >= (1024 if p <= 5 else 768) // info["threads"]
-    number = sol.tile_config   # (stands for the tiles of the mesh)
-    assert all(1 <= sol.tile_config_info(c)["ctas_per_sm"] <= 3 for c in range(n - 1) if c != number)
