@@ -655,12 +655,13 @@ int se2gpu_internal_create(const se2gpu_problem *P, int precision, int trace_cap
   TRY(dzero(h, (void **)&h->err_dev, sizeof(int)));
 
   if (precision == SE2GPU_FP64) {
-    const size_t vbytes = (size_t)nnodes * 2 * 8;
-    TRY(dzero(h, (void **)&h->f64[0][0], 5 * vbytes));   // (one allocation of all five)
-    for (int k = 1; k < 4; k++) h->f64[k / 2][k % 2] = h->f64[0][0] + (size_t)k * nnodes;
-    h->a64 = h->f64[0][0] + 4 * (size_t)nnodes;
+    // one allocation of all five, each aligned as one of its own (256 bytes)
+    const size_t vn = ((size_t)nnodes + 15) / 16 * 16;
+    TRY(dzero(h, (void **)&h->f64[0][0], 5 * vn * 16));
+    for (int k = 1; k < 4; k++) h->f64[k / 2][k % 2] = h->f64[0][0] + k * vn;
+    h->a64 = h->f64[0][0] + 4 * vn;
     // element forces of a step, written before they are read, and 1/M
-    const size_t nef = (size_t)ne * npe;
+    const size_t nef = ((size_t)ne * npe + 15) / 16 * 16;
     TRY(dalloc(h, (void **)&h->ef[0], nef * 32 + (size_t)nnodes * 8));
     h->ef[1] = h->ef[0] + nef;
     h->rmass = reinterpret_cast<double *>(h->ef[1] + nef);
