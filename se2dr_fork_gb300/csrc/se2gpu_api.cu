@@ -368,7 +368,7 @@ extern "C" void se2gpu_destroy(se2gpu_solver *h)
   void *ptrs[] = {h->f64[0][0], h->ef[0], h->Dx, h->pa, h->pminv, h->mass_bad, h->err_dev, h->mass, h->lam, h->mu, h->J00, h->J11, h->iJ00, h->iJ11, h->D, h->wq,
                   h->src_vals, h->Dd, h->iJ00d, h->iJ11d, h->stf_dev, h->traces, h->norm_part,
                   h->rec_node, h->rec_elem, h->rec_gll, h->scratch_u, h->scratch_f, h->cellc,
-                  h->tiles.bounds, h->single.bounds};
+                  h->tiles.bounds};
   for (void *p : ptrs) dfree(h, p);
   if (h->stream) cudaStreamSynchronize(h->stream);   // the frees are done before the stream goes
   delete h->src_elem_h;
@@ -437,15 +437,9 @@ static int make_const_maps(se2gpu_solver *h, const se2p::TileShape &ts, CUtensor
   return 0;
 }
 
-static void free_tiles(se2gpu_solver *h, se2gpu_tiles &t)
-{
-  dfree(h, t.bounds);
-  t.src = t.rec = t.bounds = nullptr;
-}
-
-// a configuration's kernel attributes, tensor maps, per-tile source/receiver lists and grid, into t;
-// nothing of the handle changes
-static int build_tiles(se2gpu_solver *h, int config, const se2p::TileShape &ts, se2gpu_tiles &t)
+// a configuration's kernel attributes, tensor maps, per-tile source/receiver lists (appended to tab) and
+// grid, into t; nothing of the handle changes
+static int build_tiles(se2gpu_solver *h, int config, const se2p::TileShape &ts, se2gpu_tiles &t, std::vector<int> &tab)
 {
   const bool kahan = is_kahan(h);
   memset(&t, 0, sizeof(t));
@@ -464,43 +458,47 @@ static int build_tiles(se2gpu_solver *h, int config, const se2p::TileShape &ts, 
   const int te = ts.tex, P = h->p;
   const int ntx = (h->mx + te - 1) / te, nty = (h->my + te - 1) / te, ntiles = ntx * nty;
   // tile lists: a source or receiver element appears in every tile whose owned nodes it touches, or
-  // whose nodes it touches where a tile finishes the node lines that it shares with the next ones
-  const int far = ts.halo ? 0 : 1;
+  // whose nodes it touches where a tile finishes the node lines that it shares with the next ones.  Along
+  // an axis that is the element's own tile, the next one where the element is the tile's last (the line
+  // between them is the next one's), and with shared lines the one before where it is the first.  (Every
+  // tile around tested instead, twice over: create took 380 -> 425 us with 430 elements on a small mesh.)
   auto build = [&](const std::vector<int> &elems, std::vector<int> &off, std::vector<int> &ent) {
-    auto each = [&](auto f) {   // f(tile, element index), elements ascending
-      for (int q = 0; q < (int)elems.size(); q++) {
-        const int ex = elems[q] % h->mx, ey = elems[q] / h->mx;
-        for (int ty = std::max(0, (ey - 1) / te); ty <= std::min(nty - 1, (ey + 1) / te); ty++)
-          for (int tx = std::max(0, (ex - 1) / te); tx <= std::min(ntx - 1, (ex + 1) / te); tx++) {
-            const int X0 = tx * te * P, X1 = std::min((tx + 1) * te, h->mx) * P + (((tx + 1) * te >= h->mx) ? 1 : 0);
-            const int Y0 = ty * te * P, Y1 = std::min((ty + 1) * te, h->my) * P + (((ty + 1) * te >= h->my) ? 1 : 0);
-            if (ex * P <= X1 - 1 + far && ex * P + P >= X0 && ey * P <= Y1 - 1 + far && ey * P + P >= Y0) f(ty * ntx + tx, q);
-          }
-      }
-    };
+    struct Range { int x, y, tx0, tx1, ty0, ty1; };
+    std::vector<Range> at_tiles(elems.size());
     off.assign(ntiles + 1, 0);
-    each([&](int t, int) { off[t + 1]++; });
+    for (size_t q = 0; q < elems.size(); q++) {
+      const int ey = elems[q] / h->mx, ex = elems[q] - ey * h->mx, tx = ex / te, ty = ey / te;
+      const int fx = ex - tx * te, fy = ey - ty * te;
+      const Range r = {ex * P, ey * P, tx - (!ts.halo && fx == 0 && tx > 0), tx + (fx == te - 1 && tx < ntx - 1),
+                       ty - (!ts.halo && fy == 0 && ty > 0), ty + (fy == te - 1 && ty < nty - 1)};
+      at_tiles[q] = r;
+      for (int y = r.ty0; y <= r.ty1; y++)
+        for (int x = r.tx0; x <= r.tx1; x++) off[y * ntx + x + 1]++;
+    }
     for (int t = 0; t < ntiles; t++) off[t + 1] += off[t];
     ent.assign(4 * (size_t)off[ntiles], 0);
     std::vector<int> at(off.begin(), off.end() - 1);
-    each([&](int t, int q) {
-      int *e = &ent[4 * (size_t)at[t]++];
-      e[0] = q; e[1] = elems[q] % h->mx * P; e[2] = elems[q] / h->mx * P;
-    });
+    for (size_t q = 0; q < elems.size(); q++) {   // (elements ascending in each tile)
+      const Range &r = at_tiles[q];
+      for (int y = r.ty0; y <= r.ty1; y++)
+        for (int x = r.tx0; x <= r.tx1; x++) {
+          int *e = &ent[4 * (size_t)at[y * ntx + x]++];
+          e[0] = (int)q; e[1] = r.x; e[2] = r.y;
+        }
+    }
   };
   std::vector<int> so, si, ro, ri;
   build(*h->src_elem_h, so, si);
   build(*h->rec_elem_h, ro, ri);
-  std::vector<int> tb(4 * (size_t)ntiles);   // (one table, one upload: an allocation costs about 0.1 ms)
-  for (int t = 0; t < ntiles; t++) {
-    tb[4 * (size_t)t] = so[t]; tb[4 * (size_t)t + 1] = so[t + 1];
-    tb[4 * (size_t)t + 2] = ro[t]; tb[4 * (size_t)t + 3] = ro[t + 1];
+  t.first = tab.size() / 4;
+  t.nlist = si.size() / 4;
+  tab.resize(tab.size() + 4 * (size_t)ntiles);
+  for (int k = 0; k < ntiles; k++) {
+    int *b = &tab[4 * (t.first + k)];
+    b[0] = so[k]; b[1] = so[k + 1]; b[2] = ro[k]; b[3] = ro[k + 1];
   }
-  tb.insert(tb.end(), si.begin(), si.end());
-  tb.insert(tb.end(), ri.begin(), ri.end());
-  if ((rc = upload_i(h, (int **)&t.bounds, tb.data(), tb.size()))) return rc;
-  t.src = t.bounds + ntiles;
-  t.rec = t.src + si.size() / 4;
+  tab.insert(tab.end(), si.begin(), si.end());
+  tab.insert(tab.end(), ri.begin(), ri.end());
   t.config = config;
   t.halo = ts.halo;
   t.ntx = ntx;
@@ -527,22 +525,30 @@ static int setup_f32_config(se2gpu_solver *h, int config, bool in_create = false
   if (!in_create) CK(h, cudaStreamSynchronize(h->stream));
   se2gpu_tiles t, single;
   memset(&single, 0, sizeof(single));
-  const size_t ef_bytes = ((size_t)h->mx * h->my * h->npe * (is_df(h) ? 16 : 8) + 15) / 16 * 16;
+  std::vector<int> tab;   // (one table of both, one upload: an allocation and a copy cost some 10 us)
+  int4 *dev = nullptr;
+  const size_t ef_bytes = ((size_t)h->mx * h->my * h->npe * (is_df(h) ? 16 : 8) + 255) / 256 * 256;
   void *ef = nullptr;   // element forces, where the handle has none yet
-  int rc = build_tiles(h, config, ts, t);
+  int rc = build_tiles(h, config, ts, t, tab);
   if (!rc && !ts.halo && !h->ef[0]) rc = dalloc(h, &ef, 2 * ef_bytes);
   if (!rc && one_config >= 0) {
     rc = se2p::config_shape(h->p, one_config, mode, &one);
-    if (!rc) rc = build_tiles(h, one_config, one, single);
+    if (!rc) rc = build_tiles(h, one_config, one, single, tab);
   }
+  if (!rc) rc = upload_i(h, (int **)&dev, tab.data(), tab.size());
   if (rc) {
-    free_tiles(h, t);
-    free_tiles(h, single);
+    dfree(h, dev);
     dfree(h, ef);
     return rc;
   }
-  free_tiles(h, h->tiles);
-  free_tiles(h, h->single);
+  auto place = [&](se2gpu_tiles &x) {
+    x.bounds = dev + x.first;
+    x.src = x.bounds + (size_t)x.ntx * x.nty;
+    x.rec = x.src + x.nlist;
+  };
+  place(t);
+  if (one_config >= 0) place(single);
+  dfree(h, h->tiles.bounds);
   h->tiles = t;
   h->single = single;
   if (ef) {

@@ -13,8 +13,9 @@
 // a tile configuration of the FP32 modes, set up on a handle
 struct se2gpu_tiles {
   CUtensorMap maps[2][6];        // per input buffer set: region u, cu, owned w, cw; cell constants, 1/M
-  int4 *bounds;                  // per tile: source and receiver list bounds (the allocation, with src and rec)
+  int4 *bounds;                  // per tile: source and receiver list bounds
   int4 *src, *rec;               // per-tile list entries
+  size_t first, nlist;           // place of bounds in the handle's table (tiles.bounds is its start); entries of src
   int config, ntx, nty, grid;
   bool halo;                     // else its step keeps element forces (se2gpu_f32ef.cuh, se2gpu_f32df.cuh)
 };
