@@ -468,13 +468,22 @@ int build_dft(se2nn *h)
       ext[x * 2 * m + k] = ex[k * nx + x];
       exit[k * nx + x] = exi[x * 2 * m + k];
     }
+  // one allocation and one copy of all six, each on a 256-byte boundary
+  struct { const std::vector<float> &v; bf16 **p; } parts[] = {{ext, &h->ExT}, {exit, &h->ExinvT}, {ex, &h->Ex},
+                                                               {my, &h->My}, {myi, &h->Myinv}, {exi, &h->Exinv}};
+  auto padded = [](size_t n) { return (n + 127) / 128 * 128; };
+  std::vector<float> all;
+  for (auto &q : parts) {
+    all.insert(all.end(), q.v.begin(), q.v.end());
+    all.resize(padded(all.size()));
+  }
+  bf16 *at = nullptr;
   int rc;
-  if ((rc = nalloc(h, &h->ExT, ext.size())) || (rc = upload_bf16(h, h->ExT, ext))) return rc;
-  if ((rc = nalloc(h, &h->ExinvT, exit.size())) || (rc = upload_bf16(h, h->ExinvT, exit))) return rc;
-  if ((rc = nalloc(h, &h->Ex, ex.size())) || (rc = upload_bf16(h, h->Ex, ex))) return rc;
-  if ((rc = nalloc(h, &h->My, my.size())) || (rc = upload_bf16(h, h->My, my))) return rc;
-  if ((rc = nalloc(h, &h->Myinv, myi.size())) || (rc = upload_bf16(h, h->Myinv, myi))) return rc;
-  if ((rc = nalloc(h, &h->Exinv, exi.size())) || (rc = upload_bf16(h, h->Exinv, exi))) return rc;
+  if ((rc = nalloc(h, &at, all.size())) || (rc = upload_bf16(h, at, all))) return rc;
+  for (auto &q : parts) {
+    *q.p = at;
+    at += padded(q.v.size());
+  }
   return 0;
 }
 
@@ -1142,9 +1151,13 @@ extern "C" int se2nn_create(const se2nn_config *cfg, unsigned long long seed, se
     const long cs2 = std::max((long)Bm * c.nrec * (long)c.hidden * std::max(w, h->nsub),
                               (((long)drows + 255) / 256) * std::max(h->nsub, c.hidden));
     h->partial_n = std::max(wg, std::max(cs1, cs2));
-    TRY(nalloc(h, &h->partial, (size_t)h->partial_n));
-    TRY(nalloc(h, &h->colpart, (size_t)cs1));
-    TRY(nalloc(h, &h->decpart, (size_t)Bm * c.nrec * c.hidden * h->nsub + (drows + 255) / 256 * (size_t)(h->nsub + c.hidden)));
+    // the partial sums, and those that only the fused kernels have beside them, in one allocation
+    auto padded = [](size_t n) { return (n + 63) / 64 * 64; };
+    const size_t np = padded((size_t)h->partial_n), nc = padded((size_t)cs1);
+    const size_t nd = (size_t)Bm * c.nrec * c.hidden * h->nsub + (drows + 255) / 256 * (size_t)(h->nsub + c.hidden);
+    TRY(nalloc(h, &h->partial, np + (fused_shape(h) ? nc + nd : 0)));
+    h->colpart = h->partial + np;
+    h->decpart = h->colpart + nc;
   }
   TRY(build_dft(h));
   TRY(fused_setup(h));
