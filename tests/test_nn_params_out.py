@@ -68,3 +68,23 @@ def test_device_memory_is_not_stored_to_by_the_host(net, call):
     rc = getattr(N.lib(), call)(net._h, C.cast(dev.data_ptr(), C.POINTER(C.c_float)))
     want = net.params() if call == "se2nn_get_params" else net.grads()
     assert np.array_equal(dev.cpu().numpy(), want if rc == 0 else np.full(net.nparams, 5.0, np.float32))
+
+
+@pytest.fixture(scope="module")
+def large(nn_lib):
+    # 4.2 million parameters, 17 MB: several threads
+    n = N.Network(N.Config(ny=16, nx=32, cin=16, width=64, modes=8, layers=4, nrec=4, nout=64, hidden=32, max_batch=2), seed=3)
+    n.set_params(np.random.default_rng(1).standard_normal(n.nparams).astype(np.float32))
+    return n
+
+
+@pytest.mark.parametrize("offset", [0, 1, 1024])
+@pytest.mark.parametrize("kind", ["new", "used", "half", "pinned"])
+def test_large_arrays_of_every_kind_of_host_memory(large, kind, offset):
+    assert large.nparams * 4 > 16e6
+    test_every_kind_of_host_memory(large, kind, offset)
+
+
+@pytest.mark.parametrize("call", ["se2nn_get_params", "se2nn_get_grads"])
+def test_large_device_memory_is_not_stored_to_by_the_host(large, call):
+    test_device_memory_is_not_stored_to_by_the_host(large, call)
