@@ -914,9 +914,27 @@ static se2p::Params f32_params(const se2gpu_solver *h, const se2gpu_tiles &t)
 
 se2p::Params se2gpu_internal_f32_params(se2gpu_solver *h) { return f32_params(h, h->tiles); }
 
+// FP64: v and a of the step that a block has begun and not finished -- its last one, or the one
+// whose next launch failed.  Every call that reads or advances the state begins here, so that a
+// block in which a launch failed is one of fewer steps.
+static int settle(se2gpu_solver *h)
+{
+  if (!h->unfinished) return 0;
+  auto q = f64_params(h);
+  q.ef_in = h->ef[h->cur];
+  q.stf = h->stf_dev + (size_t)(h->unfinished - 1) * h->nsrc;
+  h->launches++;
+  const cudaError_t e = se2::f64_launch_last(h->p, q, h->f64[h->cur][1], h->a64, h->stream);
+  if (e != cudaSuccess) return fail(h, SE2GPU_ERR_CUDA, "step kernel: %s", cudaGetErrorString(e));
+  h->unfinished = 0;
+  return 0;
+}
+
 // record the receivers of the last step if its row is still pending
 static int flush_record(se2gpu_solver *h)
 {
+  const int rc = settle(h);
+  if (rc) return rc;
   if (!h->pending_record) return 0;
   cudaError_t e;
   h->launches++;
@@ -960,14 +978,10 @@ static int advance_f64(se2gpu_solver *h, int nsteps)
     if (e != cudaSuccess) return fail(h, SE2GPU_ERR_CUDA, "step kernel: %s", cudaGetErrorString(e));
     if (h->pending_record) { h->rows_written++; h->pending_record = false; }
     h->cur = outb;
+    h->unfinished = k + 1;
     if (h->nrec > 0) h->pending_record = true;
   }
-  q.ef_in = h->ef[h->cur];
-  q.stf = h->stf_dev + (size_t)(nsteps - 1) * h->nsrc;
-  h->launches++;
-  cudaError_t e = se2::f64_launch_last(h->p, q, h->f64[h->cur][1], h->a64, h->stream);
-  if (e != cudaSuccess) return fail(h, SE2GPU_ERR_CUDA, "step kernel: %s", cudaGetErrorString(e));
-  return 0;
+  return settle(h);
 }
 
 // steps without a halo: START, MIDDLE per step but the last, LAST (se2gpu_f32ef.cuh); a launch that
@@ -1034,6 +1048,8 @@ extern "C" int se2gpu_advance(se2gpu_solver *h, int nsteps, const double *stf)
     return fail(h, SE2GPU_ERR_STATE, "trace buffer full: %d rows buffered, capacity %d; call se2gpu_traces",
                 h->rows_written + (h->pending_record ? 1 : 0), h->trace_cap);
   CK(h, cudaSetDevice(h->device));
+  const int rs = settle(h);
+  if (rs) return rs;
   if (h->nsrc) {
     if (nsteps > h->stf_cap) {
       CK(h, cudaStreamSynchronize(h->stream));
@@ -1098,8 +1114,9 @@ extern "C" int se2gpu_get_fields(se2gpu_solver *h, double *u, double *v, double 
 {
   if (!h) return SE2GPU_ERR_ARG;
   CK(h, cudaSetDevice(h->device));
-  CK(h, cudaStreamSynchronize(h->stream));
   int rc;
+  if ((rc = settle(h))) return rc;
+  CK(h, cudaStreamSynchronize(h->stream));
   if ((rc = check_err_flag(h))) return rc;
   const size_t n = (size_t)h->nnodes * 2;
   if (is_f64(h)) {
@@ -1151,6 +1168,8 @@ extern "C" int se2gpu_norms(se2gpu_solver *h, double out[6])
 {
   if (!h || !out) return SE2GPU_ERR_ARG;
   CK(h, cudaSetDevice(h->device));
+  const int rs = settle(h);
+  if (rs) return rs;
   const int nb = 1024;
   h->launches++;
   if (is_f64(h)) {
@@ -1182,6 +1201,8 @@ extern "C" int se2gpu_norms(se2gpu_solver *h, double out[6])
 // ---------------------------------------------------------------- internal force (packed layout)
 static int force_f64(se2gpu_solver *h, const void *u_dev, void *F_dev)
 {
+  const int rc = settle(h);   // (the element forces are overwritten here)
+  if (rc) return rc;
   auto q = f64_params(h);
   q.mode = se2::F64_FORCE;
   q.u_in = (const double2 *)u_dev;
@@ -1256,6 +1277,7 @@ extern "C" int se2gpu_info(const se2gpu_solver *h, long *ints)
 extern "C" int se2gpu_device_fields(const se2gpu_solver *h, void **u, void **v, void **a)
 {
   if (!h) return SE2GPU_ERR_ARG;
+  if (h->unfinished) return SE2GPU_ERR_STATE;   // (a launch failed; any call that reads the state finishes the step)
   if (is_f64(h)) {
     if (u) *u = f64_field(h, 0);
     if (v) *v = f64_field(h, 1);
@@ -1375,6 +1397,8 @@ extern "C" int se2gpu_checkpoint_save(se2gpu_solver *h, void *buf, long bytes)
   if (bytes < se2gpu_checkpoint_size(h)) return fail(h, SE2GPU_ERR_ARG, "checkpoint buffer of %ld bytes, %ld needed", bytes, se2gpu_checkpoint_size(h));
   if (h->rows_written > 0) return fail(h, SE2GPU_ERR_STATE, "%d trace rows are buffered; fetch them with se2gpu_traces before saving", h->rows_written);
   CK(h, cudaSetDevice(h->device));
+  const int rs = settle(h);
+  if (rs) return rs;
   CK(h, cudaStreamSynchronize(h->stream));
   int rc;
   if ((rc = check_err_flag(h))) return rc;
@@ -1409,6 +1433,7 @@ extern "C" int se2gpu_checkpoint_load(se2gpu_solver *h, const void *buf, long by
   CK(h, cudaSetDevice(h->device));
   CK(h, cudaStreamSynchronize(h->stream));
   h->rows_written = 0;
+  h->unfinished = 0;
   h->pending_record = hd.pending_record != 0;
   if (!is_f64(h)) h->rlast = hd.rlast & 1;
   const char *o = static_cast<const char *>(buf) + sizeof(hd);

@@ -37,6 +37,7 @@ struct se2gpu_solver {
   double *rmass, *Dx, *Dy, *f64_consts;
   int2 *src_xy;                  // first node of each source's element
   int cur;
+  int unfinished;                // FP64: the begun step without its v and a yet: its row of stf_dev + 1 (0: none)
   // FP32 leapfrog state (padded): u, w, cu, cw per buffer set, a of the last step
   int pitch;
   float2 *pu[2], *pw[2], *pcu[2], *pcw[2], *pa;

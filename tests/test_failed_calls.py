@@ -168,3 +168,45 @@ got.append(ens.advance(8))
 for g, w in zip(got, want):
     assert all(np.array_equal(x, y) for x, y in zip(g, w))
 """)
+
+
+@pytest.mark.parametrize("call", ["traces", "fields", "norms", "checkpoint", "force", "advance", "set_fields"])
+def test_failed_launch_in_an_fp64_block_leaves_whole_steps(run_with_fake, call):
+    """A block whose n-th dependent launch fails has made as many whole steps as its launches began,
+    whichever call comes next."""
+    run_with_fake(f"""
+su = H.Setup(S.demo(7, 6, p=3, tmax=1e30).replace(nt=1000))
+rng = np.random.default_rng(3)
+f = [rng.standard_normal(su.ndof) * s for s in (1e-6, 1e-3, 1.0)]
+stf = rng.standard_normal((5, su.nsrc))
+for n in range(5):   # four launches that finish a step and begin the next, and the last
+    sol, ref = G.Solver(su, "fp64"), G.Solver(su, "fp64")
+    for x in (sol, ref):
+        x.set_fields(*f)
+    fake.fake_launch(n)
+    try:
+        sol.advance(5, stf)
+        raise SystemExit("the launch did not fail")
+    except G.GpuError as e:
+        assert e.code == -2, e
+    fake.fake_launch(-1)
+    ref.advance(n + 1, stf[:n + 1])
+    sol.time, sol.step, sol._times = ref.time, ref.step, list(ref._times)
+    for x in (sol, ref):
+        x.got = []
+        if "{call}" == "traces":
+            x.got.append(x.traces())
+        elif "{call}" == "fields":
+            x.got += x.fields()
+        elif "{call}" == "norms":
+            x.got.append(x.norms())
+        elif "{call}" == "force":
+            x.got.append(x.assemble_linear_form(f[0]))
+        elif "{call}" == "set_fields":
+            x.set_fields(u=f[1])
+        elif "{call}" == "checkpoint" and n == 0:   # (one row pending, none written)
+            x.got.append(np.frombuffer(x.checkpoint(), dtype=np.uint8))
+        x.advance(3, stf[:3])
+        x.got += [x.traces(), *x.fields()]
+    assert len(sol.got) == len(ref.got) and all(np.array_equal(x, y) for x, y in zip(sol.got, ref.got)), n
+""")
