@@ -490,15 +490,18 @@ static int build_tiles(se2gpu_solver *h, int config, const se2p::TileShape &ts, 
   std::vector<int> so, si, ro, ri;
   build(*h->src_elem_h, so, si);
   build(*h->rec_elem_h, ro, ri);
+  // (each part of the table on a 256-byte boundary: a tile's entries are then in as few lines as can be)
+  auto padded = [](size_t n) { return (n + 15) / 16 * 16; };
   t.first = tab.size() / 4;
-  t.nlist = si.size() / 4;
-  tab.resize(tab.size() + 4 * (size_t)ntiles);
+  t.src_at = padded(ntiles);
+  t.rec_at = t.src_at + padded(si.size() / 4);
+  tab.resize(4 * (t.first + t.rec_at + padded(ri.size() / 4)));
   for (int k = 0; k < ntiles; k++) {
     int *b = &tab[4 * (t.first + k)];
     b[0] = so[k]; b[1] = so[k + 1]; b[2] = ro[k]; b[3] = ro[k + 1];
   }
-  tab.insert(tab.end(), si.begin(), si.end());
-  tab.insert(tab.end(), ri.begin(), ri.end());
+  std::copy(si.begin(), si.end(), tab.begin() + 4 * (t.first + t.src_at));
+  std::copy(ri.begin(), ri.end(), tab.begin() + 4 * (t.first + t.rec_at));
   t.config = config;
   t.halo = ts.halo;
   t.ntx = ntx;
@@ -543,8 +546,8 @@ static int setup_f32_config(se2gpu_solver *h, int config, bool in_create = false
   }
   auto place = [&](se2gpu_tiles &x) {
     x.bounds = dev + x.first;
-    x.src = x.bounds + (size_t)x.ntx * x.nty;
-    x.rec = x.src + x.nlist;
+    x.src = x.bounds + x.src_at;
+    x.rec = x.bounds + x.rec_at;
   };
   place(t);
   if (one_config >= 0) place(single);
@@ -678,13 +681,16 @@ int se2gpu_internal_create(const se2gpu_problem *P, int precision, int trace_cap
       TRY(SE2GPU_ERR_CUDA);
     }
     // the reference's scaled derivatives dN/dx = (1/J00) dN/dxi per element column, dN/dy per row; the
-    // kernels' constants; the first node of each source's element
-    const size_t ndx = (size_t)P->mx * npe, ndy = (size_t)P->my * npe;
+    // kernels' constants; the first node of each source's element: each on a 256-byte boundary but the last,
+    // which shares the constants' line
+    auto padded = [](size_t n) { return (n + 31) / 32 * 32; };
+    const size_t ndx = padded((size_t)P->mx * npe), ndy = padded((size_t)P->my * npe);
     std::vector<double> tab(ndx + ndy + 2 + P->nsrc);
     // (a division per entry made create 4 % slower at 250 x 250 elements, degree 7)
     double *o = tab.data();
     for (int e = 0; e < P->mx; e++)
       for (int i = 0; i < npe; i++) *o++ = P->iJ00[e] * P->D[i];
+    o = tab.data() + ndx;
     for (int e = 0; e < P->my; e++)
       for (int i = 0; i < npe; i++) *o++ = P->iJ11[e] * P->D[i];
     tab[ndx + ndy] = 1.0;

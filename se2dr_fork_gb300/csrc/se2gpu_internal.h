@@ -15,7 +15,7 @@ struct se2gpu_tiles {
   CUtensorMap maps[2][6];        // per input buffer set: region u, cu, owned w, cw; cell constants, 1/M
   int4 *bounds;                  // per tile: source and receiver list bounds
   int4 *src, *rec;               // per-tile list entries
-  size_t first, nlist;           // place of bounds in the handle's table (tiles.bounds is its start); entries of src
+  size_t first, src_at, rec_at;  // their places: bounds in the handle's table (tiles.bounds is its start), the lists from bounds
   int config, ntx, nty, grid;
   bool halo;                     // else its step keeps element forces (se2gpu_f32ef.cuh, se2gpu_f32df.cuh)
 };
