@@ -72,7 +72,13 @@ typedef struct se2gpu_problem {
 typedef struct se2gpu_solver se2gpu_solver;
 
 /* Allocate and upload a problem.  trace_capacity = receiver rows buffered on
-   the device between se2gpu_traces calls.  The fields start at zero. */
+   the device between se2gpu_traces calls.  The fields start at zero.
+   Device memory per node, receivers and sources aside, degree p: state, mass and cell
+   tables 96 + 16/p^2 bytes in FP64, 88 + 16/p^2 in the two-float mode, 76 + 24/p^2 in the
+   Kahan and 44 + 24/p^2 in the plain mode; and the element forces of two steps,
+   32 (1 + 1/p)^2 bytes in FP64 and the two-float mode (degrees 2 and 3 on large meshes: none) and, in
+   the plain and Kahan modes, 16 (1 + 1/p)^2 where the tile configuration keeps them (new
+   handles: small meshes only). */
 int  se2gpu_create(const se2gpu_problem *prob, int precision, int trace_capacity, se2gpu_solver **out);
 void se2gpu_destroy(se2gpu_solver *h);
 const char *se2gpu_last_error(const se2gpu_solver *h);
@@ -146,7 +152,7 @@ int se2gpu_tile_config(const se2gpu_solver *h);
 /* One configuration in full (no counterpart in the reference): info = {elements per
    tile edge, threads per CTA, owned-box buffers (2: the next tile's w arrives a tile
    ahead; 1: during the tile's element phases; 0: FP64), resident CTAs per SM on the
-   current device (0: FP64)}.  Two configurations may share edge and threads. */
+   current device (up to 3, the most that the persistent grid has; 0: FP64)}.  Two configurations may share edge and threads. */
 int se2gpu_tile_config_info(const se2gpu_solver *h, int config, int info[4]);
 
 /* ---- Checkpoint / resume (no counterpart in the reference, which restarts from

@@ -390,7 +390,7 @@ static int enqueue_steps(se2gpu_ensemble *e, int cur, int sl, int n, cudaStream_
     int chunk = 0;
     for (Group &g : e->groups)
       for (const Chunk &ch : g.chunks) {
-        static thread_local se2p::BatchArgs ba;   // 28 KB: kept off the stack
+        static thread_local se2p::BatchArgs ba;   // 27 KB: kept off the stack
         ba.maps = g.maps[cin] + 4 * (size_t)ch.first;
         ba.items = g.items + ch.item_off;
         ba.nshots = ch.nshots;

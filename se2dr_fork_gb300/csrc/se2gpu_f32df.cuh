@@ -2,12 +2,12 @@
 //
 // The same leapfrog as se2gpu_persist.cuh (state u, w with their low parts stored as Kahan terms:
 // value = hi - c) with every value of a step an unevaluated sum of two floats.  What bounds it on
-// large meshes is instruction issue (73 % of the issue slots busy, memory a quarter), so
+// large meshes is instruction issue (77 % of the issue slots busy, memory a quarter), so
 // no element is evaluated twice: as in the FP64 step (se2gpu_f64.cuh) a launch finishes the previous
 // step at the nodes of its tile, from the element forces in memory, and then leaves this step's
 // element forces there.  Only the nodes on tile edges are finished twice, where a halo of elements
 // cost a third of the element work.  The forces (16 (p+1)^2 bytes per element, two buffers) add
-// about 50 B per node and step at degree 4.  3.53M nodes, degree 4, 6 steps: 1313 -> 1243 us; degree 7
+// about 50 B per node and step at degree 4.  3.53M nodes, degree 4, 6 steps: 1313 -> 1169 us; degree 7
 // at 2.5M nodes 304 -> 176 us a step, 20000 nodes 19.4 -> 11.9 (every size: se2gpu_f32df_launch.h).
 //
 // A block of n steps: one EF_START launch (element forces of the state), n - 1 EF_MIDDLE
@@ -211,9 +211,9 @@ __global__ void __launch_bounds__(NT, df_min_blocks(P, TE, NT)) df_step(const Ef
   // first node: (u_k - u_0) + (c_0 - c_k) with the first difference split exactly by TwoSum
   // Next to issue, the fetch of its instructions bounds this part: the loops over directions and
   // points are rolled (what they index goes through the thread's own exchange rows), those over
-  // outputs too from degree 5 on, three at a time.  Unrolled, warps waited for instructions
-  // 1.45 cycles per issue, now 1.05 (degree 4, 2.5M nodes: 173 -> 159 us a step; outputs rolled at
-  // degree 5 180 -> 162, at degree 4 159 -> 161).
+  // outputs too from degree 5 on, three at a time (degree 4, 2.5M nodes: 173 -> 159 us a step, waits for
+  // instructions 1.45 -> 1.05 cycles per issue, 2.0 of 8.7 with the 28 warps that now fit; outputs rolled
+  // at degree 5 180 -> 162, at degree 4 159 -> 161).
   constexpr int DU = P >= 5 ? 3 : N1;
   const int base = (ecy * P) * RW + ecx * P;
   if (active) {

@@ -135,7 +135,10 @@ int auto_config(int p, int mode) { return default_config(p, mode, 0, 0, 1); }
 // 5.3 / 5.5 -> 5.0); 8 x 8 with one region stage, two CTAs per SM, in up to two rounds (128 x 128 8.7 -> 7.5
 // / 8.0 -> 6.6; 177 x 177 13.0 -> 12.2 / 11.5 -> 10.6; but 500 x 500 68 / 76: nothing is copied ahead).
 // Degree 7: 5 x 5 with one region stage, which leaves two (plain: three) CTAs per SM instead of one
-// (85 x 85 10.7 -> 9.1 / 10.7 -> 8.1; 143 x 143 22.5 -> 19.5 / 18.3 -> 15.9; 571 x 571 280 -> 266 / 220 -> 197).
+// (85 x 85 10.7 -> 9.1 / 10.7 -> 8.1; 143 x 143 22.5 -> 19.5 / 18.3 -> 15.9; 571 x 571 267 -> 254 / 207 -> 184; with both stages
+// 5 x 5 takes 284 / 200 there).
+// The tiles of the other degrees' large meshes leave two or three CTAs per SM with both stages; none with one was
+// built for them.
 int first_config(int p, int mode, int mx, int my, int nsm)
 {
   static const int few[8] = {3, 2, 2, 4, 3, 2, 3, 3};

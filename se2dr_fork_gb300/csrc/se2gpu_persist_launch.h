@@ -13,8 +13,8 @@ namespace se2p {
 // thread per (element, line) in order, threads >= (edge + 1)^2 (degree + 1); 1:
 // warp-aligned, 32 / (degree + 1) whole elements per warp, whose three element phases
 // synchronise within the warp, threads = 32 x warps; 2: as 0, with one region stage:
-// nothing is copied a tile ahead, but more CTAs fit an SM)).  default_config and
-// first_config choose.  The two-float mode has a list of its own (se2gpu_f32df_launch.h).
+// nothing is copied a tile ahead, but more CTAs fit an SM; the batched kernel always has two)).
+// default_config and first_config choose; what they never choose is there for the autotuner.  The two-float mode has a list of its own (se2gpu_f32df_launch.h).
 // New configurations go at the end of their degree's list: the autotuner's cache and
 // default_config refer to them by position.
 #define SE2P_CONFIGS(X)                                                                      \
@@ -37,7 +37,7 @@ struct TileShape {
   int cell_box;        // cell-constant box edge (elements, float4 each)
   int minv_w;          // 1/M box width (floats; the box is own_h high)
   size_t smem;
-  bool halo;           // recomputes a halo of elements and loads by tensor maps (all but most two-float ones)
+  bool halo;           // recomputes a halo of elements and loads by tensor maps (else: keeps element forces)
 };
 
 cudaError_t set_tables(int p, const double *D, const double *w1d);   // constant-memory D, w (current device)

@@ -216,7 +216,7 @@ __device__ __forceinline__ void x_analysis(const bf16 *sE, const bf16 *px, int n
 // through the convolution and activation: it holds them in operand registers, so results (and, on
 // their way, the pre-activations) replace them in shared memory without a block barrier; the
 // x transform at the end reads all pixels.  What bounds it is issue and the latency of dependent
-// instructions (40 instructions per value, half of them the activation, 57 % of the issue slots) at the
+// instructions (40 instructions per value, half of them the activation, 61 % of the issue slots) at the
 // warps that fit: 32 channels at a time and no second stage for the pre-activations leave three
 // CTAs per SM (80 registers, 74 KB).
 template <int W, int KIND>
