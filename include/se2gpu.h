@@ -108,7 +108,9 @@ int se2gpu_get_fields(se2gpu_solver *h, double *u, double *v, double *a);
 /* Advance nsteps steps.  stf[k*nsrc + s] is source s's source-time function at
    the time of step k (the host evaluates the STF objects, as the reference does
    per step).  One receiver row per step is buffered on the device; the call
-   fails with SE2GPU_ERR_STATE when the trace buffer would overflow. */
+   fails with SE2GPU_ERR_STATE when the trace buffer would overflow.  A call in which
+   a launch fails has advanced fewer steps, with their rows (FP32 modes: the acceleration
+   is then still that of the last complete call). */
 int se2gpu_advance(se2gpu_solver *h, int nsteps, const double *stf);
 
 /* Copy up to max_rows buffered receiver rows (oldest first) into out[row][7*nrec]
@@ -134,7 +136,8 @@ int se2gpu_info(const se2gpu_solver *h, long *ints);
 /* Device pointers of the current state.  FP64: u, v, a in the reference's
    packed layout.  FP32 modes hold the leapfrog state in rows of `pitch` nodes
    (float2 per node): u = displacement of the next step, v = half-step velocity
-   (v_k + dt/2 a_k), a = acceleration of the last step. */
+   (v_k + dt/2 a_k), a = acceleration of the last step.  (SE2GPU_ERR_STATE where a failed
+   launch left the last FP64 step to be finished by the next call that reads the state.) */
 int se2gpu_device_fields(const se2gpu_solver *h, void **u, void **v, void **a);
 
 /* Tile configurations of the step kernel (elements per tile edge, threads per
